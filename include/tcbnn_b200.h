@@ -114,8 +114,7 @@ int tcbnn_conv_prepare(const tcbnn_conv_desc* d, const uint32_t* filter_bits, vo
  * kernel (layers with tcbnn_conv_planes_bytes != 0 called with their workspace, pool == 1, channel
  * counts in multiples of 8; other calls fail) and written by tcbnn_inconv_specialized_layer;
  * tcbnn_conv_prefers_chunked_residual says for which layers it is the faster choice (every layer
- * the loader-fed kernel takes: its tile-per-group epilogue handles no other residual layout, and
- * it reads a pooled chunk-major residual in place, without the pooling pass NHWC tensors get).
+ * the loader-fed kernel takes).
  * TCBNN_RES_PROVEN, ORed into the res_out_bytes of an int16 format, says that the caller has
  * proven the bound |value| <= 32767 (e.g. C*R*S + the bound of res_in, the way the drop-in classes
  * choose int16): the layer then skips the per-value range check that sets status 2, which costs
@@ -148,9 +147,7 @@ int tcbnn_conv_layer(const tcbnn_conv_desc* d, const uint32_t* in, const void* p
  * run fastest when their input is first written out as +-1 bytes in the tensor cores' operand
  * layout by a streaming pass and the convolution kernel fetches it with bulk copies;
  * tcbnn_conv_workspace_bytes says how much device memory (256-byte aligned) that takes for a
- * descriptor, 0 when the layer has no use for it.  (Wide layers use the buffer for something
- * else: a pooled int16 residual is first reduced into it by a streaming pass.
- * tcbnn_conv_planes_bytes is the part that is the pre-expanded input: the size of the planes of
+ * descriptor, 0 when the layer has no use for it.  (tcbnn_conv_planes_bytes is the part that is the pre-expanded input: the size of the planes of
  * tcbnn_conv_layer_x, 0 for layers that take none.)  The buffer is only used during the call
  * (stream order); one buffer of the largest size serves all layers of a network on one stream.
  * With workspace == NULL this is tcbnn_conv_layer.  No reference counterpart. */
@@ -187,16 +184,11 @@ int tcbnn_conv_layer_x(const tcbnn_conv_desc* d, const uint32_t* in, const void*
  * is eligible, else the warp-level b1 MMA), 1 = always the b1 MMA, 2 = tcgen05 or an error,
  * 3 = as 2 but only the filter-stationary tcgen05 kernel with its in-kernel bit expansion (wide
  * stride-1 layers otherwise take the activation-stationary kernel, narrow ones with a workspace the
- * kernel fed from a pre-expanded input), 4 = as 0 but the loader-fed kernel moves int16 residual
- * rows straight between registers and global memory, never staging them in shared memory, 5 = as 0
- * but staging them wherever the tensors allow (0 stages them where that measured faster), 6 = as
- * 0 but the loader-fed kernel always runs one CTA per SM (0 runs layers with an n-tile of 64 as
- * two smaller CTAs per SM when they fit), 7 = as 0 but without the loader-fed kernel's
- * tile-per-group epilogues (0 uses them for layers without residuals and for chunk-major int16
- * residuals), 8 = as 0 but two CTAs per SM also for the all-warps-per-tile residual epilogues at an
- * n-tile of 64, 9 = as 0 but the loader-fed kernel's stages hold one 64-channel block each (0
- * puts four or two in a stage where three such stages fit), 10 = as 0 but every n-tile of a layer
- * gets the same number of CTAs (0 gives the n-tiles that carry a pooled residual more).
+ * kernel fed from a pre-expanded input), 6 = as 0 but the loader-fed kernel always runs one CTA per
+ * SM (0 runs layers with an n-tile of 64 as two smaller CTAs per SM when they fit), 9 = as 0 but its
+ * stages hold one 64-channel block each (0 puts four or two in a stage where three such stages fit),
+ * 10 = as 0 but every n-tile of a layer gets the same number of CTAs (0 gives the n-tiles that carry
+ * a pooled residual more); 4, 5, 7, 8 = as 0.
  * Process-wide; meant for tests and measurements.  No reference counterpart (the reference has one
  * kernel per layer type). */
 int tcbnn_set_conv_path(int path);

@@ -134,7 +134,18 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&r)[32]) {
           "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr) : "memory");
 }
-// Same for 16 and 8 columns, and a width-generic front.
+// 16 lanes x 32 consecutive columns: thread t of the warp gets, for n = 0..3 and e = 0, 1, columns
+// 8n + 2(t%4) + e of lane t/4 in r[4n + e] and of lane t/4 + 8 in r[4n + 2 + e].
+__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, int (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+          "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr) : "memory");
+}
+// Same as tmem_ld32 for 16 and 8 columns.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&r)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -150,12 +161,17 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&r)[8]) {
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
         : "r"(taddr) : "memory");
 }
-template <int N> __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, int (&r)[N]);
-template <> __device__ __forceinline__ void tmem_ld_cols<32>(uint32_t taddr, int (&r)[32]) { tmem_ld32(taddr, r); }
-template <> __device__ __forceinline__ void tmem_ld_cols<16>(uint32_t taddr, int (&r)[16]) { tmem_ld16(taddr, r); }
-template <> __device__ __forceinline__ void tmem_ld_cols<8>(uint32_t taddr, int (&r)[8]) { tmem_ld8(taddr, r); }
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// The same wait, naming the registers it makes valid: keeps their uses behind it where a later load is
+// issued before they are used.
+__device__ __forceinline__ void tmem_ld_wait16(int (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :: "memory");
 }
 
 // Shared-memory matrix descriptor, K-major, no swizzle: rows 16 B apart inside a core matrix,
@@ -189,18 +205,24 @@ __device__ __forceinline__ uint4 expand16(uint32_t h) {
 // operand bytes (measured by tcbnn_mma_peak kind 7).  Layout as for int8, K-major without
 // swizzle, except that a 16-byte core-matrix row now holds 32 channels and one MMA spans two of
 // them (`lbo` apart).
-// 8 packed bits -> 8 nibbles (bit i -> nibble i; 1 -> +1.0, 0 -> -1.0)
-__host__ __device__ __forceinline__ uint32_t expand8_f4(uint32_t b) {
-    uint32_t x = b & 0xFFu;
-    x = (x | (x << 12)) & 0x000F000Fu;
-    x = (x | (x << 6)) & 0x03030303u;
-    x = (x | (x << 3)) & 0x11111111u;
-    return 0xAAAAAAAAu ^ (x << 3);
-}
-// 32 packed bits -> 16 bytes; bits 31..24 (the chunk's channels 0-7) land in .x, 7..0 in .w.
-// Activations and filters both go through this function, so the order inside a word cancels.
+// 32 packed bits -> 16 bytes of +-1.0: bit 4*i + j of the word -> nibble i of .x/.y/.z/.w for j = 3..0
+// (1 -> +1.0, 0 -> -1.0).  Which bit lands in which nibble is free -- activations and filters both go
+// through this function, so the order inside a word cancels -- and this one costs a shift and a
+// three-input logic operation per eight values (spreading a byte's bits in order takes four times that).
 __host__ __device__ __forceinline__ uint4 expand32_f4(uint32_t w) {
-    return make_uint4(expand8_f4(w >> 24), expand8_f4(w >> 16), expand8_f4(w >> 8), expand8_f4(w));
+    return make_uint4((w & 0x88888888u) ^ 0xAAAAAAAAu, ((w << 1) & 0x88888888u) ^ 0xAAAAAAAAu,
+                      ((w << 2) & 0x88888888u) ^ 0xAAAAAAAAu, ((w << 3) & 0x88888888u) ^ 0xAAAAAAAAu);
+}
+// Output channel (within its 32) that column c of an accumulator holds.  A tcgen05.ld of shape 16x256b
+// gives a thread columns 8n + 2q and 8n + 2q + 1 of its rows (q = lane % 4, n = 0..3); with this order
+// those are two runs of four consecutive channels, 4q.. and 16 + 4q.., so that the four lanes of a
+// quad move 64 (int32) or 32 (int16) consecutive bytes of an NHWC row.  The filter blob is laid out in
+// this order (prepare_filter_f4), thresholds and bit positions follow it.
+__host__ __device__ constexpr int f4_channel_of_column(int c) {
+    return 16 * (c >> 4) + 4 * ((c >> 1) & 3) + 2 * ((c >> 3) & 1) + (c & 1);
+}
+__host__ __device__ constexpr int f4_column_of_channel(int ch) {
+    return 8 * (2 * (ch >> 4) + ((ch >> 1) & 1)) + 2 * ((ch >> 2) & 3) + (ch & 1);
 }
 // Instruction descriptor of the block-scaled kinds: e2m1 x e2m1, ue8m0 scales, K-major, M = 128,
 // K = 64, scale-factor ids 0.
@@ -221,6 +243,88 @@ __device__ __forceinline__ void mma_f4_split(uint32_t d_tmem, uint32_t a_lo, uin
         ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate),
           "r"(sfa), "r"(sfb));
 }
+// Runs of K MMAs (taps t[0..K-1] of one 64-channel block, B advancing by step_b per tap), each written
+// as one block because of what the issuing warp does between two MMAs: the tensor pipe queues only
+// two or three instructions, so whatever takes longer than that is time it idles.  The whole warp
+// executes them, the lane with leader != 0 issues; the first MMA accumulates when acc != 0, the
+// others always.
+//   mma_f4_run      nothing but the MMAs
+//   mma_f4_end      the last MMAs of a stage: two barrier tests in front of them whose results are
+//                   read behind them, then the commits of the stage and of the accumulator.  A test
+//                   takes 150-200 clocks to return while the MMAs keep the shared-memory port busy;
+//                   asked for first and read last, that time is covered.  bar_c: 0 = no commit.
+//                   Bit 0 / 1 of the result: phase par0 / par1 of barrier bar0 / bar1 is complete.
+// Measured on groups of nine with one wait and one commit per group: 61.8 -> 48.0 clocks per MMA at
+// N = 64, 70.7 -> 64.0 at N = 128, the pipe's own rate.
+#define TCBNN_F4_MMA(AOFF, PRED)                                                                     \
+    "add.u32 xa, %1, " AOFF ";\n\tmov.b64 da, {xa, %2};\n\tmov.b64 db, {xb, %4};\n\t"                \
+    "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%5], da, db, %6, [%8], [%9], " PRED ";\n\t" \
+    "add.u32 xb, xb, %10;\n\t"
+#define TCBNN_F4_HEAD                                                                                \
+    ".reg .pred pq, pt, pl;\n\t.reg .b64 da, db;\n\t.reg .b32 xa, xb;\n\t"                           \
+    "setp.ne.b32 pl, %0, 0;\n\tsetp.ne.b32 pq, %7, 0;\n\tsetp.eq.b32 pt, %0, %0;\n\tmov.u32 xb, %3;\n\t"
+#define TCBNN_F4_IN                                                                                  \
+    "r"(leader), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(d_tmem), "r"(idesc), "r"(acc), "r"(sfa), \
+        "r"(sfb), "r"(step_b)
+template <int K>
+__device__ __forceinline__ void mma_f4_run(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
+                                           uint32_t b_lo, uint32_t b_hi, uint32_t step_b, const uint32_t* t,
+                                           uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb) {
+    static_assert(K == 1 || K == 5 || K == 9, "run lengths in use");
+    if constexpr (K == 9)
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
+                     TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") TCBNN_F4_MMA("%16", "pt")
+                     TCBNN_F4_MMA("%17", "pt") TCBNN_F4_MMA("%18", "pt") TCBNN_F4_MMA("%19", "pt") "}"
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]),
+                       "r"(t[7]), "r"(t[8]) : "memory");
+    else if constexpr (K == 5)
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
+                     TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") "}"
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]) : "memory");
+    else
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") "}" ::TCBNN_F4_IN, "r"(t[0]) : "memory");
+}
+#undef TCBNN_F4_MMA
+#undef TCBNN_F4_HEAD
+#undef TCBNN_F4_IN
+#define TCBNN_F4_MMA(AOFF, PRED)                                                                     \
+    "add.u32 xa, %2, " AOFF ";\n\tmov.b64 da, {xa, %3};\n\tmov.b64 db, {xb, %5};\n\t"                \
+    "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%6], da, db, %7, [%9], [%10], " PRED ";\n\t" \
+    "add.u32 xb, xb, %11;\n\t"
+#define TCBNN_F4_HEAD                                                                                \
+    "{\n\t.reg .pred p0, p1, pq, pt, pl, pc;\n\t.reg .b64 da, db;\n\t.reg .b32 xa, xb, r1;\n\t"       \
+    "mbarrier.test_wait.parity.shared::cta.b64 p0, [%12], %13;\n\t"                                 \
+    "mbarrier.test_wait.parity.shared::cta.b64 p1, [%14], %15;\n\t"                                 \
+    "setp.ne.b32 pl, %1, 0;\n\tsetp.ne.b32 pq, %8, 0;\n\tsetp.eq.b32 pt, %1, %1;\n\tmov.u32 xb, %4;\n\t" \
+    "setp.ne.and.b32 pc, %17, 0, pl;\n\t"
+#define TCBNN_F4_TAIL                                                                                \
+    "@pl tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%16];\n\t"           \
+    "@pc tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%17];\n\t"           \
+    "selp.u32 %0, 1, 0, p0;\n\tselp.u32 r1, 2, 0, p1;\n\tor.b32 %0, %0, r1;\n\t}"
+#define TCBNN_F4_IN                                                                                  \
+    "r"(leader), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(d_tmem), "r"(idesc), "r"(acc), "r"(sfa), \
+        "r"(sfb), "r"(step_b), "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar_e), "r"(bar_c)
+template <int K>
+__device__ __forceinline__ uint32_t mma_f4_end(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
+                                               uint32_t b_lo, uint32_t b_hi, uint32_t step_b, const uint32_t* t,
+                                               uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb,
+                                               uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1,
+                                               uint32_t bar_e, uint32_t bar_c) {
+    static_assert(K == 1 || K == 4, "run lengths in use");
+    uint32_t ok;
+    if constexpr (K == 4)
+        asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_MMA("%19", "pt") TCBNN_F4_MMA("%20", "pt")
+                     TCBNN_F4_MMA("%21", "pt") TCBNN_F4_TAIL
+                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
+    else
+        asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_TAIL
+                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]) : "memory");
+    return ok;
+}
+#undef TCBNN_F4_MMA
+#undef TCBNN_F4_HEAD
+#undef TCBNN_F4_TAIL
+#undef TCBNN_F4_IN
 // Columns [col, col + 32) of the calling warp's 32 lanes of tensor memory := unit scales (every
 // byte 0x7F), so a scale reads as 1.0 wherever in the region the hardware looks it up.  Whole
 // warp; warps 0-3 of a warpgroup cover the 128 lanes between them (warp w -> lanes 32*(w%4)..).
@@ -232,10 +336,11 @@ __device__ __forceinline__ void tmem_fill_unit_scales(uint32_t tmem, uint32_t co
                      ::"r"(base + c), "r"(0x7F7F7F7Fu) : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-// fp32 accumulator holding an integer of magnitude below 2^22 -> that integer, exactly
-__device__ __forceinline__ int f4_acc_to_int(int raw) {
-    return __float_as_int(__int_as_float(raw) + 12582912.0f) - 0x4B400000;
-}
+// fp32 accumulator holding an integer of magnitude below 2^22 -> that integer, exactly; the biased
+// form leaves kF4Bias on it (its low 16 bits are those of the integer)
+constexpr int kF4Bias = 0x4B400000;
+__device__ __forceinline__ int f4_acc_to_biased(int raw) { return __float_as_int(__int_as_float(raw) + 12582912.0f); }
+__device__ __forceinline__ int f4_acc_to_int(int raw) { return f4_acc_to_biased(raw) - kF4Bias; }
 
 // Four consecutive residual channels (element index i, a multiple of 4) widened to int32.
 __device__ __forceinline__ int4 ld_res4(const void* p, int bytes, size_t i) {

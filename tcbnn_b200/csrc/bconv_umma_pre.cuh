@@ -26,13 +26,11 @@
 namespace tcbnn {
 namespace umma {
 
-constexpr int kPreEpiThreads = 512;         // epilogue threads of the one-CTA-per-SM form (16 warps)
 // One MMA-issuing warp.  (Two issuers on alternate tiles were tried and are wrong as well as no
 // faster: an mbarrier wait names its phase by parity only, so a waiter must see every phase of a
 // barrier; with two consumers alternating on the same ring slot the one that runs ahead finds the
 // parity of the phase before last already complete and reads a slot that has not been refilled.)
 constexpr int kPreMmaWarps = 1;
-constexpr int kPreThreads = kPreEpiThreads + 32 + 32 * kPreMmaWarps;
 // EPIW, the kernel's third template argument, is the number of epilogue warps: 16 (one CTA per SM,
 // all of tensor memory) or 8 (n-tile 64 only: each thread then takes 32 columns instead of 16, the
 // CTA allocates half of tensor memory and two CTAs share an SM -- twice the independent
@@ -51,10 +49,13 @@ __host__ __device__ inline long long pre_plane_positions(long long NV, int npos,
 }
 // nplane: 1 for stride 1, 4 for stride 2 (the input's four row / column parity planes)
 __host__ __device__ inline size_t pre_smem_bytes(int npos, int C, int RS, int nt, int stages, int nplane) {
-    return (size_t)stages * nplane * 2 * npos * 16 + (size_t)RS * C * nt / 2 + nt * 8 + RS * 8 + 40 * 8 + 64;
+    return (size_t)stages * nplane * 2 * npos * 16 + (size_t)RS * C * nt / 2 + nt * 8 + RS * 8 + 44 * 8 + 64;
 }
-// two buffers of a tile's int16 residual rows (128 rows x nt channels), staged in shared memory
-__host__ __device__ inline size_t pre_res_stage_bytes(int nt) { return (size_t)2 * 128 * nt * 2 + 128; }
+// kEpiTileRes: one buffer per epilogue group for the injected residual of its next tile, [chunk][128
+// pixels][16 B]
+__host__ __device__ constexpr size_t pre_res_ring_bytes(int nt, int epiw) {
+    return (size_t)(epiw / (nt <= 64 ? 4 : nt / 16)) * 128 * nt * 2 + 128;
+}
 
 // packed bits [B][H][W][C/32] -> planes [C/32][nplane][plane_positions][16 B] of +-1 nibbles, zero
 // where the raster position is padding or outside the batch.  Stride 1: one plane, the raster of
@@ -87,52 +88,47 @@ __device__ __forceinline__ void expand_raster(const ConvWsArgs& a, uint4* planes
     }
 }
 
-// Staged epilogue: int16 residual rows travel through shared memory.  The four epilogue warps that
-// share 32 rows of a tile (same TMEM lane quadrant, different column groups) form a group: the live
-// pixels among its rows are consecutive rows of the residual tensors, so the group's 128 threads
-// move them as whole 128-byte lines (cp.async in, 16-byte stores out: 4 lines per instruction) into
-// a buffer of its own whose 16-byte chunks are XOR-swizzled by row, and every thread then reads /
-// overwrites its own pixel's chunks there without bank conflicts.  The incoming rows of the next
-// tile fly while this tile is computed; the outgoing rows leave one tile late; the four groups
-// meet only among themselves (one mbarrier each), never CTA-wide.  (Without it each lane moves 16-byte pieces of its own row: 32
-// lines per instruction, which made L1TEX the busiest unit of these layers.)
-//
-// EPI selects the epilogue the kernel is compiled with, so that each carries only its own
-// registers (18 warps leave 96 per thread): 0 = plain (no residual in or out, no integer output:
-// the fp32 accumulator is compared with the fp32 threshold as it is), 1 = residual rows moved
-// directly between registers and global memory (any element size, pooled residuals, partial
-// channel ranges), 2 = staged int16 residual rows as described above.
-//
-// Tile-per-group epilogues (3 = no residual, 4 = chunk-major int16 residuals in and / or out): the
-// forms above put all 16 epilogue warps on every tile, so that a thread holds 16 or 32 of its
-// pixel's columns and pays the per-tile bookkeeping (raster position -> pixel, addresses, barrier
-// waits: some 200 instructions) for that few outputs -- most of what these warps issue.  Here a
-// group of 4 warps (8 at an n-tile of 128) owns a whole tile and the groups take tiles in turn: a
-// thread walks 64 columns of its pixel in passes of 32, the bookkeeping is paid once per 64
-// outputs, and the groups work on different accumulators at the same time (NT = 64: 4 groups on
-// 7 accumulators; NT = 128: 2 groups on 3).  With one thread per pixel every tensor is touched in
-// whole lines: chunk-major residuals, 16-byte plane slots, 8 bytes of packed bits -- so nothing is
-// staged, and a pooled residual is read in place (four lines per chunk) instead of by a pass of
-// its own.
-constexpr int kEpiPlain = 0, kEpiDirect = 1, kEpiStaged = 2, kEpiTile = 3, kEpiTileRes = 4;
+// Epilogues.  A group of 4 warps (8 at an n-tile of 128) owns a whole tile and the groups take tiles in
+// turn: a thread walks 64 columns (of one pixel, or of four pixels a quarter each) in passes of 32, so
+// that the per-tile bookkeeping (raster position -> pixel, addresses, barrier waits: some 200
+// instructions) is paid once per 64 outputs, and the groups work on different accumulators at the same
+// time (NT = 64: 4 groups on 7 accumulators; NT = 128: 2 groups on 3).  EPI selects the epilogue the
+// kernel is compiled with, so that each carries only its own registers: a thread has 96 with one CTA
+// of 18 warps per SM or two of 10, and with nearly all of L1 taken as shared memory a spilled
+// register costs a trip to L2 (28 x 28 x 128 with residuals at batch 512: eight spilled reloads per warp
+// and tile kept every warp waiting for a third of its time).
+//   kEpiTile      no residual, no integer output: the fp32 accumulator is compared with the fp32
+//                 threshold as it is.  One thread per pixel.
+//   kEpiTileRes   chunk-major int16 residuals in and / or out.  One thread per pixel: every tensor is
+//                 touched in whole lines.  The live pixels of a tile are consecutive pixels of the
+//                 tensor, so its incoming residual is one run of up to 2 KB per chunk; the group
+//                 fetches these with bulk copies into a buffer of its own as soon as it has read the
+//                 tile in front from it, so that they are in flight while it packs, stores and waits (a register-fed epilogue has 64 bytes per thread
+//                 in flight, and only while it waits).
+//   kEpiTilePool  the same with a pooled residual, or one whose buffers do not fit beside the filter
+//                 block: read in place (four lines per pooled chunk).
+//   kEpiRows2/4   everything else: NHWC residuals (int16 in: Rows2, int32 in: Rows4), NHWC saves,
+//                 integer output, mixtures with the chunk-major layout.  The accumulator is read in
+//                 the 16x256b shape: a quad of lanes holds 32 channels of four pixels, so it moves
+//                 whole 32-byte sectors of an NHWC row (f4_channel_of_column), where a thread per pixel
+//                 would move 16-byte pieces of 32 different rows.  What a later unit of work reads is
+//                 requested before the one in front is computed.  Measured on 56 x 56 x 128 -> 128, batch
+//                 256, int32 result saved (411 MB): 251 us with a thread per pixel.
+constexpr int kEpiTile = 0, kEpiTileRes = 1, kEpiRows2 = 2, kEpiRows4 = 3, kEpiTilePool = 4;
 template <int NT, int EPI, int EPIW>
 __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
-    constexpr bool RSTAGE = EPI == kEpiStaged;
     constexpr int kEpiThreads = EPIW * 32, kThreadsCta = pre_threads(EPIW);
-    static_assert(EPIW == 16 || (EPIW == 8 && NT == 64 && EPI != kEpiStaged), "8 epilogue warps: n-tile 64, no staging");
-    constexpr bool TILE = EPI == kEpiTile || EPI == kEpiTileRes;
-    constexpr int CPT = NT < 64 ? NT : 64;            // tile-per-group: columns of a tile per thread
-    constexpr int WPG = 4 * (NT / CPT);               // ... warps of a group (all rows x all columns of a tile)
-    constexpr int NG = EPIW / WPG;                    // ... groups, each on a tile of its own
+    static_assert(EPIW == 16 || (EPIW == 8 && NT == 64), "8 epilogue warps: n-tile 64");
+    constexpr bool ROWS = EPI == kEpiRows2 || EPI == kEpiRows4;
+    constexpr int CPT = NT < 64 ? NT : 64;            // columns of a tile per thread
+    constexpr int WPG = 4 * (NT / CPT);               // warps of a group (all rows x all columns of a tile)
+    constexpr int NG = EPIW / WPG;                    // groups, each on a tile of its own
     // Tensor memory: accumulators (7 at NT = 64) below column 480, the unit block scales of the
     // 4-bit MMA above it; the patch ring is as deep as shared memory allows, so that no role waits
     // on another's latency.
     constexpr uint32_t TM_COLS = EPIW == 16 ? 512 : 256, SF_COL = TM_COLS - 32;
-    constexpr int NACC = NT >= 128 ? (TILE ? 3 : 2)   // measured: deeper does not pay at NT = 128 when all warps share a tile
-                                   : ((SF_COL / NT) > 8 ? 8 : (SF_COL / NT));
+    constexpr int NACC = (SF_COL / NT) > 8 ? 8 : (SF_COL / NT);
     const int NSTAGE = a.pre_stages;
-    constexpr int COLS = NT / (EPIW / 4);             // accumulator columns per epilogue thread
-    static_assert(COLS == 8 || COLS == 16 || COLS == 32, "n-tile of 32, 64 or 128");
     constexpr int LOAD_WARP = EPIW, MMA_WARP = LOAD_WARP + 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int RS = a.R * a.S, NCB = a.C >> 6;
@@ -150,13 +146,13 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     float* sThrF = reinterpret_cast<float*>(sThr + NT);       // the thresholds as given (fp32)
     uint32_t* sTapK = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(sThrF + NT) + 7) & ~(uintptr_t)7);
     uint64_t* sBar = reinterpret_cast<uint64_t*>(sTapK + 2 * RS);
-    // barriers: a_full[8], a_empty[8], acc_full[8], acc_empty[8], epilogue groups [4], drain
-    uint32_t* sTmem = reinterpret_cast<uint32_t*>(sBar + 40);
+    // barriers: a_full[8], a_empty[8], acc_full[8], acc_empty[8], drain, res_full[NG], res_empty[NG]
+    uint32_t* sTmem = reinterpret_cast<uint32_t*>(sBar + 44);
     volatile int* sAbort = reinterpret_cast<volatile int*>(sTmem + 1);
-    unsigned char* sRes = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sTmem + 2) + 127) & ~(uintptr_t)127);
     const uint32_t bar0 = smem_u32(sBar);
-    auto BAR_EPI = [&](int g) { return bar0 + 8u * (32 + g); };    // rendezvous of an epilogue group (staged epilogue)
-    const uint32_t BAR_DRAIN = bar0 + 8u * 36;         // MMAs still in flight when the issuer gives up
+    const uint32_t BAR_DRAIN = bar0 + 8u * 32;         // MMAs still in flight when the issuer gives up
+    volatile int* sP0 = reinterpret_cast<volatile int*>(sTmem + 2);      // first pixel in each group's residual buffer
+    unsigned char* sRes = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sTmem + 6) + 127) & ~(uintptr_t)127);
     auto BAR_AFULL = [&](int s) { return bar0 + 8u * s; };
     auto BAR_AEMPTY = [&](int s) { return bar0 + 8u * (8 + s); };
     auto BAR_CFULL = [&](int b) { return bar0 + 8u * (16 + b); };
@@ -183,9 +179,9 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
 
     if (tid == 0) {
         for (int s = 0; s < 8; s++) { mbar_init(BAR_AFULL(s), 1); mbar_init(BAR_AEMPTY(s), 1); }
-        for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), TILE ? WPG : EPIW); }
-        for (int g = 0; g < 4; g++) mbar_init(BAR_EPI(g), EPIW / 4);
+        for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), WPG); }
         mbar_init(BAR_DRAIN, 1);
+        for (int g = 0; g < NG; g++) { mbar_init(bar0 + 8u * (33 + g), WPG); mbar_init(bar0 + 8u * (37 + g), WPG); }
         *sAbort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -198,12 +194,14 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             // integer form of  !((float)v < thr)  (kernel.cuh:795-796): v >= ceil(thr)
             int it = INT_MIN;
             float tf = __int_as_float(0x7FC00000);       // NaN: never "less", the bit is always set
-            if (obase + i < a.O) {
-                const float t = __ldg(a.thr + obase + i);
+            const int o = obase + (i & ~31) + f4_channel_of_column(i & 31);      // column i's channel
+            if (o < a.O) {
+                const float t = __ldg(a.thr + o);
                 tf = t;
                 if (t == t) it = t >= 2147483520.0f ? INT_MAX : t <= -2147483648.0f ? INT_MIN : (int)ceilf(t);
             }
-            sThr[i] = it;
+            // (the int16 epilogues compare values that still carry kF4Bias)
+            sThr[i] = EPI == kEpiTileRes || EPI == kEpiTilePool ? kF4Bias + min(max(it, -(1 << 23)), 1 << 23) : it;
             sThrF[i] = tf;
         }
         for (int t = tid; t < RS; t += kThreadsCta) {
@@ -295,54 +293,103 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             const uint32_t stepBlock = block_bytes >> 4;
             constexpr uint32_t IDESC = idesc_f4(NT);
             const uint32_t sfa = tmem + SF_COL, sfb = tmem + SF_COL + 16;
-            const bool rs9 = RS == 9;
             uint32_t tapk[9];                              // 3x3 filters: the tap offsets in registers
 #pragma unroll
-            for (int t = 0; t < 9; t++) tapk[t] = rs9 ? sTapK[t] : 0u;
-            const uint32_t w2 = (uint32_t)(warp - MMA_WARP);
-            uint32_t it = 0;
+            for (int t = 0; t < 9; t++) tapk[t] = t < RS ? sTapK[t] : 0u;
             bool ok = true;
             long long tr_wc = 0, tr_wa = 0;
             const long long tr_t0 = clock64();
-            // ring slot, accumulator and their phases as running counters: a division by the
-            // ring depth per stage would sit between two groups of MMAs
+            // One pass per stage of the ring.  Ring slot, accumulator and their phases are running
+            // counters (a division by the ring depth would sit between two groups of MMAs), and what
+            // the next stage needs is worked out behind the stage's first MMAs, while these keep the
+            // pipe busy: between the last MMA of a stage and the first of the next only a branch on
+            // the outcome of tests made earlier is left.
             static_assert(kPreMmaWarps == 1, "the counters below assume one issuing warp");
-            int s = 0, b = 0;
-            uint32_t sph = 0, bph = 0;
-            for (uint32_t tc = w2; (long long)mfirst + (long long)tc * mstep < mtiles && ok; tc += kPreMmaWarps) {
-                ok = a.trace ? wait.timed(BAR_CEMPTY(b), bph ^ 1, tr_wc) : wait.spin(BAR_CEMPTY(b), bph ^ 1);
-                if (!ok) break;
+            const uint32_t spt = (uint32_t)(NCB / CBS);    // stages per tile
+            const uint32_t nit = mfirst < mtiles ? (uint32_t)((mtiles - mfirst + mstep - 1) / mstep) * spt : 0u;
+            uint32_t s = 0, b = 0, sph = 0, bph = 0, left = spt;      // left: stages of this tile still to issue
+            uint32_t acc = 0, bLo = bLo0, d = tmem, aLo = aLo0;
+            // ready: bit 0 = this stage is known to be full, bit 1 = this tile's accumulator to be free,
+            // asked while the stage in front was issued (mma_f4_end); waited for only where not yet so
+            uint32_t ready = 0, need = 3u;
+            const uint32_t tap_end = sTapK[RS - 1];
+            for (uint32_t it = 0; it < nit; it++) {
+                if ((ready & need) != need) {
+                    if ((need & 2u) && !(ready & 2u)) {
+                        ok = a.trace ? wait.timed(BAR_CEMPTY(b), bph ^ 1, tr_wc) : wait.spin(BAR_CEMPTY(b), bph ^ 1);
+                        if (!ok) break;
+                    }
+                    if (!(ready & 1u)) {
+                        ok = a.trace ? wait.timed(BAR_AFULL(s), sph, tr_wa) : wait.spin(BAR_AFULL(s), sph);
+                        if (!ok) break;
+                    }
+                }
                 tc_fence_after();
-                const uint32_t d = tmem + b * NT;
-                uint32_t acc = 0;
-                uint32_t bLo = bLo0;
-                for (int cb = 0; cb < NCB && ok; cb += CBS, it++) {
-                    ok = a.trace ? wait.timed(BAR_AFULL(s), sph, tr_wa) : wait.spin(BAR_AFULL(s), sph);
-                    if (!ok) break;
-                    tc_fence_after();
-                    if (leader) {
-                    for (int sub = 0; sub < CBS; sub++) {
-                        const uint32_t aLo = aLo0 + s * stepStage + sub * stepBlock;
-                        if (rs9) {
-#pragma unroll
-                            for (int t = 0; t < 9; t++)
-                                mma_f4_split(d, aLo + tapk[t], aHi, bLo + t * stepB, bHi, IDESC, t == 0 ? acc : 1u, sfa, sfb);
-                            bLo += 9 * stepB;
-                        } else {
-                            for (int t = 0; t < RS; t++) {
-                                mma_f4_split(d, aLo + sTapK[t], aHi, bLo, bHi, IDESC, acc, sfa, sfb);
-                                acc = 1;
-                                bLo += stepB;
-                            }
-                        }
+                if (RS == 9) {
+                    for (int sub = 0; sub + 1 < CBS; sub++) {
+                        mma_f4_run<9>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk, IDESC, acc, sfa, sfb);
+                        bLo += 9 * stepB;
+                        aLo += stepBlock;
                         acc = 1;
                     }
-                    mma_commit(BAR_AEMPTY(s));          // stage free once these MMAs have read it
+                    mma_f4_run<5>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk, IDESC, acc, sfa, sfb);
+                    bLo += 5 * stepB;
+                } else {
+                    // other filters: taps in runs of five while they last, then one by one; the last is left
+                    for (int sub = 0; sub < CBS; sub++) {
+                        const int nt_ = sub + 1 == CBS ? RS - 1 : RS;
+                        int t = 0;
+                        uint32_t tk[5];                    // read one run ahead, for the same reason
+#pragma unroll
+                        for (int j = 0; j < 5; j++) tk[j] = sTapK[min(j, RS - 1)];
+                        for (; t + 5 <= nt_; t += 5) {
+                            uint32_t tn[5];
+#pragma unroll
+                            for (int j = 0; j < 5; j++) tn[j] = sTapK[min(t + 5 + j, RS - 1)];
+                            mma_f4_run<5>(leader, d, aLo, aHi, bLo, bHi, stepB, tk, IDESC, acc, sfa, sfb);
+                            bLo += 5 * stepB;
+                            acc = 1;
+#pragma unroll
+                            for (int j = 0; j < 5; j++) tk[j] = tn[j];
+                        }
+                        for (; t < nt_; t++) {             // fewer than five: tk holds them
+                            mma_f4_run<1>(leader, d, aLo, aHi, bLo, bHi, stepB, tk, IDESC, acc, sfa, sfb);
+#pragma unroll
+                            for (int j = 0; j < 4; j++) tk[j] = tk[j + 1];
+                            bLo += stepB;
+                            acc = 1;
+                        }
+                        if (sub + 1 < CBS) aLo += stepBlock;
                     }
-                    if (++s == NSTAGE) { s = 0; sph ^= 1u; }
                 }
-                if (ok && leader) mma_commit(BAR_CFULL(b));       // accumulator complete
-                if (++b == NACC) { b = 0; bph ^= 1u; }
+                asm volatile("" : "+r"(s), "+r"(b), "+r"(left), "+r"(sph), "+r"(bph));   // what follows stays behind those MMAs
+                const bool last = left == 1;
+                const bool swrap = s + 1 == (uint32_t)NSTAGE, bwrap = b + 1 == (uint32_t)NACC;
+                const uint32_t sn = swrap ? 0u : s + 1, bn = bwrap ? 0u : b + 1;
+                uint32_t sphn = swrap ? sph ^ 1u : sph, bphn = bwrap ? bph ^ 1u : bph;
+                uint32_t bar_a = BAR_AFULL(sn), bar_b = BAR_CEMPTY(bn), par_b = bphn ^ 1u;
+                uint32_t bar_e = BAR_AEMPTY(s), bar_c = last ? BAR_CFULL(b) : 0u;
+                uint32_t aLon = aLo0 + sn * stepStage, dn = last ? tmem + bn * NT : d;
+                uint32_t bLon = last ? bLo0 : bLo + (RS == 9 ? 4u : 1u) * stepB;
+                need = last ? 3u : 1u;
+                if (last) { b = bn; bph = bphn; }
+                left = last ? spt : left - 1;
+                s = sn;
+                sph = sphn;
+                const uint32_t acc_end = RS == 9 ? 1u : acc;
+                acc = last ? 0u : 1u;
+                asm volatile("" : "+r"(bar_a), "+r"(bar_b), "+r"(par_b), "+r"(bar_e), "+r"(bar_c), "+r"(aLon), "+r"(dn),
+                                  "+r"(bLon), "+r"(need), "+r"(b), "+r"(bph), "+r"(left), "+r"(s), "+r"(sph), "+r"(acc));
+                if (RS == 9) {
+                    ready = mma_f4_end<4>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk + 5, IDESC, acc_end, sfa, sfb,
+                                          bar_a, sphn, bar_b, par_b, bar_e, bar_c);
+                } else {
+                    ready = mma_f4_end<1>(leader, d, aLo, aHi, bLo, bHi, stepB, &tap_end, IDESC, acc_end, sfa, sfb,
+                                          bar_a, sphn, bar_b, par_b, bar_e, bar_c);
+                }
+                aLo = aLon;
+                d = dn;
+                bLo = bLon;
             }
             if (!ok && leader) {
                 // giving up: the MMAs already issued must have finished before tensor memory is freed
@@ -350,14 +397,14 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                 for (int i = 0; i < (1 << 20); i++)
                     if (mbar_try_wait(BAR_DRAIN, 0)) break;
             }
-            if (a.trace && blockIdx.x == 0 && leader && w2 == 0) { a.trace[3] = clock64() - tr_t0; a.trace[4] = tr_wc; a.trace[5] = tr_wa; a.trace[2] = it; }
+            if (a.trace && blockIdx.x == 0 && leader) { a.trace[3] = clock64() - tr_t0; a.trace[4] = tr_wc; a.trace[5] = tr_wa; a.trace[2] = nit; }
         }
         __syncwarp();
-    } else if (TILE && tid < kEpiThreads) {
-        // =============================== epilogue, a tile per group ==========================
-        constexpr bool RES = EPI == kEpiTileRes;
+    } else if (!ROWS && tid < kEpiThreads) {
+        // =============================== epilogue, a thread per pixel ==========================
+        constexpr bool RES = EPI == kEpiTileRes || EPI == kEpiTilePool, RING = EPI == kEpiTileRes;
         constexpr int PASSES = CPT / 32;
-        const int grp = warp / WPG, quad = warp & 3, half = (warp % WPG) >> 2;
+        const int grp = warp / WPG, wig = warp % WPG, quad = warp & 3, half = wig >> 2;
         const int row = quad * 32 + lane;
         const int Ow = (a.O + 31) >> 5;
         // Pass k of a thread covers the tile's 32-column block k (groups of 4 warps) or 2k + half
@@ -367,16 +414,46 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         const int o0 = obase + half * 32;                  // this thread's first output channel
         const int lim = (RES && a.res_in) ? min(a.residual_channels, a.res_in_ch) : 0;
         const bool has_in = RES && a.res_in && o0 < lim;
+        const bool ring = RING && obase < lim;
         const uint4* rin = reinterpret_cast<const uint4*>(a.res_in) + (size_t)(o0 >> 3) * a.res_in_npix;
         uint4* rout = reinterpret_cast<uint4*>(a.res_out) + (size_t)(o0 >> 3) * a.res_out_npix;
         bool ok = true, overflow = false;
-        uint32_t done = 0;
-        long long tr_w = 0;
-        const long long tr_t0 = clock64();
-        for (uint32_t tc = grp; (long long)mfirst + (long long)tc * mstep < mtiles && ok; tc += NG, done++) {
-            const int m = mfirst + (int)tc * mstep;
-            const int b = (int)(tc % NACC);
-            const uint32_t bph = (tc / NACC) & 1u;
+        const bool tr = a.trace != nullptr && blockIdx.x == 0;
+        uint32_t tr_w = 0;
+        const uint32_t tr_t0 = (uint32_t)clock64();
+        // ---- the group's residual buffer -----------------------------------------------------
+        const uint32_t bar_rf = bar0 + 8u * (33 + grp), bar_re = bar0 + 8u * (37 + grp);
+        unsigned char* const rbuf = sRes + (size_t)grp * (128 * NT * 2);
+        const int nchunk = ring ? min(NT, lim - obase) >> 3 : 0;
+        // output pixels in front of raster position p
+        auto live_before = [&](int p) -> int {
+            if (p >= NV) return a.B * a.OHg * a.OWg;
+            const int vy = fastdiv(p, a.pw_mul, a.pw_sh), x = p - vy * a.PW;
+            const int n = fastdiv(vy, a.vh_mul, a.vh_sh), y = vy - n * a.VH;
+            return (n * a.OHg + min(y, a.OHg)) * a.OWg + (y < a.OHg ? min(x, a.OWg) : 0);
+        };
+        // residual of m-tile `m` into the (free) buffer; the group's warps share the chunks, because a
+        // warp that issues bulk copies is busy for 100-200 clocks with each of them
+        auto request = [&](int m) {
+            const int p0 = live_before(m * 128), nl = live_before(m * 128 + 128) - p0;
+            const int mine = (nchunk - wig + WPG - 1) / WPG;             // chunks wig, wig + WPG, ..
+            if (lane == 0) {
+                if (wig == 0) sP0[grp] = p0;
+                mbar_expect_tx(bar_rf, (uint32_t)(mine * nl) * 16u);
+            }
+            __syncwarp();
+            if (nl > 0 && lane < mine)
+                bulk_g2s(smem_u32(rbuf) + (uint32_t)(wig + lane * WPG) * 2048u,
+                         reinterpret_cast<const uint4*>(a.res_in) + (size_t)((obase >> 3) + wig + lane * WPG) * a.res_in_npix + p0,
+                         (uint32_t)nl * 16u, bar_rf);
+        };
+        uint32_t rph = 0;
+        if (ring && mfirst + grp * mstep < mtiles) request(mfirst + grp * mstep);
+        static_assert(NG <= NACC, "the accumulator counters below wrap at most once per tile");
+        int b = grp;
+        uint32_t bph = 0;
+        for (int m = mfirst + grp * mstep; m < mtiles && ok; m += NG * mstep, b += NG) {
+            if (b >= NACC) { b -= NACC; bph ^= 1u; }
             // raster position -> output pixel
             const int p = m * 128 + row;
             bool live = false;
@@ -388,452 +465,359 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                 y = vy - n * a.VH;
                 live = x < a.OWg && y < a.OHg;
             }
-            const size_t opix = ((size_t)n * a.OHg + y) * a.OWg + x;
-            // injected residual of pass k (channels o0 + 32k ..): zeros where nothing is injected;
-            // 2x2 max for pooled residuals (kernel.cuh:773-783)
-            uint4 r[4];
-            auto fetch = [&](int k) {
+            const int opix = (n * a.OHg + y) * a.OWg + x;
+            // injected residual of step i (16 channels: half i & 1 of pass i >> 1): zeros where nothing
+            // is injected; 2x2 max for pooled residuals (kernel.cuh:773-783)
+            uint4 r[2];
+            auto fetch = [&](int i) {
                 const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-                if (a.residual_pool) {
-                    const size_t i00 = ((size_t)n * 2 * a.OHg + 2 * y) * 2 * a.OWg + 2 * x, rw = (size_t)2 * a.OWg;
+                const size_t i00 = ((size_t)n * 2 * a.OHg + 2 * y) * 2 * a.OWg + 2 * x, rw = (size_t)2 * a.OWg;
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        r[j] = z;
-                        if (live && o0 + 32 * HSTEP * k + 8 * j < lim) {
-                            const uint4* q = rin + (size_t)(4 * HSTEP * k + j) * a.res_in_npix + i00;
-                            const uint4 w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + rw), w3 = __ldg(q + rw + 1);
+                for (int j = 0; j < 2; j++) {
+                    r[j] = z;
+                    const int oc = 32 * HSTEP * (i >> 1) + 16 * (i & 1) + 8 * j;
+                    if (live && o0 + oc < lim) {
+                        const uint4* q = rin + (size_t)(oc >> 3) * a.res_in_npix;
+                        if (a.residual_pool) {
+                            const uint4 w0 = __ldg(q + i00), w1 = __ldg(q + i00 + 1), w2 = __ldg(q + i00 + rw), w3 = __ldg(q + i00 + rw + 1);
                             r[j].x = __vmaxs2(__vmaxs2(w0.x, w1.x), __vmaxs2(w2.x, w3.x));
                             r[j].y = __vmaxs2(__vmaxs2(w0.y, w1.y), __vmaxs2(w2.y, w3.y));
                             r[j].z = __vmaxs2(__vmaxs2(w0.z, w1.z), __vmaxs2(w2.z, w3.z));
                             r[j].w = __vmaxs2(__vmaxs2(w0.w, w1.w), __vmaxs2(w2.w, w3.w));
+                        } else {
+                            r[j] = __ldg(q + opix);
                         }
                     }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; j++)
-                        r[j] = (live && o0 + 32 * HSTEP * k + 8 * j < lim)
-                                   ? __ldg(rin + (size_t)(4 * HSTEP * k + j) * a.res_in_npix + opix) : z;
                 }
             };
-            if (RES && has_in) fetch(0);                   // flies while the accumulator is awaited
-            ok = (a.trace && blockIdx.x == 0) ? wait.timed(BAR_CFULL(b), bph, tr_w) : wait.relaxed(BAR_CFULL(b), bph);
+            if (EPI == kEpiTilePool && has_in) fetch(0);          // flies while the accumulator is awaited
+            ok = tr ? wait.relaxed_timed(BAR_CFULL(b), bph, tr_w) : wait.relaxed(BAR_CFULL(b), bph);
             if (!ok) break;
+            uint32_t rslot = 0;
+            if (ring) {
+                ok = tr ? wait.relaxed_timed(bar_rf, rph, tr_w) : wait.relaxed(bar_rf, rph);
+                if (!ok) break;
+                rph ^= 1u;
+                rslot = smem_u32(rbuf) + (uint32_t)(opix - sP0[grp]) * 16u;
+            }
             tc_fence_after();
-            uint32_t words[PASSES];
-#pragma unroll
+            int v0[16];                                    // (residual epilogues: the columns on their way)
+#pragma unroll 1
             for (int k = 0; k < PASSES; k++) {
-                int v[32];
-                tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + b * NT + (HSTEP * k + half) * 32, v);
-                tmem_ld_wait();
-                if (k == PASSES - 1) {
-                    tc_fence_before();                     // this warp is done with the accumulator
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
-                }
+                const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + b * NT + (HSTEP * k + half) * 32;
                 uint32_t word = 0;                         // channel c of the pass at bit 31 - c
-                if (!RES) {
+                if constexpr (!RES) {
+                    int v[32];
+                    tmem_ld32(taddr, v);
+                    tmem_ld_wait();
+                    if (k == PASSES - 1) {
+                        tc_fence_before();                 // this warp is done with the accumulator
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+                    }
                     // the reference's comparison as it stands, !((float)value < threshold)
                     // (kernel.cuh:795-796), on the fp32 accumulator
                     const float4* tf4 = reinterpret_cast<const float4*>(sThrF + (HSTEP * k + half) * 32);
 #pragma unroll
                     for (int j = 0; j < 8; j++) {
                         const float4 th = tf4[j];
-                        if (!(__int_as_float(v[4 * j]) < th.x)) word |= 0x80000000u >> (4 * j);
-                        if (!(__int_as_float(v[4 * j + 1]) < th.y)) word |= 0x80000000u >> (4 * j + 1);
-                        if (!(__int_as_float(v[4 * j + 2]) < th.z)) word |= 0x80000000u >> (4 * j + 2);
-                        if (!(__int_as_float(v[4 * j + 3]) < th.w)) word |= 0x80000000u >> (4 * j + 3);
+                        if (!(__int_as_float(v[4 * j]) < th.x)) word |= 0x80000000u >> f4_channel_of_column(4 * j);
+                        if (!(__int_as_float(v[4 * j + 1]) < th.y)) word |= 0x80000000u >> f4_channel_of_column(4 * j + 1);
+                        if (!(__int_as_float(v[4 * j + 2]) < th.z)) word |= 0x80000000u >> f4_channel_of_column(4 * j + 2);
+                        if (!(__int_as_float(v[4 * j + 3]) < th.w)) word |= 0x80000000u >> f4_channel_of_column(4 * j + 3);
                     }
                 } else {
+                    // 16 columns (two chunks) at a time, the next 16 on their way meanwhile: fewer
+                    // registers alive at once.  Values carry kF4Bias throughout.
+                    auto step = [&](int (&v)[16], const int h) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = f4_acc_to_int(v[j]);   // fp32 accumulators, exact integers
-                    if (has_in) {
+                        for (int j = 0; j < 16; j++) v[j] = f4_acc_to_biased(v[j]);
+                        auto add8 = [&](int j, const uint4& q) {
+                            const uint32_t rw[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                            for (int e = 0; e < 8; e++)
+                                v[f4_column_of_channel(8 * j + e)] += (e & 1) ? (int)rw[e >> 1] >> 16 : (int)(short)(rw[e >> 1] & 0xFFFFu);
+                        };
+                        const int c0 = (half + HSTEP * k) * 4 + 2 * h;       // first chunk of this step
+                        if constexpr (RING) {
+                            if (ring) {
+                                if (live) {
+#pragma unroll
+                                    for (int j = 0; j < 2; j++) {
+                                        if (c0 + j < nchunk) {
+                                            uint4 q;
+                                            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q.x), "=r"(q.y), "=r"(q.z), "=r"(q.w)
+                                                         : "r"(rslot + (uint32_t)(c0 + j) * 2048u) : "memory");
+                                            add8(j, q);
+                                        }
+                                    }
+                                }
+                                if (h == 1 && k == PASSES - 1) {         // buffer read: refill it for the group's next tile
+                                    __syncwarp();
+                                    if (lane == 0) mbar_arrive(bar_re);
+                                    if (m + NG * mstep < mtiles) {
+                                        ok = wait(bar_re, rph ^ 1u);
+                                        if (ok) request(m + NG * mstep);
+                                    }
+                                }
+                            }
+                        } else if (has_in) {
+#pragma unroll
+                            for (int j = 0; j < 2; j++) add8(j, r[j]);
+                            if (2 * k + h + 1 < 2 * PASSES) fetch(2 * k + h + 1);   // flies during this step's arithmetic
+                        }
+                        const int4* th4 = reinterpret_cast<const int4*>(sThr + (HSTEP * k + half) * 32 + 16 * h);
 #pragma unroll
                         for (int j = 0; j < 4; j++) {
-                            v[8 * j] += (int)(short)(r[j].x & 0xFFFFu);
-                            v[8 * j + 1] += (int)(short)(r[j].x >> 16);
-                            v[8 * j + 2] += (int)(short)(r[j].y & 0xFFFFu);
-                            v[8 * j + 3] += (int)(short)(r[j].y >> 16);
-                            v[8 * j + 4] += (int)(short)(r[j].z & 0xFFFFu);
-                            v[8 * j + 5] += (int)(short)(r[j].z >> 16);
-                            v[8 * j + 6] += (int)(short)(r[j].w & 0xFFFFu);
-                            v[8 * j + 7] += (int)(short)(r[j].w >> 16);
+                            const int4 th = th4[j];
+                            if (v[4 * j] >= th.x) word |= 0x80000000u >> (16 * h + f4_channel_of_column(4 * j));
+                            if (v[4 * j + 1] >= th.y) word |= 0x80000000u >> (16 * h + f4_channel_of_column(4 * j + 1));
+                            if (v[4 * j + 2] >= th.z) word |= 0x80000000u >> (16 * h + f4_channel_of_column(4 * j + 2));
+                            if (v[4 * j + 3] >= th.w) word |= 0x80000000u >> (16 * h + f4_channel_of_column(4 * j + 3));
                         }
-                        if (k + 1 < PASSES) fetch(k + 1);  // the next pass's residual flies during this one's arithmetic
-                    }
-                    const int4* th4 = reinterpret_cast<const int4*>(sThr + (HSTEP * k + half) * 32);
+                        if (a.res_out && live) {
+                            if (!a.res_out_proven) {       // a real branch: three instructions per value
+                                uint32_t ovf = 0;          // |v| of every value ORed together
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const int4 th = th4[j];
-                        if (v[4 * j] >= th.x) word |= 0x80000000u >> (4 * j);
-                        if (v[4 * j + 1] >= th.y) word |= 0x80000000u >> (4 * j + 1);
-                        if (v[4 * j + 2] >= th.z) word |= 0x80000000u >> (4 * j + 2);
-                        if (v[4 * j + 3] >= th.w) word |= 0x80000000u >> (4 * j + 3);
-                    }
-                    if (a.res_out && live) {
-                        if (!a.res_out_proven) {           // a real branch: two instructions per value
-                            uint32_t ovf = 0;              // |v| of every value ORed together
+                                for (int j = 0; j < 16; j++) ovf |= (uint32_t)((v[j] - kF4Bias) ^ ((v[j] - kF4Bias) >> 31));
+                                overflow |= ovf > 32767u;  // some value outside [-32768, 32767]
+                            }
 #pragma unroll
-                            for (int j = 0; j < 32; j++) ovf |= (uint32_t)(v[j] ^ (v[j] >> 31));
-                            overflow |= ovf > 32767u;      // some value outside [-32768, 32767]
+                            for (int j = 0; j < 2; j++) {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int kk = 0; kk < 4; kk++)
+                                    w[kk] = __byte_perm((uint32_t)v[f4_column_of_channel(8 * j + 2 * kk)],
+                                                        (uint32_t)v[f4_column_of_channel(8 * j + 2 * kk + 1)], 0x5410);
+                                rout[(size_t)(4 * HSTEP * k + 2 * h + j) * a.res_out_npix + opix] = make_uint4(w[0], w[1], w[2], w[3]);
+                            }
                         }
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int kk = 0; kk < 4; kk++)
-                                w[kk] = ((uint32_t)v[8 * j + 2 * kk] & 0xFFFFu) | ((uint32_t)v[8 * j + 2 * kk + 1] << 16);
-                            rout[(size_t)(4 * HSTEP * k + j) * a.res_out_npix + opix] = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
+                    };
+                    int v1[16];
+                    if (k == 0) tmem_ld16(taddr, v0);
+                    tmem_ld_wait16(v0);
+                    tmem_ld16(taddr + 16, v1);
+                    step(v0, 0);
+                    tmem_ld_wait16(v1);
+                    if (k == PASSES - 1) {
+                        tc_fence_before();                 // this warp is done with the accumulator
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+                    } else {
+                        tmem_ld16(taddr + HSTEP * 32, v0);
                     }
+                    step(v1, 1);
                 }
-                words[k] = word;
-                if (a.nxt && live) store_next_planes(a, n, y, x, o0 + 32 * HSTEP * k, word, 32);
-            }
-            if (live) {
-                // bits of channel o live at bit 31 - o%32 of word o/32
-                uint32_t* wp = a.out + (size_t)n * a.out_image_stride + ((size_t)y * a.OWg + x) * Ow + (o0 >> 5);
-                if (PASSES == 2 && HSTEP == 1 && (reinterpret_cast<uintptr_t>(wp) & 7) == 0) {
-                    *reinterpret_cast<uint2*>(wp) = make_uint2(words[0], words[PASSES - 1]);
-                } else {
-#pragma unroll
-                    for (int k = 0; k < PASSES; k++) wp[HSTEP * k] = words[k];
+                if (live) {
+                    // bits of channel o live at bit 31 - o%32 of word o/32
+                    a.out[(size_t)n * a.out_image_stride + ((size_t)y * a.OWg + x) * Ow + ((o0 + 32 * HSTEP * k) >> 5)] = word;
+                    if (a.nxt) store_next_planes(a, n, y, x, o0 + 32 * HSTEP * k, word);
                 }
             }
         }
+        if (ring && !ok) {
+            // giving up: a request may be in flight; wait (bounded) for it before the CTA exits
+            for (int i = 0; i < (1 << 20); i++)
+                if (mbar_try_wait(bar_rf, rph)) break;
+        }
         if (overflow) atomicExch(a.err_flag, 2);
-        if (a.trace && blockIdx.x == 0 && tid == 0) { a.trace[6] = clock64() - tr_t0; a.trace[7] = tr_w; a.trace[8] = done; }
-    } else if (!TILE && tid < kEpiThreads) {
-        // =============================== epilogue ===========================================
-        constexpr int NQ = COLS / 8;                       // 8-channel groups (one uint4 of int16) per thread
-        const int row = tid & 127, quad = warp & 3, cg = warp >> 2;
+        if (tr && tid == 0) {
+            a.trace[6] = (uint32_t)clock64() - tr_t0;
+            a.trace[7] = tr_w;
+            a.trace[8] = mfirst < mtiles ? (mtiles - mfirst + NG * mstep - 1) / (NG * mstep) : 0;
+        }
+    } else if (ROWS && tid < kEpiThreads) {
+        // =============================== epilogue, a quad per row piece ========================
+        constexpr int RB = EPI == kEpiRows2 ? 2 : 4;       // bytes of an injected residual value
+        constexpr int PASSES = CPT / 32, HSTEP = WPG / 4;
+        // A unit of work is 16 rows x 32 columns, two per pass.  Residual values are requested one unit
+        // ahead (int32, 16 registers) or two (int16, 8 registers each).
+        constexpr int NU = 2 * PASSES, AHEAD = RB == 4 ? 1 : 2, RREG = 4 * RB;
+        const int grp = warp / WPG, quad = warp & 3, half = (warp % WPG) >> 2;
+        // the row whose packed word this lane ends up with, and the quad's four rows
+        const int row = quad * 32 + (lane >> 2) + 8 * (lane & 3), q4 = lane & 3;
         const int Ow = (a.O + 31) >> 5;
+        const int o0 = obase + half * 32;
         const int lim = a.res_in ? min(a.residual_channels, a.res_in_ch) : 0;
-        const int o0 = obase + cg * COLS;                  // this thread's first output channel
-        const bool res16 = EPI == kEpiDirect && a.res_in && a.res_in_bytes == 2 && (a.res_in_ch & 7) == 0 && (lim & 7) == 0;
-        uint32_t tc = 0;
+        // element (pixel, channel o): pixel * stride + o (NHWC), or chunk-major [o/8][pixel][8]
+        const size_t in_ps = a.res_in_chunked ? 8 : (size_t)a.res_in_ch, out_ps = a.res_out_chunked ? 8 : (size_t)a.O;
+        auto in_off = [&](int o) { return a.res_in_chunked ? (size_t)(o >> 3) * a.res_in_npix * 8 + (o & 7) : (size_t)o; };
+        auto out_off = [&](int o) { return a.res_out_chunked ? (size_t)(o >> 3) * a.res_out_npix * 8 + (o & 7) : (size_t)o; };
         bool ok = true, overflow = false;
-        long long tr_w = 0;
-        const long long tr_t0 = clock64();
-        struct Pix { bool live; int n, y, x; size_t opix; };
-        auto locate = [&](int m) {
-            Pix q{false, 0, 0, 0, 0};
+        const bool tr = a.trace != nullptr && blockIdx.x == 0;
+        uint32_t tr_w = 0;
+        const uint32_t tr_t0 = (uint32_t)clock64();
+        int b = grp;
+        uint32_t bph = 0;
+        for (int m = mfirst + grp * mstep; m < mtiles && ok; m += NG * mstep, b += NG) {
+            if (b >= NACC) { b -= NACC; bph ^= 1u; }
             const int p = m * 128 + row;
+            bool live = false;
+            int n = 0, y = 0, x = 0;
             if (p < NV) {
                 const int vy = fastdiv(p, a.pw_mul, a.pw_sh);
-                q.x = p - vy * a.PW;
-                q.n = fastdiv(vy, a.vh_mul, a.vh_sh);
-                q.y = vy - q.n * a.VH;
-                q.live = q.x < a.OWg && q.y < a.OHg;
+                x = p - vy * a.PW;
+                n = fastdiv(vy, a.vh_mul, a.vh_sh);
+                y = vy - n * a.VH;
+                live = x < a.OWg && y < a.OHg;
             }
-            q.opix = ((size_t)q.n * a.OHg + q.y) * a.OWg + q.x;
-            return q;
-        };
-        // ---- staged residual rows (RSTAGE; the host enables it only for int16 tensors, an n-tile
-        //      that lies entirely inside or outside the injected channels, NT of 64 or 128) --------
-        constexpr uint32_t ROWB = NT * 2;                  // bytes of one pixel's residual segment
-        constexpr int NCOPY = (32 * ROWB) / (128 * 16);    // 16-byte pieces per thread and tile (group: 32 rows, 128 threads)
-        const int gtid = cg * 32 + lane;                   // this thread's index in its group
-        const int grow0 = quad * 32;                       // the group's first row of a tile
-        const bool st_in = RSTAGE && a.res_in && obase < lim;
-        const bool st_out = RSTAGE && a.res_out;
-        // output pixels in front of raster position p (live pixels are consecutive tensor rows)
-        auto live_before = [&](int p) -> long long {
-            if (p >= NV) return (long long)a.B * a.OHg * a.OWg;
-            const int vy = fastdiv(p, a.pw_mul, a.pw_sh), x = p - vy * a.PW;
-            const int n = fastdiv(vy, a.vh_mul, a.vh_sh), y = vy - n * a.VH;
-            return ((long long)n * a.OHg + min(y, a.OHg)) * a.OWg + (y < a.OHg ? min(x, a.OWg) : 0);
-        };
-        // shared-memory address of 16-byte chunk `c` of staged row `r`: chunks XOR-swizzled by row
-        auto st_addr = [&](int buf, int r, int c) -> uint32_t {
-            return smem_u32(sRes) + (uint32_t)(quad * 2 + buf) * (32u * ROWB) + (uint32_t)r * ROWB +
-                   (uint32_t)(((c & ~7) | ((c ^ r) & 7)) << 4);
-        };
-        // bytes of a pixel's incoming segment: the whole n-tile, or the part of it that receives a
-        // residual (a producer with fewer channels, e.g. 64 of this layer's 128); a multiple of 16
-        const uint32_t rowb_in = st_in ? (uint32_t)min(NT, lim - obase) * 2u : ROWB;
-        auto issue_in = [&](long long p0, int nl, int buf) {   // cp.async of a tile's incoming rows
-            if (!st_in) return;
-            const char* g = reinterpret_cast<const char*>(a.res_in) + ((size_t)p0 * a.res_in_ch + obase) * 2;
+            // pixel index of this lane's row (-1: not an output) and of the quad's rows; the same in
+            // the residual's grid
+            const int opix = live ? (n * a.OHg + y) * a.OWg + x : -1;
+            const uint32_t ipix = a.residual_pool ? (uint32_t)((n * 2 * a.OHg + 2 * y) * 2) * a.OWg + 2 * x : (uint32_t)opix;
+            auto orow = [&](int i) { return __shfl_sync(0xffffffffu, opix, (lane & ~3) | i); };
+            auto irow = [&](int i) { return __shfl_sync(0xffffffffu, ipix, (lane & ~3) | i); };
+            uint32_t r[AHEAD][RREG];
+            // residual of unit u (rows 2(u&1), 2(u&1)+1 of the quad's four, pass u/2) into q
+            auto fetch = [&](int u, uint32_t (&q)[RREG]) {
 #pragma unroll
-            for (int k = 0; k < NCOPY; k++) {
-                // the same thread -> (row, chunk) map as store_out: a thread refills exactly the
-                // bytes it has just drained, whatever the width of the incoming rows
-                const uint32_t off = (uint32_t)(gtid + k * 128) * 16u;
-                const int r = off / ROWB, c = (off % ROWB) >> 4;
-                if (r < nl && (uint32_t)(c << 4) < rowb_in)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st_addr(buf, r, c)),
-                                 "l"(g + (size_t)r * a.res_in_ch * 2 + (c << 4)) : "memory");
-            }
-        };
-        auto store_out = [&](long long p0, int nl, int buf) {  // a tile's outgoing rows, whole lines
-            if (!st_out) return;
-            char* g = reinterpret_cast<char*>(a.res_out) + ((size_t)p0 * a.O + obase) * 2;
+                for (int i = 0; i < 2; i++) {
+                    const bool rlive = orow(2 * (u & 1) + i) >= 0;
+                    const uint32_t rpix = irow(2 * (u & 1) + i);
 #pragma unroll
-            for (int k = 0; k < NCOPY; k++) {
-                const uint32_t off = (uint32_t)(gtid + k * 128) * 16u;
-                const int r = off / ROWB, c = (off % ROWB) >> 4;
-                if (r < nl) {
-                    uint4 v4;
-                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v4.x), "=r"(v4.y), "=r"(v4.z), "=r"(v4.w)
-                                 : "r"(st_addr(buf, r, c)) : "memory");
-                    *reinterpret_cast<uint4*>(g + (size_t)r * a.O * 2 + (c << 4)) = v4;
-                }
-            }
-        };
-        uint32_t eph = 0;                                  // phase of the epilogue rendezvous
-        auto rendezvous = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(BAR_EPI(quad));
-            const bool r = wait(BAR_EPI(quad), eph);
-            eph ^= 1;
-            return r;
-        };
-        // int16 residual of channels [o0, o0+COLS) of one pixel, packed (zeros where nothing is
-        // injected); 2x2 max for pooled residuals (kernel.cuh:773-783)
-        auto fetch16 = [&](uint4 (&r)[NQ], const Pix& q) {
-            const short* base = reinterpret_cast<const short*>(a.res_in);
-            const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-            if (a.res_in_chunked) {
-                // [channel chunk][pixel][8 channels]: consecutive lanes (pixels) read consecutive
-                // 16 bytes, so a warp's load touches four whole lines instead of 32 pieces of lines
-                const uint4* cb = reinterpret_cast<const uint4*>(a.res_in) + (size_t)(o0 >> 3) * a.res_in_npix;
-                if (a.residual_pool) {
-                    const size_t i00 = ((size_t)q.n * 2 * a.OHg + 2 * q.y) * 2 * a.OWg + 2 * q.x, rw = (size_t)2 * a.OWg;
-#pragma unroll
-                    for (int j = 0; j < NQ; j++) {
-                        r[j] = z;
-                        if (q.live && o0 + 8 * j < lim) {
-                            const uint4* p = cb + (size_t)j * a.res_in_npix + i00;
-                            const uint4 w0 = __ldg(p), w1 = __ldg(p + 1), w2 = __ldg(p + rw), w3 = __ldg(p + rw + 1);
-                            r[j].x = __vmaxs2(__vmaxs2(w0.x, w1.x), __vmaxs2(w2.x, w3.x));
-                            r[j].y = __vmaxs2(__vmaxs2(w0.y, w1.y), __vmaxs2(w2.y, w3.y));
-                            r[j].z = __vmaxs2(__vmaxs2(w0.z, w1.z), __vmaxs2(w2.z, w3.z));
-                            r[j].w = __vmaxs2(__vmaxs2(w0.w, w1.w), __vmaxs2(w2.w, w3.w));
+                    for (int g = 0; g < 2; g++) {
+                        const int o = o0 + 32 * HSTEP * (u >> 1) + 16 * g + 4 * q4;
+                        const bool on = rlive && o < lim;
+                        if constexpr (RB == 4) {
+                            int4 w = make_int4(0, 0, 0, 0);
+                            if (on) {
+                                const int* src = reinterpret_cast<const int*>(a.res_in) + (size_t)rpix * in_ps + in_off(o);
+                                if (a.residual_pool) {
+                                    const size_t dn = (size_t)2 * a.OWg * in_ps;
+                                    w = max4(max4(ld_res4(src, 4, 0), ld_res4(src, 4, in_ps)), max4(ld_res4(src, 4, dn), ld_res4(src, 4, dn + in_ps)));
+                                } else {
+                                    w = ld_res4(src, 4, 0);
+                                }
+                            }
+                            q[i * 8 + g * 4] = w.x; q[i * 8 + g * 4 + 1] = w.y; q[i * 8 + g * 4 + 2] = w.z; q[i * 8 + g * 4 + 3] = w.w;
+                        } else {
+                            uint2 w = make_uint2(0u, 0u);
+                            if (on) {
+                                const short* src = reinterpret_cast<const short*>(a.res_in) + (size_t)rpix * in_ps + in_off(o);
+                                auto ld = [&](size_t off) { return __ldg(reinterpret_cast<const uint2*>(src + off)); };
+                                w = ld(0);
+                                if (a.residual_pool) {     // 2x2 max (kernel.cuh:773-783)
+                                    const size_t dn = (size_t)2 * a.OWg * in_ps;
+                                    const uint2 w1 = ld(in_ps), w2 = ld(dn), w3 = ld(dn + in_ps);
+                                    w.x = __vmaxs2(__vmaxs2(w.x, w1.x), __vmaxs2(w2.x, w3.x));
+                                    w.y = __vmaxs2(__vmaxs2(w.y, w1.y), __vmaxs2(w2.y, w3.y));
+                                }
+                            }
+                            q[i * 4 + g * 2] = w.x; q[i * 4 + g * 2 + 1] = w.y;
                         }
                     }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < NQ; j++)
-                        r[j] = (q.live && o0 + 8 * j < lim) ? __ldg(cb + (size_t)j * a.res_in_npix + q.opix) : z;
                 }
-            } else if (a.residual_pool) {
-                const size_t b00 = (((size_t)q.n * 2 * a.OHg + 2 * q.y) * 2 * a.OWg + 2 * q.x) * a.res_in_ch + o0;
-                const size_t rowp = (size_t)2 * a.OWg * a.res_in_ch;
+            };
+            const bool has_in = o0 < lim;
+            if (has_in) {                                  // flies while the accumulator is awaited
 #pragma unroll
-                for (int h = 0; h < NQ; h += 2) {              // 8 loads in flight at a time
-                    uint4 w[4][2];
-#pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        const bool on = h + j < NQ && q.live && o0 + 8 * (h + j) < lim;
-                        const short* s = base + b00 + 8 * (h + j);
-                        w[0][j] = on ? __ldg(reinterpret_cast<const uint4*>(s)) : z;
-                        w[1][j] = on ? __ldg(reinterpret_cast<const uint4*>(s + a.res_in_ch)) : z;
-                        w[2][j] = on ? __ldg(reinterpret_cast<const uint4*>(s + rowp)) : z;
-                        w[3][j] = on ? __ldg(reinterpret_cast<const uint4*>(s + rowp + a.res_in_ch)) : z;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 2; j++) {
-                        if (h + j >= NQ) continue;
-                        r[h + j].x = __vmaxs2(__vmaxs2(w[0][j].x, w[1][j].x), __vmaxs2(w[2][j].x, w[3][j].x));
-                        r[h + j].y = __vmaxs2(__vmaxs2(w[0][j].y, w[1][j].y), __vmaxs2(w[2][j].y, w[3][j].y));
-                        r[h + j].z = __vmaxs2(__vmaxs2(w[0][j].z, w[1][j].z), __vmaxs2(w[2][j].z, w[3][j].z));
-                        r[h + j].w = __vmaxs2(__vmaxs2(w[0][j].w, w[1][j].w), __vmaxs2(w[2][j].w, w[3][j].w));
-                    }
-                }
-            } else {
-                const short* s = base + q.opix * a.res_in_ch + o0;
-#pragma unroll
-                for (int j = 0; j < NQ; j++)
-                    r[j] = (q.live && o0 + 8 * j < lim) ? __ldg(reinterpret_cast<const uint4*>(s + 8 * j)) : z;
+                for (int i = 0; i < AHEAD; i++)
+                    if (i < NU) fetch(i, r[i]);
             }
-        };
-        auto add16 = [&](int (&v)[COLS], const uint4 (&r)[NQ]) {
-#pragma unroll
-            for (int j = 0; j < NQ; j++) {
-                v[8 * j] += (int)(short)(r[j].x & 0xFFFFu);
-                v[8 * j + 1] += (int)(short)(r[j].x >> 16);
-                v[8 * j + 2] += (int)(short)(r[j].y & 0xFFFFu);
-                v[8 * j + 3] += (int)(short)(r[j].y >> 16);
-                v[8 * j + 4] += (int)(short)(r[j].z & 0xFFFFu);
-                v[8 * j + 5] += (int)(short)(r[j].z >> 16);
-                v[8 * j + 6] += (int)(short)(r[j].w & 0xFFFFu);
-                v[8 * j + 7] += (int)(short)(r[j].w >> 16);
-            }
-        };
-        // packed output bits (and the next layer's planes) of this thread's channels of one pixel
-        auto store_bits = [&](const Pix& q, uint32_t word) {
-            // bits of channel o live at bit 31 - o%32 of word o/32 (little-endian bytes)
-            unsigned char* wp = reinterpret_cast<unsigned char*>(
-                a.out + (size_t)q.n * a.out_image_stride + ((size_t)q.y * a.OWg + q.x) * Ow + (o0 >> 5));
-            if (COLS == 32) *reinterpret_cast<uint32_t*>(wp) = word;
-            else if (COLS == 16) *reinterpret_cast<unsigned short*>(wp + ((o0 & 16) ? 0 : 2)) = (unsigned short)word;
-            else wp[3 - ((o0 & 31) >> 3)] = (unsigned char)word;
-            if (a.nxt) store_next_planes(a, q.n, q.y, q.x, o0, word, COLS);
-        };
-        constexpr bool plain = EPI == kEpiPlain;
-        uint4 rnext[NQ];
-#pragma unroll
-        for (int j = 0; j < NQ; j++) rnext[j] = make_uint4(0u, 0u, 0u, 0u);
-        Pix cur = locate(mfirst);
-        if (res16 && mfirst < mtiles) fetch16(rnext, cur);
-        // first pixel and number of live pixels of the group's rows of the current, previous and next tile
-        long long p0_cur = 0, p0_prev = 0, p0_next = 0;
-        int nl_cur = 0, nl_prev = -1, nl_next = 0;
-        if (RSTAGE && mfirst < mtiles) {
-            p0_cur = live_before(mfirst * 128 + grow0);
-            nl_cur = (int)(live_before(mfirst * 128 + grow0 + 32) - p0_cur);
-            issue_in(p0_cur, nl_cur, 0);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        }
-        int b = 0, mprev = -1;
-        uint32_t bph = 0;
-        for (int m = mfirst; m < mtiles && ok; m += mstep, tc++) {
-            const Pix q = cur;
-            uint4 rcur[NQ];
-#pragma unroll
-            for (int j = 0; j < NQ; j++) rcur[j] = rnext[j];
-            if (m + mstep < mtiles) {                      // next tile's row: its residual flies during this tile
-                cur = locate(m + mstep);
-                if (res16) fetch16(rnext, cur);
-            }
-            ok = wait.timed(BAR_CFULL(b), bph, tr_w);
+            ok = tr ? wait.relaxed_timed(BAR_CFULL(b), bph, tr_w) : wait.relaxed(BAR_CFULL(b), bph);
             if (!ok) break;
             tc_fence_after();
-            int v[COLS];
-            tmem_ld_cols<COLS>(tmem + ((uint32_t)(quad * 32) << 16) + b * NT + cg * COLS, v);
-            tmem_ld_wait();
-            tc_fence_before();                             // this warp is done with the accumulator
-            __syncwarp();
-            if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
-            if (++b == NACC) { b = 0; bph ^= 1; }
-            if (plain) {
-                // no residual and no integer output: the reference's comparison as it stands,
-                // !((float)value < threshold) (kernel.cuh:795-796), on the fp32 accumulator
-                uint32_t word = 0;
-                const float4* tf4 = reinterpret_cast<const float4*>(sThrF + cg * COLS);
-#pragma unroll
-                for (int j = 0; j < COLS / 4; j++) {
-                    const float4 th = tf4[j];
-                    if (!(__int_as_float(v[4 * j]) < th.x)) word |= (1u << (COLS - 1)) >> (4 * j);
-                    if (!(__int_as_float(v[4 * j + 1]) < th.y)) word |= (1u << (COLS - 1)) >> (4 * j + 1);
-                    if (!(__int_as_float(v[4 * j + 2]) < th.z)) word |= (1u << (COLS - 1)) >> (4 * j + 2);
-                    if (!(__int_as_float(v[4 * j + 3]) < th.w)) word |= (1u << (COLS - 1)) >> (4 * j + 3);
+            uint32_t w0 = 0, w1 = 0;                       // this lane's channels' bits of rows 0 and 1 of a pass
+#pragma unroll 1
+            for (int u = 0; u < NU; u++) {
+                const int k = u >> 1, h = u & 1;
+                const int cb = HSTEP * k + half;           // 32-column block of the accumulator
+                const int o = o0 + 32 * HSTEP * k + 4 * q4;
+                int v[16];
+                tmem_ld_16x256b_x4(tmem + ((uint32_t)(quad * 32 + 16 * h) << 16) + b * NT + cb * 32, v);
+                tmem_ld_wait();
+                if (u == NU - 1) {
+                    tc_fence_before();                     // this warp is done with the accumulator
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
                 }
-                if (q.live) store_bits(q, word);
-                mprev = m;
-                continue;
-            }
+                // values of row i of this unit, channel run g: four consecutive channels
+                int4 c[2][2];
+                const int op[2] = {orow(2 * h), orow(2 * h + 1)};
 #pragma unroll
-            for (int j = 0; j < COLS; j++) v[j] = f4_acc_to_int(v[j]);     // fp32 accumulators, exact integers
-            if (q.live && a.acc_out) {
-                int4* dst = reinterpret_cast<int4*>(a.acc_out + q.opix * a.O + o0);
+                for (int i = 0; i < 2; i++)
 #pragma unroll
-                for (int j = 0; j < COLS / 4; j++)
-                    dst[j] = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            }
-            const int sbuf = (int)(tc & 1);
-            int lrow = 0;
-            if (RSTAGE) {
-                // this tile's incoming rows have landed (mine: wait_group; everyone's: rendezvous),
-                // and every thread has written its part of the previous tile's outgoing rows
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-                ok = rendezvous();
-                if (!ok) break;
-                if (nl_prev >= 0) store_out(p0_prev, nl_prev, sbuf ^ 1);
-                if (m + mstep < mtiles) {
-                    p0_next = live_before((m + mstep) * 128 + grow0);
-                    nl_next = (int)(live_before((m + mstep) * 128 + grow0 + 32) - p0_next);
-                    issue_in(p0_next, nl_next, sbuf ^ 1);  // the buffer this thread has just drained
-                }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                lrow = (int)((long long)q.opix - p0_cur);
-                if (st_in && q.live && o0 < lim) {
-                    uint4 r[NQ];
-#pragma unroll
-                    for (int j = 0; j < NQ; j++) {
-                        r[j] = make_uint4(0u, 0u, 0u, 0u);
-                        if (o0 + 8 * j < lim)
-                            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r[j].x), "=r"(r[j].y), "=r"(r[j].z), "=r"(r[j].w)
-                                         : "r"(st_addr(sbuf, lrow, cg * NQ + j)) : "memory");
-                    }
-                    add16(v, r);
-                }
-            } else if (res16) {
-                add16(v, rcur);
-            } else if (a.res_in && q.live && o0 < lim) {
-#pragma unroll
-                for (int j = 0; j < COLS / 4; j++) {
-                    const int o = o0 + 4 * j;
-                    if (o >= lim) continue;
-                    int4 r;
-                    if (a.residual_pool) {
-                        const size_t b00 = (((size_t)q.n * 2 * a.OHg + 2 * q.y) * 2 * a.OWg + 2 * q.x) * a.res_in_ch + o;
-                        const size_t rowp = (size_t)2 * a.OWg * a.res_in_ch;
-                        r = max4(max4(ld_res4(a.res_in, a.res_in_bytes, b00),
-                                      ld_res4(a.res_in, a.res_in_bytes, b00 + a.res_in_ch)),
-                                 max4(ld_res4(a.res_in, a.res_in_bytes, b00 + rowp),
-                                      ld_res4(a.res_in, a.res_in_bytes, b00 + rowp + a.res_in_ch)));
-                    } else {
-                        r = ld_res4(a.res_in, a.res_in_bytes, q.opix * a.res_in_ch + o);
-                    }
-                    v[4 * j] += r.x; v[4 * j + 1] += r.y; v[4 * j + 2] += r.z; v[4 * j + 3] += r.w;
-                }
-            }
-            uint32_t word = 0;                             // channel c of this thread at bit COLS-1-c
-            const int4* th4 = reinterpret_cast<const int4*>(sThr + cg * COLS);
-#pragma unroll
-            for (int j = 0; j < COLS / 4; j++) {
-                const int4 th = th4[j];
-                if (v[4 * j] >= th.x) word |= (1u << (COLS - 1)) >> (4 * j);
-                if (v[4 * j + 1] >= th.y) word |= (1u << (COLS - 1)) >> (4 * j + 1);
-                if (v[4 * j + 2] >= th.z) word |= (1u << (COLS - 1)) >> (4 * j + 2);
-                if (v[4 * j + 3] >= th.w) word |= (1u << (COLS - 1)) >> (4 * j + 3);
-            }
-            if (a.res_out && q.live) {
-                const size_t idx = q.opix * a.O + o0;
-                if (a.res_out_bytes == 2) {
-                    uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<short*>(a.res_out) + idx);
-                    if (!a.res_out_proven) {               // a real branch: two instructions per value
-                        uint32_t ovf = 0;                  // |v| of every value ORed together
-#pragma unroll
-                        for (int j = 0; j < COLS; j++) ovf |= (uint32_t)(v[j] ^ (v[j] >> 31));
-                        overflow |= ovf > 32767u;          // some value outside [-32768, 32767]
-                    }
-#pragma unroll
-                    for (int j = 0; j < NQ; j++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int kk = 0; kk < 4; kk++) {
-                            const int lo = v[8 * j + 2 * kk], hi = v[8 * j + 2 * kk + 1];
-                            w[kk] = ((uint32_t)lo & 0xFFFFu) | ((uint32_t)hi << 16);
+                    for (int g = 0; g < 2; g++) {
+                        c[i][g] = make_int4(f4_acc_to_int(v[8 * g + 2 * i]), f4_acc_to_int(v[8 * g + 2 * i + 1]),
+                                            f4_acc_to_int(v[8 * g + 4 + 2 * i]), f4_acc_to_int(v[8 * g + 4 + 2 * i + 1]));
+                        if (a.acc_out && op[i] >= 0)
+                            *reinterpret_cast<int4*>(a.acc_out + (size_t)op[i] * a.O + o + 16 * g) = c[i][g];
+                        if (has_in) {
+                            const uint32_t* q = r[0] + (i * 2 + g) * RB;
+                            if constexpr (RB == 4) {
+                                c[i][g].x += (int)q[0]; c[i][g].y += (int)q[1]; c[i][g].z += (int)q[2]; c[i][g].w += (int)q[3];
+                            } else {
+                                c[i][g].x += (int)(short)(q[0] & 0xFFFFu); c[i][g].y += (int)q[0] >> 16;
+                                c[i][g].z += (int)(short)(q[1] & 0xFFFFu); c[i][g].w += (int)q[1] >> 16;
+                            }
                         }
-                        if (RSTAGE)                        // into the staged row, in place of what was read
-                            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(st_addr(sbuf, lrow, cg * NQ + j)),
-                                         "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
-                        else if (a.res_out_chunked)
-                            reinterpret_cast<uint4*>(a.res_out)[(size_t)((o0 >> 3) + j) * a.res_out_npix + q.opix] =
-                                make_uint4(w[0], w[1], w[2], w[3]);
-                        else
-                            dst[j] = make_uint4(w[0], w[1], w[2], w[3]);
                     }
-                } else {
-                    int4* dst = reinterpret_cast<int4*>(reinterpret_cast<int*>(a.res_out) + idx);
+                if (has_in) {                              // a later unit's residual flies during what follows
+                    if constexpr (AHEAD == 2) {
 #pragma unroll
-                    for (int j = 0; j < COLS / 4; j++)
-                        dst[j] = make_int4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                        for (int j = 0; j < RREG; j++) r[0][j] = r[AHEAD - 1][j];
+                    }
+                    if (u + AHEAD < NU) fetch(u + AHEAD, r[AHEAD - 1]);
+                }
+                uint32_t w[2] = {0u, 0u};
+#pragma unroll
+                for (int g = 0; g < 2; g++) {
+                    const int2 ta = *reinterpret_cast<const int2*>(sThr + cb * 32 + 16 * g + 2 * q4);
+                    const int2 tb = *reinterpret_cast<const int2*>(sThr + cb * 32 + 16 * g + 8 + 2 * q4);
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        uint32_t nib = c[i][g].x >= ta.x ? 8u : 0u;
+                        if (c[i][g].y >= ta.y) nib |= 4u;
+                        if (c[i][g].z >= tb.x) nib |= 2u;
+                        if (c[i][g].w >= tb.y) nib |= 1u;
+                        w[i] |= nib << (28 - 16 * g - 4 * q4);
+                    }
+                }
+                if (a.res_out) {
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        if (op[i] < 0) continue;
+#pragma unroll
+                        for (int g = 0; g < 2; g++) {
+                            const size_t idx = (size_t)op[i] * out_ps + out_off(o + 16 * g);
+                            if (a.res_out_bytes == 2) {
+                                if (!a.res_out_proven) {
+                                    const uint32_t ovf = (uint32_t)(c[i][g].x ^ (c[i][g].x >> 31)) | (uint32_t)(c[i][g].y ^ (c[i][g].y >> 31)) |
+                                                         (uint32_t)(c[i][g].z ^ (c[i][g].z >> 31)) | (uint32_t)(c[i][g].w ^ (c[i][g].w >> 31));
+                                    overflow |= ovf > 32767u;              // some value outside [-32768, 32767]
+                                }
+                                *reinterpret_cast<uint2*>(reinterpret_cast<short*>(a.res_out) + idx) =
+                                    make_uint2(__byte_perm((uint32_t)c[i][g].x, (uint32_t)c[i][g].y, 0x5410),
+                                               __byte_perm((uint32_t)c[i][g].z, (uint32_t)c[i][g].w, 0x5410));
+                            } else {
+                                *reinterpret_cast<int4*>(reinterpret_cast<int*>(a.res_out) + idx) = c[i][g];
+                            }
+                        }
+                    }
+                }
+                if (h == 0) {
+                    w0 = w[0]; w1 = w[1];
+                    continue;
+                }
+                // every lane of a quad has its channels' bits of all four rows: lane i collects row i
+                const bool up = (q4 & 2) != 0, odd = (q4 & 1) != 0;
+                uint32_t k0 = up ? w[0] : w0, k1 = up ? w[1] : w1;
+                k0 |= __shfl_xor_sync(0xffffffffu, up ? w0 : w[0], 2);
+                k1 |= __shfl_xor_sync(0xffffffffu, up ? w1 : w[1], 2);
+                uint32_t word = odd ? k1 : k0;
+                word |= __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 1);
+                if (live) {
+                    a.out[(size_t)n * a.out_image_stride + ((size_t)y * a.OWg + x) * Ow + ((o0 + 32 * HSTEP * k) >> 5)] = word;
+                    if (a.nxt) store_next_planes(a, n, y, x, o0 + 32 * HSTEP * k, word);
                 }
             }
-            if (q.live) store_bits(q, word);
-            mprev = m;
-            p0_prev = p0_cur; nl_prev = nl_cur;
-            p0_cur = p0_next; nl_cur = nl_next;
-        }
-        if (RSTAGE) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");      // nothing of this thread's in flight at exit
-            if (ok && mprev >= 0 && rendezvous()) store_out(p0_prev, nl_prev, (int)((tc - 1) & 1));
         }
         if (overflow) atomicExch(a.err_flag, 2);
-        if (a.trace && blockIdx.x == 0 && tid == 0) { a.trace[6] = clock64() - tr_t0; a.trace[7] = tr_w; a.trace[8] = tc; }
+        if (tr && tid == 0) {
+            a.trace[6] = (uint32_t)clock64() - tr_t0;
+            a.trace[7] = tr_w;
+            a.trace[8] = mfirst < mtiles ? (mtiles - mfirst + NG * mstep - 1) / (NG * mstep) : 0;
+        }
     }
     tc_fence_before();
     __syncthreads();

@@ -55,7 +55,7 @@ struct ConvWsArgs {
     int nxt_nplane;           // 1, or 4 when that layer has stride 2 (one plane per row / column parity)
     const void* res_in; int res_in_bytes, res_in_ch, residual_channels, residual_pool;
     // int16 residual tensors may be laid out by 8-channel chunk, [ch/8][pixels][8], instead of NHWC
-    // (bconv_umma_pre.cuh, direct epilogue only): npix = pixels of the whole tensor
+    // (bconv_umma_pre.cuh only): npix = pixels of the whole tensor
     int res_in_chunked, res_out_chunked; long long res_in_npix, res_out_npix;
     uint32_t* out; long long out_image_stride;
     void* res_out; int res_out_bytes; int32_t* acc_out;
@@ -122,30 +122,22 @@ __device__ __forceinline__ void prepare_filter_f4(const uint32_t* fbits, int O, 
         const int tap = (int)(r % RS); r /= RS;
         const int cb = (int)(r % ncb);
         const int tile = (int)(r / ncb);
-        const int o = tile * nt + n;
+        const int o = tile * nt + (n & ~31) + f4_channel_of_column(n & 31);
         out[i] = expand32_f4(fbits[((size_t)o * RS + tap) * Cw + cb * 2 + c2]);
     }
 }
 
-// Writes the +-1 nibbles of `nbits` output channels (8, 16 or 32; first channel o0, a multiple of
-// nbits; channel c at bit nbits-1-c of `word`) of output pixel (n, y, x) into the next layer's
-// planes: one 16-byte slot per raster position and 32-channel chunk (expand32_f4 order).
-__device__ __forceinline__ void store_next_planes(const ConvWsArgs& a, int n, int y, int x, int o0,
-                                                  uint32_t word, int nbits) {
+// Writes the +-1 nibbles of 32 output channels (o0, a multiple of 32, .. o0 + 31; channel c at bit
+// 31 - c of `word`) of output pixel (n, y, x) into the next layer's planes: one 16-byte slot per
+// raster position and 32-channel chunk.
+__device__ __forceinline__ void store_next_planes(const ConvWsArgs& a, int n, int y, int x, int o0, uint32_t word) {
     int pl = 0;
     if (a.nxt_nplane == 4) {                    // stride-2 consumer: pixel (y, x) lives in plane (y&1, x&1) at (y/2, x/2)
         pl = (y & 1) * 2 + (x & 1);
         y >>= 1; x >>= 1;
     }
-    uint4* base = a.nxt + ((size_t)(o0 >> 5) * a.nxt_nplane + pl) * a.nxt_positions + a.nxt_front +
-                  ((long long)n * a.nxt_VH + y) * a.nxt_PW + x;
-    if (nbits == 32) {
-        base[0] = expand32_f4(word);
-    } else if (nbits == 16) {                   // half a chunk: channels 0-15 are its first 8 bytes
-        reinterpret_cast<uint2*>(base)[(o0 >> 4) & 1] = make_uint2(expand8_f4(word >> 8), expand8_f4(word));
-    } else {                                    // 8 channels: one 32-bit word of the slot
-        reinterpret_cast<uint32_t*>(base)[(o0 >> 3) & 3] = expand8_f4(word);
-    }
+    a.nxt[((size_t)(o0 >> 5) * a.nxt_nplane + pl) * a.nxt_positions + a.nxt_front +
+          ((long long)n * a.nxt_VH + y) * a.nxt_PW + x] = expand32_f4(word);
 }
 
 struct WsWait {
@@ -179,7 +171,14 @@ struct WsWait {
         atomicExch(err, 1);
         return false;
     }
-    // same, adding the cycles spent waiting to `acc` (tracing)
+    // relaxed, adding the cycles spent waiting to `acc` (tracing)
+    __device__ __forceinline__ bool relaxed_timed(uint32_t bar, uint32_t parity, uint32_t& acc) const {
+        const uint32_t t0 = (uint32_t)clock64();
+        const bool ok = relaxed(bar, parity);
+        acc += (uint32_t)clock64() - t0;
+        return ok;
+    }
+    // the plain wait with the same
     __device__ __forceinline__ bool timed(uint32_t bar, uint32_t parity, long long& acc) const {
         const long long t0 = clock64();
         const bool ok = (*this)(bar, parity);
@@ -628,7 +627,7 @@ __device__ void conv_umma_ws_cta(const ConvWsArgs& a, unsigned char* smem) {
                 if (a.nxt) {
 #pragma unroll
                     for (int k = 0; k < NB_PER; k++)
-                        store_next_planes(a, n, y, x, obase + (grp + k * EPI_GROUPS) * 32, words[k], 32);
+                        store_next_planes(a, n, y, x, obase + (grp + k * EPI_GROUPS) * 32, words[k]);
                 }
             }
             tr_body += clock64() - e0;

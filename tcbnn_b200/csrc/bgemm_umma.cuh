@@ -52,13 +52,10 @@ struct GemmUmmaArgs {
     long long* trace;          // null, or 16 counters: CTA 0 writes [9..15] (clocks; see the C header)
 };
 
-// bit i of b set -> nibble i of the result = 0xF (the nibble order of expand8_f4)
-__device__ __forceinline__ uint32_t nibble_mask8(uint32_t b) {
-    uint32_t x = b & 0xFFu;
-    x = (x | (x << 12)) & 0x000F000Fu;
-    x = (x | (x << 6)) & 0x03030303u;
-    x = (x | (x << 3)) & 0x11111111u;
-    return x * 0xFu;
+// zeroes the nibbles of the bits that are clear in m (nibble order of expand32_f4)
+__device__ __forceinline__ uint4 keep32_f4(uint4 e, uint32_t m) {
+    return make_uint4(e.x & (((m >> 3) & 0x11111111u) * 0xFu), e.y & (((m >> 2) & 0x11111111u) * 0xFu),
+                      e.z & (((m >> 1) & 0x11111111u) * 0xFu), e.w & ((m & 0x11111111u) * 0xFu));
 }
 
 // packed bits [rows][ld words] (bit k of a row at bit 31 - k%32 of word k/32) -> units; one launch
@@ -101,11 +98,7 @@ __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_r
             if (r < rows && k0 < K) {
                 e = expand32_f4(w[j]);
                 const int valid = K - k0;                                // elements of this chunk that exist
-                if (valid < 32) {                                        // the rest is padding: 0, not -1
-                    const uint32_t m = 0xFFFFFFFFu << (32 - valid);
-                    e.x &= nibble_mask8(m >> 24); e.y &= nibble_mask8(m >> 16);
-                    e.z &= nibble_mask8(m >> 8);  e.w &= nibble_mask8(m);
-                }
+                if (valid < 32) e = keep32_f4(e, 0xFFFFFFFFu << (32 - valid));   // the rest is padding: 0, not -1
             }
             out[(size_t)kb * 256 + (c & 1) * 128 + row] = e;
         }

@@ -85,11 +85,9 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
          "  uint4* nxt; long long nxt_positions, nxt_front; int nxt_PW, nxt_VH; int res_out_chunked; };\n"
          // 32 packed bits -> 32 nibbles of +1 / -1 (e2m1), the order the conv kernels' filters use
          // (expand32_f4 in bconv_umma.cuh)
-         "__device__ __forceinline__ uint32_t expand8_f4(uint32_t b) {\n"
-         "  uint32_t x = b & 0xFFu; x = (x | (x << 12)) & 0x000F000Fu; x = (x | (x << 6)) & 0x03030303u;\n"
-         "  x = (x | (x << 3)) & 0x11111111u; return 0xAAAAAAAAu ^ (x << 3); }\n"
          "__device__ __forceinline__ uint4 expand32_f4(uint32_t w) {\n"
-         "  return make_uint4(expand8_f4(w >> 24), expand8_f4(w >> 16), expand8_f4(w >> 8), expand8_f4(w)); }\n";
+         "  return make_uint4((w & 0x88888888u) ^ 0xAAAAAAAAu, ((w << 1) & 0x88888888u) ^ 0xAAAAAAAAu,\n"
+         "                    ((w << 2) & 0x88888888u) ^ 0xAAAAAAAAu, ((w << 3) & 0x88888888u) ^ 0xAAAAAAAAu); }\n";
     for (int half = 0; half < nhalf; half++) {
     const int OB = 64 * half, O = Oall - OB < 64 ? Oall - OB : 64;
     // VEC (stride 4 only, image rows a multiple of 4 pixels, aligned base): a thread's taps of one

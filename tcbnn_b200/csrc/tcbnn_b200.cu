@@ -442,8 +442,6 @@ PreparedLayout prepared_layout(const tcbnn_conv_desc* d) {
             }
         }
     }
-    // the loader-fed kernel pre-pools an injected residual too (scratch behind its planes)
-    if (L.pre_nt && d->pool == 1) L.pool_bytes = (size_t)d->B * d->OH * d->OW * d->O * 2;
     L.prepool_bytes = 0;
     if (d->pool != 1 && (L.umma_nt || L.as_npos || L.pre_nt))
         L.prepool_bytes = ((size_t)d->B * OHu * OWu * ((d->O + 31) / 32) * 4 + 255) & ~(size_t)255;
@@ -451,12 +449,10 @@ PreparedLayout prepared_layout(const tcbnn_conv_desc* d) {
     return L;
 }
 
-// Scratch in front of a pooled layer's pre-pool bits: the input planes of the loader-fed kernel
-// followed by its pooled-residual scratch, or the activation-stationary kernel's pooled residual.
-size_t planes_padded(const PreparedLayout& L) { return (L.pre_bytes + 255) & ~(size_t)255; }
+// Scratch in front of a pooled layer's pre-pool bits: the input planes of the loader-fed kernel, or the
+// activation-stationary kernel's pooled residual.
 size_t main_ws_bytes(const PreparedLayout& L) {
-    if (L.pre_bytes) return planes_padded(L) + ((L.pool_bytes + 255) & ~(size_t)255);
-    return (L.pool_bytes + 255) & ~(size_t)255;
+    return ((L.pre_bytes ? L.pre_bytes : L.pool_bytes) + 255) & ~(size_t)255;
 }
 
 template <int PPT>
@@ -483,18 +479,9 @@ int launch_inconv_tiled(const InConvArgs& c, size_t smem, int sms, cudaStream_t 
 }
 
 int g_conv_two_ctas = 1;  // loader-fed kernel, n-tile 64: two CTAs of eight epilogue warps per SM when they fit
-int g_conv_res_stage = 1; // loader-fed kernel: stage int16 residual rows in shared memory when possible
-int g_conv_tile = 1;      // loader-fed kernel: the tile-per-group epilogues where the tensors allow them
 int g_conv_cbs = 1;       // loader-fed kernel: four or two 64-channel blocks per stage where they fit
 int g_conv_uneven = 1;    // loader-fed kernel: more CTAs for the n-tiles that carry a pooled residual
 
-// The tile-per-group epilogues of the loader-fed kernel take residuals only in the chunk-major
-// int16 layout and write no int32 accumulators.
-bool pre_tile_ok(const void* res_in, int res_in_bytes, int res_in_chunked, const void* res_out, int res_out_bytes,
-                 int res_out_chunked, const void* acc_out) {
-    return g_conv_tile && !acc_out && (!res_in || (res_in_chunked && res_in_bytes == 2)) &&
-           (!res_out || (res_out_chunked && res_out_bytes == 2));
-}
 int g_conv_path = 0;     // 0 auto, 1 warp-level b1 MMA, 2 tcgen05 (error if not eligible), 3 = 2 without the activation-stationary kernel
 
 template <int NT, int STRIDE>
@@ -551,7 +538,7 @@ int launch_conv_umma_pre_k(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream
     if (per > mtiles) per = mtiles;
     long long grid = per * a.ntiles_n;
     a.nt_heavy = 0; a.per_heavy = a.per_light = (int)per;
-    if (EPI == umma::kEpiTileRes && g_conv_uneven && a.res_in && a.residual_pool) {
+    if (EPI == umma::kEpiTilePool && g_conv_uneven && a.res_in && a.residual_pool) {
         // A pooled residual injected into the first channels only (the first block of a stage):
         // the n-tiles it falls into take about 1.75 times as long per tile as the others when the
         // tile's own MMAs are few (measured at 14 x 14 x 256: 0.141 ms against 0.081 for the same
@@ -576,25 +563,53 @@ int launch_conv_umma_pre_k(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream
 
 // n-tile 64: two CTAs of eight epilogue warps per SM when the filter block and a patch ring of at
 // least three stages fit half of the shared memory.  Measured at batch 1024, 56 x 56 x 64 -> 64
-// (two CTAs / one): all-warps-per-tile epilogues 0.119 / 0.154 ms plain and 0.40 / 0.33 with
-// residual rows moved directly (32 columns of residual per thread spill), so those stay on one
-// CTA; tile-per-group epilogues 0.105 / 0.143 plain and 0.223 / 0.255 with chunk-major residuals.
-template <int EPI>
-int launch_conv_umma_pre_64(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st) {
-    if (g_conv_two_ctas && (EPI == umma::kEpiPlain || EPI == umma::kEpiTile || EPI == umma::kEpiTileRes || g_conv_two_ctas == 2)) {
-        int stages = a.pre_stages;
-        const int nplane = (a.stride == 2 ? 4 : 1) * a.pre_cbs;
-        while (stages > 3 && umma::pre_smem_bytes(a.NPOS, a.C, a.R * a.S, 64, stages, nplane) > 113 * 1024) stages--;
-        const size_t need = umma::pre_smem_bytes(a.NPOS, a.C, a.R * a.S, 64, stages, nplane);
-        if (need <= 113 * 1024) {
-            a.pre_stages = stages;
-            return launch_conv_umma_pre_k<64, EPI, 8>(a, need, sms, st);
+// (two CTAs / one): 0.105 / 0.143 ms plain and 0.223 / 0.255 with chunk-major residuals.
+template <int NT, int EPI>
+int launch_conv_umma_pre_epi(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st) {
+    if constexpr (NT == 64) {
+        if (g_conv_two_ctas) {
+            int stages = a.pre_stages;
+            const int nplane = (a.stride == 2 ? 4 : 1) * a.pre_cbs;
+            while (stages > 3 && umma::pre_smem_bytes(a.NPOS, a.C, a.R * a.S, 64, stages, nplane) > 113 * 1024) stages--;
+            const size_t need = umma::pre_smem_bytes(a.NPOS, a.C, a.R * a.S, 64, stages, nplane);
+            if (need <= 113 * 1024) {
+                a.pre_stages = stages;
+                return launch_conv_umma_pre_k<64, EPI, 8>(a, need, sms, st);
+            }
         }
     }
-    return launch_conv_umma_pre_k<64, EPI, 16>(a, smem, sms, st);
+    return launch_conv_umma_pre_k<NT, EPI, 16>(a, smem, sms, st);
 }
 
-// npos, C, RS of the layer are needed to size the patch ring again when the residual rows are staged
+// kEpiTileRes with an injected residual: its buffers take precedence over the patch ring's depth down
+// to three stages.  *fits = false: no room for them.
+template <int NT>
+int launch_conv_umma_pre_ring(umma::ConvWsArgs& a, int sms, cudaStream_t st, bool* fits) {
+    const int RS = a.R * a.S, np = a.stride == 2 ? 4 : 1;
+    auto need = [&](int stages, int cbs, int epiw) {
+        return umma::pre_smem_bytes(a.NPOS, a.C, RS, NT, stages, np * cbs) + umma::pre_res_ring_bytes(NT, epiw);
+    };
+    *fits = true;
+    if constexpr (NT == 64) {
+        int stages = a.pre_stages;
+        while (stages > 3 && need(stages, a.pre_cbs, 8) > 113 * 1024) stages--;
+        if (g_conv_two_ctas && need(stages, a.pre_cbs, 8) <= 113 * 1024) {
+            a.pre_stages = stages;
+            return launch_conv_umma_pre_k<64, umma::kEpiTileRes, 8>(a, need(stages, a.pre_cbs, 8), sms, st);
+        }
+    }
+    // (an issuer that waits and commits four times as often costs more than the buffers bring: 7 x 7 x
+    // 512 at batch 1024 takes 0.106 ms with them and one block per stage, 0.086 without and four)
+    int stages = a.pre_stages > 3 ? a.pre_stages : 3;
+    while (stages > 3 && need(stages, a.pre_cbs, 16) > 227 * 1024) stages--;
+    if (need(stages, a.pre_cbs, 16) <= 227 * 1024) {
+        a.pre_stages = stages;
+        return launch_conv_umma_pre_k<NT, umma::kEpiTileRes, 16>(a, need(stages, a.pre_cbs, 16), sms, st);
+    }
+    *fits = false;
+    return 0;
+}
+
 template <int NT>
 int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st, bool expand) {
     if (expand) {
@@ -603,47 +618,19 @@ int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t
                                                                    a.pre_front);
         if (launch_check("conv_layer (input expansion)")) return 1;
     }
-    if (pre_tile_ok(a.res_in, a.res_in_bytes, a.res_in_chunked, a.res_out, a.res_out_bytes, a.res_out_chunked, a.acc_out)) {
-        const bool plain = !a.res_in && !a.res_out;
-        if constexpr (NT == 64) {
-            return plain ? launch_conv_umma_pre_64<umma::kEpiTile>(a, smem, sms, st)
-                         : launch_conv_umma_pre_64<umma::kEpiTileRes>(a, smem, sms, st);
-        } else {
-            return plain ? launch_conv_umma_pre_k<NT, umma::kEpiTile, 16>(a, smem, sms, st)
-                         : launch_conv_umma_pre_k<NT, umma::kEpiTileRes, 16>(a, smem, sms, st);
+    if (!a.res_in && !a.res_out && !a.acc_out) return launch_conv_umma_pre_epi<NT, umma::kEpiTile>(a, smem, sms, st);
+    if (!a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked))
+    {
+        if (!a.res_in) return launch_conv_umma_pre_epi<NT, umma::kEpiTileRes>(a, smem, sms, st);
+        if (!a.residual_pool) {
+            bool fits;
+            const int rc = launch_conv_umma_pre_ring<NT>(a, sms, st, &fits);
+            if (fits) return rc;
         }
+        return launch_conv_umma_pre_epi<NT, umma::kEpiTilePool>(a, smem, sms, st);
     }
-    if constexpr (NT >= 64) {
-        // int16 residual rows through shared memory (see conv_umma_pre_cta) when the tensors allow
-        // it and the two row buffers fit beside a patch ring of at least two stages.  Measured at
-        // batch 1024 (staged / direct): 28 x 28 x 128 0.186 / 0.215 ms, 14 x 14 x 256 0.112 /
-        // 0.138, 7 x 7 x 512 0.127 / 0.120, 56 x 56 x 64 (n-tile 64) 0.425 / 0.327 -- the once-per-tile
-        // rendezvous of the 16 epilogue warps costs more than the narrow rows save there.
-        const int lim = a.res_in ? (a.residual_channels < a.res_in_ch ? a.residual_channels : a.res_in_ch) : 0;
-        const bool in_ok = !a.res_in || (a.res_in_bytes == 2 && !a.res_in_chunked && !a.residual_pool && a.res_in_ch % 8 == 0 &&
-                                         ((uintptr_t)a.res_in & 15) == 0 && lim % 8 == 0);
-        const bool out_ok = !a.res_out || (a.res_out_bytes == 2 && !a.res_out_chunked && ((uintptr_t)a.res_out & 15) == 0);
-        if ((a.res_in || a.res_out) && in_ok && out_ok && g_conv_res_stage && (NT >= 128 || g_conv_res_stage == 2)) {
-            int stages = a.pre_stages;
-            const int RS = a.R * a.S;
-            const int nplane = (a.stride == 2 ? 4 : 1) * a.pre_cbs;
-            while (stages > 2 && umma::pre_smem_bytes(a.NPOS, a.C, RS, NT, stages, nplane) + umma::pre_res_stage_bytes(NT) > 227 * 1024)
-                stages--;
-            const size_t need = umma::pre_smem_bytes(a.NPOS, a.C, RS, NT, stages, nplane) + umma::pre_res_stage_bytes(NT);
-            if (need <= 227 * 1024) {
-                a.pre_stages = stages;
-                return launch_conv_umma_pre_k<NT, umma::kEpiStaged, 16>(a, need, sms, st);
-            }
-        }
-    }
-    const bool plain = !a.res_in && !a.res_out && !a.acc_out;
-    if constexpr (NT == 64) {
-        return plain ? launch_conv_umma_pre_64<umma::kEpiPlain>(a, smem, sms, st)
-                     : launch_conv_umma_pre_64<umma::kEpiDirect>(a, smem, sms, st);
-    } else {
-        return plain ? launch_conv_umma_pre_k<NT, umma::kEpiPlain, 16>(a, smem, sms, st)
-                     : launch_conv_umma_pre_k<NT, umma::kEpiDirect, 16>(a, smem, sms, st);
-    }
+    if (a.res_in && a.res_in_bytes == 4) return launch_conv_umma_pre_epi<NT, umma::kEpiRows4>(a, smem, sms, st);
+    return launch_conv_umma_pre_epi<NT, umma::kEpiRows2>(a, smem, sms, st);
 }
 
 // The *_bytes arguments of the conv entry points name the residual's element format: 4 = int32
@@ -655,47 +642,6 @@ bool residual_format(int code, int* bytes, int* chunked, int* proven = nullptr) 
     *chunked = fmt == TCBNN_RES_INT16_CHUNKED;
     *bytes = *chunked ? 2 : fmt;
     return fmt == 2 || fmt == 4 || fmt == TCBNN_RES_INT16_CHUNKED;
-}
-
-// 2x2 max of a chunked int16 residual [ch/8][B*2P*2Q][8] -> NHWC [B][P][Q][ch].  A block takes 32
-// consecutive output pixels x all chunks: it reads chunk by chunk (consecutive lanes = consecutive
-// pixels: whole lines), turns the tile through shared memory (16-byte slots XOR-swizzled by pixel),
-// and writes pixel by pixel (consecutive lanes = consecutive chunks of a row: whole lines again).
-constexpr int kPoolChunkedMaxCh8 = 32;
-__global__ void __launch_bounds__(256) k_pool_residual16_chunked(const uint4* in, uint4* out, int B, int P, int Q, int ch8) {
-    __shared__ uint4 tile[32 * kPoolChunkedMaxCh8];
-    const long long npix = (long long)B * P * Q, npix_in = npix * 4;
-    const long long ntiles = (npix + 31) / 32;
-    const int units = 32 * ch8;
-    const int swz = (ch8 & (ch8 - 1)) == 0 ? (ch8 < 8 ? ch8 - 1 : 7) : 0;    // power-of-two chunk counts only
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const long long pix0 = t * 32;
-        for (int u = threadIdx.x; u < units; u += 256) {
-            const int c = u >> 5, pl = u & 31;
-            const long long pix = pix0 + pl;
-            uint4 m = make_uint4(0u, 0u, 0u, 0u);
-            if (pix < npix) {
-                long long r = pix;
-                const int x = (int)(r % Q); r /= Q;
-                const int y = (int)(r % P);
-                const long long n = r / P;
-                const uint4* s0 = in + (long long)c * npix_in + (n * 2 * P + 2 * y) * 2 * Q + 2 * x;
-                const uint4* s1 = s0 + 2 * Q;
-                const uint4 a = __ldg(s0), b = __ldg(s0 + 1), e = __ldg(s1), f = __ldg(s1 + 1);
-                m.x = __vmaxs2(__vmaxs2(a.x, b.x), __vmaxs2(e.x, f.x));
-                m.y = __vmaxs2(__vmaxs2(a.y, b.y), __vmaxs2(e.y, f.y));
-                m.z = __vmaxs2(__vmaxs2(a.z, b.z), __vmaxs2(e.z, f.z));
-                m.w = __vmaxs2(__vmaxs2(a.w, b.w), __vmaxs2(e.w, f.w));
-            }
-            tile[pl * ch8 + (c ^ (pl & swz))] = m;
-        }
-        __syncthreads();
-        for (int u = threadIdx.x; u < units; u += 256) {
-            const int pl = u / ch8, c = u - pl * ch8;
-            if (pix0 + pl < npix) out[(pix0 + pl) * ch8 + c] = tile[pl * ch8 + (c ^ (pl & swz))];
-        }
-        __syncthreads();
-    }
 }
 
 // 2x2 max of an int16 residual [B][2P][2Q][ch] -> [B][P][Q][ch] (kernel.cuh:773-783), 8 channels
@@ -1453,26 +1399,6 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
                     if (need <= 227 * 1024) { a.pre_cbs = 2; a.pre_stages = 2; pre_smem = need; }
                 }
             }
-            // a pooled int16 residual is reduced by a streaming pass first when the workspace has
-            // the room behind the planes: four scattered loads per value in the epilogue cost more
-            const size_t pooled_res_bytes = (size_t)d->B * d->OH * d->OW * (size_t)res_in_ch * 2;
-            // (the tile-per-group epilogues read a pooled chunk-major residual in place: whole lines)
-            if (res_in && residual_pool && res_in_bytes == 2 && res_in_ch % 8 == 0 && !pooled &&
-                !pre_tile_ok(res_in, res_in_bytes, res_in_chunked, res_out, res_out_bytes, res_out_chunked, acc_out) &&
-                (!res_in_chunked || res_in_ch / 8 <= kPoolChunkedMaxCh8) &&
-                pooled_res_bytes <= L.pool_bytes && workspace_bytes >= planes_padded(L) + pooled_res_bytes) {
-                char* pooled_res = (char*)workspace + planes_padded(L);
-                const long long units = (long long)d->B * d->OH * d->OW * (res_in_ch / 8);
-                if (res_in_chunked)
-                    k_pool_residual16_chunked<<<elementwise_grid(units, sms), 256, 0, st>>>(
-                        (const uint4*)res_in, (uint4*)pooled_res, d->B, d->OH, d->OW, res_in_ch / 8);   // (res_in_ch / 8 <= 32: checked above)
-                else
-                    k_pool_residual16<<<elementwise_grid(units, sms), 256, 0, st>>>((const uint4*)res_in, (uint4*)pooled_res,
-                                                                                 d->B, d->OH, d->OW, res_in_ch / 8);
-                if (launch_check("conv_layer (residual pooling)")) return 1;
-                a.res_in = pooled_res; a.residual_pool = 0;
-                a.res_in_chunked = 0; a.res_in_npix = (long long)d->B * d->OH * d->OW;     // the pooled copy is NHWC
-            }
             if (L.pre_nt == 32) return launch_conv_umma_pre<32>(a, pre_smem, sms, st, !workspace_ready);
             if (L.pre_nt == 64) return launch_conv_umma_pre<64>(a, pre_smem, sms, st, !workspace_ready);
             if (L.pre_nt == 128) return launch_conv_umma_pre<128>(a, pre_smem, sms, st, !workspace_ready);
@@ -1551,13 +1477,10 @@ int tcbnn_conv_prefers_chunked_residual(const tcbnn_conv_desc* d) {
 int tcbnn_set_conv_path(int path) {
     if (path < 0 || path > 10)
         return fail("set_conv_path: 0 = automatic, 1 = warp-level b1 MMA, 2 = tcgen05, 3 = tcgen05 filter-stationary kernel only, "
-                    "4 / 5 = automatic with residual staging never / wherever possible, 6 = automatic, one CTA per SM only, "
-                    "7 = automatic without the tile-per-group epilogues, 8 = automatic, two CTAs per SM wherever they fit, "
+                    "4, 5, 7, 8 = automatic, 6 = automatic, one CTA per SM only, "
                     "9 = automatic, one 64-channel block per stage, 10 = automatic, every n-tile the same number of CTAs");
     g_conv_path = path >= 4 ? 0 : path;
-    g_conv_res_stage = path == 4 ? 0 : path == 5 ? 2 : 1;
-    g_conv_two_ctas = path == 6 ? 0 : path == 8 ? 2 : 1;
-    g_conv_tile = path == 7 ? 0 : 1;
+    g_conv_two_ctas = path == 6 ? 0 : 1;
     g_conv_cbs = path == 9 ? 0 : 1;
     g_conv_uneven = path == 10 ? 0 : 1;
     return 0;
