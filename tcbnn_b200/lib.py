@@ -100,6 +100,18 @@ def check(rc):
         raise TcbnnError(load().tcbnn_last_error().decode())
 
 
+_bound = {}
+
+
+def bound(name):
+    """The entry point as a ctypes function, looked up once."""
+    f = _bound.get(name)
+    if f is None:
+        f = _bound[name] = getattr(load(), name)
+    return f
+
+
 def call(name, *args):
     """Call an int-returning entry point and raise on a non-zero status."""
-    check(getattr(load(), name)(*args))
+    if (_bound.get(name) or bound(name))(*args) != 0:
+        raise TcbnnError(load().tcbnn_last_error().decode())

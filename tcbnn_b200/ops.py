@@ -9,19 +9,27 @@ from . import lib as _l
 from .lib import ConvDesc
 
 
+# Pointers and streams are handed to ctypes as plain ints (its declared argument types convert them):
+# a call's cost on the host is what a small layer's time is made of.
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_current_device = torch._C._cuda_getDevice
+
+
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _raw_stream(_current_device())
 
 
 def _need_cuda(*ts):
     for t in ts:
-        if t is not None and not t.is_cuda:
+        if t is None:
+            continue
+        if not t.is_cuda:
             raise _l.TcbnnError("tcbnn_b200 ops need CUDA tensors (no CPU path exists)")
-        if t is not None and not t.is_contiguous():
+        if not t.is_contiguous():
             raise _l.TcbnnError("tcbnn_b200 ops need contiguous tensors")
 
 
@@ -83,11 +91,11 @@ def gemm_workspace(M, N, K, device):
 def gemm_launches(M, N, K, workspace):
     """Kernels a GEMM-family call of this shape launches with this workspace tensor."""
     nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    return _l.load().tcbnn_gemm_launches(M, N, K, C.c_size_t(nbytes))
+    return _l.load().tcbnn_gemm_launches(M, N, K, nbytes)
 
 
 def _ws(ws):
-    return (_ptr(ws), C.c_size_t(ws.numel() * 4 if ws is not None else 0))
+    return (ws.data_ptr(), ws.numel() * 4) if ws is not None else (None, 0)
 
 
 def bgemm(A, B, K, out=None, workspace=None):
@@ -106,7 +114,9 @@ def fc_layer(A, W, thr, K, out=None, workspace=None):
     M, lda = A.shape
     N, ldw = W.shape
     if out is None:
-        out = torch.zeros((M, step128_words(N)), dtype=torch.int32, device=A.device)
+        # the kernels store every word of a row that holds columns; words behind them read as zero
+        words = step128_words(N)
+        out = (torch.empty if words == (N + 31) // 32 else torch.zeros)((M, words), dtype=torch.int32, device=A.device)
     _l.call("tcbnn_fc_layer", _ptr(A), _ptr(W), _ptr(thr), M, K, N, lda, ldw, _ptr(out),
             out.shape[1], *_ws(workspace), _stream())
     return out
@@ -160,6 +170,11 @@ def conv_workspace(d, device):
     return t
 
 
+def shared_scratch(device):
+    """The tensor conv_workspace() currently hands out on this device, or None."""
+    return _scratch.get((device.type, device.index))
+
+
 def conv_layer(d, x, prepared, thr, res_in=None, residual_channels=0, residual_pool=False,
                out=None, out_image_stride=None, save_residual=False, want_acc=False,
                res_out_buf=None, residual_dtype=torch.int32, workspace=None, workspace_ready=False,
@@ -181,29 +196,36 @@ def conv_layer(d, x, prepared, thr, res_in=None, residual_channels=0, residual_p
     Ow = (d.O + 31) // 32
     stride = out_image_stride or d.OH * d.OW * Ow
     if out is None:
-        out = torch.zeros((d.B, stride), dtype=torch.int32, device=x.device)
+        # a dense output is stored word by word by the layer; padding between images reads as zero
+        dense = stride == d.OH * d.OW * Ow
+        out = (torch.empty if dense else torch.zeros)((d.B, stride), dtype=torch.int32, device=x.device)
     P, Q = d.pool * d.OH, d.pool * d.OW
     res_out = res_out_buf
     if res_out is None and save_residual:
         res_out = torch.empty((d.B, P, Q, d.O), dtype=residual_dtype, device=x.device)
     acc_out = torch.empty((d.B, P, Q, d.O), dtype=torch.int32, device=x.device) if want_acc else None
+    name, args = conv_call(d, x, prepared, thr, res_in, residual_channels, residual_pool, out, stride, res_out, acc_out,
+                           workspace, workspace_ready, next_layer, res_in_chunked, res_out_chunked, res_out_proven)
+    _l.call(name, *args, _stream())
+    return out, res_out, acc_out
+
+
+def conv_call(d, x, prepared, thr, res_in, residual_channels, residual_pool, out, stride, res_out, acc_out,
+              workspace, workspace_ready, next_layer, res_in_chunked, res_out_chunked, res_out_proven):
+    """(entry point, its arguments without the stream) of a conv_layer call on these tensors."""
     res_in_ch = res_in.shape[-1] if res_in is not None else 0
     args = (C.byref(d), _ptr(x), _ptr(prepared), _ptr(thr), _ptr(res_in),
             _residual_code(res_in, res_in_chunked),
-            res_in_ch, residual_channels, int(bool(residual_pool)), _ptr(out),
-            C.c_longlong(stride), _ptr(res_out),
+            res_in_ch, residual_channels, int(bool(residual_pool)), _ptr(out), stride, _ptr(res_out),
             _residual_code(res_out, res_out_chunked, res_out_proven), _ptr(acc_out))
     if next_layer is not None or workspace_ready:
         nd, npl = next_layer if next_layer is not None else (None, None)
-        _l.call("tcbnn_conv_layer_x", *args, _ptr(workspace),
-                C.c_size_t(workspace.numel() if workspace is not None else 0), int(bool(workspace_ready)),
-                C.byref(nd) if nd is not None else None, _ptr(npl),
-                C.c_size_t(npl.numel() if npl is not None else 0), _stream())
-    elif workspace is not None:
-        _l.call("tcbnn_conv_layer_w", *args, _ptr(workspace), C.c_size_t(workspace.numel()), _stream())
-    else:
-        _l.call("tcbnn_conv_layer", *args, _stream())
-    return out, res_out, acc_out
+        return "tcbnn_conv_layer_x", args + (
+            _ptr(workspace), workspace.numel() if workspace is not None else 0, int(bool(workspace_ready)),
+            C.byref(nd) if nd is not None else None, _ptr(npl), npl.numel() if npl is not None else 0)
+    if workspace is not None:
+        return "tcbnn_conv_layer_w", args + (_ptr(workspace), workspace.numel())
+    return "tcbnn_conv_layer", args
 
 
 def _residual_code(t, chunked, proven=False):
@@ -296,24 +318,26 @@ def inconv_layer(d, x, filter_bits, thr, out=None, out_image_stride=None, save_r
     acc_out = torch.empty((d.B, P, Q, d.O), dtype=torch.float32, device=x.device) if want_acc else None
     if next_layer is not None and specialized is None:
         raise _l.TcbnnError("inconv_layer: next_layer needs the specialised kernel")
+    name, args = inconv_call(d, x, filter_bits, thr, out, stride, res_out, acc_out, lut, specialized, next_layer, res_out_chunked)
+    _l.call(name, *args, _stream())
+    return out, res_out, acc_out
+
+
+def inconv_call(d, x, filter_bits, thr, out, stride, res_out, acc_out, lut, specialized, next_layer, res_out_chunked):
+    """(entry point, its arguments without the stream) of an inconv_layer call on these tensors."""
+    res_bytes = res_out.element_size() if res_out is not None else 4
     if specialized is not None:
         u8 = lut is not None
         nd, npl = next_layer if next_layer is not None else (None, None)
-        _l.call("tcbnn_inconv_specialized_layer_x", specialized.handle, C.byref(d),
-                None if u8 else _ptr(x), _ptr(x) if u8 else None, _ptr(lut), _ptr(out),
-                C.c_longlong(stride), _ptr(res_out),
-                _residual_code(res_out, res_out_chunked), _ptr(acc_out),
-                C.byref(nd) if nd is not None else None, _ptr(npl),
-                C.c_size_t(npl.numel() if npl is not None else 0), _stream())
-    elif lut is not None:
-        _l.call("tcbnn_inconv_layer_u8", C.byref(d), _ptr(x), _ptr(lut), _ptr(filter_bits), _ptr(thr),
-                _ptr(out), C.c_longlong(stride), _ptr(res_out),
-                res_out.element_size() if res_out is not None else 4, _ptr(acc_out), _stream())
-    else:
-        _l.call("tcbnn_inconv_layer", C.byref(d), _ptr(x), _ptr(filter_bits), _ptr(thr), _ptr(out),
-                C.c_longlong(stride), _ptr(res_out),
-                res_out.element_size() if res_out is not None else 4, _ptr(acc_out), _stream())
-    return out, res_out, acc_out
+        return "tcbnn_inconv_specialized_layer_x", (
+            specialized.handle, C.byref(d), None if u8 else _ptr(x), _ptr(x) if u8 else None, _ptr(lut), _ptr(out),
+            stride, _ptr(res_out), _residual_code(res_out, res_out_chunked), _ptr(acc_out),
+            C.byref(nd) if nd is not None else None, _ptr(npl), npl.numel() if npl is not None else 0)
+    if lut is not None:
+        return "tcbnn_inconv_layer_u8", (C.byref(d), _ptr(x), _ptr(lut), _ptr(filter_bits), _ptr(thr), _ptr(out), stride,
+                                         _ptr(res_out), res_bytes, _ptr(acc_out))
+    return "tcbnn_inconv_layer", (C.byref(d), _ptr(x), _ptr(filter_bits), _ptr(thr), _ptr(out), stride, _ptr(res_out),
+                                  res_bytes, _ptr(acc_out))
 
 
 def mma_peak(kind, warps_per_sm=32, iters=4000):

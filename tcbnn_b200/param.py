@@ -73,7 +73,29 @@ def _dev():
     return torch.device("cuda", torch.cuda.current_device())
 
 
-class In128LayerParam:
+class _Layer:
+    """What the layer classes share: forward() makes one call of the C ABI whose arguments are worked
+    out once (_call_args) and kept until an attribute of the object is set -- a buffer, the live batch,
+    a hand-over -- so that a pass over a network of small layers is not spent on preparing arguments."""
+
+    def __setattr__(self, name, value):
+        self.__dict__[name] = value
+        self.__dict__["_call"] = None
+
+    def forward(self):
+        c = self.__dict__.get("_call")
+        if c is None or not self._call_valid(c):
+            name, args, keep = self._call_args()
+            # `keep`: tensors and descriptors the arguments point into
+            c = self.__dict__["_call"] = (ops._l.bound(name), args, keep)
+        if c[0](*c[1], ops._stream()) != 0:
+            raise ops._l.TcbnnError(ops._l.load().tcbnn_last_error().decode())
+
+    def _call_valid(self, c):
+        return True
+
+
+class In128LayerParam(_Layer):
     """param.h:115-222.  fp32 [input_height][input_width] -> bit rows."""
 
     def __init__(self, name, input_height, input_width):
@@ -102,9 +124,9 @@ class In128LayerParam:
         src = src.reshape(-1, self.input_width)
         self.input_gpu[:src.shape[0]].copy_(src, non_blocking=True)
 
-    def forward(self):
-        ops._l.call("tcbnn_pack_rows", ops._ptr(self.input_gpu), self.live, self.input_width,
-                    self.output_gpu.shape[1], ops._ptr(self.output_gpu), ops._stream())
+    def _call_args(self):
+        x, out = self.input_gpu, self.output_gpu
+        return "tcbnn_pack_rows", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out)), (x, out)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -116,7 +138,7 @@ class In128LayerParam:
         return ops.unpack_rows(self.output_gpu, self.output_width).cpu().numpy()
 
 
-class Fc128LayerParam:
+class Fc128LayerParam(_Layer):
     """param.h:224-385.  Hidden FC layer: bit GEMM + threshold + repack."""
 
     def __init__(self, name, input_height, input_width, weight_width):
@@ -155,9 +177,11 @@ class Fc128LayerParam:
     def kernel_launches(self):
         return self.launches
 
-    def forward(self):
-        ops.fc_layer(self.input_gpu[:self.live], self.weight_gpu, self.bn_gpu, self.input_width,
-                     out=self.output_gpu[:self.live], workspace=self.workspace)
+    def _call_args(self):
+        a, w, thr, out, ws = self.input_gpu, self.weight_gpu, self.bn_gpu, self.output_gpu, self.workspace
+        ops._need_cuda(a, w, thr)
+        return "tcbnn_fc_layer", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
+                                  a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws)), (a, w, thr, out, ws)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -169,7 +193,7 @@ class Fc128LayerParam:
         return ops.unpack_rows(self.output_gpu, self.output_width).cpu().numpy()
 
 
-class Out128LayerParam:
+class Out128LayerParam(_Layer):
     """param.h:388-531.  Output layer: bit GEMM + per-class scale and bias -> fp32 logits."""
 
     def __init__(self, name, input_height, input_width, weight_width):
@@ -203,9 +227,13 @@ class Out128LayerParam:
     def kernel_launches(self):
         return self.launches
 
-    def forward(self):
-        ops.out_layer(self.input_gpu[:self.live], self.weight_gpu, self.bn_scale_gpu, self.bn_bias_gpu,
-                      self.input_width, out=self.output_gpu[:self.live], workspace=self.workspace)
+    def _call_args(self):
+        a, w, out, ws = self.input_gpu, self.weight_gpu, self.output_gpu, self.workspace
+        scale, bias = self.bn_scale_gpu, self.bn_bias_gpu
+        ops._need_cuda(a, w, scale, bias)
+        return "tcbnn_out_layer", (ops._ptr(a), ops._ptr(w), ops._ptr(scale), ops._ptr(bias), self.live, self.input_width,
+                                   w.shape[0], a.shape[1], w.shape[1], ops._ptr(out), out.shape[1],
+                                   *ops._ws(ws)), (a, w, scale, bias, out, ws)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -214,7 +242,7 @@ class Out128LayerParam:
         return self.output_gpu[:self.live].cpu().numpy()
 
 
-class InConv128LayerParam:
+class InConv128LayerParam(_Layer):
     """param.h:701-870.  First conv layer on fp32 NCHW images."""
 
     def __init__(self, name, input_height, input_width, filter_height, filter_width,
@@ -308,12 +336,16 @@ class InConv128LayerParam:
         src = src.reshape((-1,) + tuple(self.input_gpu.shape[1:]))
         self.input_gpu[:src.shape[0]].copy_(src, non_blocking=True)
 
-    def forward(self):
-        ops.inconv_layer(self.desc, self.input_gpu, self.filter_gpu, self.bn_gpu, out=self.output_gpu,
-                         res_out_buf=self.output_residual_gpu, lut=self.input_lut_gpu,
-                         specialized=self.specialized,
-                         next_layer=self.next_layer if self.specialized is not None else None,
-                         res_out_chunked=self.residual_chunked)
+    def _call_args(self):
+        d, x, f, thr, lut = self.desc, self.input_gpu, self.filter_gpu, self.bn_gpu, self.input_lut_gpu
+        out, res, spec = self.output_gpu, self.output_residual_gpu, self.specialized
+        nxt = self.next_layer if spec is not None else None
+        ops._need_cuda(x, f, thr, lut)
+        if (x.dtype == torch.uint8) != (lut is not None):
+            raise ops._l.TcbnnError("%s: uint8 images need a lut, fp32 images must not have one" % self.name)
+        name, args = ops.inconv_call(d, x, f, thr, out, d.OH * d.OW * ((d.O + 31) // 32), res, None, lut, spec, nxt,
+                                     self.residual_chunked)
+        return name, args, (d, x, f, thr, lut, out, res, spec, nxt)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -330,7 +362,7 @@ class InConv128LayerParam:
         return ops.unpack_rows(self.output_gpu[:d.B].reshape(rows, -1), d.O).reshape(d.B, d.OH, d.OW, d.O).cpu().numpy()
 
 
-class Conv128LayerParam:
+class Conv128LayerParam(_Layer):
     """param.h:872-1065.  Binary conv layer with threshold / OR-pool / residual fused."""
 
     def __init__(self, name, input_height, input_width, filter_height, filter_width,
@@ -393,6 +425,7 @@ class Conv128LayerParam:
         if n != self.desc.B and self.input_planes is not None:
             self.input_planes.zero_()
         self.desc.B = n
+        self._call = None                # the scratch a call needs depends on the batch
 
     def set_input_gpu(self, t):
         d = self.desc
@@ -440,18 +473,24 @@ class Conv128LayerParam:
         pools_output = self.desc.pool != 1 and has_ws          # tcgen05 on the pre-pool grid + OR-pooling pass
         return 1 + int(own_expand) + int(pools_output)
 
-    def forward(self):
-        ops.conv_layer(self.desc, self.input_gpu, self.prepared, self.bn_gpu,
-                       res_in=self.input_residual_gpu if self.inject_residual else None,
-                       residual_channels=self.residual_channels, residual_pool=self.residual_pool,
-                       out=self.output_gpu, out_image_stride=self.out_image_stride,
-                       res_out_buf=self.output_residual_gpu,
-                       workspace=self.input_planes, workspace_ready=self.input_planes is not None,
-                       next_layer=self.next_layer,
-                       res_in_chunked=self.input_residual_chunked and self.inject_residual,
-                       res_out_chunked=self.residual_chunked,
-                       # int16 was chosen from the bound fan-in + bound of the injected residual
-                       res_out_proven=self.residual_bound is not None and self.residual_bound <= 32767)
+    def _call_args(self):
+        d, x, prep, thr = self.desc, self.input_gpu, self.prepared, self.bn_gpu
+        res_in = self.input_residual_gpu if self.inject_residual else None
+        out, res_out, planes, nxt = self.output_gpu, self.output_residual_gpu, self.input_planes, self.next_layer
+        ops._need_cuda(x, prep, thr, res_in)
+        # planes that a producer fills, or the scratch shared by the layers that bring none
+        ws = planes if planes is not None else ops.conv_workspace(d, x.device)
+        name, args = ops.conv_call(d, x, prep, thr, res_in, self.residual_channels, self.residual_pool, out,
+                                   self.out_image_stride, res_out, None, ws, planes is not None, nxt,
+                                   self.input_residual_chunked and self.inject_residual, self.residual_chunked,
+                                   # int16 was chosen from the bound fan-in + bound of the injected residual
+                                   self.residual_bound is not None and self.residual_bound <= 32767)
+        return name, args, (ws, d, x, prep, thr, res_in, out, res_out, nxt)
+
+    def _call_valid(self, c):
+        # the shared scratch is replaced when a larger layer asks for it
+        ws = c[2][0]
+        return ws is None or ws is self.__dict__.get("input_planes") or ws is ops.shared_scratch(ws.device)
 
     def get_output_gpu(self):
         return self.output_gpu
