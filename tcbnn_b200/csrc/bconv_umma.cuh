@@ -270,7 +270,7 @@ template <int K>
 __device__ __forceinline__ void mma_f4_run(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                            uint32_t b_lo, uint32_t b_hi, uint32_t step_b, const uint32_t* t,
                                            uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb) {
-    static_assert(K == 1 || K == 5 || K == 9, "run lengths in use");
+    static_assert(K == 1 || K == 4 || K == 5 || K == 9, "run lengths in use");
     if constexpr (K == 9)
         asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
                      TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") TCBNN_F4_MMA("%16", "pt")
@@ -281,6 +281,10 @@ __device__ __forceinline__ void mma_f4_run(uint32_t leader, uint32_t d_tmem, uin
         asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
                      TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") "}"
                      ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]) : "memory");
+    else if constexpr (K == 4)
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
+                     TCBNN_F4_MMA("%14", "pt") "}"
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
     else
         asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") "}" ::TCBNN_F4_IN, "r"(t[0]) : "memory");
 }
@@ -310,12 +314,15 @@ __device__ __forceinline__ uint32_t mma_f4_end(uint32_t leader, uint32_t d_tmem,
                                                uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb,
                                                uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1,
                                                uint32_t bar_e, uint32_t bar_c) {
-    static_assert(K == 1 || K == 4, "run lengths in use");
+    static_assert(K == 1 || K == 3 || K == 4, "run lengths in use");
     uint32_t ok;
     if constexpr (K == 4)
         asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_MMA("%19", "pt") TCBNN_F4_MMA("%20", "pt")
                      TCBNN_F4_MMA("%21", "pt") TCBNN_F4_TAIL
                      : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
+    else if constexpr (K == 3)
+        asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_MMA("%19", "pt") TCBNN_F4_MMA("%20", "pt") TCBNN_F4_TAIL
+                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]) : "memory");
     else
         asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_TAIL
                      : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]) : "memory");

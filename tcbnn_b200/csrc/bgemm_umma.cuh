@@ -6,16 +6,23 @@
 // One streaming pass first writes both operands as +-1 nibbles (0 for padding: rows past the end,
 // bits past K) in 4 KB units [128-row tile][64-bit k-block][32-bit chunk][row][16 B], the
 // no-swizzle K-major operand layout, so that a unit is one bulk copy and one MMA operand.
-// The GEMM CTA owns a 128 x 128 or a 256 x 128 tile (one or two 128-row sub-tiles of A against one
-// tile of W) over a range of k-blocks:
+// The GEMM is persistent: a CTA per SM walks over 128 x 128 or 256 x 128 tiles (one or two 128-row
+// sub-tiles of A against one tile of W), each over a range of k-blocks:
 //
-//   warps 0-7  epilogue : after the last k-block, tcgen05.ld and either finish the layer (one
-//                         split: int32 / threshold bits / scale + bias straight from the
-//                         accumulator) or store int32 partial sums for gemm_splitk_finish
+//   warps 0-7  epilogue : tcgen05.ld and either finish the layer (one split: int32 / threshold bits /
+//                         scale + bias straight from the accumulator) or store int32 partial sums for
+//                         gemm_splitk_finish.  128 x 128 tiles alternate between two accumulators, so
+//                         that a tile is finished while the next one is computed
 //   warp  8    loader A : one lane, one bulk copy per sub-tile and stage (a stage holds up to
 //                         kGemmKU consecutive k-blocks, contiguous in the expanded operand)
 //   warp  9    MMA      : converged warp, elected lane: one N=128 MMA per sub-tile and k-block
 //   warp  10   loader W : one lane, one bulk copy per stage
+//
+// Loaders and issuer run ahead across tile boundaries, so set-up, first loads and epilogue of all
+// but a CTA's last tile are hidden: as one CTA per tile (two per SM) the MLP's hidden layer, 8192 x 1024
+// x 1024, spent 23 us on 3.3 us of MMAs.  W's rows are laid out in the order of
+// f4_channel_of_column within each 32, so that integer and float results leave in whole sectors (the
+// 16x256b read of the accumulator, see there).
 //
 // A thread that issues a bulk copy is busy for 100-200 clocks per copy whatever its size, and
 // copies issued by different warps overlap (tcbnn_bulk_copy_rate measures both): hence few, large
@@ -29,15 +36,12 @@ namespace umma {
 constexpr int kGemmThreads = 352;
 constexpr int kGemmUnit = 4096;                        // 128 rows x 64 k, 4 bits each
 constexpr int kGemmKU = 4;                             // k-blocks per stage
-// Per tile shape (PAIR: 256 x 128, else 128 x 128): ring depth, bytes of a stage, tensor-memory
-// columns (accumulators, then 32 columns of unit scales at the top).  The ring sizes also fix how
-// many CTAs share an SM: one 256 x 128 CTA (all 512 columns), two 128 x 128 CTAs (256 each), so
-// that no CTA ever waits for tensor memory held by a neighbour.
-// stages: 4 for a 256 x 128 CTA; 128 x 128 CTAs take 3 when two of them share an SM, 6 alone
+// Per tile shape (PAIR: 256 x 128, else 128 x 128): ring depth and bytes of a stage.  One CTA per SM
+// takes all of tensor memory: accumulators, then 32 columns of unit scales at the top.
+__host__ __device__ constexpr int gemm_stages(bool pair) { return pair ? 4 : 6; }
 __host__ __device__ constexpr int gemm_stage_bytes(bool pair) { return (pair ? 3 : 2) * kGemmKU * kGemmUnit; }
-__host__ __device__ constexpr uint32_t gemm_tmem_cols(bool pair) { return pair ? 512u : 256u; }
-__host__ __device__ constexpr size_t gemm_smem(bool pair, int stages) {
-    return (size_t)stages * gemm_stage_bytes(pair) + 32 * 8 + 64;
+__host__ __device__ constexpr size_t gemm_smem(bool pair) {
+    return (size_t)gemm_stages(pair) * gemm_stage_bytes(pair) + 32 * 8 + 64 + 8 * 128 * 4;    // ring, barriers, thresholds per epilogue warp
 }
 
 struct GemmUmmaArgs {
@@ -47,7 +51,6 @@ struct GemmUmmaArgs {
     int32_t* partial;          // [splits][M][N], used when splits > 1
     // splits == 1: the layer is finished in the epilogue (GemmMode of bnn_layers.cuh)
     int mode; void* out; int ldo; const float* p0; const float* p1;
-    int nst;                   // stages in the ring (the launch's dynamic shared memory holds them)
     int* status;               // set to 1 when a bounded wait gives up
     long long* trace;          // null, or 16 counters: CTA 0 writes [9..15] (clocks; see the C header)
 };
@@ -67,8 +70,10 @@ __device__ __forceinline__ uint4 keep32_f4(uint4 e, uint32_t m) {
 __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_rows, int a_ld, int RT_a,
                                                  const uint32_t* w_bits, int w_rows, int w_ld, int RT_w,
                                                  int K, int KB, uint4* out_a, uint4* out_w) {
-    // the GEMM that consumes these units may be set up meanwhile (it waits before its first copy)
+    // the GEMM that consumes these units may be set up meanwhile (it waits before its first copy);
+    // this pass itself is a programmatic dependent of whatever wrote A
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int KG = (KB + 3) >> 2;
     const int tasks = (RT_a + RT_w) * KG;
     const int t = threadIdx.x, row = t >> 1, half = t & 1;
@@ -79,7 +84,7 @@ __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_r
         const uint32_t* bits = isw ? w_bits : a_bits;
         const int rows = isw ? w_rows : a_rows, ld = isw ? w_ld : a_ld;
         uint4* out = (isw ? out_w : out_a) + (size_t)rt * KB * 256;      // 256 slots of 16 bytes per unit
-        const int r = rt * 128 + row;
+        const int r = rt * 128 + (isw ? (row & ~31) + f4_channel_of_column(row & 31) : row);
         const int w0 = kg * 8 + half * 4;                                // first 32-bit chunk of this thread
         uint32_t w[4] = {0u, 0u, 0u, 0u};
         if (r < rows) {
@@ -107,32 +112,43 @@ __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_r
 
 template <bool PAIR>
 __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned char* smem) {
-    constexpr int STAGE = gemm_stage_bytes(PAIR);
-    const int NST = g.nst;                              // at most 8
-    constexpr uint32_t TM_COLS = gemm_tmem_cols(PAIR), SF_COL = TM_COLS - 32;
+    constexpr int STAGE = gemm_stage_bytes(PAIR), NST = gemm_stages(PAIR);
+    constexpr int NACC = PAIR ? 1 : 2;                  // accumulators of 256 / 128 columns
+    constexpr uint32_t TM_COLS = 512, SF_COL = TM_COLS - 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const long long tr_cta0 = clock64();
     uint64_t* sBar = reinterpret_cast<uint64_t*>(smem + (size_t)NST * STAGE);
-    // barriers: full[NST] | empty[NST] | acc_full | drain
-    uint32_t* sTmem = reinterpret_cast<uint32_t*>(sBar + 2 * NST + 2);
+    // barriers: full[NST] | empty[NST] | acc_full[NACC] | acc_empty[NACC] | drain
+    uint32_t* sTmem = reinterpret_cast<uint32_t*>(sBar + 2 * NST + 2 * NACC + 1);
     volatile int* sAbort = reinterpret_cast<volatile int*>(sTmem + 1);
+    float* sThr = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(sTmem + 2) + 15) & ~(uintptr_t)15);
     const uint32_t bar0 = smem_u32(sBar);
     auto BAR_FULL = [&](int s) { return bar0 + 8u * s; };
     auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (NST + s); };
-    const uint32_t BAR_ACC = bar0 + 8u * (2 * NST), BAR_DRAIN = bar0 + 8u * (2 * NST + 1);
+    auto BAR_CFULL = [&](int b) { return bar0 + 8u * (2 * NST + b); };
+    auto BAR_CEMPTY = [&](int b) { return bar0 + 8u * (2 * NST + NACC + b); };
+    const uint32_t BAR_DRAIN = bar0 + 8u * (2 * NST + 2 * NACC);
 
-    // tile of this CTA: blockIdx.x = (split * tiles_m + tm) * NT + tn; tm counts pairs of sub-tiles when PAIR
+    // tile t = (split * tiles_m + tm) * NT + tn; tm counts pairs of sub-tiles when PAIR
     const int tiles_m = PAIR ? (g.MT + 1) >> 1 : g.MT;
-    const int tn = blockIdx.x % g.NT;
-    const int tm = (blockIdx.x / g.NT) % tiles_m;
-    const int split = blockIdx.x / (g.NT * tiles_m);
-    const int kb0 = split * g.per, kb1 = min(g.KB, kb0 + g.per);
-    const int rt0 = PAIR ? tm * 2 : tm;                 // first 128-row tile of A
-    const bool two = PAIR && rt0 + 1 < g.MT;            // second 128-row sub-tile exists
+    const int ntiles = tiles_m * g.NT * g.splits;
+    struct Tile { int tn, rt0, split, kb0, kb1; bool two; };
+    auto tile = [&](int t) {
+        Tile q;
+        q.tn = t % g.NT;
+        const int tm = (t / g.NT) % tiles_m;
+        q.split = t / (g.NT * tiles_m);
+        q.kb0 = q.split * g.per;
+        q.kb1 = min(g.KB, q.kb0 + g.per);
+        q.rt0 = PAIR ? tm * 2 : tm;                     // first 128-row tile of A
+        q.two = PAIR && q.rt0 + 1 < g.MT;               // second 128-row sub-tile exists
+        return q;
+    };
 
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
         for (int s = 0; s < NST; s++) { mbar_init(BAR_FULL(s), 2); mbar_init(BAR_EMPTY(s), 1); }
-        mbar_init(BAR_ACC, 1);
+        for (int b = 0; b < NACC; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), 8); }
         mbar_init(BAR_DRAIN, 1);
         *sAbort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -162,23 +178,26 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             uint32_t ph = 0, issued = 0;
             bool ok = true;
             long long tr_w = 0;
-            for (int kb = kb0; kb < kb1; kb += kGemmKU) {
-                const uint32_t nkb = (uint32_t)min(kGemmKU, kb1 - kb);
-                ok = tr ? wait.timed(BAR_EMPTY(s), ph ^ 1, tr_w) : wait(BAR_EMPTY(s), ph ^ 1);
-                if (!ok) break;
-                const uint32_t dst = smem_u32(smem + (size_t)s * STAGE);
-                if (isw) {
-                    mbar_expect_tx(BAR_FULL(s), nkb * kGemmUnit);
-                    bulk_g2s(dst + OFF_W, g.ew + ((size_t)tn * g.KB + kb) * kGemmUnit, nkb * kGemmUnit, BAR_FULL(s));
-                } else {
-                    mbar_expect_tx(BAR_FULL(s), (two ? 2u : 1u) * nkb * kGemmUnit);
-                    bulk_g2s(dst, g.ea + ((size_t)rt0 * g.KB + kb) * kGemmUnit, nkb * kGemmUnit, BAR_FULL(s));
-                    if (two)
-                        bulk_g2s(dst + kGemmKU * kGemmUnit, g.ea + ((size_t)(rt0 + 1) * g.KB + kb) * kGemmUnit,
-                                 nkb * kGemmUnit, BAR_FULL(s));
+            for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+                const Tile q = tile(t);
+                const unsigned char* src = isw ? g.ew + (size_t)q.tn * g.KB * kGemmUnit : g.ea + (size_t)q.rt0 * g.KB * kGemmUnit;
+                for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
+                    const uint32_t bytes = (uint32_t)min(kGemmKU, q.kb1 - kb) * kGemmUnit;
+                    ok = tr ? wait.timed(BAR_EMPTY(s), ph ^ 1, tr_w) : wait(BAR_EMPTY(s), ph ^ 1);
+                    if (!ok) break;
+                    const uint32_t dst = smem_u32(smem + (size_t)s * STAGE);
+                    if (isw) {
+                        mbar_expect_tx(BAR_FULL(s), bytes);
+                        bulk_g2s(dst + OFF_W, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
+                    } else {
+                        mbar_expect_tx(BAR_FULL(s), (q.two ? 2u : 1u) * bytes);
+                        bulk_g2s(dst, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
+                        if (q.two)
+                            bulk_g2s(dst + kGemmKU * kGemmUnit, src + (size_t)(g.KB + kb) * kGemmUnit, bytes, BAR_FULL(s));
+                    }
+                    issued++;
+                    if (++s == NST) { s = 0; ph ^= 1; }
                 }
-                issued++;
-                if (++s == NST) { s = 0; ph ^= 1; }
             }
             if (tr && !isw) g.trace[10] = tr_w;
             if (!ok) {
@@ -196,40 +215,80 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         __syncwarp();
     } else if (warp == 9) {
         // =============================== MMA issuer =========================================
-        const bool leader = elect_one();
+        // (what the next stage needs is worked out and asked for while this one's MMAs are queued: the
+        // same scheme as in bconv_umma_pre.cuh, reasons there)
+        const uint32_t leader = elect_one() ? 1u : 0u;
         constexpr uint32_t IDESC = idesc_f4(128);
         const uint64_t desc0 = smem_desc(smem_u32(smem), 128 * 16, 128u);
         const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
         constexpr uint32_t stepStage = STAGE >> 4, stepUnit = kGemmUnit >> 4, offW = OFF_W >> 4,
                            offA2 = (kGemmKU * kGemmUnit) >> 4;
+        const uint32_t units[4] = {0u, stepUnit, 2 * stepUnit, 3 * stepUnit};
         const uint32_t sfa = tmem + SF_COL, sfb = tmem + SF_COL + 16;
-        int s = 0;
-        uint32_t ph = 0;
+        uint32_t s = 0, ph = 0, b = 0, bph = 0, ready = 0, need = 3u;
         bool ok = true;
         long long tr_w = 0;
         const long long tr_t0 = clock64();
-        for (int kb = kb0; kb < kb1 && ok; kb += kGemmKU) {
-            const int nkb = min(kGemmKU, kb1 - kb);
-            ok = tr ? wait.timed(BAR_FULL(s), ph, tr_w) : wait.spin(BAR_FULL(s), ph);
-            if (!ok) break;
-            tc_fence_after();
-            if (leader) {
-                const uint32_t a = lo0 + s * stepStage, b = a + offW;
-#pragma unroll
-                for (int j = 0; j < kGemmKU; j++) {
-                    if (j < nkb) {
-                        const uint32_t acc = (kb > kb0 || j > 0) ? 1u : 0u;
-                        mma_f4_split(tmem, a + j * stepUnit, hi, b + j * stepUnit, hi, IDESC, acc, sfa, sfb);
-                        if (two)
-                            mma_f4_split(tmem + 128, a + offA2 + j * stepUnit, hi, b + j * stepUnit, hi, IDESC, acc, sfa, sfb);
-                    }
+        int t = blockIdx.x, tr_kb = 0;
+        Tile q = tile(t < ntiles ? t : 0);
+        int kb = q.kb0;
+        while (t < ntiles) {
+            if ((ready & need) != need) {
+                if ((need & 2u) && !(ready & 2u)) {
+                    ok = wait.spin(BAR_CEMPTY(b), bph ^ 1);
+                    if (!ok) break;
                 }
-                mma_commit(BAR_EMPTY(s));
+                if (!(ready & 1u)) {
+                    ok = tr ? wait.timed(BAR_FULL(s), ph, tr_w) : wait.spin(BAR_FULL(s), ph);
+                    if (!ok) break;
+                }
             }
-            if (++s == NST) { s = 0; ph ^= 1; }
+            tc_fence_after();
+            const int nkb = min(kGemmKU, q.kb1 - kb);
+            uint32_t acc = kb > q.kb0 ? 1u : 0u;
+            const uint32_t d = tmem + b * 128;
+            uint32_t aLo = lo0 + s * stepStage, bLo = aLo + offW;
+            if (nkb == kGemmKU) {
+                if (q.two) mma_f4_run<4>(leader, d + 128, aLo + offA2, hi, bLo, hi, stepUnit, units, IDESC, acc, sfa, sfb);
+                mma_f4_run<1>(leader, d, aLo, hi, bLo, hi, stepUnit, units, IDESC, acc, sfa, sfb);
+            } else {
+                for (int j = 0; j < nkb; j++) {
+                    const uint32_t o = j * stepUnit;
+                    if (q.two) mma_f4_run<1>(leader, d + 128, aLo + offA2, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
+                    if (j + 1 < nkb) mma_f4_run<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
+                    if (j + 1 < nkb) acc = 1;
+                }
+            }
+            asm volatile("" : "+r"(s), "+r"(b), "+r"(ph), "+r"(bph), "+r"(kb));   // what follows stays behind those MMAs
+            tr_kb += nkb;
+            const bool last = kb + nkb >= q.kb1;
+            const uint32_t sc = s, bc = b;
+            s = s + 1 == (uint32_t)NST ? 0u : s + 1;
+            ph ^= s == 0 ? 1u : 0u;
+            if (last) {
+                b = b + 1 == (uint32_t)NACC ? 0u : b + 1;
+                bph ^= b == 0 ? 1u : 0u;
+            }
+            const uint32_t bar_c = last ? BAR_CFULL(bc) : 0u;
+            need = last ? 3u : 1u;
+            // (while a tile is being issued, its own accumulator is what bar1 names; the answer counts
+            // only at the first stage of a tile)
+            if (nkb == kGemmKU)
+                ready = mma_f4_end<3>(leader, d, aLo, hi, bLo + stepUnit, hi, stepUnit, units + 1, IDESC, 1u, sfa, sfb,
+                                      BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
+            else {
+                const uint32_t o = (nkb - 1) * stepUnit;
+                ready = mma_f4_end<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb,
+                                      BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
+            }
+            if (last) {
+                t += gridDim.x;
+                if (t < ntiles) { q = tile(t); kb = q.kb0; }
+            } else {
+                kb += kGemmKU;
+            }
         }
-        if (ok && leader) mma_commit(BAR_ACC);
-        if (tr && leader) { g.trace[11] = clock64() - tr_t0; g.trace[12] = tr_w; g.trace[14] = kb1 - kb0; }
+        if (tr && leader) { g.trace[11] = clock64() - tr_t0; g.trace[12] = tr_w; g.trace[14] = tr_kb; }
         if (!ok && leader) {
             // giving up: the MMAs already issued must have finished before tensor memory is freed
             mma_commit(BAR_DRAIN);
@@ -239,58 +298,124 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         __syncwarp();
     } else if (warp < 8) {
         // =============================== epilogue ===========================================
-        const int sub = warp >> 2, quad = warp & 3;
-        const int m = (rt0 + sub) * 128 + quad * 32 + lane;
-        const bool have = sub == 0 || two;
-        const long long tr_t0 = clock64();
-        const bool acc_ok = wait.relaxed(BAR_ACC, 0);
-        if (g.trace != nullptr && blockIdx.x == 0 && tid == 0) g.trace[13] = clock64() - tr_t0;
-        const long long tr_t1 = clock64();
-        if (acc_ok && have) {
+        const int quad = warp & 3, q4 = lane & 3;
+        long long tr_w = 0, tr_body = 0;
+        int b = 0;
+        uint32_t bph = 0;
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            const Tile q = tile(t);
+            const int sub = PAIR ? warp >> 2 : 0;       // 256 x 128: a warpgroup per sub-tile; 128 x 128: per column half
+            const int nb0 = PAIR ? 0 : (warp >> 2) * 2, nb1 = PAIR ? 4 : nb0 + 2;
+            const int m0 = (q.rt0 + sub) * 128 + quad * 32;                  // this warp's rows
+            const bool have = sub == 0 || q.two;
+            // thresholds of this warp's columns, in the accumulator's column order, while it is awaited
+            // (a threshold per column straight from global memory costs a trip to L2 each: 6800 clocks
+            // per tile).  NaN behind the last column: never reached.
+            float* const thr = sThr + warp * 128;
+            if (g.splits == 1 && g.mode == GEMM_FC_BITS) {
+                __syncwarp();
+                for (int nb = nb0; nb < nb1; nb++) {
+                    const int n = q.tn * 128 + nb * 32 + f4_channel_of_column(lane);
+                    thr[nb * 32 + lane] = n < g.N ? __ldg(g.p0 + n) : __int_as_float(0x7FC00000);
+                }
+                __syncwarp();
+            }
+            const long long e0 = clock64();
+            if (!wait.relaxed(BAR_CFULL(b), bph)) break;
+            const long long e1 = clock64();
+            tr_w += e1 - e0;
             tc_fence_after();
-            const bool vec = (g.N & 3) == 0;
+            const uint32_t tcol = tmem + ((uint32_t)(quad * 32) << 16) + b * 128 + sub * 128;
+            if (have) {
+                const bool ints = g.splits > 1 || g.mode == GEMM_INT32;
+                if (!ints && g.mode == GEMM_FC_BITS) {
+                    const int m = m0 + lane;
+#pragma unroll 1
+                    for (int nb = nb0; nb < nb1; nb++) {
+                        const int n0 = q.tn * 128 + nb * 32;
+                        if (n0 >= g.N) break;
+                        int v[32];
+                        tmem_ld32(tcol + nb * 32, v);
+                        tmem_ld_wait();
+                        // (float)K - 2*(float)c >= thr[n] (kernel.cuh:210-213): the accumulator is that value
+                        uint32_t word = 0;
+                        const float4* t4 = reinterpret_cast<const float4*>(thr + nb * 32);
 #pragma unroll
-            for (int nb = 0; nb < 4; nb++) {
-                int v[32];
-                tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + sub * 128 + nb * 32, v);
-                tmem_ld_wait();
-                const int n0 = tn * 128 + nb * 32;
-                if (m >= g.M || n0 >= g.N) continue;
-                if (g.splits > 1 || g.mode == GEMM_INT32) {
-                    // int32 sums: the split-K partials, or C itself
-                    int32_t* dst = g.splits > 1 ? g.partial + ((size_t)split * g.M + m) * g.N + n0
-                                                : reinterpret_cast<int32_t*>(g.out) + (size_t)m * g.ldo + n0;
-                    const bool v4 = g.splits > 1 ? vec : ((g.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0);
+                        for (int j = 0; j < 8; j++) {
+                            const float4 th = t4[j];
+                            if (__int_as_float(v[4 * j]) >= th.x) word |= 0x80000000u >> f4_channel_of_column(4 * j);
+                            if (__int_as_float(v[4 * j + 1]) >= th.y) word |= 0x80000000u >> f4_channel_of_column(4 * j + 1);
+                            if (__int_as_float(v[4 * j + 2]) >= th.z) word |= 0x80000000u >> f4_channel_of_column(4 * j + 2);
+                            if (__int_as_float(v[4 * j + 3]) >= th.w) word |= 0x80000000u >> f4_channel_of_column(4 * j + 3);
+                        }
+                        if (m < g.M) reinterpret_cast<uint32_t*>(g.out)[(size_t)m * g.ldo + (n0 >> 5)] = word;
+                    }
+                } else {
+                    // int32 sums (the split-K partials, or C itself), or scale and bias (kernel.cuh:270-273,
+                    // fused multiply-add): rows of four consecutive columns per lane
+                    uint32_t* dst = g.splits > 1 ? reinterpret_cast<uint32_t*>(g.partial) + (size_t)q.split * g.M * g.N
+                                                 : reinterpret_cast<uint32_t*>(g.out);
+                    const int ld = g.splits > 1 ? g.N : g.ldo;
+                    const bool v4 = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+#pragma unroll 1
+                    for (int nb = nb0; nb < nb1; nb++) {
+                        const int n0 = q.tn * 128 + nb * 32 + 4 * q4;
+                        float4 sc[2], bi[2];
+                        if (!ints) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const int c0 = f4_acc_to_int(v[4 * j]), c1 = f4_acc_to_int(v[4 * j + 1]);
-                        const int c2 = f4_acc_to_int(v[4 * j + 2]), c3 = f4_acc_to_int(v[4 * j + 3]);
-                        if (v4 && n0 + 4 * j + 3 < g.N) {
-                            *reinterpret_cast<int4*>(dst + 4 * j) = make_int4(c0, c1, c2, c3);
-                        } else {
-                            const int cc[4] = {c0, c1, c2, c3};
+                            for (int gg = 0; gg < 2; gg++) {
+                                const int n = n0 + 16 * gg;
+                                sc[gg] = make_float4(n < g.N ? __ldg(g.p0 + n) : 0.f, n + 1 < g.N ? __ldg(g.p0 + n + 1) : 0.f,
+                                                     n + 2 < g.N ? __ldg(g.p0 + n + 2) : 0.f, n + 3 < g.N ? __ldg(g.p0 + n + 3) : 0.f);
+                                bi[gg] = make_float4(n < g.N ? __ldg(g.p1 + n) : 0.f, n + 1 < g.N ? __ldg(g.p1 + n + 1) : 0.f,
+                                                     n + 2 < g.N ? __ldg(g.p1 + n + 2) : 0.f, n + 3 < g.N ? __ldg(g.p1 + n + 3) : 0.f);
+                            }
+                        }
 #pragma unroll
-                            for (int k = 0; k < 4; k++)
-                                if (n0 + 4 * j + k < g.N) dst[4 * j + k] = cc[k];
+                        for (int h = 0; h < 2; h++) {
+                            int v[16];
+                            tmem_ld_16x256b_x4(tcol + ((uint32_t)(16 * h) << 16) + nb * 32, v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 2; i++) {
+                                const int m = m0 + 16 * h + 8 * i + (lane >> 2);
+                                if (m >= g.M) continue;
+#pragma unroll
+                                for (int gg = 0; gg < 2; gg++) {
+                                    const int n = n0 + 16 * gg;
+                                    const int r0 = v[8 * gg + 2 * i], r1 = v[8 * gg + 2 * i + 1];
+                                    const int r2 = v[8 * gg + 4 + 2 * i], r3 = v[8 * gg + 4 + 2 * i + 1];
+                                    uint4 w;
+                                    if (ints)
+                                        w = make_uint4((uint32_t)f4_acc_to_int(r0), (uint32_t)f4_acc_to_int(r1),
+                                                       (uint32_t)f4_acc_to_int(r2), (uint32_t)f4_acc_to_int(r3));
+                                    else
+                                        w = make_uint4(__float_as_uint(fmaf(__int_as_float(r0), sc[gg].x, bi[gg].x)),
+                                                       __float_as_uint(fmaf(__int_as_float(r1), sc[gg].y, bi[gg].y)),
+                                                       __float_as_uint(fmaf(__int_as_float(r2), sc[gg].z, bi[gg].z)),
+                                                       __float_as_uint(fmaf(__int_as_float(r3), sc[gg].w, bi[gg].w)));
+                                    uint32_t* o = dst + (size_t)m * ld + n;
+                                    if (v4 && n + 3 < g.N) {
+                                        *reinterpret_cast<uint4*>(o) = w;
+                                    } else {
+                                        if (n < g.N) o[0] = w.x;
+                                        if (n + 1 < g.N) o[1] = w.y;
+                                        if (n + 2 < g.N) o[2] = w.z;
+                                        if (n + 3 < g.N) o[3] = w.w;
+                                    }
+                                }
+                            }
                         }
                     }
-                } else if (g.mode == GEMM_FC_BITS) {
-                    // (float)K - 2*(float)c >= thr[n] (kernel.cuh:210-213): the accumulator is that value
-                    uint32_t word = 0;
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (n0 + j < g.N && __int_as_float(v[j]) >= __ldg(g.p0 + n0 + j)) word |= 0x80000000u >> j;
-                    reinterpret_cast<uint32_t*>(g.out)[(size_t)m * g.ldo + (n0 >> 5)] = word;
-                } else {
-                    // scale and bias (kernel.cuh:270-273), fused multiply-add
-                    float* dst = reinterpret_cast<float*>(g.out) + (size_t)m * g.ldo + n0;
-#pragma unroll
-                    for (int j = 0; j < 32; j++)
-                        if (n0 + j < g.N) dst[j] = fmaf(__int_as_float(v[j]), __ldg(g.p0 + n0 + j), __ldg(g.p1 + n0 + j));
                 }
             }
+            tc_fence_before();                          // this warp is done with the accumulator
+            __syncwarp();
+            if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+            tr_body += clock64() - e1;
+            if (++b == NACC) { b = 0; bph ^= 1u; }
         }
-        if (g.trace != nullptr && blockIdx.x == 0 && tid == 0) g.trace[15] = clock64() - tr_t1;
+        if (tr && tid == 0) { g.trace[13] = tr_w; g.trace[15] = tr_body; }
     }
     tc_fence_before();
     __syncthreads();

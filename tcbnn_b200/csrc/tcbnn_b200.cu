@@ -2,6 +2,7 @@
 // include/tcbnn_b200.h for the contract of each entry point).
 #include "../../include/tcbnn_b200.h"
 #include "bnn_layers.cuh"
+#include "bgemm_small.cuh"
 #include "bconv_umma.cuh"
 #include "bconv_umma_ws.cuh"
 #include "bconv_umma_as.cuh"
@@ -14,6 +15,7 @@
 #include <cstring>
 #include <atomic>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 using namespace tcbnn;
@@ -70,6 +72,24 @@ int configure_once(bool (&done)[64], F&& configure) {
     return 0;
 }
 
+// Launches `kernel` as a programmatic dependent of whatever precedes it in the stream: its blocks may
+// be set up while that still runs, and it waits (griddepcontrol.wait) before it touches anything that
+// an earlier launch writes or reads.  Every kernel launched this way executes that wait.
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 constexpr int kThreads = 256;          // 8 warps per CTA
 constexpr int kCtasPerSm = 2;          // 16 resident warps per SM, up to 128 registers each
 
@@ -88,10 +108,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_conv(ConvArgs c) { con
 __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_inconv(InConvArgs c) { inconv_layer(c); }
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 k_pack_rows(const float* x, int rows, int cols, int ld, uint32_t* out) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the consumer waits before it reads
     pack_rows(x, rows, cols, ld, out);
 }
 __global__ void __launch_bounds__(kThreads, 8)
 k_pack_rows_vec(const float* x, int rows, int cols, int ld, uint32_t* out) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the consumer waits before it reads
     pack_rows_vec(x, rows, cols, ld, out);
 }
 __global__ void k_unpack_rows(const uint32_t* in, int rows, int cols, int ld, float* out) {
@@ -109,6 +131,12 @@ __global__ void k_pack_inconv_filter(const float* F, int RS, int O, uint32_t* ou
 __global__ void k_conv_prepare(const uint32_t* fbits, int O, int R, int S, int Cw, int W_in, int KP,
                                uint32_t* wq, uint32_t* ktab, int* pwt, int* pwtot) {
     conv_prepare(fbits, O, R, S, Cw, W_in, KP, wq, ktab, pwt, pwtot);
+}
+
+template <int MT, int NTL>
+__global__ void __launch_bounds__(32 * kSmallMaxWarps, 1) k_gemm_small(GemmArgs g, int KW, int NW) {
+    extern __shared__ __align__(16) int small_red[];
+    gemm_small_block<MT, NTL>(g, KW, NW, small_red);
 }
 
 int launch_check(const char* what) {
@@ -137,6 +165,43 @@ int gemm_splits(int M, int N, int K, int sms) {
     return s < 1 ? 1 : (int)s;
 }
 
+// splits a call without the tcgen05 path uses, given its scratch
+int gemm_use_splits(int M, int N, int K, int sms, size_t workspace_bytes) {
+    const int s = gemm_splits(M, N, K, sms);
+    const long long blocks = (long long)((M + 15) / 16) * ((N + 7) / 8);
+    if (s <= 1 || K < (1 << 17) || blocks >= sms / 4) return 1;
+    return workspace_bytes >= (size_t)s * M * N * sizeof(int32_t) ? s : 1;
+}
+
+// ---- b1 GEMM of small problems (bgemm_small.cuh) -------------------------------------------
+template <int MT, int NTL>
+int launch_gemm_small(const GemmArgs& g, int KW, int NW, cudaStream_t st) {
+    const int ncols = g.mode == GEMM_FC_BITS ? (g.N + 31) & ~31 : g.N;
+    const long long grid = (long long)((g.M + 16 * MT - 1) / (16 * MT)) * ((ncols + 8 * NTL * NW - 1) / (8 * NTL * NW));
+    if (grid >= (1LL << 31)) return fail("gemm: more than 2^31 tiles");
+    const cudaError_t e = launch_dependent(k_gemm_small<MT, NTL>, (unsigned)grid, 32 * KW * NW,
+                                           (size_t)KW * NW * 16 * MT * (8 * NTL + 2) * 4, st, g, KW, NW);
+    if (e != cudaSuccess) return fail("gemm (small): %s", cudaGetErrorString(e));
+    return 0;
+}
+
+// The tile: as large as still leaves every SM two blocks (fewer loads per MMA), but 16 rows where M has
+// no more.  K is cut into as many slices as it has 256-bit steps, up to 8; column groups fill the
+// block up to 8 warps where K is too short for that.  (Long K on few tiles: 16 slices.)
+int run_gemm_small(const GemmArgs& g, int sms, cudaStream_t st) {
+    const int steps = (g.K + 255) / 256;
+    auto tiles = [&](int rows, int cols) { return (long long)((g.M + rows - 1) / rows) * ((g.N + cols - 1) / cols); };
+    int KW = 1;
+    while (KW < 8 && KW < steps) KW *= 2;
+    if (steps >= 64 && tiles(16, 8) * 8 <= 16LL * sms) KW = 16;
+    const int NWmax = 8 / KW > 1 ? 8 / KW : 1;
+    auto groups = [&](int cols) { int nw = 1; while (nw < NWmax && nw * cols < g.N) nw *= 2; return nw; };
+    if (g.M <= 16 || tiles(32, 16) < sms) return launch_gemm_small<1, 1>(g, KW, groups(8), st);
+    if (KW > 8) KW = 8;
+    if (tiles(32, 32) < 2LL * sms) return launch_gemm_small<2, 2>(g, KW, groups(16), st);
+    return launch_gemm_small<2, 4>(g, KW, groups(32), st);
+}
+
 // ---- tcgen05 bit GEMM (bgemm_umma.cuh) -----------------------------------------------------
 long long* g_conv_trace = nullptr;   // device buffer for per-role cycle counters, or null
 int g_gemm_force_pair = -1, g_gemm_force_splits = -1;   // tcbnn_set_gemm_plan: -1 = from the model
@@ -156,16 +221,16 @@ __global__ void __launch_bounds__(umma::kGemmThreads, 1) k_gemm_umma(umma::GemmU
 struct GemmUmmaPlan {
     bool use;
     bool pair;            // 256 x 128 tiles (two sub-tiles of A per CTA) instead of 128 x 128
-    int stages;           // ring depth; fixes the dynamic shared memory and with it the CTAs per SM
     int MT, NT, KB, splits, per;
     size_t off_ea, off_ew, off_partial, bytes;
 };
 
 // Tile shape and split count of the tcgen05 path from a clock model of its launches, calibrated
-// on the kernel's own cycle counters (tcbnn_conv_set_trace): a k-block costs a lone 128 x 128 CTA
-// about 150 clocks, each of two such CTAs sharing an SM 250, a 256 x 128 CTA 180 (the loads, not
-// the MMAs, set the pace); set-up and epilogue cost a CTA 6500, 8000 and 11000 clocks; more than
-// one split adds the finishing launch and the partial sums' round trip.
+// on the kernel's own cycle counters (tcbnn_conv_set_trace): a k-block costs a CTA that owns 128 x 128
+// tiles about 140 clocks (loads and operand reads share the shared-memory port), 256 x 128 tiles 180;
+// set-up, first loads and the last epilogue are paid once per CTA, the 256 x 128 epilogue (one
+// accumulator) once per tile; more than one split adds the finishing launch and the partial sums'
+// round trip.
 GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
     GemmUmmaPlan p = {};
     // below 2^30 multiply-adds the single launch of the warp-level kernel wins (measured; a plan
@@ -184,22 +249,13 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
             const int splits = (p.KB + per - 1) / per;                    // no empty split
             if (splits != want && want > 1) continue;
             if (g_gemm_force_splits > 0 && want != (g_gemm_force_splits < p.KB ? g_gemm_force_splits : p.KB)) continue;
-            const long long ctas = tiles * splits;
-            const bool shared_sm = !pair && ctas > sms;                   // two 128 x 128 CTAs per SM
-            const long long resident = (long long)sms * (shared_sm ? 2 : 1);
-            const long long waves = (ctas + resident - 1) / resident;
-            const double kblock = pair ? 180.0 : (shared_sm ? 250.0 : 150.0);
-            const double fixed = pair ? 11000.0 : (shared_sm ? 8000.0 : 6500.0);
-            double clk = (double)waves * (per * kblock + fixed);
+            const long long waves = (tiles * splits + sms - 1) / sms;
+            double clk = pair ? (double)waves * (per * 180.0 + 3000.0) + 6000.0 : (double)waves * per * 140.0 + 7000.0;
             if (splits > 1) clk += 12000.0 + 6.0 * splits * (double)M * N * 4.0 / 3000.0;
             if (clk < best) { best = clk; p.pair = pair != 0; p.splits = splits; p.per = per; }
         }
     }
     if (p.splits < 1) { p.use = false; return p; }      // a forced plan no slicing of K gives
-    {
-        const long long ctas = (long long)(p.pair ? (p.MT + 1) / 2 : p.MT) * p.NT * p.splits;
-        p.stages = p.pair ? 4 : (ctas > sms ? 3 : 6);
-    }
     size_t o = 0;
     p.off_ea = o;      o += (size_t)p.MT * p.KB * umma::kGemmUnit;  o = (o + 255) & ~(size_t)255;
     p.off_ew = o;      o += (size_t)p.NT * p.KB * umma::kGemmUnit;  o = (o + 255) & ~(size_t)255;
@@ -212,27 +268,26 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, int
     static bool configured[64] = {false};
     if (configure_once(configured, [] {
             cudaError_t e = cudaFuncSetAttribute(k_gemm_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)umma::gemm_smem(true, 4));
+                                                 (int)umma::gemm_smem(true));
             if (e != cudaSuccess) return e;
             return cudaFuncSetAttribute(k_gemm_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)umma::gemm_smem(false, 6));
+                                        (int)umma::gemm_smem(false));
         }))
         return 1;
     char* w = (char*)workspace;
     {
         const long long tasks = (long long)(p.MT + p.NT) * ((p.KB + 3) / 4);   // one CTA per task, up to 8 per SM
         const int grid = (int)(tasks < (long long)sms * 8 ? tasks : (long long)sms * 8);
-        k_expand_rows<<<grid, 256, 0, st>>>(g.A, g.M, g.lda, p.MT, g.W, g.N, g.ldw, p.NT, g.K, p.KB,
-                                            (uint4*)(w + p.off_ea), (uint4*)(w + p.off_ew));
+        const cudaError_t e = launch_dependent(k_expand_rows, grid, 256, 0, st, g.A, g.M, g.lda, p.MT, g.W, g.N, g.ldw, p.NT,
+                                               g.K, p.KB, (uint4*)(w + p.off_ea), (uint4*)(w + p.off_ew));
+        if (e != cudaSuccess) return fail("gemm (operand expansion): %s", cudaGetErrorString(e));
     }
-    if (launch_check("gemm (operand expansion)")) return 1;
     umma::GemmUmmaArgs a;
     a.ea = (const unsigned char*)(w + p.off_ea); a.ew = (const unsigned char*)(w + p.off_ew);
     a.M = g.M; a.N = g.N; a.KB = p.KB; a.MT = p.MT; a.NT = p.NT; a.splits = p.splits; a.per = p.per;
     a.partial = p.splits > 1 ? (int32_t*)(w + p.off_partial) : nullptr;
     a.mode = g.mode; a.out = g.out; a.ldo = g.ldo; a.p0 = g.p0; a.p1 = g.p1;
     a.trace = g_conv_trace;
-    a.nst = p.stages;
     {
         static int* status_addr[64] = {nullptr};
         int dev = 0;
@@ -250,18 +305,10 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, int
     {
         // a programmatic dependent of the expansion launch: set-up (barriers, tensor memory, unit
         // scales) overlaps the expansion pass, the kernel waits for it before its first copy
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)((p.pair ? (p.MT + 1) / 2 : p.MT) * p.NT * p.splits));
-        cfg.blockDim = dim3(umma::kGemmThreads);
-        cfg.dynamicSmemBytes = umma::gemm_smem(p.pair, p.stages);
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e = p.pair ? cudaLaunchKernelEx(&cfg, k_gemm_umma<true>, a)
-                                     : cudaLaunchKernelEx(&cfg, k_gemm_umma<false>, a);
+        const long long tiles = (long long)(p.pair ? (p.MT + 1) / 2 : p.MT) * p.NT * p.splits;
+        const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
+        const cudaError_t e = launch_dependent(p.pair ? k_gemm_umma<true> : k_gemm_umma<false>, grid, umma::kGemmThreads,
+                                               umma::gemm_smem(p.pair), st, a);
         if (e != cudaSuccess) return fail("gemm (tcgen05): %s", cudaGetErrorString(e));
     }
     if (launch_check("gemm (tcgen05)")) return 1;
@@ -288,16 +335,11 @@ int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t s
     const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms);
     if (plan.use && g_gemm_path != 1 && workspace && workspace_bytes >= plan.bytes && ((uintptr_t)workspace & 255) == 0)
         return run_gemm_umma(g, plan, workspace, sms, st);
-    int splits = gemm_splits(g.M, g.N, g.K, sms);
-    const size_t need = (size_t)splits * g.M * g.N * sizeof(int32_t);
-    if (splits > 1 && (workspace == nullptr || workspace_bytes < need)) splits = 1;
+    // Slices of K on different SMs with a finishing launch pay only where K is very long and there is
+    // next to no M x N to spread over the GPU; everything else finishes inside one launch.
+    int splits = gemm_use_splits(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0);
+    if (splits == 1) return run_gemm_small(g, sms, st);
     const long long tiles = (long long)((g.M + 31) / 32) * ((g.N + 31) / 32);
-    if (splits == 1) {
-        g.splits = 1;
-        g.partial = nullptr;
-        k_gemm<<<warp_grid(tiles, sms), kThreads, 0, st>>>(g);
-        return launch_check("gemm");
-    }
     GemmArgs p = g;
     p.mode = GEMM_PARTIAL;
     p.splits = splits;
@@ -1101,8 +1143,7 @@ int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes) {
     if (M <= 0 || N <= 0 || K <= 0 || sm_count(&sms)) return 0;
     const GemmUmmaPlan plan = gemm_umma_plan(M, N, K, sms);
     if (plan.use && g_gemm_path != 1 && workspace_bytes >= plan.bytes) return plan.splits > 1 ? 3 : 2;   // expansion, GEMM, finish
-    const int s = gemm_splits(M, N, K, sms);
-    return (s > 1 && workspace_bytes >= (size_t)s * M * N * sizeof(int32_t)) ? 2 : 1;
+    return gemm_use_splits(M, N, K, sms, workspace_bytes) > 1 ? 2 : 1;
 }
 
 int tcbnn_set_gemm_path(int path) {
