@@ -63,6 +63,9 @@ __host__ __device__ constexpr size_t pre_res_ring_bytes(int nt, int epiw) {
 // raster position (vr, vx) of the OUTPUT grid, so that a filter tap is again a fixed offset.
 __device__ __forceinline__ void expand_raster(const ConvWsArgs& a, uint4* planes, long long plane_positions,
                                               long long front) {
+    // a programmatic dependent of the bits' producer; the convolution that follows is one of this pass
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int NCB = a.C >> 6, Cw = a.C >> 5;
     const int nplane = a.stride == 2 ? 4 : 1;
     const long long total = plane_positions * NCB * nplane;
@@ -146,12 +149,13 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     float* sThrF = reinterpret_cast<float*>(sThr + NT);       // the thresholds as given (fp32)
     uint32_t* sTapK = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(sThrF + NT) + 7) & ~(uintptr_t)7);
     uint64_t* sBar = reinterpret_cast<uint64_t*>(sTapK + 2 * RS);
-    // barriers: a_full[8], a_empty[8], acc_full[8], acc_empty[8], drain, res_full[NG], res_empty[NG]
+    // barriers: a_full[8], a_empty[8], acc_full[8], acc_empty[8], drain, res_full[NG], res_empty[NG], filter
     uint32_t* sTmem = reinterpret_cast<uint32_t*>(sBar + 44);
     volatile int* sAbort = reinterpret_cast<volatile int*>(sTmem + 1);
     const uint32_t bar0 = smem_u32(sBar);
     const uint32_t BAR_DRAIN = bar0 + 8u * 32;         // MMAs still in flight when the issuer gives up
     volatile int* sP0 = reinterpret_cast<volatile int*>(sTmem + 2);      // first pixel in each group's residual buffer
+    const uint32_t BAR_FILTER = bar0 + 8u * 41;        // the filter block has landed
     unsigned char* sRes = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sTmem + 6) + 127) & ~(uintptr_t)127);
     auto BAR_AFULL = [&](int s) { return bar0 + 8u * s; };
     auto BAR_AEMPTY = [&](int s) { return bar0 + 8u * (8 + s); };
@@ -177,20 +181,46 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     const int mtiles = (NV + 127) / 128;
     const int obase = nt * NT;
 
+    // Launched as a programmatic dependent: everything up to griddepcontrol.wait may run while the
+    // launch in front is still running, so it touches nothing but this CTA's own memory.
     if (tid == 0) {
         for (int s = 0; s < 8; s++) { mbar_init(BAR_AFULL(s), 1); mbar_init(BAR_AEMPTY(s), 1); }
         for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), WPG); }
         mbar_init(BAR_DRAIN, 1);
+        mbar_init(BAR_FILTER, 1);
         for (int g = 0; g < NG; g++) { mbar_init(bar0 + 8u * (33 + g), WPG); mbar_init(bar0 + 8u * (37 + g), WPG); }
         *sAbort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MMA_WARP) tmem_alloc(smem_u32(sTmem), TM_COLS);
-    {
-        const uint4* src = a.wf4 + (size_t)nt * RS * (a.C >> 5) * NT;
-        const int nB = RS * (a.C >> 5) * NT;
-        for (int i = tid; i < nB; i += kThreadsCta) sB[i] = __ldg(src + i);
-        for (int i = tid; i < NT; i += kThreadsCta) {
+    for (int t = tid; t < RS; t += kThreadsCta) {
+        // offset of the tap's operand inside a stage, in 16-byte units
+        const int r = t / a.S, sx = t % a.S;
+        if (NPLANE == 4) {
+            const int ty = r - a.pad_h, tx = sx - a.pad_w;
+            const int py = ty & 1, px = tx & 1;
+            const int dy = (ty - py) / 2, dx = (tx - px) / 2;
+            sTapK[t] = (uint32_t)(py * 2 + px) * (plane_bytes >> 4) + (uint32_t)((dy + a.back_y) * a.PW + (dx + a.back_x));
+        } else {
+            sTapK[t] = (uint32_t)(r * a.PW + sx);
+        }
+    }
+    fence_proxy_async();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *sTmem;
+    // Only now that this CTA has its tensor memory may the next launch's CTAs come: one of them could
+    // otherwise take it first and wait for this grid, which would wait for it.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp < 4) tmem_fill_unit_scales(tmem, SF_COL);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid < kEpiThreads) {
+        // thresholds, in the accumulator's column order
+        for (int i = tid; i < NT; i += kEpiThreads) {
             // integer form of  !((float)v < thr)  (kernel.cuh:795-796): v >= ceil(thr)
             int it = INT_MIN;
             float tf = __int_as_float(0x7FC00000);       // NaN: never "less", the bit is always set
@@ -204,28 +234,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             sThr[i] = EPI == kEpiTileRes || EPI == kEpiTilePool ? kF4Bias + min(max(it, -(1 << 23)), 1 << 23) : it;
             sThrF[i] = tf;
         }
-        for (int t = tid; t < RS; t += kThreadsCta) {
-            // offset of the tap's operand inside a stage, in 16-byte units
-            const int r = t / a.S, sx = t % a.S;
-            if (NPLANE == 4) {
-                const int ty = r - a.pad_h, tx = sx - a.pad_w;
-                const int py = ty & 1, px = tx & 1;
-                const int dy = (ty - py) / 2, dx = (tx - px) / 2;
-                sTapK[t] = (uint32_t)(py * 2 + px) * (plane_bytes >> 4) + (uint32_t)((dy + a.back_y) * a.PW + (dx + a.back_x));
-            } else {
-                sTapK[t] = (uint32_t)(r * a.PW + sx);
-            }
-        }
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
     }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *sTmem;
-    if (warp < 4) tmem_fill_unit_scales(tmem, SF_COL);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
     const WsWait wait{sAbort, a.err_flag};
 
     if (warp == LOAD_WARP) {
@@ -236,6 +246,16 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         // per 64-channel block): one lane issuing them all took longer than the stage's MMAs.
         {
             constexpr int kIssueLanes = 8;
+            {
+                // the filter block, in eight pieces (a multiple of 16 bytes each): one trip to L2 for the
+                // issuer instead of one per 16 bytes and thread
+                const uint32_t nB = (uint32_t)(RS * (a.C >> 5) * NT), part = (nB + kIssueLanes - 1) / kIssueLanes;
+                if (lane == 0) mbar_expect_tx(BAR_FILTER, nB * 16u);
+                __syncwarp();
+                const uint32_t first = (uint32_t)lane * part;
+                if (lane < kIssueLanes && first < nB)
+                    bulk_g2s(smem_u32(sB + first), a.wf4 + (size_t)nt * nB + first, min(part, nB - first) * 16u, BAR_FILTER);
+            }
             const long long back = (long long)a.back_y * a.PW + a.back_x;
             const int ncopy = CBS * NPLANE * 2;
             uint32_t it = 0, sph = 0;
@@ -264,6 +284,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                 }
             }
             if (!ok && lane == 0) {
+                for (int i = 0; i < (1 << 20); i++)
+                    if (mbar_try_wait(BAR_FILTER, 0)) break;
                 // giving up: wait (bounded) for the copies still in flight before the CTA exits;
                 // stages below `s` were last filled in this pass over the ring, the others in the one before
                 for (int s2 = 0; s2 < NSTAGE; s2++) {
@@ -313,7 +335,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             // asked while the stage in front was issued (mma_f4_end); waited for only where not yet so
             uint32_t ready = 0, need = 3u;
             const uint32_t tap_end = sTapK[RS - 1];
-            for (uint32_t it = 0; it < nit; it++) {
+            ok = wait(BAR_FILTER, 0);
+            for (uint32_t it = 0; it < nit && ok; it++) {
                 if ((ready & need) != need) {
                     if ((need & 2u) && !(ready & 2u)) {
                         ok = a.trace ? wait.timed(BAR_CEMPTY(b), bph ^ 1, tr_wc) : wait.spin(BAR_CEMPTY(b), bph ^ 1);

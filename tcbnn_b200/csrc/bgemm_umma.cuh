@@ -145,7 +145,6 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         return q;
     };
 
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
         for (int s = 0; s < NST; s++) { mbar_init(BAR_FULL(s), 2); mbar_init(BAR_EMPTY(s), 1); }
         for (int b = 0; b < NACC; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), 8); }
@@ -159,6 +158,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *sTmem;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // (not before the allocation: see bconv_umma_pre.cuh)
     if (warp < 4) tmem_fill_unit_scales(tmem, SF_COL);
     tc_fence_before();
     __syncthreads();

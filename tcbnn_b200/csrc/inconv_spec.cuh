@@ -235,6 +235,8 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
     }   // channel groups
     // two blocks per SM: at most 128 registers per thread (the sums take O of them)
     emit(s, "extern \"C\" __global__ void __launch_bounds__(%d, 2) tcbnn_spec(SpecArgs c) {\n", kSpecThreads);
+    // the layer behind may be set up meanwhile (it waits for this grid before it reads anything)
+    s += " asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
     if (want_u8)
         s += " __shared__ float slut[768];\n"
              " for (int i = threadIdx.x; i < 768; i += blockDim.x) slut[i] = __ldg(c.lut + i);\n"

@@ -599,8 +599,9 @@ int launch_conv_umma_pre_k(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream
             }
         }
     }
-    k_conv_umma_pre<NT, EPI, EPIW><<<(int)grid, umma::pre_threads(EPIW), smem, st>>>(a);
-    return launch_check("conv_layer (tcgen05, pre-expanded input)");
+    const cudaError_t e = launch_dependent(k_conv_umma_pre<NT, EPI, EPIW>, (unsigned)grid, umma::pre_threads(EPIW), smem, st, a);
+    if (e != cudaSuccess) return fail("conv_layer (tcgen05, pre-expanded input): %s", cudaGetErrorString(e));
+    return 0;
 }
 
 // n-tile 64: two CTAs of eight epilogue warps per SM when the filter block and a patch ring of at
@@ -656,9 +657,9 @@ template <int NT>
 int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st, bool expand) {
     if (expand) {
         const long long units = a.pre_positions * (a.C >> 6) * (a.stride == 2 ? 4 : 1);
-        k_expand_raster<<<elementwise_grid(units, sms), 256, 0, st>>>(a, const_cast<uint4*>(a.pre), a.pre_positions,
-                                                                   a.pre_front);
-        if (launch_check("conv_layer (input expansion)")) return 1;
+        const cudaError_t e = launch_dependent(k_expand_raster, (unsigned)elementwise_grid(units, sms), 256, 0, st, a,
+                                               const_cast<uint4*>(a.pre), a.pre_positions, a.pre_front);
+        if (e != cudaSuccess) return fail("conv_layer (input expansion): %s", cudaGetErrorString(e));
     }
     if (!a.res_in && !a.res_out && !a.acc_out) return launch_conv_umma_pre_epi<NT, umma::kEpiTile>(a, smem, sms, st);
     if (!a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked))
@@ -714,6 +715,8 @@ __global__ void __launch_bounds__(256) k_pool_residual16(const uint4* in, uint4*
 // grid, this pass reduces it.
 __global__ void __launch_bounds__(256) k_pool_bits(const uint32_t* in, uint32_t* out, int B, int P, int Q, int Ow,
                                                   long long out_image_stride) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a programmatic dependent, like what follows it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long total = (long long)B * P * Q * Ow;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -1309,8 +1312,10 @@ static int expand_for_next(const tcbnn_conv_desc* next, const uint32_t* bits, co
     umma::fastdiv_setup(a.VH, &a.vh_mul, &a.vh_sh);
     int sms;
     if (sm_count(&sms)) return 1;
-    k_expand_raster<<<elementwise_grid(nx.positions * (next->C >> 6) * nx.nplane, sms), 256, 0, st>>>(a, nx.planes, nx.positions, nx.front);
-    return launch_check("expansion for the next layer");
+    const cudaError_t e = launch_dependent(k_expand_raster, (unsigned)elementwise_grid(nx.positions * (next->C >> 6) * nx.nplane, sms),
+                                           256, 0, st, a, nx.planes, nx.positions, nx.front);
+    if (e != cudaSuccess) return fail("expansion for the next layer: %s", cudaGetErrorString(e));
+    return 0;
 }
 
 static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const void* prepared,
@@ -1453,9 +1458,9 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
       };
       if (launch_tc()) return 1;
       if (pooled) {
-          k_pool_bits<<<elementwise_grid((long long)d->B * d->OH * d->OW * Ow, sms), 256, 0, st>>>(
-              prepool, out, d->B, d->OH, d->OW, Ow, out_image_stride);
-          return launch_check("conv_layer (OR pooling)");
+          const cudaError_t e = launch_dependent(k_pool_bits, (unsigned)elementwise_grid((long long)d->B * d->OH * d->OW * Ow, sms), 256,
+                                                 0, st, prepool, out, d->B, d->OH, d->OW, Ow, out_image_stride);
+          if (e != cudaSuccess) return fail("conv_layer (OR pooling): %s", cudaGetErrorString(e));
       }
       return 0;
     }
