@@ -182,7 +182,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     const int obase = nt * NT;
 
     // Launched as a programmatic dependent: everything up to griddepcontrol.wait may run while the
-    // launch in front is still running, so it touches nothing but this CTA's own memory.
+    // launch in front is still running, so it touches nothing but this CTA's own memory and the filter.
     if (tid == 0) {
         for (int s = 0; s < 8; s++) { mbar_init(BAR_AFULL(s), 1); mbar_init(BAR_AEMPTY(s), 1); }
         for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), WPG); }
@@ -217,6 +217,18 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    constexpr int kIssueLanes = 8;
+    if (warp == LOAD_WARP) {
+        // The filter block, in eight pieces (a multiple of 16 bytes each).  Before the wait: the blob is
+        // written by tcbnn_conv_prepare alone, whose last operation is no kernel, so that nothing behind
+        // it starts before the blob is complete.
+        const uint32_t nB = (uint32_t)(RS * (a.C >> 5) * NT), part = (nB + kIssueLanes - 1) / kIssueLanes;
+        if (lane == 0) mbar_expect_tx(BAR_FILTER, nB * 16u);
+        __syncwarp();
+        const uint32_t first = (uint32_t)lane * part;
+        if (lane < kIssueLanes && first < nB)
+            bulk_g2s(smem_u32(sB + first), a.wf4 + (size_t)nt * nB + first, min(part, nB - first) * 16u, BAR_FILTER);
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid < kEpiThreads) {
         // thresholds, in the accumulator's column order
@@ -245,17 +257,6 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         // size, and a stage of a stride-2 layer is 8 to 32 copies (four parity planes x two chunks
         // per 64-channel block): one lane issuing them all took longer than the stage's MMAs.
         {
-            constexpr int kIssueLanes = 8;
-            {
-                // the filter block, in eight pieces (a multiple of 16 bytes each): one trip to L2 for the
-                // issuer instead of one per 16 bytes and thread
-                const uint32_t nB = (uint32_t)(RS * (a.C >> 5) * NT), part = (nB + kIssueLanes - 1) / kIssueLanes;
-                if (lane == 0) mbar_expect_tx(BAR_FILTER, nB * 16u);
-                __syncwarp();
-                const uint32_t first = (uint32_t)lane * part;
-                if (lane < kIssueLanes && first < nB)
-                    bulk_g2s(smem_u32(sB + first), a.wf4 + (size_t)nt * nB + first, min(part, nB - first) * 16u, BAR_FILTER);
-            }
             const long long back = (long long)a.back_y * a.PW + a.back_x;
             const int ncopy = CBS * NPLANE * 2;
             uint32_t it = 0, sph = 0;

@@ -710,24 +710,35 @@ __global__ void __launch_bounds__(256) k_pool_residual16(const uint4* in, uint4*
     }
 }
 
+// the next layer's input planes, as its descriptor lays them out
+struct NextPlanes { uint4* planes; long long positions, front; int PW, VH, nplane; };
+
 // OR over 2x2 windows of packed output bits [B][2P][2Q][Ow] -> [B][P][Q][Ow] (kernel.cuh:756-770
 // pools by OR-ing the window's bits): the tcgen05 kernels compute a pooled layer on its pre-pool
 // grid, this pass reduces it.
+// With `nx` (planes set) it also writes the pooled output as the next layer's pre-expanded input, which
+// saves that layer's own pass over it.
 __global__ void __launch_bounds__(256) k_pool_bits(const uint32_t* in, uint32_t* out, int B, int P, int Q, int Ow,
-                                                  long long out_image_stride) {
+                                                  long long out_image_stride, NextPlanes nx) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a programmatic dependent, like what follows it
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long total = (long long)B * P * Q * Ow;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
-        const int w = (int)(i % Ow);
-        long long r = i / Ow;
-        const int x = (int)(r % Q); r /= Q;
-        const int y = (int)(r % P);
-        const long long n = r / P;
+        const unsigned long long q = total < (1LL << 32) ? (unsigned)i / (unsigned)Ow : (unsigned long long)i / Ow;
+        const int w = (int)(i - (long long)q * Ow);
+        const unsigned pix = (unsigned)q, row = pix / (unsigned)Q;       // (fewer than 2^31 pixels: conv_check)
+        const int x = (int)(pix - row * Q), y = (int)(row % (unsigned)P);
+        const long long n = row / (unsigned)P;
         const uint32_t* s0 = in + ((n * 2 * P + 2 * y) * 2 * Q + 2 * x) * Ow + w;
         const uint32_t* s1 = s0 + (long long)2 * Q * Ow;
-        out[n * out_image_stride + ((long long)y * Q + x) * Ow + w] = __ldg(s0) | __ldg(s0 + Ow) | __ldg(s1) | __ldg(s1 + Ow);
+        const uint32_t v = __ldg(s0) | __ldg(s0 + Ow) | __ldg(s1) | __ldg(s1 + Ow);
+        out[n * out_image_stride + ((long long)y * Q + x) * Ow + w] = v;
+        if (nx.planes) {
+            const bool par = nx.nplane == 4;               // stride-2 consumer: one plane per row / column parity
+            const int pl = par ? (y & 1) * 2 + (x & 1) : 0, py = par ? y >> 1 : y, px = par ? x >> 1 : x;
+            nx.planes[((size_t)w * nx.nplane + pl) * nx.positions + nx.front + (n * nx.VH + py) * nx.PW + px] = umma::expand32_f4(v);
+        }
     }
 }
 
@@ -1229,7 +1240,6 @@ int tcbnn_conv_prepare(const tcbnn_conv_desc* d, const uint32_t* filter_bits, vo
         filter_bits, d->O, d->R, d->S, (d->C + 31) / 32, d->W, L.KP, (uint32_t*)(p + L.off_wq),
         (uint32_t*)(p + L.off_ktab), (int*)(p + L.off_pwt), (int*)(p + L.off_pwtot));
     if (launch_check("conv_prepare")) return 1;
-    CUDA_TRY(cudaMemsetAsync(p + L.off_err, 0, 256, (cudaStream_t)stream));
     if (L.umma_nt) {
         const long long units = (long long)d->O * d->R * d->S * (d->C / 16);
         k_prepare_filter_ws<<<elementwise_grid(units, sms), 256, 0, (cudaStream_t)stream>>>(
@@ -1248,6 +1258,9 @@ int tcbnn_conv_prepare(const tcbnn_conv_desc* d, const uint32_t* filter_bits, vo
             filter_bits, d->O, d->R * d->S, d->C, umma::kAsNT, (uint4*)(p + L.off_wi8_as));
         if (launch_check("conv_prepare (int8 filter, 128-channel tiles)")) return 1;
     }
+    // last, and no kernel: the convolutions read the blob ahead of their place in the stream (programmatic
+    // launches), which a memset in front of them rules out until the blob is complete
+    CUDA_TRY(cudaMemsetAsync(p + L.off_err, 0, 256, (cudaStream_t)stream));
     return 0;
 }
 
@@ -1281,9 +1294,6 @@ int tcbnn_conv_layer_w(const tcbnn_conv_desc* d, const uint32_t* in, const void*
                               residual_pool, out, out_image_stride, res_out, res_out_bytes, acc_out,
                               workspace, workspace_bytes, 0, nullptr, nullptr, 0, stream);
 }
-
-// the next layer's input planes, as its descriptor lays them out
-struct NextPlanes { uint4* planes; long long positions, front; int PW, VH, nplane; };
 
 // Checks that `next` can take `d`'s output as pre-expanded input and describes its planes.
 static int next_planes_of(const tcbnn_conv_desc* d, int out_h, int out_w, const tcbnn_conv_desc* next,
@@ -1459,7 +1469,8 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
       if (launch_tc()) return 1;
       if (pooled) {
           const cudaError_t e = launch_dependent(k_pool_bits, (unsigned)elementwise_grid((long long)d->B * d->OH * d->OW * Ow, sms), 256,
-                                                 0, st, prepool, out, d->B, d->OH, d->OW, Ow, out_image_stride);
+                                                 0, st, prepool, out, d->B, d->OH, d->OW, Ow, out_image_stride, nx ? *nx : NextPlanes{});
+          if (nx) *fed = true;
           if (e != cudaSuccess) return fail("conv_layer (OR pooling): %s", cudaGetErrorString(e));
       }
       return 0;
@@ -1688,12 +1699,20 @@ int tcbnn_inconv_specialized_layer_x(void* handle, const tcbnn_conv_desc* d, con
         }
     }
     void* params[] = {&c};
-    const unsigned grid = (c.total + spec::kSpecThreads - 1) / spec::kSpecThreads;
+    // Blocks of 64 threads fill the SMs more evenly at the start and the end of the launch (3 x 3 x 128 at
+    // batch 1024 of 32 x 32: 83.9 us against 87.6, one 224 x 224 image through 7 x 7 x 64: 15.3 / 17.0); warps of
+    // a large block stay closer together in the code, which pays once that no longer fits the
+    // instruction cache and the launch is long (7 x 7 x 64 at batch 1024: 543 us at 256 threads, 561 at 64).
+    int spec_sms;
+    if (sm_count(&spec_sms)) return 1;
+    const bool long_code = (size_t)d->R * d->S * (d->O < 64 ? d->O : 64) * 16 > 32 * 1024;
+    const unsigned threads = long_code && c.total > 2u * spec::kSpecThreads * (unsigned)spec_sms ? spec::kSpecThreads : 64u;
+    const unsigned grid = (c.total + threads - 1) / threads;
     // aligned row loads when the geometry allows (stride 4, rows a multiple of 4 pixels, aligned base)
     const bool vec = h->sw == 4 && d->W % 4 == 0 && (x ? ((uintptr_t)x & 15) == 0 : ((uintptr_t)x8 & 3) == 0);
     const int variant = (x ? 0 : 2) + (vec ? 1 : 0);
     if (spec_build(h, variant, false)) return 1;       // first use compiles it (checked under the handle's lock)
-    CUDA_TRY(cudaLaunchKernel((const void*)h->kernel[variant], dim3(grid, (h->O + 63) / 64), dim3(spec::kSpecThreads),
+    CUDA_TRY(cudaLaunchKernel((const void*)h->kernel[variant], dim3(grid, (h->O + 63) / 64), dim3(threads),
                               params, 0, (cudaStream_t)stream));
     if (launch_check("inconv_specialized_layer")) return 1;
     if (expand_after) return expand_for_next(next, out, nx, (cudaStream_t)stream);

@@ -746,7 +746,7 @@ public:
                 if (p->fast_handle && p->fast_next == NULL) { slot = &p->fast_next; pslot = &p->fast_next_planes; bslot = &p->fast_next_planes_bytes; }
             } else if (pr.kind == tcbnn_dropin::kLayerConv) {
                 Conv128LayerParam* p = (Conv128LayerParam*)pr.host;
-                if (p->pool_height == 1 && !p->ahead_fc && p->fast_next == NULL) { slot = &p->fast_next; pslot = &p->fast_next_planes; bslot = &p->fast_next_planes_bytes; }
+                if (!p->ahead_fc && p->fast_next == NULL) { slot = &p->fast_next; pslot = &p->fast_next_planes; bslot = &p->fast_next_planes_bytes; }
             }
             if (slot) {
                 const size_t ws = tcbnn_conv_workspace_bytes(&fast_desc);

@@ -527,7 +527,7 @@ public:
     // this layer also writes its output as the consumer's pre-expanded input
     void hand_over_to(Conv128LayerParam* consumer) {
         const bool dense = out_image_stride == (long long)desc.OH * desc.OW * Ow();
-        if (desc.pool != 1 || !dense) return;
+        if (!dense) return;
         Planes* p = new Planes();
         if (!p->create(&consumer->desc)) { delete p; return; }
         next = &consumer->desc; next_planes = p; consumer->input_planes.reset_to(p);

@@ -273,7 +273,7 @@ class Network:
             kind = type(prod).__name__
             if kind == "Conv128LayerParam":
                 dense = prod.out_image_stride == prod.desc.OH * prod.desc.OW * ((prod.desc.O + 31) // 32)
-                if prod.desc.pool != 1 or not dense:
+                if not dense:
                     continue
             elif kind == "InConv128LayerParam":
                 if getattr(prod, "specialized", None) is None:
