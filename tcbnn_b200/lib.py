@@ -111,7 +111,15 @@ def bound(name):
     return f
 
 
+# process-wide settings: what is recorded of earlier calls (models.Network) does not outlive a change
+_SETTINGS = {"tcbnn_set_conv_path", "tcbnn_set_gemm_path", "tcbnn_set_gemm_plan", "tcbnn_conv_set_trace"}
+settings_generation = 0
+
+
 def call(name, *args):
     """Call an int-returning entry point and raise on a non-zero status."""
+    if name in _SETTINGS:
+        global settings_generation
+        settings_generation += 1
     if (_bound.get(name) or bound(name))(*args) != 0:
         raise TcbnnError(load().tcbnn_last_error().decode())
