@@ -580,15 +580,19 @@ int launch_conv_umma_pre_k(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream
     if (per > mtiles) per = mtiles;
     long long grid = per * a.ntiles_n;
     a.nt_heavy = 0; a.per_heavy = a.per_light = (int)per;
-    if (EPI == umma::kEpiTilePool && g_conv_uneven && a.res_in && a.residual_pool) {
-        // A pooled residual injected into the first channels only (the first block of a stage):
-        // the n-tiles it falls into take about 1.75 times as long per tile as the others when the
-        // tile's own MMAs are few (measured at 14 x 14 x 256: 0.141 ms against 0.081 for the same
-        // layer without pooling), so they get that many more CTAs each.
+    if (EPI != umma::kEpiTile && g_conv_uneven && a.res_in && a.residual_pool) {
+        // A pooled residual injected into the first channels only (the first block of a stage): a tile
+        // of the n-tiles it falls into takes longer than one of the others, the more so the fewer its
+        // own MMAs are, so they get that many more CTAs each.  Measured with weights of 1 / 1.75 / 2.5 / 3.5:
+        // 14 x 14 x 256 at batch 1024, int16: 130 / 106 / 99 / 104 us; 16 x 16 x 256 at batch 201, int32: 80 / 66 /
+        // 63 / 52; 72 MMAs per tile, 8 x 8 x 512, int32, 1 / 1.4 / 1.75 / 2.5: 41 / 37 / 36 / 39 and 7 x 7 x 512, int16: 81 / 89
+        // / 99 / 128.
         const int lim = a.residual_channels < a.res_in_ch ? a.residual_channels : a.res_in_ch;
         const int heavy = (lim + NT - 1) / NT, light = a.ntiles_n - heavy;
-        if (heavy > 0 && light > 0 && (a.C >> 6) * a.R * a.S <= 36) {
-            long long pl = (long long)((double)budget / (1.75 * heavy + light));
+        const bool few = (a.C >> 6) * a.R * a.S <= 36;
+        const double weight = a.res_in_bytes == 4 ? (few ? 3.5 : 1.6) : (few ? 2.5 : 1.0);
+        if (heavy > 0 && light > 0 && weight > 1.0) {
+            long long pl = (long long)((double)budget / (weight * heavy + light));
             if (pl < 1) pl = 1;
             long long ph = (budget - light * pl) / heavy;
             if (ph > mtiles) ph = mtiles;
