@@ -14,6 +14,8 @@ C ABI.  Differences that follow from the B200 design, not from the interface:
     buffers, so a serving loop with a ragged last batch keeps its layer objects (the reference
     fixes the batch at construction, param.h:875-881).
 """
+import copy
+
 import numpy as np
 import torch
 
@@ -93,6 +95,18 @@ class _Layer:
 
     def _call_valid(self, c):
         return True
+
+    def part(self, first, n):
+        """A layer object with this one's weights for n images of the batch, its activations in this
+        one's buffers."""
+        c = copy.copy(self)
+        if hasattr(self, "desc"):
+            c.desc = type(self.desc).from_buffer_copy(self.desc)
+            c.desc.B = n
+        else:
+            c.live = n
+        c._call = None
+        return c
 
 
 class In128LayerParam(_Layer):

@@ -155,6 +155,29 @@ def test_host_feeder_overlapped_copies_give_each_batch_its_own_logits(cuda):
         assert np.array_equal(last.numpy(), expect[-1])
 
 
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("which,parts", [("resnet18", 2), ("resnet18", 5), ("vgg_cifar", 3), ("mlp", 2)])
+def test_host_feeder_computes_the_last_batch_in_parts(cuda, which, parts, graph):
+    """A large last batch is computed part by part (two even parts, a shorter last one, one image each)
+    behind its copy: every batch's logits equal the whole-batch pass's, on two runs of one feeder."""
+    spec = {"resnet18": models.resnet18_spec(5, image=64, classes=100), "vgg_cifar": models.vgg_cifar_spec(7),
+            "mlp": models.mlp_spec(6)}[which]
+    bound = models.SYNTHETIC_IMAGE_ABS_BOUND if which == "resnet18" else None
+    w = models.synthetic_weights(spec, 75)
+    xs = [np.ascontiguousarray(models.synthetic_input(spec, 76 + i)) for i in range(2)]
+    expect = [models.Network(spec, w, x, input_abs_bound=bound).forward().cpu().numpy() for x in xs]
+    feeder = models.HostFeeder(models.Network(spec, w, xs[0], input_abs_bound=bound), graph=graph)
+    feeder.PART_BYTES = xs[0].nbytes // parts
+    assert len(feeder._cuts()) == parts
+    for _ in range(2):
+        got = []
+        last = torch.empty(expect[0].shape, dtype=torch.float32).pin_memory()
+        feeder.run([torch.from_numpy(x).pin_memory() for x in xs], lambda out: got.append(out.clone()), last)
+        torch.cuda.synchronize()
+        assert all(np.array_equal(g.cpu().numpy(), e) for g, e in zip(got, expect))
+        assert np.array_equal(last.numpy(), expect[-1])
+
+
 @pytest.mark.parametrize("which", ["resnet18", "vgg_cifar", "mlp"])
 def test_set_batch_runs_ragged_batches_on_the_same_objects(cuda, which):
     """Layer objects built for 8 images process 5, then 8, then 3 images (Network.set_batch)
