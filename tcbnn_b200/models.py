@@ -404,13 +404,14 @@ class HostFeeder:
     on its own stream while batch i is being computed (two device input buffers).  Every batch
     still pays its own copy; only the waiting is overlapped.
 
-    The last batch has no copy to hide its compute behind, so a large one arrives and is computed in
-    parts: the compute of a part runs while the next one is copied, and only the last part's is left
-    (ResNet-18, three batches of 256 byte images: 2742 us, 2090 of them copies)."""
+    Large batches arrive and are computed in parts: the first compute then waits for a part's copy
+    instead of a batch's, and only a part's compute is left once the last copy is done (ResNet-18, three
+    batches of 256 byte images, 2090 us of copies: 2742 us by whole batches)."""
 
     # A part is worth its own pass when copying it takes longer than the layers' latency, about 150 us
-    # (16 MiB at 55 GB/s: 305); more than eight add passes and no overlap.
-    PART_BYTES, MAX_PARTS = 16 << 20, 8
+    # (16 MiB at 55 GB/s: 305).  At most four: smaller passes fill the GPU less well (128 images of
+    # ResNet-18 take 340 us, 256 take 628), and where the compute is the longer side that counts.
+    PART_BYTES, MAX_PARTS = 16 << 20, 4
 
     def __init__(self, net, graph=True):
         """graph: run each forward pass as a CUDA-graph replay (Network.forward_graph)."""
@@ -424,6 +425,7 @@ class HostFeeder:
         self.read_stream = torch.cuda.Stream()
         self.computed = torch.cuda.Event()
         self.read_done = torch.cuda.Event()
+        self.staged, self.stage_free = [None, None], [torch.cuda.Event(), torch.cuda.Event()]
         self.n = 0
         self.pending = None
         self.part_copied = [[torch.cuda.Event() for _ in range(self.MAX_PARTS)] for _ in range(2)]
@@ -463,15 +465,15 @@ class HostFeeder:
     def run(self, batches, on_result=None, result_host=None):
         """batches: iterable of pinned host tensors; on_result(logits_device) is called after
         each forward pass has been queued.  result_host: pinned host tensor that receives every
-        batch's logits; that device->host read runs on a third stream, beside the next batch's
-        compute and input copy, and the next pass's output layer waits for it."""
+        batch's logits; that device->host read runs on a third stream, from a copy on the device,
+        beside the next batch's compute and input copy."""
         main = torch.cuda.current_stream()
         for ev in self.free:
             ev.record(main)
         self.read_done.record(main)
         it = iter(batches)
         nxt = next(it, None)
-        slot = 0
+        slot = stage = 0
         if nxt is not None:
             self._enqueue_copy(slot, nxt)
         while nxt is not None:
@@ -481,9 +483,8 @@ class HostFeeder:
                 slot ^= 1
                 self._enqueue_copy(slot, nxt)
             self.first.input_gpu = self.bufs[cur_slot]
-            main.wait_event(self.read_done)          # the logits buffer is about to be rewritten
             cuts = self._cuts()
-            if nxt is None and len(cuts) > 1:
+            if len(cuts) > 1:
                 out = self._run_parts(main, cur_slot, cuts)
             else:
                 main.wait_event(self.copied[cur_slot])
@@ -492,9 +493,17 @@ class HostFeeder:
             if on_result is not None:
                 on_result(out)
             if result_host is not None:
+                # (two staging buffers: waiting for the read itself, which shares PCIe with the input
+                # copies, held the next pass back by 65 us at batch 256)
+                if self.staged[stage] is None or self.staged[stage].shape != out.shape:
+                    self.staged[stage] = torch.empty_like(out)
+                main.wait_event(self.stage_free[stage])
+                self.staged[stage].copy_(out)
                 self.computed.record(main)
                 with torch.cuda.stream(self.read_stream):
                     self.read_stream.wait_event(self.computed)
-                    result_host.copy_(out, non_blocking=True)
+                    result_host.copy_(self.staged[stage], non_blocking=True)
+                    self.stage_free[stage].record(self.read_stream)
                     self.read_done.record(self.read_stream)
+                stage ^= 1
         main.wait_event(self.read_done)

@@ -157,9 +157,9 @@ def test_host_feeder_overlapped_copies_give_each_batch_its_own_logits(cuda):
 
 @pytest.mark.parametrize("graph", [False, True])
 @pytest.mark.parametrize("which,parts", [("resnet18", 2), ("resnet18", 5), ("vgg_cifar", 3), ("mlp", 2)])
-def test_host_feeder_computes_the_last_batch_in_parts(cuda, which, parts, graph):
-    """A large last batch is computed part by part (two even parts, a shorter last one, one image each)
-    behind its copy: every batch's logits equal the whole-batch pass's, on two runs of one feeder."""
+def test_host_feeder_computes_large_batches_in_parts(cuda, which, parts, graph):
+    """Large batches are computed part by part (two even parts, a shorter last one, one image each)
+    behind their copies: every batch's logits equal the whole-batch pass's, on two runs of one feeder."""
     spec = {"resnet18": models.resnet18_spec(5, image=64, classes=100), "vgg_cifar": models.vgg_cifar_spec(7),
             "mlp": models.mlp_spec(6)}[which]
     bound = models.SYNTHETIC_IMAGE_ABS_BOUND if which == "resnet18" else None
@@ -168,6 +168,8 @@ def test_host_feeder_computes_the_last_batch_in_parts(cuda, which, parts, graph)
     expect = [models.Network(spec, w, x, input_abs_bound=bound).forward().cpu().numpy() for x in xs]
     feeder = models.HostFeeder(models.Network(spec, w, xs[0], input_abs_bound=bound), graph=graph)
     feeder.PART_BYTES = xs[0].nbytes // parts
+    feeder.MAX_PARTS = 5
+    feeder.part_copied = [[torch.cuda.Event() for _ in range(5)] for _ in range(2)]
     assert len(feeder._cuts()) == parts
     for _ in range(2):
         got = []
