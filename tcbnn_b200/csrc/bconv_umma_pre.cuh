@@ -32,7 +32,8 @@ namespace umma {
 // parity of the phase before last already complete and reads a slot that has not been refilled.)
 constexpr int kPreMmaWarps = 1;
 // EPIW, the kernel's third template argument, is the number of epilogue warps: 16 (one CTA per SM,
-// all of tensor memory) or 8 (n-tile 64 only: each thread then takes 32 columns instead of 16, the
+// all of tensor memory), a single group of 4 or 8 (launches with one tile per CTA, where only latency
+// counts: registers for all of a tile's residual at once, and the epilogue rehearsed) or 8 (n-tile 64 only: each thread then takes 32 columns instead of 16, the
 // CTA allocates half of tensor memory and two CTAs share an SM -- twice the independent
 // loader / issuer / epilogue pipelines, so that one CTA's barrier round trips and epilogue
 // latency are covered by the other's work, and half the per-thread bookkeeping per output).
@@ -121,11 +122,12 @@ constexpr int kEpiTile = 0, kEpiTileRes = 1, kEpiRows2 = 2, kEpiRows4 = 3, kEpiT
 template <int NT, int EPI, int EPIW>
 __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     constexpr int kEpiThreads = EPIW * 32, kThreadsCta = pre_threads(EPIW);
-    static_assert(EPIW == 16 || (EPIW == 8 && NT == 64), "8 epilogue warps: n-tile 64");
     constexpr bool ROWS = EPI == kEpiRows2 || EPI == kEpiRows4;
     constexpr int CPT = NT < 64 ? NT : 64;            // columns of a tile per thread
     constexpr int WPG = 4 * (NT / CPT);               // warps of a group (all rows x all columns of a tile)
     constexpr int NG = EPIW / WPG;                    // groups, each on a tile of its own
+    constexpr bool SINGLE = NG == 1;
+    static_assert(EPIW == 16 || (EPIW == 8 && NT == 64) || (SINGLE && !ROWS), "forms in use");
     // Tensor memory: accumulators (7 at NT = 64) below column 480, the unit block scales of the
     // 4-bit MMA above it; the patch ring is as deep as shared memory allows, so that no role waits
     // on another's latency.
@@ -229,8 +231,16 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         if (lane < kIssueLanes && first < nB)
             bulk_g2s(smem_u32(sB + first), a.wf4 + (size_t)nt * nB + first, min(part, nB - first) * 16u, BAR_FILTER);
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid < kEpiThreads) {
+    // Rehearsal (single-group CTAs): the epilogue runs its loop once without effect (nothing read from or
+    // written to global memory, no barrier touched) before it waits for the launch in front.  Its code
+    // then comes from the instruction cache when it counts: fetching it from L2 as it is first executed
+    // costs a microsecond and more of such a layer's 5 to 9.  `opaque` keeps the compiler from making a
+    // copy of the loop body for it.  (The MMA issuer gains nothing by it; a CTA of several groups loses 7 %
+    // in its residual epilogues to the extra predicates, on a long run of tiles.)
+    auto opaque = [](uint32_t v) { asm volatile("" : "+r"(v)); return v; };
+    // epilogue threads, behind their rehearsal
+    auto epilogue_start = [&]() {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         // thresholds, in the accumulator's column order
         for (int i = tid; i < NT; i += kEpiThreads) {
             // integer form of  !((float)v < thr)  (kernel.cuh:795-796): v >= ceil(thr)
@@ -247,7 +257,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             sThrF[i] = tf;
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-    }
+    };
     const WsWait wait{sAbort, a.err_flag};
 
     if (warp == LOAD_WARP) {
@@ -259,6 +269,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         {
             const long long back = (long long)a.back_y * a.PW + a.back_x;
             const int ncopy = CBS * NPLANE * 2;
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             uint32_t it = 0, sph = 0;
             int s = 0;
             bool ok = true;
@@ -472,17 +483,22 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                          (uint32_t)nl * 16u, bar_rf);
         };
         uint32_t rph = 0;
-        if (ring && mfirst + grp * mstep < mtiles) request(mfirst + grp * mstep);
         static_assert(NG <= NACC, "the accumulator counters below wrap at most once per tile");
         int b = grp;
         uint32_t bph = 0;
-        for (int m = mfirst + grp * mstep; m < mtiles && ok; m += NG * mstep, b += NG) {
+        uint32_t dry = SINGLE ? opaque(1u) : 0u;
+        if (!SINGLE) {
+            epilogue_start();
+            if (ring && mfirst + grp * mstep < mtiles) request(mfirst + grp * mstep);
+        }
+#pragma unroll 1
+        for (int m = mfirst + grp * mstep; (m < mtiles || dry) && ok; m += NG * mstep, b += NG) {
             if (b >= NACC) { b -= NACC; bph ^= 1u; }
             // raster position -> output pixel
             const int p = m * 128 + row;
             bool live = false;
             int n = 0, y = 0, x = 0;
-            if (p < NV) {
+            if (p < NV && !dry) {
                 const int vy = fastdiv(p, a.pw_mul, a.pw_sh);
                 x = p - vy * a.PW;
                 n = fastdiv(vy, a.vh_mul, a.vh_sh);
@@ -492,8 +508,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             const int opix = (n * a.OHg + y) * a.OWg + x;
             // injected residual of step i (16 channels: half i & 1 of pass i >> 1): zeros where nothing
             // is injected; 2x2 max for pooled residuals (kernel.cuh:773-783)
-            uint4 r[2];
-            auto fetch = [&](int i) {
+            uint4 r[SINGLE ? 2 * PASSES : 1][2];
+            auto fetch = [&](int i, uint4 (&r)[2]) {
                 const uint4 z = make_uint4(0u, 0u, 0u, 0u);
                 const size_t i00 = ((size_t)n * 2 * a.OHg + 2 * y) * 2 * a.OWg + 2 * x, rw = (size_t)2 * a.OWg;
 #pragma unroll
@@ -514,11 +530,14 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     }
                 }
             };
-            if (EPI == kEpiTilePool && has_in) fetch(0);          // flies while the accumulator is awaited
-            ok = tr ? wait.relaxed_timed(BAR_CFULL(b), bph, tr_w) : wait.relaxed(BAR_CFULL(b), bph);
+            if (EPI == kEpiTilePool && has_in) {           // flies while the accumulator is awaited
+#pragma unroll
+                for (int i = 0; i < (SINGLE ? 2 * PASSES : 1); i++) fetch(i, r[i]);
+            }
+            if (!dry) ok = tr ? wait.relaxed_timed(BAR_CFULL(b), bph, tr_w) : SINGLE ? wait(BAR_CFULL(b), bph) : wait.relaxed(BAR_CFULL(b), bph);
             if (!ok) break;
-            uint32_t rslot = 0;
-            if (ring) {
+            uint32_t rslot = smem_u32(rbuf);
+            if (ring && !dry) {
                 ok = tr ? wait.relaxed_timed(bar_rf, rph, tr_w) : wait.relaxed(bar_rf, rph);
                 if (!ok) break;
                 rph ^= 1u;
@@ -526,7 +545,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             }
             tc_fence_after();
             int v0[16];                                    // (residual epilogues: the columns on their way)
-#pragma unroll 1
+#pragma unroll (SINGLE ? PASSES : 1)
             for (int k = 0; k < PASSES; k++) {
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + b * NT + (HSTEP * k + half) * 32;
                 uint32_t word = 0;                         // channel c of the pass at bit 31 - c
@@ -537,7 +556,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (k == PASSES - 1) {
                         tc_fence_before();                 // this warp is done with the accumulator
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+                        if (lane == 0 && !dry) mbar_arrive(BAR_CEMPTY(b));
                     }
                     // the reference's comparison as it stands, !((float)value < threshold)
                     // (kernel.cuh:795-796), on the fp32 accumulator
@@ -565,7 +584,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                         const int c0 = (half + HSTEP * k) * 4 + 2 * h;       // first chunk of this step
                         if constexpr (RING) {
                             if (ring) {
-                                if (live) {
+                                if (live || dry) {
 #pragma unroll
                                     for (int j = 0; j < 2; j++) {
                                         if (c0 + j < nchunk) {
@@ -578,8 +597,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                                 }
                                 if (h == 1 && k == PASSES - 1) {         // buffer read: refill it for the group's next tile
                                     __syncwarp();
-                                    if (lane == 0) mbar_arrive(bar_re);
-                                    if (m + NG * mstep < mtiles) {
+                                    if (lane == 0 && !dry) mbar_arrive(bar_re);
+                                    if (m + NG * mstep < mtiles && !dry) {
                                         ok = wait(bar_re, rph ^ 1u);
                                         if (ok) request(m + NG * mstep);
                                     }
@@ -587,8 +606,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                             }
                         } else if (has_in) {
 #pragma unroll
-                            for (int j = 0; j < 2; j++) add8(j, r[j]);
-                            if (2 * k + h + 1 < 2 * PASSES) fetch(2 * k + h + 1);   // flies during this step's arithmetic
+                            for (int j = 0; j < 2; j++) add8(j, r[SINGLE ? 2 * k + h : 0][j]);
+                            if (!SINGLE && 2 * k + h + 1 < 2 * PASSES) fetch(2 * k + h + 1, r[0]);   // flies during this step's arithmetic
                         }
                         const int4* th4 = reinterpret_cast<const int4*>(sThr + (HSTEP * k + half) * 32 + 16 * h);
 #pragma unroll
@@ -599,12 +618,12 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                             if (v[4 * j + 2] >= th.z) word |= 0x80000000u >> (16 * h + f4_channel_of_column(4 * j + 2));
                             if (v[4 * j + 3] >= th.w) word |= 0x80000000u >> (16 * h + f4_channel_of_column(4 * j + 3));
                         }
-                        if (a.res_out && live) {
+                        if (a.res_out && (live || dry)) {
                             if (!a.res_out_proven) {       // a real branch: three instructions per value
                                 uint32_t ovf = 0;          // |v| of every value ORed together
 #pragma unroll
                                 for (int j = 0; j < 16; j++) ovf |= (uint32_t)((v[j] - kF4Bias) ^ ((v[j] - kF4Bias) >> 31));
-                                overflow |= ovf > 32767u;  // some value outside [-32768, 32767]
+                                overflow |= ovf > 32767u && live;  // some value outside [-32768, 32767]
                             }
 #pragma unroll
                             for (int j = 0; j < 2; j++) {
@@ -613,7 +632,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                                 for (int kk = 0; kk < 4; kk++)
                                     w[kk] = __byte_perm((uint32_t)v[f4_column_of_channel(8 * j + 2 * kk)],
                                                         (uint32_t)v[f4_column_of_channel(8 * j + 2 * kk + 1)], 0x5410);
-                                rout[(size_t)(4 * HSTEP * k + 2 * h + j) * a.res_out_npix + opix] = make_uint4(w[0], w[1], w[2], w[3]);
+                                if (live) rout[(size_t)(4 * HSTEP * k + 2 * h + j) * a.res_out_npix + opix] = make_uint4(w[0], w[1], w[2], w[3]);
                             }
                         }
                     };
@@ -626,7 +645,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (k == PASSES - 1) {
                         tc_fence_before();                 // this warp is done with the accumulator
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+                        if (lane == 0 && !dry) mbar_arrive(BAR_CEMPTY(b));
                     } else {
                         tmem_ld16(taddr + HSTEP * 32, v0);
                     }
@@ -637,6 +656,13 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     a.out[(size_t)n * a.out_image_stride + ((size_t)y * a.OWg + x) * Ow + ((o0 + 32 * HSTEP * k) >> 5)] = word;
                     if (a.nxt) store_next_planes(a, n, y, x, o0 + 32 * HSTEP * k, word);
                 }
+            }
+            if (dry) {
+                dry = opaque(0u);
+                epilogue_start();
+                m = mfirst + (grp - NG) * mstep;
+                b = grp - NG;
+                if (ring && m + NG * mstep < mtiles) request(m + NG * mstep);
             }
         }
         if (ring && !ok) {
@@ -673,6 +699,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         const uint32_t tr_t0 = (uint32_t)clock64();
         int b = grp;
         uint32_t bph = 0;
+        epilogue_start();
         for (int m = mfirst + grp * mstep; m < mtiles && ok; m += NG * mstep, b += NG) {
             if (b >= NACC) { b -= NACC; bph ^= 1u; }
             const int p = m * 128 + row;

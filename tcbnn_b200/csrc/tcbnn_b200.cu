@@ -555,7 +555,7 @@ int launch_conv_umma_ws(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t 
 }
 
 template <int NT, int EPI, int EPIW>
-__global__ void __launch_bounds__(umma::pre_threads(EPIW), EPIW == 8 ? 2 : 1) k_conv_umma_pre(umma::ConvWsArgs a) {
+__global__ void __launch_bounds__(umma::pre_threads(EPIW), EPIW == 8 && NT == 64 ? 2 : 1) k_conv_umma_pre(umma::ConvWsArgs a) {
     extern __shared__ __align__(128) unsigned char dyn_smem_pre[];
     umma::conv_umma_pre_cta<NT, EPI, EPIW>(a, dyn_smem_pre);
 }
@@ -569,18 +569,18 @@ int launch_conv_umma_pre_k(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream
     static bool configured[64] = {false};
     if (configure_once(configured, [] {
             return cudaFuncSetAttribute(k_conv_umma_pre<NT, EPI, EPIW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        EPIW == 8 ? 113 * 1024 : 227 * 1024);
+                                        EPIW == 8 && NT == 64 ? 113 * 1024 : 227 * 1024);
         }))
         return 1;
     a.ntiles_n = a.O / NT;
     if (a.ntiles_n > sms) return fail("conv_layer: more n-tiles than SMs");
     const long long mtiles = (a.NV + 127) / 128;
-    const long long budget = (long long)(EPIW == 8 ? 2 : 1) * sms;        // one or two CTAs per SM
+    const long long budget = (long long)(EPIW == 8 && NT == 64 ? 2 : 1) * sms;        // one or two CTAs per SM
     long long per = budget / a.ntiles_n;                                  // CTAs per n-tile
     if (per > mtiles) per = mtiles;
     long long grid = per * a.ntiles_n;
     a.nt_heavy = 0; a.per_heavy = a.per_light = (int)per;
-    if (EPI != umma::kEpiTile && g_conv_uneven && a.res_in && a.residual_pool) {
+    if (EPI != umma::kEpiTile && g_conv_uneven && a.res_in && a.residual_pool && per < mtiles) {
         // A pooled residual injected into the first channels only (the first block of a stage): a tile
         // of the n-tiles it falls into takes longer than one of the others, the more so the fewer its
         // own MMAs are, so they get that many more CTAs each.  Measured with weights of 1 / 1.75 / 2.5 / 3.5:
@@ -665,9 +665,15 @@ int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t
                                                const_cast<uint4*>(a.pre), a.pre_positions, a.pre_front);
         if (e != cudaSuccess) return fail("conv_layer (input expansion): %s", cudaGetErrorString(e));
     }
-    if (!a.res_in && !a.res_out && !a.acc_out) return launch_conv_umma_pre_epi<NT, umma::kEpiTile>(a, smem, sms, st);
-    if (!a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked))
-    {
+    const bool plain = !a.res_in && !a.res_out && !a.acc_out;
+    const bool chunked = !a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked);
+    // A tile per CTA and none to spare: the form for latency (one image through ResNet-18: 135 -> 115 us)
+    constexpr int kSingle = NT == 128 ? 8 : 4;
+    if ((plain || chunked) && (a.NV + 127) / 128 * (a.O / NT) <= sms)
+        return plain ? launch_conv_umma_pre_k<NT, umma::kEpiTile, kSingle>(a, smem, sms, st)
+                     : launch_conv_umma_pre_k<NT, umma::kEpiTilePool, kSingle>(a, smem, sms, st);
+    if (plain) return launch_conv_umma_pre_epi<NT, umma::kEpiTile>(a, smem, sms, st);
+    if (chunked) {
         if (!a.res_in) return launch_conv_umma_pre_epi<NT, umma::kEpiTileRes>(a, smem, sms, st);
         if (!a.residual_pool) {
             bool fits;
