@@ -184,11 +184,12 @@ int tcbnn_conv_layer_x(const tcbnn_conv_desc* d, const uint32_t* in, const void*
  * is eligible, else the warp-level b1 MMA), 1 = always the b1 MMA, 2 = tcgen05 or an error,
  * 3 = as 2 but only the filter-stationary tcgen05 kernel with its in-kernel bit expansion (wide
  * stride-1 layers otherwise take the activation-stationary kernel, narrow ones with a workspace the
- * kernel fed from a pre-expanded input), 6 = as 0 but the loader-fed kernel always runs one CTA per
- * SM (0 runs layers with an n-tile of 64 as two smaller CTAs per SM when they fit), 9 = as 0 but its
+ * kernel fed from a pre-expanded input), 6 = as 0 but the loader-fed kernel always runs one CTA of
+ * 16 epilogue warps per SM (0 runs layers with an n-tile of 64 as two smaller CTAs per SM when they
+ * fit, and launches with a tile per CTA with one epilogue group), 7 = as 0 without the latter, 9 = as 0 but its
  * stages hold one 64-channel block each (0 puts four or two in a stage where three such stages fit),
  * 10 = as 0 but every n-tile of a layer gets the same number of CTAs (0 gives the n-tiles that carry
- * a pooled residual more); 4, 5, 7, 8 = as 0.
+ * a pooled residual more); 4, 5, 8 = as 0.
  * Process-wide; meant for tests and measurements.  No reference counterpart (the reference has one
  * kernel per layer type). */
 int tcbnn_set_conv_path(int path);

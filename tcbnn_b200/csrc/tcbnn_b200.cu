@@ -522,6 +522,7 @@ int launch_inconv_tiled(const InConvArgs& c, size_t smem, int sms, cudaStream_t 
 
 int g_conv_two_ctas = 1;  // loader-fed kernel, n-tile 64: two CTAs of eight epilogue warps per SM when they fit
 int g_conv_cbs = 1;       // loader-fed kernel: four or two 64-channel blocks per stage where they fit
+int g_conv_single = 1;    // loader-fed kernel: single-group CTAs where every tile has one to itself
 int g_conv_uneven = 1;    // loader-fed kernel: more CTAs for the n-tiles that carry a pooled residual
 
 int g_conv_path = 0;     // 0 auto, 1 warp-level b1 MMA, 2 tcgen05 (error if not eligible), 3 = 2 without the activation-stationary kernel
@@ -669,7 +670,7 @@ int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t
     const bool chunked = !a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked);
     // A tile per CTA and none to spare: the form for latency (one image through ResNet-18: 135 -> 115 us)
     constexpr int kSingle = NT == 128 ? 8 : 4;
-    if ((plain || chunked) && (a.NV + 127) / 128 * (a.O / NT) <= sms)
+    if (g_conv_single && (plain || chunked) && (a.NV + 127) / 128 * (a.O / NT) <= sms)
         return plain ? launch_conv_umma_pre_k<NT, umma::kEpiTile, kSingle>(a, smem, sms, st)
                      : launch_conv_umma_pre_k<NT, umma::kEpiTilePool, kSingle>(a, smem, sms, st);
     if (plain) return launch_conv_umma_pre_epi<NT, umma::kEpiTile>(a, smem, sms, st);
@@ -1544,10 +1545,11 @@ int tcbnn_conv_prefers_chunked_residual(const tcbnn_conv_desc* d) {
 int tcbnn_set_conv_path(int path) {
     if (path < 0 || path > 10)
         return fail("set_conv_path: 0 = automatic, 1 = warp-level b1 MMA, 2 = tcgen05, 3 = tcgen05 filter-stationary kernel only, "
-                    "4, 5, 7, 8 = automatic, 6 = automatic, one CTA per SM only, "
+                    "4, 5, 8 = automatic, 6 = automatic, one CTA of 16 epilogue warps per SM only, 7 = automatic without single-group CTAs, "
                     "9 = automatic, one 64-channel block per stage, 10 = automatic, every n-tile the same number of CTAs");
     g_conv_path = path >= 4 ? 0 : path;
     g_conv_two_ctas = path == 6 ? 0 : 1;
+    g_conv_single = path == 6 || path == 7 ? 0 : 1;
     g_conv_cbs = path == 9 ? 0 : 1;
     g_conv_uneven = path == 10 ? 0 : 1;
     return 0;

@@ -364,8 +364,9 @@ def gemm_status():
 
 def set_conv_path(path):
     """0 = automatic, 1 = warp-level b1 MMA, 2 = tcgen05 (error when a layer is not eligible),
-    3 = tcgen05 without the activation-stationary kernel, 6 = one CTA per SM only, 9 = one 64-channel
-    block per stage, 10 = every n-tile the same number of CTAs; 4, 5, 7, 8 = automatic
+    3 = tcgen05 without the activation-stationary kernel, 6 = one CTA of 16 epilogue warps per SM only,
+    7 = without single-group CTAs, 9 = one 64-channel block per stage, 10 = every n-tile the same
+    number of CTAs; 4, 5, 8 = automatic
     (tcbnn_set_conv_path)."""
     _l.call("tcbnn_set_conv_path", int(path))
 

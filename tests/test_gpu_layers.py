@@ -644,6 +644,35 @@ def test_conv_layer_reports_int16_overflow_on_tile_epilogue(cuda):
     assert ops.conv_status(d, prep) == 0          # reading clears it
 
 
+@pytest.mark.parametrize("C,O,stride,mode", [(64, 32, 1, "plain"), (64, 64, 1, "pool"), (128, 128, 2, "none"), (128, 256, 1, "pool")])
+@pytest.mark.parametrize("more", [0, 1])
+def test_conv_layer_one_tile_per_cta_and_one_more(cuda, C, O, stride, mode, more):
+    """The last size whose tiles all have a CTA of their own, and the first that has a tile too many:
+    output bits and chunk-major int16 residuals against the oracle."""
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    ntiles = max(1, O // 128) if C > 64 else O // min(O, 128)
+    P = 7                                                     # raster of 8 x 8 positions per image
+    B = sms // ntiles * 128 // 64 + more
+    H = P * stride
+    g = util.rng(C + O + stride + more)
+    x, f = util.rand_words(g, (B, H, H, C // 32)), util.rand_words(g, (O, 9, C // 32))
+    thr = (g.standard_normal(O) * np.sqrt(C * 9) * 0.5).astype(np.float32)
+    res_in = {"none": None, "plain": (B, P, P, O), "pool": (B, 2 * P, 2 * P, O // 2)}[mode]
+    if res_in is not None:
+        res_in = g.integers(-300, 300, size=res_in).astype(np.int32)
+    rc = res_in.shape[-1] if res_in is not None else 0
+    eo, er, _ = orc.conv_layer(x, f, thr, C, 3, 3, stride, stride, True, 1, res_in=res_in, residual_channels=rc,
+                               residual_pool=mode == "pool", save_residual=True)
+    d = ops.conv_desc(B, H, H, C, O, 3, 3, stride, stride)
+    prep = ops.conv_prepare(d, dev(f, cuda))
+    r16 = ops.nhwc_to_chunked(dev(res_in.astype(np.int16), cuda)) if res_in is not None else None
+    go, gr, _ = ops.conv_layer(d, dev(x, cuda), prep, dev(thr, cuda), res_in=r16, residual_channels=rc,
+                               residual_pool=mode == "pool", save_residual=True, residual_dtype=torch.int16,
+                               res_in_chunked=r16 is not None, res_out_chunked=True)
+    assert np.array_equal(ops.chunked_to_nhwc(gr).cpu().numpy().astype(np.int32), er)
+    assert np.array_equal(host_u32(go), eo) and ops.conv_status(d, prep) == 0
+
+
 def test_specialized_first_layer_writes_chunked_residual(cuda):
     g = util.rng(123)
     B, H = 3, 36
