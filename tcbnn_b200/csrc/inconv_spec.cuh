@@ -49,15 +49,22 @@ struct SpecArgs {
     int res_out_chunked;      // int16 residual laid out [channel chunk of 8][pixel][8] instead of NHWC
 };
 
-// One kernel per (input type, load style), compiled when first used: a 7x7x64 kernel takes
-// 1.5 - 4 s to compile and most callers only ever use one of the four.
+// One kernel per form of call -- input type, load style, residual format, accumulators -- compiled when
+// first used: a 7x7x64 kernel takes 0.7 - 1.5 s to compile, half as much again with every output's code
+// in it, and most callers only ever use one.
+constexpr int kResNone = 0, kResChunked = 1, kResInt16 = 2, kResInt32 = 3;
+constexpr int kSpecVariants = 64;
+// vec: aligned row loads; res_vec: the residual tensor is 16-byte aligned with rows in multiples of that
+inline int spec_variant(bool u8, bool vec, int res, bool acc, bool res_vec) {
+    return (vec ? 1 : 0) | (u8 ? 2 : 0) | (res << 2) | (acc ? 16 : 0) | (res_vec && res ? 32 : 0);
+}
 struct SpecHandle {
     int O, R, S, sh, sw, pad_h, pad_w, pool;
     std::vector<unsigned char> codes;
     std::vector<uint32_t> thr_bits;
     std::mutex mu;
-    cudaLibrary_t lib[4] = {nullptr, nullptr, nullptr, nullptr};       // index = u8 * 2 + vec
-    cudaKernel_t kernel[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaLibrary_t lib[kSpecVariants] = {};             // by spec_variant
+    cudaKernel_t kernel[kSpecVariants] = {};
 };
 
 inline void emit(std::string& s, const char* fmt, ...) {
@@ -70,10 +77,11 @@ inline void emit(std::string& s, const char* fmt, ...) {
 }
 
 // codes[tap][o] = b0<<2 | b1<<1 | b2 (bit 1 = '+'), thr_bits[o] = the threshold's bit pattern
-// variant = u8 * 2 + vec: which of the four kernels the source defines (entry point tcbnn_spec)
+// variant: which of the handle's kernels the source defines (spec_variant; entry point tcbnn_spec)
 inline std::string generate_source(const SpecHandle& h, const std::vector<unsigned char>& codes,
                                    const std::vector<uint32_t>& thr_bits, int variant) {
-    const bool want_u8 = (variant & 2) != 0, want_vec = (variant & 1) != 0;
+    const bool want_u8 = (variant & 2) != 0, want_vec = (variant & 1) != 0, want_acc = (variant & 16) != 0, res_vec = (variant & 32) != 0;
+    const int res = (variant >> 2) & 3;
     // Output channels are handled 64 at a time: blockIdx.y picks the group (its own code path).
     const int Oall = h.O, RS = h.R * h.S, OwAll = (Oall + 31) / 32, nhalf = (Oall + 63) / 64;
     std::string s;
@@ -198,65 +206,59 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
         emit(s, "       pl[(size_t)%d * c.nxt_positions] = expand32_f4(w%d);\n", OB / 32 + k, k);
     s += "     }\n   } }\n";
     // residual = (int)acc (kernel.cuh:666-668), optional fp32 accumulators
-    s += " const size_t opix = ((size_t)n * P + y) * Q + x;\n"
-         " if (c.res_out) {\n"
-         "  if (c.res_out_bytes == 2) {\n"
-         "   short* r = reinterpret_cast<short*>(c.res_out) + opix * c.res_out_ld + OBASE;\n";
-    if (O % 8 == 0) {
+    if (res || want_acc) s += " const size_t opix = ((size_t)n * P + y) * Q + x;\n";
+    auto pack16 = [&](int j) {                              // channels 8j .. 8j + 7 as int16
+        s += "make_uint4(";
+        for (int k = 0; k < 4; k++)
+            emit(s, "((uint32_t)(int)a%d & 0xFFFFu) | ((uint32_t)(int)a%d << 16)%s", 8 * j + 2 * k, 8 * j + 2 * k + 1, k < 3 ? ", " : ");\n");
+    };
+    if (res == kResChunked) {
         // chunk-major layout [channel chunk of 8][pixel][8]: consecutive threads (pixels) store
         // consecutive 16 bytes, whole lines per warp
-        emit(s, "   if (c.res_out_chunked) {\n    uint4* d4 = reinterpret_cast<uint4*>(c.res_out) + (size_t)%d * c.total + opix;\n", OB / 8);
-        for (int j = 0; j < O / 8; j++) {
-            emit(s, "    d4[(size_t)%d * c.total] = make_uint4(", j);
-            for (int k = 0; k < 4; k++)
-                emit(s, "((uint32_t)(int)a%d & 0xFFFFu) | ((uint32_t)(int)a%d << 16)%s", 8 * j + 2 * k, 8 * j + 2 * k + 1,
-                     k < 3 ? ", " : ");\n");
+        emit(s, " uint4* d4 = reinterpret_cast<uint4*>(c.res_out) + (size_t)%d * c.total + opix;\n", OB / 8);
+        for (int j = 0; j < O / 8; j++) { emit(s, " d4[(size_t)%d * c.total] = ", j); pack16(j); }
+    } else if (res == kResInt16) {
+        s += " short* r = reinterpret_cast<short*>(c.res_out) + opix * c.res_out_ld + OBASE;\n";
+        if (res_vec && O % 8 == 0) {
+            s += " uint4* d4 = reinterpret_cast<uint4*>(r);\n";
+            for (int j = 0; j < O / 8; j++) { emit(s, " d4[%d] = ", j); pack16(j); }
+        } else {
+            for (int o = 0; o < O; o++) emit(s, " r[%d] = (short)(int)a%d;\n", o, o);
         }
-        s += "   } else\n";
-        s += "   if ((c.res_out_ld & 7) == 0 && (reinterpret_cast<size_t>(c.res_out) & 15) == 0) {\n"
-             "    uint4* d4 = reinterpret_cast<uint4*>(r);\n";
-        for (int j = 0; j < O / 8; j++) {
-            emit(s, "    d4[%d] = make_uint4(", j);
-            for (int k = 0; k < 4; k++)
-                emit(s, "((uint32_t)(int)a%d & 0xFFFFu) | ((uint32_t)(int)a%d << 16)%s", 8 * j + 2 * k, 8 * j + 2 * k + 1,
-                     k < 3 ? ", " : ");\n");
-        }
-        s += "   } else\n";
-    }
-    s += "   {\n";
-    for (int o = 0; o < O; o++) emit(s, "    r[%d] = (short)(int)a%d;\n", o, o);
-    s += "   }\n  } else {\n   int* r = reinterpret_cast<int*>(c.res_out) + opix * c.res_out_ld + OBASE;\n";
-    if (O % 16 == 0) {
-        // A warp's 16-byte pieces of 32 different rows take L1 a cycle per row (3 x 3 x 128 at batch 1024:
-        // 213 us with the int32 residual, 76 without).  Quads of lanes exchange their pieces first, so
-        // that a store covers 64 consecutive bytes of each row.  Full warps only.
-        s += "   if ((c.res_out_ld & 3) == 0 && (reinterpret_cast<size_t>(c.res_out) & 15) == 0 && __activemask() == 0xffffffffu) {\n"
-             "    const unsigned l = threadIdx.x & 3u; const unsigned lane0 = threadIdx.x & 28u; int* p4[4];\n"
-             "    for (int k = 0; k < 4; k++) p4[k] = reinterpret_cast<int*>(c.res_out) + (size_t)__shfl_sync(0xffffffffu, (unsigned)opix, lane0 + k) * c.res_out_ld + OBASE + 4 * l;\n";
-        for (int g = 0; g < O / 16; g++) {
-            s += "    { int4 q[4] = {";
-            for (int k = 0; k < 4; k++) {
-                const int o = 16 * g + 4 * k;
-                emit(s, "make_int4((int)a%d, (int)a%d, (int)a%d, (int)a%d)%s", o, o + 1, o + 2, o + 3, k < 3 ? ", " : "};\n");
+    } else if (res == kResInt32) {
+        s += " int* r = reinterpret_cast<int*>(c.res_out) + opix * c.res_out_ld + OBASE;\n";
+        if (res_vec && O % 16 == 0) {
+            // A warp's 16-byte pieces of 32 different rows take L1 a cycle per row (3 x 3 x 128 at batch
+            // 1024: 213 us with the int32 residual, 76 without).  Quads of lanes exchange their pieces
+            // first, so that a store covers 64 consecutive bytes of each row.  Full warps only.
+            s += " if (__activemask() == 0xffffffffu) {\n"
+                 "  const unsigned l = threadIdx.x & 3u; const unsigned lane0 = threadIdx.x & 28u; int* p4[4];\n"
+                 "  for (int k = 0; k < 4; k++) p4[k] = reinterpret_cast<int*>(c.res_out) + (size_t)__shfl_sync(0xffffffffu, (unsigned)opix, lane0 + k) * c.res_out_ld + OBASE + 4 * l;\n";
+            for (int g = 0; g < O / 16; g++) {
+                s += "  { int4 q[4] = {";
+                for (int k = 0; k < 4; k++) {
+                    const int o = 16 * g + 4 * k;
+                    emit(s, "make_int4((int)a%d, (int)a%d, (int)a%d, (int)a%d)%s", o, o + 1, o + 2, o + 3, k < 3 ? ", " : "};\n");
+                }
+                emit(s, "   quad_transpose(q, l); for (int k = 0; k < 4; k++) *reinterpret_cast<int4*>(p4[k] + %d) = q[k]; }\n", 16 * g);
             }
-            emit(s, "     quad_transpose(q, l); for (int k = 0; k < 4; k++) *reinterpret_cast<int4*>(p4[k] + %d) = q[k]; }\n", 16 * g);
+            s += " } else\n";
         }
-        s += "   } else\n";
+        s += " {\n";
+        if (res_vec && O % 4 == 0) {
+            s += "  int4* d4 = reinterpret_cast<int4*>(r);\n";
+            for (int j = 0; j < O / 4; j++)
+                emit(s, "  d4[%d] = make_int4((int)a%d, (int)a%d, (int)a%d, (int)a%d);\n", j, 4 * j, 4 * j + 1, 4 * j + 2, 4 * j + 3);
+        } else {
+            for (int o = 0; o < O; o++) emit(s, "  r[%d] = (int)a%d;\n", o, o);
+        }
+        s += " }\n";
     }
-    if (O % 4 == 0) {
-        s += "   if ((c.res_out_ld & 3) == 0 && (reinterpret_cast<size_t>(c.res_out) & 15) == 0) {\n"
-             "    int4* d4 = reinterpret_cast<int4*>(r);\n";
-        for (int j = 0; j < O / 4; j++)
-            emit(s, "    d4[%d] = make_int4((int)a%d, (int)a%d, (int)a%d, (int)a%d);\n", j, 4 * j, 4 * j + 1, 4 * j + 2, 4 * j + 3);
-        s += "   } else\n";
+    if (want_acc) {
+        emit(s, " float* q = c.acc_out + opix * %d + OBASE;\n", Oall);
+        for (int o = 0; o < O; o++) emit(s, " q[%d] = a%d;\n", o, o);
     }
-    s += "   {\n";
-    for (int o = 0; o < O; o++) emit(s, "    r[%d] = (int)a%d;\n", o, o);
-    s += "   }\n";
-    s += "  }\n }\n if (c.acc_out) {\n";
-    emit(s, "  float* q = c.acc_out + opix * %d + OBASE;\n", Oall);
-    for (int o = 0; o < O; o++) emit(s, "  q[%d] = a%d;\n", o, o);
-    s += " }\n}\n";
+    s += "}\n";
     }   // channel groups
     // two blocks per SM: at most 128 registers per thread (the sums take O of them)
     emit(s, "extern \"C\" __global__ void __launch_bounds__(%d, 2) tcbnn_spec(SpecArgs c) {\n", kSpecThreads);

@@ -1617,7 +1617,7 @@ int tcbnn_inconv_layer_u8(const tcbnn_conv_desc* d, const uint8_t* x, const floa
 }
 
 // ---- first layer specialised to one filter (run-time compiled) -----------------------------
-// Compiles (and loads, unless only_compile) one variant of the handle's kernel; variant = u8 * 2 + vec.
+// Compiles (and loads, unless only_compile) one variant of the handle's kernel (spec::spec_variant).
 static int spec_build(spec::SpecHandle* h, int variant, bool only_compile) {
     std::lock_guard<std::mutex> lock(h->mu);
     if (h->kernel[variant]) return 0;
@@ -1722,7 +1722,9 @@ int tcbnn_inconv_specialized_layer_x(void* handle, const tcbnn_conv_desc* d, con
     const unsigned grid = (c.total + threads - 1) / threads;
     // aligned row loads when the geometry allows (stride 4, rows a multiple of 4 pixels, aligned base)
     const bool vec = h->sw == 4 && d->W % 4 == 0 && (x ? ((uintptr_t)x & 15) == 0 : ((uintptr_t)x8 & 3) == 0);
-    const int variant = (x ? 0 : 2) + (vec ? 1 : 0);
+    const int res = !res_out ? spec::kResNone : res_out_chunked ? spec::kResChunked : res_out_bytes == 2 ? spec::kResInt16 : spec::kResInt32;
+    const bool res_vec = ((uintptr_t)res_out & 15) == 0 && d->O * res_out_bytes % 16 == 0;
+    const int variant = spec::spec_variant(x == nullptr, vec, res, acc_out != nullptr, res_vec);
     if (spec_build(h, variant, false)) return 1;       // first use compiles it (checked under the handle's lock)
     CUDA_TRY(cudaLaunchKernel((const void*)h->kernel[variant], dim3(grid, (h->O + 63) / 64), dim3(threads),
                               params, 0, (cudaStream_t)stream));
@@ -1734,7 +1736,7 @@ int tcbnn_inconv_specialized_layer_x(void* handle, const tcbnn_conv_desc* d, con
 int tcbnn_inconv_release(void* handle) {
     if (!handle) return 0;
     spec::SpecHandle* h = (spec::SpecHandle*)handle;
-    for (int v = 0; v < 4; v++)
+    for (int v = 0; v < spec::kSpecVariants; v++)
         if (h->lib[v]) cudaLibraryUnload(h->lib[v]);
     delete h;
     return 0;
@@ -1752,7 +1754,8 @@ int tcbnn_inconv_specialize_selftest(const tcbnn_conv_desc* d, unsigned seed, lo
     for (auto& c : h.codes) { s = s * 1664525u + 1013904223u; c = (unsigned char)((s >> 24) & 7u); }
     for (auto& t : h.thr_bits) { s = s * 1664525u + 1013904223u; t = 0x40000000u ^ (s & 0x807FFFFFu); }
     // the uint8 variant with row loads where the stride allows them, the plain fp32 one otherwise
-    const int variant = d->stride_w == 4 ? 3 : 0;
+    const int variant = d->stride_w == 4 ? spec::spec_variant(true, true, spec::kResInt16, false, d->O % 8 == 0)
+                                         : spec::spec_variant(false, false, spec::kResInt32, true, d->O % 4 == 0);
     if (source_bytes) *source_bytes = (long long)spec::generate_source(h, h.codes, h.thr_bits, variant).size();
     return spec_build(&h, variant, true);
 }
