@@ -363,7 +363,10 @@ class Network:
         graph = torch.cuda.CUDAGraph()
         try:
             with torch.cuda.stream(torch.cuda.Stream()):
-                # thread_local: other threads' calls are left alone, as in forward_graph()
+                # thread_local: only this thread's calls are checked during the capture; another
+                # thread (e.g. a communicator's watchdog polling its events) is left alone.  (Not
+                # torch.cuda.graph: it collects garbage and empties the allocator's cache first, 50 to
+                # 100 ms per graph, and the launches allocate nothing.)
                 graph.capture_begin(capture_error_mode="thread_local")
                 try:
                     for l in self.layers:
@@ -388,12 +391,9 @@ class Network:
             for l in self.layers:
                 l.forward()
             torch.cuda.synchronize()
-            g = torch.cuda.CUDAGraph()
-            # thread_local: only this thread's calls are checked during the capture; another
-            # thread (e.g. a communicator's watchdog polling its events) is left alone
-            with torch.cuda.graph(g, capture_error_mode="thread_local"):
-                for l in self.layers:
-                    l.forward()
+            g = self._record()
+            if g is None:
+                raise lib.TcbnnError("the layers' launches could not be recorded as a graph on this stream")
             graphs[key] = g
         g.replay()
         return self.layers[-1].get_output_gpu()
