@@ -79,6 +79,21 @@ int tcbnn_bgemm(const uint32_t* A, const uint32_t* B, int M, int N, int K, int l
 int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
                    int lda, int ldw, uint32_t* out, int ldo, void* workspace,
                    size_t workspace_bytes, void* stream);
+/* The same with operands in the tcgen05 GEMM's own form ("units": +-1 4-bit values in 4 KB blocks), for
+ * chains of FC layers.  tcbnn_fc_units_bytes(M, N, K, rows) is the size of `rows` rows of K for a layer of
+ * that shape, 0 where the layer does not run on that kernel.  w_units: the layer's weight, expanded once
+ * by tcbnn_fc_expand_weight; a_units: its input, written by the producer; next_units: the output
+ * bits also go there, as the next layer's a_units (K = N here).  tcbnn_pack_rows_x writes the first
+ * layer's.  Buffers are 256-byte aligned and zeroed by the caller once; A, W and out are as above, and are
+ * what a call uses whose shape takes another kernel.  Any of the three may be NULL.  No reference
+ * counterpart. */
+size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows);
+int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units, void* stream);
+int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
+                     int lda, int ldw, uint32_t* out, int ldo, void* workspace, size_t workspace_bytes,
+                     const void* a_units, const void* w_units, void* next_units, void* stream);
+int tcbnn_pack_rows_x(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
+                      void* stream);
 /* Output layer: out[m][n] = fma((float)(K - 2*popc), scale[n], bias[n]), fp32 [M][ldo].
  * Out128LayerFMT, kernel.cuh:230-280. */
 int tcbnn_out_layer(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,

@@ -51,6 +51,7 @@ struct GemmUmmaArgs {
     int32_t* partial;          // [splits][M][N], used when splits > 1
     // splits == 1: the layer is finished in the epilogue (GemmMode of bnn_layers.cuh)
     int mode; void* out; int ldo; const float* p0; const float* p1;
+    uint4* nxt; int nxt_KB;    // threshold bits also as the next layer's expanded A operand, or null
     int* status;               // set to 1 when a bounded wait gives up
     long long* trace;          // null, or 16 counters: CTA 0 writes [9..15] (clocks; see the C header)
 };
@@ -59,6 +60,14 @@ struct GemmUmmaArgs {
 __device__ __forceinline__ uint4 keep32_f4(uint4 e, uint32_t m) {
     return make_uint4(e.x & (((m >> 3) & 0x11111111u) * 0xFu), e.y & (((m >> 2) & 0x11111111u) * 0xFu),
                       e.z & (((m >> 1) & 0x11111111u) * 0xFu), e.w & ((m & 0x11111111u) * 0xFu));
+}
+
+// Chunk c (32 bits of K) of row r of an expanded operand with KB k-blocks; `valid` elements exist, the rest
+// is padding: 0, not -1.
+__device__ __forceinline__ void store_unit_chunk(uint4* units, int KB, int r, int c, uint32_t word, int valid) {
+    uint4 e = expand32_f4(word);
+    if (valid < 32) e = keep32_f4(e, 0xFFFFFFFFu << (32 - valid));
+    units[((size_t)(r >> 7) * KB + (c >> 1)) * 256 + (c & 1) * 128 + (r & 127)] = e;
 }
 
 // packed bits [rows][ld words] (bit k of a row at bit 31 - k%32 of word k/32) -> units; one launch
@@ -348,7 +357,10 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                             if (__int_as_float(v[4 * j + 2]) >= th.z) word |= 0x80000000u >> f4_channel_of_column(4 * j + 2);
                             if (__int_as_float(v[4 * j + 3]) >= th.w) word |= 0x80000000u >> f4_channel_of_column(4 * j + 3);
                         }
-                        if (m < g.M) reinterpret_cast<uint32_t*>(g.out)[(size_t)m * g.ldo + (n0 >> 5)] = word;
+                        if (m < g.M) {
+                            reinterpret_cast<uint32_t*>(g.out)[(size_t)m * g.ldo + (n0 >> 5)] = word;
+                            if (g.nxt) store_unit_chunk(g.nxt, g.nxt_KB, m, n0 >> 5, word, g.N - n0);
+                        }
                     }
                 } else {
                     // int32 sums (the split-K partials, or C itself), or scale and bias (kernel.cuh:270-273,

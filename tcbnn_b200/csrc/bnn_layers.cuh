@@ -486,8 +486,10 @@ __device__ __forceinline__ uint32_t spread4(uint32_t b) {
 // used -- with 64 warps per SM that keeps up to 256 KB in flight.  Four ballots give one bit per
 // (lane, component); lane L interleaves eight lanes' four bits into word L & 3 of block L >> 2.
 // rows * ceil(blocks / 8) must fit in 31 bits (the caller checks).
+// also(row, chunk, word): what else becomes of each word that holds columns.
+template <class F>
 __device__ __forceinline__ void pack_rows_vec(const float* x, int rows, int cols, int ld_words,
-                                              uint32_t* out) {
+                                              uint32_t* out, F&& also) {
     constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const unsigned blocks = (unsigned)ld_words >> 2, chunks = (blocks + U - 1) / U;
@@ -513,7 +515,10 @@ __device__ __forceinline__ void pack_rows_vec(const float* x, int rows, int cols
         const int sh = 8 * (lane & 3);
         const uint32_t v = spread4(m0 >> sh) | (spread4(m1 >> sh) << 1) | (spread4(m2 >> sh) << 2) |
                            (spread4(m3 >> sh) << 3);           // column k of the word at bit k
-        if (blk0 + myu < blocks) out[(size_t)row * ld_words + blk0 * 4 + lane] = __brev(v);   // 128 contiguous bytes
+        if (blk0 + myu < blocks) {
+            out[(size_t)row * ld_words + blk0 * 4 + lane] = __brev(v);       // 128 contiguous bytes
+            if ((int)(blk0 * 4 + lane) * 32 < cols) also((int)row, (int)blk0 * 4 + lane, __brev(v));
+        }
     }
 }
 

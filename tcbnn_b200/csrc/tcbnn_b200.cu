@@ -112,9 +112,12 @@ k_pack_rows(const float* x, int rows, int cols, int ld, uint32_t* out) {
     pack_rows(x, rows, cols, ld, out);
 }
 __global__ void __launch_bounds__(kThreads, 8)
-k_pack_rows_vec(const float* x, int rows, int cols, int ld, uint32_t* out) {
+k_pack_rows_vec(const float* x, int rows, int cols, int ld, uint32_t* out, uint4* units) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the consumer waits before it reads
-    pack_rows_vec(x, rows, cols, ld, out);
+    pack_rows_vec(x, rows, cols, ld, out, [&](int row, int c, uint32_t word) {
+        // the FC layer behind takes its operand expanded (bgemm_umma.cuh)
+        if (units) umma::store_unit_chunk(units, (cols + 63) >> 6, row, c, word, cols - c * 32);
+    });
 }
 __global__ void k_unpack_rows(const uint32_t* in, int rows, int cols, int ld, float* out) {
     unpack_rows(in, rows, cols, ld, out);
@@ -264,7 +267,21 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
     return p;
 }
 
-int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, int sms, cudaStream_t st) {
+// Operands that are expanded already, and where the threshold bits go expanded (tcbnn_fc_layer_x)
+struct GemmUnits { const void* a; const void* w; void* next; };
+
+// packed rows -> units, for either operand (null units: not that one)
+int expand_units(const uint32_t* a_bits, int M, int lda, void* a_units, const uint32_t* w_bits, int N, int ldw, void* w_units, int K,
+                 int sms, cudaStream_t st) {
+    const int KB = (K + 63) / 64, RTa = a_units ? (M + 127) / 128 : 0, RTw = w_units ? (N + 127) / 128 : 0;
+    const long long tasks = (long long)(RTa + RTw) * ((KB + 3) / 4);       // one CTA per task, up to 8 per SM
+    const cudaError_t e = launch_dependent(k_expand_rows, (unsigned)(tasks < (long long)sms * 8 ? tasks : (long long)sms * 8), 256, 0, st,
+                                           a_bits, M, lda, RTa, w_bits, N, ldw, RTw, K, KB, (uint4*)a_units, (uint4*)w_units);
+    if (e != cudaSuccess) return fail("gemm (operand expansion): %s", cudaGetErrorString(e));
+    return 0;
+}
+
+int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, const GemmUnits& u, int sms, cudaStream_t st) {
     static bool configured[64] = {false};
     if (configure_once(configured, [] {
             cudaError_t e = cudaFuncSetAttribute(k_gemm_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -275,15 +292,11 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, int
         }))
         return 1;
     char* w = (char*)workspace;
-    {
-        const long long tasks = (long long)(p.MT + p.NT) * ((p.KB + 3) / 4);   // one CTA per task, up to 8 per SM
-        const int grid = (int)(tasks < (long long)sms * 8 ? tasks : (long long)sms * 8);
-        const cudaError_t e = launch_dependent(k_expand_rows, grid, 256, 0, st, g.A, g.M, g.lda, p.MT, g.W, g.N, g.ldw, p.NT,
-                                               g.K, p.KB, (uint4*)(w + p.off_ea), (uint4*)(w + p.off_ew));
-        if (e != cudaSuccess) return fail("gemm (operand expansion): %s", cudaGetErrorString(e));
-    }
+    if ((!u.a || !u.w) && expand_units(g.A, g.M, g.lda, u.a ? nullptr : w + p.off_ea, g.W, g.N, g.ldw, u.w ? nullptr : w + p.off_ew, g.K, sms, st))
+        return 1;
     umma::GemmUmmaArgs a;
-    a.ea = (const unsigned char*)(w + p.off_ea); a.ew = (const unsigned char*)(w + p.off_ew);
+    a.ea = (const unsigned char*)(u.a ? u.a : w + p.off_ea); a.ew = (const unsigned char*)(u.w ? u.w : w + p.off_ew);
+    a.nxt = (uint4*)u.next; a.nxt_KB = (g.N + 63) / 64;
     a.M = g.M; a.N = g.N; a.KB = p.KB; a.MT = p.MT; a.NT = p.NT; a.splits = p.splits; a.per = p.per;
     a.partial = p.splits > 1 ? (int32_t*)(w + p.off_partial) : nullptr;
     a.mode = g.mode; a.out = g.out; a.ldo = g.ldo; a.p0 = g.p0; a.p1 = g.p1;
@@ -323,7 +336,7 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, int
 
 int g_gemm_path = 0;     // 0 automatic, 1 warp-level b1 MMA only
 
-int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st, const GemmUnits& u = GemmUnits{}) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) return fail("gemm: M, N, K must be positive");
     if ((g.lda & 1) || (g.ldw & 1)) return fail("gemm: lda and ldw must be even (64-bit loads)");
     if (g.lda * 32 < g.K || g.ldw * 32 < g.K) return fail("gemm: leading dimension shorter than K");
@@ -333,8 +346,16 @@ int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t s
     int sms;
     if (sm_count(&sms)) return 1;
     const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms);
-    if (plan.use && g_gemm_path != 1 && workspace && workspace_bytes >= plan.bytes && ((uintptr_t)workspace & 255) == 0)
-        return run_gemm_umma(g, plan, workspace, sms, st);
+    if (plan.use && g_gemm_path != 1 && workspace && workspace_bytes >= plan.bytes && ((uintptr_t)workspace & 255) == 0) {
+        // (the epilogue writes the next operand where it finishes the layer itself)
+        const GemmUnits mine{u.a, u.w, plan.splits == 1 ? u.next : nullptr};
+        if (run_gemm_umma(g, plan, workspace, mine, sms, st)) return 1;
+        return u.next && !mine.next ? expand_units((const uint32_t*)g.out, g.M, g.ldo, u.next, nullptr, 0, 0, nullptr, g.N, sms, st) : 0;
+    }
+    if (u.next) {
+        if (run_gemm(g, workspace, workspace_bytes, st)) return 1;
+        return expand_units((const uint32_t*)g.out, g.M, g.ldo, u.next, nullptr, 0, 0, nullptr, g.N, sms, st);
+    }
     // Slices of K on different SMs with a finishing launch pay only where K is very long and there is
     // next to no M x N to spread over the GPU; everything else finishes inside one launch.
     int splits = gemm_use_splits(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0);
@@ -1101,6 +1122,11 @@ int tcbnn_version(void) { return 100; }
 const char* tcbnn_last_error(void) { return g_err; }
 
 int tcbnn_pack_rows(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* stream) {
+    return tcbnn_pack_rows_x(x, rows, cols, ld_words, out, nullptr, stream);
+}
+
+int tcbnn_pack_rows_x(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units, void* stream) {
+    if ((uintptr_t)units & 255) return fail("pack_rows: units must be 256-byte aligned");
     if (rows <= 0 || cols <= 0) return fail("pack_rows: empty input");
     if ((ld_words & 3) || ld_words * 32 < cols) return fail("pack_rows: ld_words must be a multiple of 4 and cover cols");
     if ((uintptr_t)out & 15) return fail("pack_rows: output must be 16-byte aligned");
@@ -1112,10 +1138,12 @@ int tcbnn_pack_rows(const float* x, int rows, int cols, int ld_words, uint32_t* 
         // memory-bound and light on registers: all 64 warps an SM holds (8 CTAs)
         long long ctas = (vtasks + kThreads / 32 - 1) / (kThreads / 32);
         if (ctas > 8LL * sms) ctas = 8LL * sms;
-        k_pack_rows_vec<<<(int)ctas, kThreads, 0, (cudaStream_t)stream>>>(x, rows, cols, ld_words, out);
+        k_pack_rows_vec<<<(int)ctas, kThreads, 0, (cudaStream_t)stream>>>(x, rows, cols, ld_words, out, (uint4*)units);
+        return launch_check("pack_rows");
     } else
         k_pack_rows<<<warp_grid(tasks, sms), kThreads, 0, (cudaStream_t)stream>>>(x, rows, cols, ld_words, out);
-    return launch_check("pack_rows");
+    if (launch_check("pack_rows")) return 1;
+    return units ? expand_units(out, rows, ld_words, units, nullptr, 0, 0, nullptr, cols, sms, (cudaStream_t)stream) : 0;
 }
 
 int tcbnn_unpack_rows(const uint32_t* in, int rows, int cols, int ld_words, float* out, void* stream) {
@@ -1209,6 +1237,30 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
     if (ldo * 32 < N) return fail("fc_layer: ldo too small");
     GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows) {
+    int sms;
+    if (M <= 0 || N <= 0 || K <= 0 || rows <= 0 || sm_count(&sms) || !gemm_umma_plan(M, N, K, sms).use) return 0;
+    return (size_t)((rows + 127) / 128) * ((K + 63) / 64) * umma::kGemmUnit;
+}
+
+int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units, void* stream) {
+    if (N <= 0 || K <= 0 || (ldw & 1) || ldw * 32 < K || ((uintptr_t)W & 7)) return fail("fc_expand_weight: bad sizes or alignment");
+    if (!units || ((uintptr_t)units & 255)) return fail("fc_expand_weight: units must be 256-byte aligned");
+    int sms;
+    if (sm_count(&sms)) return 1;
+    return expand_units(nullptr, 0, 0, nullptr, W, N, ldw, units, K, sms, (cudaStream_t)stream);
+}
+
+int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N, int lda, int ldw, uint32_t* out,
+                     int ldo, void* workspace, size_t workspace_bytes, const void* a_units, const void* w_units, void* next_units,
+                     void* stream) {
+    if (ldo * 32 < N) return fail("fc_layer: ldo too small");
+    if (((uintptr_t)a_units | (uintptr_t)w_units | (uintptr_t)next_units) & 255) return fail("fc_layer: units must be 256-byte aligned");
+    if (next_units && (ldo & 1)) return fail("fc_layer: next_units needs an even ldo");
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr};
+    return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream, GemmUnits{a_units, w_units, next_units});
 }
 
 int tcbnn_out_layer(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,

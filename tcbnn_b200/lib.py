@@ -37,6 +37,10 @@ SIGNATURES = {
     "tcbnn_gemm_status": (_I, [C.POINTER(C.c_int)]),
     "tcbnn_bgemm": (_I, [_P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
     "tcbnn_fc_layer": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
+    "tcbnn_fc_units_bytes": (_SZ, [_I, _I, _I, _I]),
+    "tcbnn_fc_expand_weight": (_I, [_P, _I, _I, _I, _P, _P]),
+    "tcbnn_fc_layer_x": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P, _P, _P]),
+    "tcbnn_pack_rows_x": (_I, [_P, _I, _I, _I, _P, _P, _P]),
     "tcbnn_out_layer": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
     "tcbnn_conv_shape": (_I, [C.POINTER(ConvDesc)]),
     "tcbnn_conv_prepared_bytes": (_SZ, [C.POINTER(ConvDesc)]),

@@ -263,6 +263,7 @@ class Network:
             prev = obj
         if handover:
             self._wire_handover()
+            self._wire_units()
             self._wire_residual_layouts()
 
     def _wire_handover(self):
@@ -286,6 +287,31 @@ class Network:
                 continue
             prod.next_layer = (cons.desc, planes)
             cons.input_planes = planes
+
+    def _wire_units(self):
+        """FC layers on the tcgen05 GEMM: the weight is expanded once, and a producer that packs bits
+        (the input layer, another FC layer) writes the expanded input too."""
+        for prod, cons in zip(self.layers, self.layers[1:]):
+            if type(cons).__name__ != "Fc128LayerParam":
+                continue
+            M, K, N, dev = cons.input_height, cons.input_width, cons.weight_width, cons.weight_gpu.device
+            cons.weight_units = ops.fc_units(M, N, K, N, dev)
+            if cons.weight_units is None:
+                continue
+            ops.fc_expand_weight(cons.weight_gpu, K, cons.weight_units)
+            if type(prod).__name__ in ("In128LayerParam", "Fc128LayerParam"):
+                cons.units_room = ops.fc_units(M, N, K, M, dev)
+            cons.units_versions = cons.versions()
+        self._use_units()
+
+    def _use_units(self):
+        """Producers write expanded inputs while the live batch has their consumer on the kernel that
+        reads them."""
+        for prod, cons in zip(self.layers, self.layers[1:]):
+            room = getattr(cons, "units_room", None)
+            if room is not None:
+                used = ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0
+                cons.input_units = prod.next_units = room if used else None
 
     def _wire_residual_layouts(self):
         """An int16 residual tensor is kept in the chunk-major layout (TCBNN_RES_INT16_CHUNKED)
@@ -316,6 +342,7 @@ class Network:
             if getattr(cons, "input_planes", None) is not None:
                 cons.input_planes = ops.new_planes(cons.desc, cons.input_gpu.device)
                 prod.next_layer = (cons.desc, cons.input_planes)
+        p._use_units()
         return p
 
     def set_input(self, x):
@@ -327,6 +354,7 @@ class Network:
         The logits of the live images are the first n rows of the output."""
         for l in self.layers:
             l.set_batch(n)
+        self._use_units()
         self.live_batch = n
 
     _pass = None           # (layers' calls, settings, device, graph or None, passes seen) of the last pass

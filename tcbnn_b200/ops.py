@@ -94,6 +94,22 @@ def gemm_launches(M, N, K, workspace):
     return _l.load().tcbnn_gemm_launches(M, N, K, nbytes)
 
 
+def fc_units(M, N, K, rows, device):
+    """Zeroed room for `rows` expanded rows of K (tcbnn_fc_layer_x) of an FC layer of that shape, or None
+    where the layer does not run on the kernel that takes them."""
+    n = fc_units_bytes(M, N, K, rows)
+    return torch.zeros((n,), dtype=torch.uint8, device=device) if n else None
+
+
+def fc_units_bytes(M, N, K, rows):
+    return _l.load().tcbnn_fc_units_bytes(M, N, K, rows)
+
+
+def fc_expand_weight(W, K, units):
+    _need_cuda(W)
+    _l.call("tcbnn_fc_expand_weight", _ptr(W), W.shape[0], K, W.shape[1], _ptr(units), _stream())
+
+
 def _ws(ws):
     return (ws.data_ptr(), ws.numel() * 4) if ws is not None else (None, 0)
 

@@ -87,9 +87,9 @@ class _Layer:
     def forward(self):
         c = self.__dict__.get("_call")
         if c is None or not self._call_valid(c):
-            name, args, keep = self._call_args()
-            # `keep`: tensors and descriptors the arguments point into
-            c = self.__dict__["_call"] = (ops._l.bound(name), args, keep)
+            name, *rest = self._call_args()
+            # after the arguments: tensors and descriptors they point into, what _call_valid looks at
+            c = self.__dict__["_call"] = (ops._l.bound(name), *rest)
         if c[0](*c[1], ops._stream()) != 0:
             raise ops._l.TcbnnError(ops._l.load().tcbnn_last_error().decode())
 
@@ -138,9 +138,12 @@ class In128LayerParam(_Layer):
         src = src.reshape(-1, self.input_width)
         self.input_gpu[:src.shape[0]].copy_(src, non_blocking=True)
 
+    next_units = None      # the FC layer behind takes its input expanded (Fc128LayerParam.input_units)
+
     def _call_args(self):
-        x, out = self.input_gpu, self.output_gpu
-        return "tcbnn_pack_rows", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out)), (x, out)
+        x, out, nxt = self.input_gpu, self.output_gpu, self.next_units
+        return "tcbnn_pack_rows_x", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out),
+                                     ops._ptr(nxt)), (x, out, nxt)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -188,14 +191,42 @@ class Fc128LayerParam(_Layer):
             raise ValueError("%s: input rows of %d words do not cover K=%d" % (self.name, t.shape[1], K))
         self.input_gpu = t
 
+    # Operands in the GEMM kernel's own form (tcbnn_fc_layer_x), wired by models.Network: this layer's
+    # weight, its input as the producer writes it (units_room; input_units while the live batch takes that
+    # kernel), and the next FC layer's input.  They follow the packed operands: another input or weight
+    # tensor, or one written to since, drops them.
+    units_room = input_units = weight_units = next_units = units_versions = None
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name == "input_gpu":
+            self.units_room = self.input_units = None
+        elif name == "weight_gpu":
+            self.weight_units = None
+
+    def versions(self):
+        """Changes when torch writes to the packed operands (tensors of inference mode do not say)."""
+        return tuple(0 if t.is_inference() else t._version for t in (self.input_gpu, self.weight_gpu))
+
+    def _call_valid(self, c):
+        return c[3] == self.versions()
+
     def kernel_launches(self):
-        return self.launches
+        # the operand expansion is not launched where both operands come expanded; where a finishing
+        # launch computes the bits (launches == 3), the next layer's input is expanded from them
+        return (self.launches - int(self.input_units is not None and self.weight_units is not None)
+                + int(self.next_units is not None and self.launches == 3))
 
     def _call_args(self):
         a, w, thr, out, ws = self.input_gpu, self.weight_gpu, self.bn_gpu, self.output_gpu, self.workspace
         ops._need_cuda(a, w, thr)
-        return "tcbnn_fc_layer", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
-                                  a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws)), (a, w, thr, out, ws)
+        versions = self.versions()
+        if self.units_versions is not None and self.units_versions != versions:
+            self.units_room = self.input_units = self.weight_units = None
+        u = (self.input_units, self.weight_units, self.next_units)
+        return "tcbnn_fc_layer_x", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
+                                    a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws),
+                                    *(ops._ptr(t) for t in u)), (a, w, thr, out, ws, u), versions
 
     def get_output_gpu(self):
         return self.output_gpu

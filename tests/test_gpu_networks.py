@@ -38,6 +38,30 @@ def test_mlp(cuda):
     _compare(models.mlp_spec(256), 5, cuda)
 
 
+@pytest.mark.parametrize("batch, widths", [(1401, (784, 1031, 999, 1100)), (1400, (845, 1024, 928, 1500))])
+def test_fc_layers_hand_their_operands_over_expanded(cuda, batch, widths):
+    # ragged rows and columns (words and k-blocks half used), either packing kernel of the input layer
+    spec = models.mlp_spec(batch, widths[0])
+    for l, n in zip(spec["layers"][1:-1], widths[1:]):
+        l["N"] = n
+    _compare(spec, 17, cuda)
+    w, x = models.synthetic_weights(spec, 17), models.synthetic_input(spec, 18)
+    net = models.Network(spec, w, x)
+    assert all(l.input_units is not None for l in net.layers[1:-1])
+    want = net.forward().clone()
+    net.set_batch(batch - 200)                       # other rows of the last tile, or another kernel
+    assert torch.equal(net.forward()[:batch - 200], want[:batch - 200])
+    net.set_batch(40)
+    assert torch.equal(net.forward()[:40], want[:40])
+    net.set_batch(batch)
+    fc = net.layers[2]
+    fc.weight_gpu.copy_(torch.zeros_like(fc.weight_gpu))       # a weight written to in place counts
+    changed = net.forward().clone()
+    plain = models.Network(spec, w, x, handover=False)
+    plain.layers[2].weight_gpu.zero_()
+    assert torch.equal(changed, plain.forward()) and not torch.equal(changed, want)
+
+
 def test_vgg_cifar(cuda):
     _compare(models.vgg_cifar_spec(8), 10, cuda)
 
