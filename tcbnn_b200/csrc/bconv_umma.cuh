@@ -270,7 +270,7 @@ template <int K>
 __device__ __forceinline__ void mma_f4_run(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                            uint32_t b_lo, uint32_t b_hi, uint32_t step_b, const uint32_t* t,
                                            uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb) {
-    static_assert(K == 1 || K == 5 || K == 9, "run lengths in use");
+    static_assert(K == 1 || K == 4 || K == 5 || K == 9, "run lengths in use");
     if constexpr (K == 9)
         asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
                      TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") TCBNN_F4_MMA("%16", "pt")
@@ -281,71 +281,16 @@ __device__ __forceinline__ void mma_f4_run(uint32_t leader, uint32_t d_tmem, uin
         asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
                      TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") "}"
                      ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]) : "memory");
+    else if constexpr (K == 4)
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
+                     TCBNN_F4_MMA("%14", "pt") "}"
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
     else
         asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") "}" ::TCBNN_F4_IN, "r"(t[0]) : "memory");
 }
 #undef TCBNN_F4_MMA
 #undef TCBNN_F4_HEAD
 #undef TCBNN_F4_IN
-// Two accumulators side by side, D0 += A B0 and D1 += A B1 with D1 128 columns behind D0 and B1 `b1` behind
-// B0: A stays in the collector from the first MMA to the second, which leaves 12 KB instead of 16 to read
-// from shared memory per step.  A and both Bs advance by step_b.
-#define TCBNN_F4_PAIR(D, B, BHI, ID, SFA, SFB, PRED)                                           \
-    "mov.b64 da, {xa, " BHI "};\n\tmov.b64 db, {xb, " BHI "};\n\tadd.u32 xc, xb, " B ";\n\tmov.b64 dc, {xc, " BHI "};\n\t" \
-    "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32.collector::a::fill [" D "], da, db, " ID ", [" SFA "], [" SFB "], " PRED ";\n\t" \
-    "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32.collector::a::lastuse [xd], da, dc, " ID ", [" SFA "], [" SFB "], " PRED ";\n\t"
-#define TCBNN_F4_RUN2(PRED) TCBNN_F4_PAIR("%4", "%10", "%2", "%5", "%7", "%8", PRED) \
-    "add.u32 xa, xa, %9;\n\tadd.u32 xb, xb, %9;\n\t"
-template <int K>
-__device__ __forceinline__ void mma_f4_pair_run(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t hi, uint32_t b_lo,
-                                                uint32_t b1, uint32_t step, uint32_t idesc, uint32_t acc, uint32_t sfa,
-                                                uint32_t sfb) {
-    static_assert(K == 1 || K == 2, "run lengths in use");
-#define TCBNN_F4_HEAD2                                                                               \
-    "{\n\t.reg .pred pq, pt, pl;\n\t.reg .b64 da, db, dc;\n\t.reg .b32 xa, xb, xc, xd;\n\t"          \
-    "setp.ne.b32 pl, %0, 0;\n\tsetp.ne.b32 pq, %6, 0;\n\tsetp.eq.b32 pt, %0, %0;\n\t"              \
-    "mov.u32 xa, %1;\n\tmov.u32 xb, %3;\n\tadd.u32 xd, %4, 128;\n\t"
-#define TCBNN_F4_IN2                                                                                 \
-    "r"(leader), "r"(a_lo), "r"(hi), "r"(b_lo), "r"(d_tmem), "r"(idesc), "r"(acc), "r"(sfa), "r"(sfb), "r"(step), "r"(b1)
-    if constexpr (K == 2)
-        asm volatile(TCBNN_F4_HEAD2 TCBNN_F4_RUN2("pq") TCBNN_F4_RUN2("pt") "}" ::TCBNN_F4_IN2 : "memory");
-    else
-        asm volatile(TCBNN_F4_HEAD2 TCBNN_F4_RUN2("pq") "}" ::TCBNN_F4_IN2 : "memory");
-}
-#undef TCBNN_F4_HEAD2
-#undef TCBNN_F4_RUN2
-#define TCBNN_F4_END2(PRED) TCBNN_F4_PAIR("%5", "%11", "%3", "%6", "%8", "%9", PRED) \
-    "add.u32 xa, xa, %10;\n\tadd.u32 xb, xb, %10;\n\t"
-#define TCBNN_F4_HEAD2                                                                               \
-    "{\n\t.reg .pred p0, p1, pq, pt, pl, pc;\n\t.reg .b64 da, db, dc;\n\t.reg .b32 xa, xb, xc, xd, r1;\n\t" \
-    "mbarrier.test_wait.parity.shared::cta.b64 p0, [%12], %13;\n\t"                                 \
-    "mbarrier.test_wait.parity.shared::cta.b64 p1, [%14], %15;\n\t"                                 \
-    "setp.ne.b32 pl, %1, 0;\n\tsetp.ne.b32 pq, %7, 0;\n\tsetp.eq.b32 pt, %1, %1;\n\t"              \
-    "mov.u32 xa, %2;\n\tmov.u32 xb, %4;\n\tadd.u32 xd, %5, 128;\n\tsetp.ne.and.b32 pc, %17, 0, pl;\n\t"
-#define TCBNN_F4_TAIL2                                                                               \
-    "@pl tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%16];\n\t"           \
-    "@pc tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%17];\n\t"           \
-    "selp.u32 %0, 1, 0, p0;\n\tselp.u32 r1, 2, 0, p1;\n\tor.b32 %0, %0, r1;\n\t}"
-template <int K>
-__device__ __forceinline__ uint32_t mma_f4_pair_end(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t hi,
-                                                    uint32_t b_lo, uint32_t b1, uint32_t step, uint32_t idesc, uint32_t acc,
-                                                    uint32_t sfa, uint32_t sfb, uint32_t bar0, uint32_t par0, uint32_t bar1,
-                                                    uint32_t par1, uint32_t bar_e, uint32_t bar_c) {
-    static_assert(K == 1 || K == 2, "run lengths in use");
-    uint32_t ok;
-    if constexpr (K == 2)
-        asm volatile(TCBNN_F4_HEAD2 TCBNN_F4_END2("pq") TCBNN_F4_END2("pt") TCBNN_F4_TAIL2
-                     : "=&r"(ok) : TCBNN_F4_IN2, "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar_e), "r"(bar_c) : "memory");
-    else
-        asm volatile(TCBNN_F4_HEAD2 TCBNN_F4_END2("pq") TCBNN_F4_TAIL2
-                     : "=&r"(ok) : TCBNN_F4_IN2, "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar_e), "r"(bar_c) : "memory");
-    return ok;
-}
-#undef TCBNN_F4_PAIR
-#undef TCBNN_F4_END2
-#undef TCBNN_F4_HEAD2
-#undef TCBNN_F4_TAIL2
-#undef TCBNN_F4_IN2
 #define TCBNN_F4_MMA(AOFF, PRED)                                                                     \
     "add.u32 xa, %2, " AOFF ";\n\tmov.b64 da, {xa, %3};\n\tmov.b64 db, {xb, %5};\n\t"                \
     "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%6], da, db, %7, [%9], [%10], " PRED ";\n\t" \

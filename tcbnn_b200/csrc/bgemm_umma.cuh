@@ -6,18 +6,17 @@
 // One streaming pass first writes both operands as +-1 nibbles (0 for padding: rows past the end,
 // bits past K) in 4 KB units [128-row tile][64-bit k-block][32-bit chunk][row][16 B], the
 // no-swizzle K-major operand layout, so that a unit is one bulk copy and one MMA operand.
-// The GEMM is persistent: a CTA per SM walks over 128 x 128 or 128 x 256 tiles (a 128-row tile of
-// A against one or two of W), each over a range of k-blocks:
+// The GEMM is persistent: a CTA per SM walks over 128 x 128 or 256 x 128 tiles (one or two 128-row
+// sub-tiles of A against one tile of W), each over a range of k-blocks:
 //
 //   warps 0-7  epilogue : tcgen05.ld and either finish the layer (one split: int32 / threshold bits /
 //                         scale + bias straight from the accumulator) or store int32 partial sums for
 //                         gemm_splitk_finish.  128 x 128 tiles alternate between two accumulators, so
 //                         that a tile is finished while the next one is computed
-//   warp  8    loader A : one lane, one bulk copy per stage (a stage holds up to
+//   warp  8    loader A : one lane, one bulk copy per sub-tile and stage (a stage holds up to
 //                         kGemmKU consecutive k-blocks, contiguous in the expanded operand)
-//   warp  9    MMA      : converged warp, elected lane: one N=128 MMA per sub-tile and k-block, the two
-//                         of a 128 x 256 tile back to back with A kept in the collector
-//   warp  10   loader W : one lane, one bulk copy per sub-tile and stage
+//   warp  9    MMA      : converged warp, elected lane: one N=128 MMA per sub-tile and k-block
+//   warp  10   loader W : one lane, one bulk copy per stage
 //
 // Loaders and issuer run ahead across tile boundaries, so set-up, first loads and epilogue of all
 // but a CTA's last tile are hidden: as one CTA per tile (two per SM) the MLP's hidden layer, 8192 x 1024
@@ -37,7 +36,7 @@ namespace umma {
 constexpr int kGemmThreads = 352;
 constexpr int kGemmUnit = 4096;                        // 128 rows x 64 k, 4 bits each
 constexpr int kGemmKU = 4;                             // k-blocks per stage
-// Per tile shape (PAIR: 128 x 256, else 128 x 128): ring depth and bytes of a stage.  One CTA per SM
+// Per tile shape (PAIR: 256 x 128, else 128 x 128): ring depth and bytes of a stage.  One CTA per SM
 // takes all of tensor memory: accumulators, then 32 columns of unit scales at the top.
 __host__ __device__ constexpr int gemm_stages(bool pair) { return pair ? 4 : 6; }
 __host__ __device__ constexpr int gemm_stage_bytes(bool pair) { return (pair ? 3 : 2) * kGemmKU * kGemmUnit; }
@@ -139,19 +138,19 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     auto BAR_CEMPTY = [&](int b) { return bar0 + 8u * (2 * NST + NACC + b); };
     const uint32_t BAR_DRAIN = bar0 + 8u * (2 * NST + 2 * NACC);
 
-    // tile t = (split * MT + tm) * tiles_n + tn; tn counts pairs of sub-tiles when PAIR
-    const int tiles_n = PAIR ? (g.NT + 1) >> 1 : g.NT;
-    const int ntiles = g.MT * tiles_n * g.splits;
-    struct Tile { int tn, rt, split, kb0, kb1; bool two; };
+    // tile t = (split * tiles_m + tm) * NT + tn; tm counts pairs of sub-tiles when PAIR
+    const int tiles_m = PAIR ? (g.MT + 1) >> 1 : g.MT;
+    const int ntiles = tiles_m * g.NT * g.splits;
+    struct Tile { int tn, rt0, split, kb0, kb1; bool two; };
     auto tile = [&](int t) {
         Tile q;
-        const int r = t / tiles_n, n = t - r * tiles_n;
-        q.split = r / g.MT;
-        q.rt = r - q.split * g.MT;
+        q.tn = t % g.NT;
+        const int tm = (t / g.NT) % tiles_m;
+        q.split = t / (g.NT * tiles_m);
         q.kb0 = q.split * g.per;
         q.kb1 = min(g.KB, q.kb0 + g.per);
-        q.tn = PAIR ? n * 2 : n;                        // first 128-column tile of W
-        q.two = PAIR && q.tn + 1 < g.NT;                // second 128-column sub-tile exists
+        q.rt0 = PAIR ? tm * 2 : tm;                     // first 128-row tile of A
+        q.two = PAIR && q.rt0 + 1 < g.MT;               // second 128-row sub-tile exists
         return q;
     };
 
@@ -177,7 +176,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     // Launched as a programmatic dependent of the expansion pass, the CTA has come this far while
     // that pass was still running; its units are complete (and visible) once this returns.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    constexpr uint32_t OFF_W = kGemmKU * kGemmUnit;     // W's place inside a stage
+    constexpr uint32_t OFF_W = (PAIR ? 2u : 1u) * kGemmKU * kGemmUnit;     // W's place inside a stage
     const bool tr = g.trace != nullptr && blockIdx.x == 0;
 
     if (warp == 8 || warp == 10) {
@@ -190,20 +189,20 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             long long tr_w = 0;
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 const Tile q = tile(t);
-                const unsigned char* src = isw ? g.ew + (size_t)q.tn * g.KB * kGemmUnit : g.ea + (size_t)q.rt * g.KB * kGemmUnit;
+                const unsigned char* src = isw ? g.ew + (size_t)q.tn * g.KB * kGemmUnit : g.ea + (size_t)q.rt0 * g.KB * kGemmUnit;
                 for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
                     const uint32_t bytes = (uint32_t)min(kGemmKU, q.kb1 - kb) * kGemmUnit;
                     ok = tr ? wait.timed(BAR_EMPTY(s), ph ^ 1, tr_w) : wait(BAR_EMPTY(s), ph ^ 1);
                     if (!ok) break;
                     const uint32_t dst = smem_u32(smem + (size_t)s * STAGE);
-                    if (!isw) {
+                    if (isw) {
                         mbar_expect_tx(BAR_FULL(s), bytes);
-                        bulk_g2s(dst, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
+                        bulk_g2s(dst + OFF_W, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
                     } else {
                         mbar_expect_tx(BAR_FULL(s), (q.two ? 2u : 1u) * bytes);
-                        bulk_g2s(dst + OFF_W, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
+                        bulk_g2s(dst, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
                         if (q.two)
-                            bulk_g2s(dst + 2 * OFF_W, src + (size_t)(g.KB + kb) * kGemmUnit, bytes, BAR_FULL(s));
+                            bulk_g2s(dst + kGemmKU * kGemmUnit, src + (size_t)(g.KB + kb) * kGemmUnit, bytes, BAR_FULL(s));
                     }
                     issued++;
                     if (++s == NST) { s = 0; ph ^= 1; }
@@ -231,7 +230,8 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         constexpr uint32_t IDESC = idesc_f4(128);
         const uint64_t desc0 = smem_desc(smem_u32(smem), 128 * 16, 128u);
         const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
-        constexpr uint32_t stepStage = STAGE >> 4, stepUnit = kGemmUnit >> 4, offW = OFF_W >> 4;
+        constexpr uint32_t stepStage = STAGE >> 4, stepUnit = kGemmUnit >> 4, offW = OFF_W >> 4,
+                           offA2 = (kGemmKU * kGemmUnit) >> 4;
         const uint32_t units[4] = {0u, stepUnit, 2 * stepUnit, 3 * stepUnit};
         const uint32_t sfa = tmem + SF_COL, sfb = tmem + SF_COL + 16;
         uint32_t s = 0, ph = 0, b = 0, bph = 0, ready = 0, need = 3u;
@@ -257,22 +257,15 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             uint32_t acc = kb > q.kb0 ? 1u : 0u;
             const uint32_t d = tmem + b * 128;
             uint32_t aLo = lo0 + s * stepStage, bLo = aLo + offW;
-            const bool two = PAIR && q.two;
-            if (two) {
-                if (nkb == kGemmKU)
-                    mma_f4_pair_run<2>(leader, d, aLo, hi, bLo, offW, stepUnit, IDESC, acc, sfa, sfb);
-                else
-                    for (int j = 0; j + 1 < nkb; j++) {
-                        mma_f4_pair_run<1>(leader, d, aLo + j * stepUnit, hi, bLo + j * stepUnit, offW, stepUnit, IDESC, acc, sfa, sfb);
-                        acc = 1;
-                    }
-            } else if (nkb == kGemmKU) {
+            if (nkb == kGemmKU) {
+                if (q.two) mma_f4_run<4>(leader, d + 128, aLo + offA2, hi, bLo, hi, stepUnit, units, IDESC, acc, sfa, sfb);
                 mma_f4_run<1>(leader, d, aLo, hi, bLo, hi, stepUnit, units, IDESC, acc, sfa, sfb);
             } else {
-                for (int j = 0; j + 1 < nkb; j++) {
+                for (int j = 0; j < nkb; j++) {
                     const uint32_t o = j * stepUnit;
-                    mma_f4_run<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
-                    acc = 1;
+                    if (q.two) mma_f4_run<1>(leader, d + 128, aLo + offA2, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
+                    if (j + 1 < nkb) mma_f4_run<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
+                    if (j + 1 < nkb) acc = 1;
                 }
             }
             asm volatile("" : "+r"(s), "+r"(b), "+r"(ph), "+r"(bph), "+r"(kb));   // what follows stays behind those MMAs
@@ -289,19 +282,14 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             need = last ? 3u : 1u;
             // (while a tile is being issued, its own accumulator is what bar1 names; the answer counts
             // only at the first stage of a tile)
-            const uint32_t o = (nkb - 1) * stepUnit, o2 = 2 * stepUnit;
-            if (two && nkb == kGemmKU)
-                ready = mma_f4_pair_end<2>(leader, d, aLo + o2, hi, bLo + o2, offW, stepUnit, IDESC, 1u, sfa, sfb,
-                                           BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
-            else if (two)
-                ready = mma_f4_pair_end<1>(leader, d, aLo + o, hi, bLo + o, offW, stepUnit, IDESC, acc, sfa, sfb,
-                                           BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
-            else if (nkb == kGemmKU)
+            if (nkb == kGemmKU)
                 ready = mma_f4_end<3>(leader, d, aLo, hi, bLo + stepUnit, hi, stepUnit, units + 1, IDESC, 1u, sfa, sfb,
                                       BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
-            else
+            else {
+                const uint32_t o = (nkb - 1) * stepUnit;
                 ready = mma_f4_end<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb,
                                       BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
+            }
             if (last) {
                 t += gridDim.x;
                 if (t < ntiles) { q = tile(t); kb = q.kb0; }
@@ -325,9 +313,9 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         uint32_t bph = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
             const Tile q = tile(t);
-            const int sub = PAIR ? warp >> 2 : 0;       // 128 x 256: a warpgroup per sub-tile; 128 x 128: per column half
+            const int sub = PAIR ? warp >> 2 : 0;       // 256 x 128: a warpgroup per sub-tile; 128 x 128: per column half
             const int nb0 = PAIR ? 0 : (warp >> 2) * 2, nb1 = PAIR ? 4 : nb0 + 2;
-            const int m0 = q.rt * 128 + quad * 32, tn = q.tn + sub;          // this warp's rows, its column tile
+            const int m0 = (q.rt0 + sub) * 128 + quad * 32;                  // this warp's rows
             const bool have = sub == 0 || q.two;
             // thresholds of this warp's columns, in the accumulator's column order, while it is awaited
             // (a threshold per column straight from global memory costs a trip to L2 each: 6800 clocks
@@ -336,7 +324,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             if (g.splits == 1 && g.mode == GEMM_FC_BITS) {
                 __syncwarp();
                 for (int nb = nb0; nb < nb1; nb++) {
-                    const int n = tn * 128 + nb * 32 + f4_channel_of_column(lane);
+                    const int n = q.tn * 128 + nb * 32 + f4_channel_of_column(lane);
                     thr[nb * 32 + lane] = n < g.N ? __ldg(g.p0 + n) : __int_as_float(0x7FC00000);
                 }
                 __syncwarp();
@@ -353,7 +341,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                     const int m = m0 + lane;
 #pragma unroll 1
                     for (int nb = nb0; nb < nb1; nb++) {
-                        const int n0 = tn * 128 + nb * 32;
+                        const int n0 = q.tn * 128 + nb * 32;
                         if (n0 >= g.N) break;
                         int v[32];
                         tmem_ld32(tcol + nb * 32, v);
@@ -383,7 +371,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                     const bool v4 = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
 #pragma unroll 1
                     for (int nb = nb0; nb < nb1; nb++) {
-                        const int n0 = tn * 128 + nb * 32 + 4 * q4;
+                        const int n0 = q.tn * 128 + nb * 32 + 4 * q4;
                         float4 sc[2], bi[2];
                         if (!ints) {
 #pragma unroll

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(umma::kGemmThreads, 1) k_gemm_umma(umma::GemmU
 
 struct GemmUmmaPlan {
     bool use;
-    bool pair;            // 128 x 256 tiles (two sub-tiles of W per CTA) instead of 128 x 128
+    bool pair;            // 256 x 128 tiles (two sub-tiles of A per CTA) instead of 128 x 128
     int MT, NT, KB, splits, per;
     size_t off_ea, off_ew, off_partial, bytes;
 };
@@ -245,8 +245,8 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
     double best = 1e30;
     for (int pair = 0; pair < 2; pair++) {
         if (g_gemm_force_pair >= 0 && pair != g_gemm_force_pair) continue;
-        if (pair && p.NT < 2 && g_gemm_force_pair < 0) continue;
-        const long long tiles = (long long)p.MT * (pair ? (p.NT + 1) / 2 : p.NT);
+        if (pair && p.MT < 2 && g_gemm_force_pair < 0) continue;
+        const long long tiles = (long long)(pair ? (p.MT + 1) / 2 : p.MT) * p.NT;
         for (int want = 1; want <= 32 && (want <= (p.KB + 3) / 4 || g_gemm_force_splits > 0); want++) {
             const int per = (p.KB + want - 1) / want;
             const int splits = (p.KB + per - 1) / per;                    // no empty split
@@ -318,7 +318,7 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, con
     {
         // a programmatic dependent of the expansion launch: set-up (barriers, tensor memory, unit
         // scales) overlaps the expansion pass, the kernel waits for it before its first copy
-        const long long tiles = (long long)p.MT * (p.pair ? (p.NT + 1) / 2 : p.NT) * p.splits;
+        const long long tiles = (long long)(p.pair ? (p.MT + 1) / 2 : p.MT) * p.NT * p.splits;
         const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
         const cudaError_t e = launch_dependent(p.pair ? k_gemm_umma<true> : k_gemm_umma<false>, grid, umma::kGemmThreads,
                                                umma::gemm_smem(p.pair), st, a);
