@@ -36,13 +36,12 @@ namespace umma {
 constexpr int kGemmThreads = 352;
 constexpr int kGemmUnit = 4096;                        // 128 rows x 64 k, 4 bits each
 constexpr int kGemmKU = 4;                             // k-blocks per stage
-// Per tile shape (PAIR: 256 x 128, else 128 x 128): ring depth and bytes of a stage.  One CTA per SM
-// takes all of tensor memory: accumulators, then 32 columns of unit scales at the top.
-__host__ __device__ constexpr int gemm_stages(bool pair) { return pair ? 4 : 6; }
-__host__ __device__ constexpr int gemm_stage_bytes(bool pair) { return (pair ? 3 : 2) * kGemmKU * kGemmUnit; }
-__host__ __device__ constexpr size_t gemm_smem(bool pair) {
-    return (size_t)gemm_stages(pair) * gemm_stage_bytes(pair) + 32 * 8 + 64 + 8 * 128 * 4;    // ring, barriers, thresholds per epilogue warp
-}
+// Ring depth and bytes of a stage (A and W).  One CTA per SM takes all of tensor memory: accumulators,
+// then 32 columns of unit scales at the top.
+constexpr int kGemmStages = 6;
+constexpr int kGemmStageBytes = 2 * kGemmKU * kGemmUnit;
+// ring, barriers, thresholds per epilogue warp
+constexpr size_t kGemmSmem = (size_t)kGemmStages * kGemmStageBytes + 32 * 8 + 64 + 8 * 128 * 4;
 
 struct GemmUmmaArgs {
     const unsigned char* ea;   // expanded A: [MT][KB] units
@@ -119,9 +118,91 @@ __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_r
     }
 }
 
+// ---- a pair of CTAs on one 256 x 256 tile (cta_group::2) ------------------------------------------
+// Each CTA holds its 128 rows of A, half of W's 256 rows and its 128 x 256 accumulator; the leader (even
+// rank) issues MMAs that read both shared memories.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// arrives on the leader's copy of a barrier
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
+                 "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar) : "memory");
+}
+// WsWait with the bound in clocks, about a second: a CTA also waits for its partner
+struct GemmPairWait {
+    volatile int* abort;
+    int* err;
+    __device__ __forceinline__ bool poll(uint32_t bar, uint32_t parity, bool sleep) const {
+        const long long t0 = clock64();
+        for (int i = 0; i < (1 << 28); i++) {
+            if (mbar_test_wait(bar, parity)) return true;
+            if (sleep) __nanosleep(64);
+            if ((i & 63) == 63 && (*abort || clock64() - t0 > (1LL << 31))) break;
+        }
+        *abort = 1;
+        atomicExch(err, 1);
+        return false;
+    }
+    __device__ __forceinline__ bool operator()(uint32_t bar, uint32_t parity) const { return poll(bar, parity, false); }
+    __device__ __forceinline__ bool spin(uint32_t bar, uint32_t parity) const { return poll(bar, parity, false); }
+    __device__ __forceinline__ bool relaxed(uint32_t bar, uint32_t parity) const { return poll(bar, parity, true); }
+    __device__ __forceinline__ bool timed(uint32_t bar, uint32_t parity, long long& acc) const {
+        const long long t0 = clock64();
+        const bool ok = poll(bar, parity, false);
+        acc += clock64() - t0;
+        return ok;
+    }
+};
+// K MMAs of 256 x 256 x 64, A and W advancing by `step` alike; with END what mma_f4_end does (the commits
+// arrive in both CTAs).
+#define TCBNN_F4_PAIR_MMA(PRED)                                                                      \
+    "mov.b64 da, {xa, %3};\n\tmov.b64 db, {xb, %3};\n\t"                                            \
+    "@pl tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%5], da, db, %6, [%8], [%9], " PRED ";\n\t" \
+    "add.u32 xa, xa, %10;\n\tadd.u32 xb, xb, %10;\n\t"
+#define TCBNN_F4_PAIR_HEAD                                                                           \
+    "{\n\t.reg .pred p0, p1, pq, pt, pl, pc;\n\t.reg .b64 da, db;\n\t.reg .b32 xa, xb, r1;\n\t.reg .b16 both;\n\t" \
+    "setp.ne.b32 pl, %1, 0;\n\tsetp.ne.b32 pq, %7, 0;\n\tsetp.eq.b32 pt, %1, %1;\n\t"              \
+    "mov.u32 xa, %2;\n\tmov.u32 xb, %4;\n\t"
+#define TCBNN_F4_PAIR_TEST                                                                           \
+    "mbarrier.test_wait.parity.shared::cta.b64 p0, [%11], %12;\n\t"                                 \
+    "mbarrier.test_wait.parity.shared::cta.b64 p1, [%13], %14;\n\tsetp.ne.and.b32 pc, %16, 0, pl;\n\tmov.b16 both, 3;\n\t"
+#define TCBNN_F4_PAIR_TAIL                                                                           \
+    "@pl tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%15], both;\n\t" \
+    "@pc tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%16], both;\n\t" \
+    "selp.u32 %0, 1, 0, p0;\n\tselp.u32 r1, 2, 0, p1;\n\tor.b32 %0, %0, r1;\n\t}"
+#define TCBNN_F4_PAIR_IN                                                                             \
+    "r"(leader), "r"(a_lo), "r"(hi), "r"(b_lo), "r"(d_tmem), "r"(idesc), "r"(acc), "r"(sfa), "r"(sfb), "r"(step)
+__device__ __forceinline__ void mma_f4_pair_run(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
+                                                uint32_t step, uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb) {
+    uint32_t none;
+    asm volatile(TCBNN_F4_PAIR_HEAD TCBNN_F4_PAIR_MMA("pq") "mov.u32 %0, 0;\n\t}" : "=&r"(none) : TCBNN_F4_PAIR_IN : "memory");
+}
+template <int K>
+__device__ __forceinline__ uint32_t mma_f4_pair_end(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
+                                                    uint32_t step, uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb,
+                                                    uint32_t bar0, uint32_t par0, uint32_t bar1, uint32_t par1, uint32_t bar_e,
+                                                    uint32_t bar_c) {
+    static_assert(K == 1 || K == 3, "run lengths in use");
+    uint32_t ok;
+    if constexpr (K == 3)
+        asm volatile(TCBNN_F4_PAIR_HEAD TCBNN_F4_PAIR_TEST TCBNN_F4_PAIR_MMA("pq") TCBNN_F4_PAIR_MMA("pt") TCBNN_F4_PAIR_MMA("pt")
+                     TCBNN_F4_PAIR_TAIL : "=&r"(ok) : TCBNN_F4_PAIR_IN, "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar_e),
+                     "r"(bar_c) : "memory");
+    else
+        asm volatile(TCBNN_F4_PAIR_HEAD TCBNN_F4_PAIR_TEST TCBNN_F4_PAIR_MMA("pq") TCBNN_F4_PAIR_TAIL
+                     : "=&r"(ok) : TCBNN_F4_PAIR_IN, "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar_e), "r"(bar_c) : "memory");
+    return ok;
+}
+#undef TCBNN_F4_PAIR_MMA
+#undef TCBNN_F4_PAIR_HEAD
+#undef TCBNN_F4_PAIR_TEST
+#undef TCBNN_F4_PAIR_TAIL
+#undef TCBNN_F4_PAIR_IN
+
 template <bool PAIR>
 __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned char* smem) {
-    constexpr int STAGE = gemm_stage_bytes(PAIR), NST = gemm_stages(PAIR);
+    constexpr int STAGE = kGemmStageBytes, NST = kGemmStages;
     constexpr int NACC = PAIR ? 1 : 2;                  // accumulators of 256 / 128 columns
     constexpr uint32_t TM_COLS = 512, SF_COL = TM_COLS - 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -138,30 +219,40 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     auto BAR_CEMPTY = [&](int b) { return bar0 + 8u * (2 * NST + NACC + b); };
     const uint32_t BAR_DRAIN = bar0 + 8u * (2 * NST + 2 * NACC);
 
-    // tile t = (split * tiles_m + tm) * NT + tn; tm counts pairs of sub-tiles when PAIR
-    const int tiles_m = PAIR ? (g.MT + 1) >> 1 : g.MT;
-    const int ntiles = tiles_m * g.NT * g.splits;
-    struct Tile { int tn, rt0, split, kb0, kb1; bool two; };
+    // tile t = (split * tiles_m + tm) * tiles_n + tn; both count pairs when PAIR, and a pair of CTAs walks
+    // over the tiles together
+    const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
+    const int t_first = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, t_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int tiles_m = PAIR ? (g.MT + 1) >> 1 : g.MT, tiles_n = PAIR ? (g.NT + 1) >> 1 : g.NT;
+    const int ntiles = tiles_m * tiles_n * g.splits;
+    struct Tile { int tn, rt, split, kb0, kb1; };
     auto tile = [&](int t) {
         Tile q;
-        q.tn = t % g.NT;
-        const int tm = (t / g.NT) % tiles_m;
-        q.split = t / (g.NT * tiles_m);
+        const int r = t / tiles_n, n = t - r * tiles_n;
+        q.split = r / tiles_m;
+        const int m = r - q.split * tiles_m;
         q.kb0 = q.split * g.per;
         q.kb1 = min(g.KB, q.kb0 + g.per);
-        q.rt0 = PAIR ? tm * 2 : tm;                     // first 128-row tile of A
-        q.two = PAIR && q.rt0 + 1 < g.MT;               // second 128-row sub-tile exists
+        q.rt = PAIR ? m * 2 + rank : m;                 // this CTA's 128-row tile of A
+        q.tn = PAIR ? n * 2 : n;                        // first 128-column tile
         return q;
     };
 
     if (tid == 0) {
-        for (int s = 0; s < NST; s++) { mbar_init(BAR_FULL(s), 2); mbar_init(BAR_EMPTY(s), 1); }
-        for (int b = 0; b < NACC; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), 8); }
+        for (int s = 0; s < NST; s++) { mbar_init(BAR_FULL(s), PAIR && rank == 0 ? 3 : 2); mbar_init(BAR_EMPTY(s), 1); }
+        for (int b = 0; b < NACC; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), PAIR ? 16 : 8); }
         mbar_init(BAR_DRAIN, 1);
         *sAbort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 9) tmem_alloc(smem_u32(sTmem), TM_COLS);
+    if (warp == 9) {
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(sTmem)), "r"(TM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            tmem_alloc(smem_u32(sTmem), TM_COLS);
+        }
+    }
     fence_proxy_async();
     tc_fence_before();
     __syncthreads();
@@ -171,12 +262,13 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     if (warp < 4) tmem_fill_unit_scales(tmem, SF_COL);
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();                 // the partner's barriers and scales are set up as well
     tc_fence_after();
-    const WsWait wait{sAbort, g.status};
+    const typename std::conditional<PAIR, GemmPairWait, WsWait>::type wait{sAbort, g.status};
     // Launched as a programmatic dependent of the expansion pass, the CTA has come this far while
     // that pass was still running; its units are complete (and visible) once this returns.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    constexpr uint32_t OFF_W = (PAIR ? 2u : 1u) * kGemmKU * kGemmUnit;     // W's place inside a stage
+    constexpr uint32_t OFF_W = kGemmKU * kGemmUnit;     // W's place inside a stage
     const bool tr = g.trace != nullptr && blockIdx.x == 0;
 
     if (warp == 8 || warp == 10) {
@@ -187,22 +279,20 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             uint32_t ph = 0, issued = 0;
             bool ok = true;
             long long tr_w = 0;
-            for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+            for (int t = t_first; t < ntiles && ok; t += t_step) {
                 const Tile q = tile(t);
-                const unsigned char* src = isw ? g.ew + (size_t)q.tn * g.KB * kGemmUnit : g.ea + (size_t)q.rt0 * g.KB * kGemmUnit;
+                const int tile128 = isw ? q.tn + rank : q.rt;
+                const bool exists = tile128 < (isw ? g.NT : g.MT);   // (else: sums that nobody stores)
+                const unsigned char* src = (isw ? g.ew : g.ea) + (size_t)tile128 * g.KB * kGemmUnit;
                 for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
                     const uint32_t bytes = (uint32_t)min(kGemmKU, q.kb1 - kb) * kGemmUnit;
                     ok = tr ? wait.timed(BAR_EMPTY(s), ph ^ 1, tr_w) : wait(BAR_EMPTY(s), ph ^ 1);
                     if (!ok) break;
-                    const uint32_t dst = smem_u32(smem + (size_t)s * STAGE);
-                    if (isw) {
+                    if (!PAIR || exists) {
                         mbar_expect_tx(BAR_FULL(s), bytes);
-                        bulk_g2s(dst + OFF_W, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
+                        bulk_g2s(smem_u32(smem + (size_t)s * STAGE) + (isw ? OFF_W : 0u), src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
                     } else {
-                        mbar_expect_tx(BAR_FULL(s), (q.two ? 2u : 1u) * bytes);
-                        bulk_g2s(dst, src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
-                        if (q.two)
-                            bulk_g2s(dst + kGemmKU * kGemmUnit, src + (size_t)(g.KB + kb) * kGemmUnit, bytes, BAR_FULL(s));
+                        mbar_arrive(BAR_FULL(s));
                     }
                     issued++;
                     if (++s == NST) { s = 0; ph ^= 1; }
@@ -216,9 +306,23 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                 for (int s2 = 0; s2 < NST; s2++) {
                     const bool this_pass = s2 < s;
                     if (!this_pass && issued < (uint32_t)NST) continue;
-                    for (int i = 0; i < (1 << 20); i++)
-                        if (mbar_try_wait(BAR_FULL(s2), this_pass ? ph : ph ^ 1)) break;
+                    for (int i = 0; i < (PAIR ? 1 << 16 : 1 << 20); i++)
+                        if (PAIR ? mbar_test_wait(BAR_FULL(s2), this_pass ? ph : ph ^ 1) : mbar_try_wait(BAR_FULL(s2), this_pass ? ph : ph ^ 1)) break;
                 }
+            }
+        }
+        __syncwarp();
+    } else if (PAIR && warp == 9 && rank == 1) {
+        // =============================== relay: this CTA's stage is there ===================
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        for (int t = t_first; t < ntiles && ok; t += t_step) {
+            const Tile q = tile(t);
+            for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
+                ok = wait.spin(BAR_FULL(s), ph);
+                if (!ok) break;
+                if (lane == 0) mbar_arrive_leader(BAR_FULL(s));
+                if (++s == (uint32_t)NST) { s = 0; ph ^= 1; }
             }
         }
         __syncwarp();
@@ -227,18 +331,17 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         // (what the next stage needs is worked out and asked for while this one's MMAs are queued: the
         // same scheme as in bconv_umma_pre.cuh, reasons there)
         const uint32_t leader = elect_one() ? 1u : 0u;
-        constexpr uint32_t IDESC = idesc_f4(128);
+        constexpr uint32_t IDESC = PAIR ? idesc_f4(256) + ((128u >> 4) << 24) : idesc_f4(128);   // (M = 256: one step up)
         const uint64_t desc0 = smem_desc(smem_u32(smem), 128 * 16, 128u);
         const uint32_t hi = (uint32_t)(desc0 >> 32), lo0 = (uint32_t)desc0;
-        constexpr uint32_t stepStage = STAGE >> 4, stepUnit = kGemmUnit >> 4, offW = OFF_W >> 4,
-                           offA2 = (kGemmKU * kGemmUnit) >> 4;
+        constexpr uint32_t stepStage = STAGE >> 4, stepUnit = kGemmUnit >> 4, offW = OFF_W >> 4;
         const uint32_t units[4] = {0u, stepUnit, 2 * stepUnit, 3 * stepUnit};
         const uint32_t sfa = tmem + SF_COL, sfb = tmem + SF_COL + 16;
         uint32_t s = 0, ph = 0, b = 0, bph = 0, ready = 0, need = 3u;
         bool ok = true;
         long long tr_w = 0;
         const long long tr_t0 = clock64();
-        int t = blockIdx.x, tr_kb = 0;
+        int t = t_first, tr_kb = 0;
         Tile q = tile(t < ntiles ? t : 0);
         int kb = q.kb0;
         while (t < ntiles) {
@@ -257,15 +360,18 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             uint32_t acc = kb > q.kb0 ? 1u : 0u;
             const uint32_t d = tmem + b * 128;
             uint32_t aLo = lo0 + s * stepStage, bLo = aLo + offW;
-            if (nkb == kGemmKU) {
-                if (q.two) mma_f4_run<4>(leader, d + 128, aLo + offA2, hi, bLo, hi, stepUnit, units, IDESC, acc, sfa, sfb);
+            if constexpr (PAIR) {
+                for (int j = 0; j < (nkb == kGemmKU ? 1 : nkb - 1); j++) {
+                    mma_f4_pair_run(leader, d, aLo + j * stepUnit, bLo + j * stepUnit, hi, stepUnit, IDESC, acc, sfa, sfb);
+                    acc = 1;
+                }
+            } else if (nkb == kGemmKU) {
                 mma_f4_run<1>(leader, d, aLo, hi, bLo, hi, stepUnit, units, IDESC, acc, sfa, sfb);
             } else {
-                for (int j = 0; j < nkb; j++) {
+                for (int j = 0; j + 1 < nkb; j++) {
                     const uint32_t o = j * stepUnit;
-                    if (q.two) mma_f4_run<1>(leader, d + 128, aLo + offA2, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
-                    if (j + 1 < nkb) mma_f4_run<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
-                    if (j + 1 < nkb) acc = 1;
+                    mma_f4_run<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb);
+                    acc = 1;
                 }
             }
             asm volatile("" : "+r"(s), "+r"(b), "+r"(ph), "+r"(bph), "+r"(kb));   // what follows stays behind those MMAs
@@ -282,16 +388,23 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             need = last ? 3u : 1u;
             // (while a tile is being issued, its own accumulator is what bar1 names; the answer counts
             // only at the first stage of a tile)
-            if (nkb == kGemmKU)
+            const uint32_t o = (nkb - 1) * stepUnit;
+            if constexpr (PAIR) {
+                if (nkb == kGemmKU)
+                    ready = mma_f4_pair_end<3>(leader, d, aLo + stepUnit, bLo + stepUnit, hi, stepUnit, IDESC, 1u, sfa, sfb,
+                                               BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
+                else
+                    ready = mma_f4_pair_end<1>(leader, d, aLo + o, bLo + o, hi, stepUnit, IDESC, acc, sfa, sfb,
+                                               BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
+            } else if (nkb == kGemmKU) {
                 ready = mma_f4_end<3>(leader, d, aLo, hi, bLo + stepUnit, hi, stepUnit, units + 1, IDESC, 1u, sfa, sfb,
                                       BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
-            else {
-                const uint32_t o = (nkb - 1) * stepUnit;
+            } else {
                 ready = mma_f4_end<1>(leader, d, aLo, hi, bLo + o, hi, stepUnit, &o, IDESC, acc, sfa, sfb,
                                       BAR_FULL(s), ph, BAR_CEMPTY(b), bph ^ 1u, BAR_EMPTY(sc), bar_c);
             }
             if (last) {
-                t += gridDim.x;
+                t += t_step;
                 if (t < ntiles) { q = tile(t); kb = q.kb0; }
             } else {
                 kb += kGemmKU;
@@ -300,9 +413,12 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         if (tr && leader) { g.trace[11] = clock64() - tr_t0; g.trace[12] = tr_w; g.trace[14] = tr_kb; }
         if (!ok && leader) {
             // giving up: the MMAs already issued must have finished before tensor memory is freed
-            mma_commit(BAR_DRAIN);
+            if constexpr (PAIR)
+                asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(BAR_DRAIN) : "memory");
+            else
+                mma_commit(BAR_DRAIN);
             for (int i = 0; i < (1 << 20); i++)
-                if (mbar_try_wait(BAR_DRAIN, 0)) break;
+                if (PAIR ? mbar_test_wait(BAR_DRAIN, 0) : mbar_try_wait(BAR_DRAIN, 0)) break;
         }
         __syncwarp();
     } else if (warp < 8) {
@@ -311,12 +427,12 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         long long tr_w = 0, tr_body = 0;
         int b = 0;
         uint32_t bph = 0;
-        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        for (int t = t_first; t < ntiles; t += t_step) {
             const Tile q = tile(t);
-            const int sub = PAIR ? warp >> 2 : 0;       // 256 x 128: a warpgroup per sub-tile; 128 x 128: per column half
+            const int sub = PAIR ? warp >> 2 : 0;       // pair: a warpgroup per 128 columns; alone: per 64
             const int nb0 = PAIR ? 0 : (warp >> 2) * 2, nb1 = PAIR ? 4 : nb0 + 2;
-            const int m0 = (q.rt0 + sub) * 128 + quad * 32;                  // this warp's rows
-            const bool have = sub == 0 || q.two;
+            const int m0 = q.rt * 128 + quad * 32, tn = q.tn + sub;          // this warp's rows, its column tile
+            const bool have = !PAIR || (q.rt < g.MT && tn < g.NT);
             // thresholds of this warp's columns, in the accumulator's column order, while it is awaited
             // (a threshold per column straight from global memory costs a trip to L2 each: 6800 clocks
             // per tile).  NaN behind the last column: never reached.
@@ -324,7 +440,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             if (g.splits == 1 && g.mode == GEMM_FC_BITS) {
                 __syncwarp();
                 for (int nb = nb0; nb < nb1; nb++) {
-                    const int n = q.tn * 128 + nb * 32 + f4_channel_of_column(lane);
+                    const int n = tn * 128 + nb * 32 + f4_channel_of_column(lane);
                     thr[nb * 32 + lane] = n < g.N ? __ldg(g.p0 + n) : __int_as_float(0x7FC00000);
                 }
                 __syncwarp();
@@ -341,7 +457,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                     const int m = m0 + lane;
 #pragma unroll 1
                     for (int nb = nb0; nb < nb1; nb++) {
-                        const int n0 = q.tn * 128 + nb * 32;
+                        const int n0 = tn * 128 + nb * 32;
                         if (n0 >= g.N) break;
                         int v[32];
                         tmem_ld32(tcol + nb * 32, v);
@@ -371,7 +487,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                     const bool v4 = (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
 #pragma unroll 1
                     for (int nb = nb0; nb < nb1; nb++) {
-                        const int n0 = q.tn * 128 + nb * 32 + 4 * q4;
+                        const int n0 = tn * 128 + nb * 32 + 4 * q4;
                         float4 sc[2], bi[2];
                         if (!ints) {
 #pragma unroll
@@ -423,7 +539,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             }
             tc_fence_before();                          // this warp is done with the accumulator
             __syncwarp();
-            if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+            if (lane == 0) { if constexpr (PAIR) mbar_arrive_leader(BAR_CEMPTY(b)); else mbar_arrive(BAR_CEMPTY(b)); }
             tr_body += clock64() - e1;
             if (++b == NACC) { b = 0; bph ^= 1u; }
         }
@@ -431,7 +547,12 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) tmem_dealloc(tmem, TM_COLS);
+    if constexpr (PAIR) {
+        cluster_sync();                                 // nothing of the partner's reaches into this CTA any more
+        if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
+    } else if (warp == 9) {
+        tmem_dealloc(tmem, TM_COLS);
+    }
     if (g.trace != nullptr && blockIdx.x == 0 && tid == 0) g.trace[9] = clock64() - tr_cta0;
 }
 

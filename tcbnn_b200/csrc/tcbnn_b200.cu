@@ -215,15 +215,18 @@ __global__ void __launch_bounds__(256) k_expand_rows(const uint32_t* a_bits, int
                                                      int K, int KB, uint4* out_a, uint4* out_w) {
     umma::expand_rows_pair(a_bits, a_rows, a_ld, RT_a, w_bits, w_rows, w_ld, RT_w, K, KB, out_a, out_w);
 }
-template <bool PAIR>
 __global__ void __launch_bounds__(umma::kGemmThreads, 1) k_gemm_umma(umma::GemmUmmaArgs g) {
     extern __shared__ __align__(128) unsigned char dyn_smem_gemm[];
-    umma::gemm_umma_cta<PAIR>(g, dyn_smem_gemm);
+    umma::gemm_umma_cta<false>(g, dyn_smem_gemm);
+}
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(umma::kGemmThreads, 1) k_gemm_umma_pair(umma::GemmUmmaArgs g) {
+    extern __shared__ __align__(128) unsigned char dyn_smem_gemm[];
+    umma::gemm_umma_cta<true>(g, dyn_smem_gemm);
 }
 
 struct GemmUmmaPlan {
     bool use;
-    bool pair;            // 256 x 128 tiles (two sub-tiles of A per CTA) instead of 128 x 128
+    bool pair;            // 256 x 256 tiles on pairs of SMs instead of 128 x 128 on one
     int MT, NT, KB, splits, per;
     size_t off_ea, off_ew, off_partial, bytes;
 };
@@ -245,15 +248,16 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
     double best = 1e30;
     for (int pair = 0; pair < 2; pair++) {
         if (g_gemm_force_pair >= 0 && pair != g_gemm_force_pair) continue;
-        if (pair && p.MT < 2 && g_gemm_force_pair < 0) continue;
-        const long long tiles = (long long)(pair ? (p.MT + 1) / 2 : p.MT) * p.NT;
+        if (pair && (p.MT < 2 || p.NT < 2) && g_gemm_force_pair < 0) continue;
+        const long long tiles = pair ? (long long)((p.MT + 1) / 2) * ((p.NT + 1) / 2) : (long long)p.MT * p.NT;
         for (int want = 1; want <= 32 && (want <= (p.KB + 3) / 4 || g_gemm_force_splits > 0); want++) {
             const int per = (p.KB + want - 1) / want;
             const int splits = (p.KB + per - 1) / per;                    // no empty split
             if (splits != want && want > 1) continue;
             if (g_gemm_force_splits > 0 && want != (g_gemm_force_splits < p.KB ? g_gemm_force_splits : p.KB)) continue;
-            const long long waves = (tiles * splits + sms - 1) / sms;
-            double clk = pair ? (double)waves * (per * 180.0 + 3000.0) + 6000.0 : (double)waves * per * 140.0 + 7000.0;
+            const int slots = pair ? sms / 2 : sms;
+            const long long waves = (tiles * splits + slots - 1) / slots;
+            double clk = pair ? (double)waves * (per * 150.0 + 3000.0) + 6000.0 : (double)waves * per * 140.0 + 7000.0;
             if (splits > 1) clk += 12000.0 + 6.0 * splits * (double)M * N * 4.0 / 3000.0;
             if (clk < best) { best = clk; p.pair = pair != 0; p.splits = splits; p.per = per; }
         }
@@ -284,11 +288,9 @@ int expand_units(const uint32_t* a_bits, int M, int lda, void* a_units, const ui
 int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, const GemmUnits& u, int sms, cudaStream_t st) {
     static bool configured[64] = {false};
     if (configure_once(configured, [] {
-            cudaError_t e = cudaFuncSetAttribute(k_gemm_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)umma::gemm_smem(true));
+            cudaError_t e = cudaFuncSetAttribute(k_gemm_umma_pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)umma::kGemmSmem);
             if (e != cudaSuccess) return e;
-            return cudaFuncSetAttribute(k_gemm_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)umma::gemm_smem(false));
+            return cudaFuncSetAttribute(k_gemm_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)umma::kGemmSmem);
         }))
         return 1;
     char* w = (char*)workspace;
@@ -318,10 +320,11 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, con
     {
         // a programmatic dependent of the expansion launch: set-up (barriers, tensor memory, unit
         // scales) overlaps the expansion pass, the kernel waits for it before its first copy
-        const long long tiles = (long long)(p.pair ? (p.MT + 1) / 2 : p.MT) * p.NT * p.splits;
-        const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-        const cudaError_t e = launch_dependent(p.pair ? k_gemm_umma<true> : k_gemm_umma<false>, grid, umma::kGemmThreads,
-                                               umma::gemm_smem(p.pair), st, a);
+        const long long tiles = (p.pair ? (long long)((p.MT + 1) / 2) * ((p.NT + 1) / 2) : (long long)p.MT * p.NT) * p.splits;
+        const long long slots = p.pair ? sms / 2 : sms;
+        const unsigned grid = (unsigned)(tiles < slots ? tiles : slots) * (p.pair ? 2u : 1u);
+        const cudaError_t e = launch_dependent(p.pair ? k_gemm_umma_pair : k_gemm_umma, grid, umma::kGemmThreads,
+                                               umma::kGemmSmem, st, a);
         if (e != cudaSuccess) return fail("gemm (tcgen05): %s", cudaGetErrorString(e));
     }
     if (launch_check("gemm (tcgen05)")) return 1;
