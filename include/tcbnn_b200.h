@@ -53,8 +53,8 @@ size_t tcbnn_gemm_workspace_bytes(int M, int N, int K);
  * counterparts. */
 int tcbnn_set_gemm_path(int path);
 int tcbnn_gemm_status(int* status);
-/* Overrides what the tcgen05 GEMM derives from its cost model: `pair` 1 = CTAs own 256 x 128
- * tiles, 0 = 128 x 128, -1 = automatic; `splits` 1..32 = that many slices of K (1: the GEMM's own
+/* Overrides what the tcgen05 GEMM derives from its cost model: `pair` 1 = pairs of CTAs own
+ * 256 x 256 tiles, 0 = single ones 128 x 128, -1 = automatic; `splits` 1..32 = that many slices of K (1: the GEMM's own
  * epilogue finishes the layer; more: int32 partial sums and a finishing pass), -1 = automatic.
  * A forced plan also waives the M*N*K >= 2^30 rule.  A workspace sized by
  * tcbnn_gemm_workspace_bytes AFTER this call fits the forced plan.

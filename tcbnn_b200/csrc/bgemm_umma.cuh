@@ -6,17 +6,24 @@
 // One streaming pass first writes both operands as +-1 nibbles (0 for padding: rows past the end,
 // bits past K) in 4 KB units [128-row tile][64-bit k-block][32-bit chunk][row][16 B], the
 // no-swizzle K-major operand layout, so that a unit is one bulk copy and one MMA operand.
-// The GEMM is persistent: a CTA per SM walks over 128 x 128 or 256 x 128 tiles (one or two 128-row
-// sub-tiles of A against one tile of W), each over a range of k-blocks:
+// The GEMM is persistent: a CTA per SM walks over 128 x 128 tiles, or a pair of CTAs over 256 x 256
+// tiles (PAIR), each over a range of k-blocks:
 //
 //   warps 0-7  epilogue : tcgen05.ld and either finish the layer (one split: int32 / threshold bits /
 //                         scale + bias straight from the accumulator) or store int32 partial sums for
 //                         gemm_splitk_finish.  128 x 128 tiles alternate between two accumulators, so
 //                         that a tile is finished while the next one is computed
-//   warp  8    loader A : one lane, one bulk copy per sub-tile and stage (a stage holds up to
+//   warp  8    loader A : one lane, one bulk copy per stage (a stage holds up to
 //                         kGemmKU consecutive k-blocks, contiguous in the expanded operand)
-//   warp  9    MMA      : converged warp, elected lane: one N=128 MMA per sub-tile and k-block
+//   warp  9    MMA      : converged warp, elected lane: one MMA per k-block (in the second CTA of a pair
+//                         the relay that tells the first that a stage has arrived)
 //   warp  10   loader W : one lane, one bulk copy per stage
+//
+// A 128 x 128 tile reads 8 KB of operands per k-block and has 8 KB copied in, which fills the
+// shared-memory port for 128 clocks (136 measured) where its MMA takes 64.  A pair does four times the work on
+// twice the SMs: each reads its 128 rows of A and half of W, 4 + 4 KB, and receives as much, for an MMA that
+// takes 128 (131-152 measured).  8192 x 8192 x 8192 with threshold bits 204 -> 186 us against 256 x 128
+// tiles on one SM (28 KB and 220 clocks per k-block), the kernel itself 0.79 of the MMA rate.
 //
 // Loaders and issuer run ahead across tile boundaries, so set-up, first loads and epilogue of all
 // but a CTA's last tile are hidden: as one CTA per tile (two per SM) the MLP's hidden layer, 8192 x 1024
@@ -120,20 +127,24 @@ __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_r
 
 // ---- a pair of CTAs on one 256 x 256 tile (cta_group::2) ------------------------------------------
 // Each CTA holds its 128 rows of A, half of W's 256 rows and its 128 x 256 accumulator; the leader (even
-// rank) issues MMAs that read both shared memories.
+// rank) issues MMAs that read both shared memories.  A bulk copy completes on a barrier of the CTA it
+// writes to, so the second CTA relays: its warp 9 waits for a stage and arrives on the leader's barrier.
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// arrives on the leader's copy of a barrier
+// Arrives on the leader's copy of a barrier.  (The relay has written nothing itself; with .release.cluster
+// each arrival took about 1400 clocks, and a k-block 360 instead of 135.)
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
     asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
-                 "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar) : "memory");
+                 "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar) : "memory");
 }
-// WsWait with the bound in clocks, about a second: a CTA also waits for its partner
+// WsWait with the bound in clocks, about a second, as a CTA waits for its partner too.  Polls rather than
+// suspends: a stage passes through three barriers on its way (360 clocks per k-block with try_wait).
 struct GemmPairWait {
     volatile int* abort;
     int* err;
     __device__ __forceinline__ bool poll(uint32_t bar, uint32_t parity, bool sleep) const {
+        if (mbar_test_wait(bar, parity)) return true;
         const long long t0 = clock64();
         for (int i = 0; i < (1 << 28); i++) {
             if (mbar_test_wait(bar, parity)) return true;
@@ -314,15 +325,17 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
         __syncwarp();
     } else if (PAIR && warp == 9 && rank == 1) {
         // =============================== relay: this CTA's stage is there ===================
-        uint32_t s = 0, ph = 0;
-        bool ok = true;
-        for (int t = t_first; t < ntiles && ok; t += t_step) {
-            const Tile q = tile(t);
-            for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
-                ok = wait.spin(BAR_FULL(s), ph);
-                if (!ok) break;
-                if (lane == 0) mbar_arrive_leader(BAR_FULL(s));
-                if (++s == (uint32_t)NST) { s = 0; ph ^= 1; }
+        if (lane == 0) {
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (int t = t_first; t < ntiles && ok; t += t_step) {
+                const Tile q = tile(t);
+                for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
+                    ok = wait.spin(BAR_FULL(s), ph);
+                    if (!ok) break;
+                    mbar_arrive_leader(BAR_FULL(s));
+                    if (++s == (uint32_t)NST) { s = 0; ph ^= 1; }
+                }
             }
         }
         __syncwarp();

@@ -233,8 +233,8 @@ struct GemmUmmaPlan {
 
 // Tile shape and split count of the tcgen05 path from a clock model of its launches, calibrated
 // on the kernel's own cycle counters (tcbnn_conv_set_trace): a k-block costs a CTA that owns 128 x 128
-// tiles about 140 clocks (loads and operand reads share the shared-memory port), 256 x 128 tiles 180;
-// set-up, first loads and the last epilogue are paid once per CTA, the 256 x 128 epilogue (one
+// tiles about 140 clocks (loads and operand reads share the shared-memory port), a pair that owns 256 x 256
+// tiles 150; set-up, first loads and the last epilogue are paid once per CTA, the pair's epilogue (one
 // accumulator) once per tile; more than one split adds the finishing launch and the partial sums'
 // round trip.
 GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {

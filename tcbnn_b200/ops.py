@@ -368,7 +368,7 @@ def set_gemm_path(path):
 
 
 def set_gemm_plan(pair=-1, splits=-1):
-    """Force the tcgen05 GEMM's tile shape (1: 256 x 128, 0: 128 x 128) and split count; -1 = automatic."""
+    """Force the tcgen05 GEMM's tile shape (1: 256 x 256 on two SMs, 0: 128 x 128) and split count; -1 = automatic."""
     _l.call("tcbnn_set_gemm_plan", int(pair), int(splits))
 
 
