@@ -483,7 +483,7 @@ __device__ __forceinline__ uint32_t spread4(uint32_t b) {
 // The same packing for rows whose length is a multiple of 4 floats on a 16-byte aligned base: a
 // lane reads 16 bytes (four consecutive columns), a warp one 128-column block per load, and a
 // task is eight consecutive blocks of one row, all eight loads (4 KB) issued before the first is
-// used -- with 64 warps per SM that keeps up to 256 KB in flight.  Four ballots give one bit per
+// used -- with 48 warps per SM that keeps up to 192 KB in flight.  Four ballots give one bit per
 // (lane, component); lane L interleaves eight lanes' four bits into word L & 3 of block L >> 2.
 // rows * ceil(blocks / 8) must fit in 31 bits (the caller checks).
 // also(row, chunk, word): what else becomes of each word that holds columns.
