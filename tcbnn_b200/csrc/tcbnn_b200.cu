@@ -190,9 +190,13 @@ int launch_gemm_small(const GemmArgs& g, int KW, int NW, cudaStream_t st) {
     return 0;
 }
 
-// The tile: as large as still leaves every SM two blocks (fewer loads per MMA), but 16 rows where M has
-// no more.  K is cut into as many slices as it has 256-bit steps, up to 8; column groups fill the
-// block up to 8 warps where K is too short for that.  (Long K on few tiles: 16 slices.)
+// The tile: as large as still leaves every SM enough blocks (fewer loads per MMA), but 16 rows where M has
+// no more and 16 columns where N has no more.  Enough is the more, the shorter K is: a block is one chain of
+// load, MMA, exchange and store, and with one 256-bit step per warp the chain is all there is.  Measured
+// crossings in tiles per SM, 16 x 8 to 32 x 16 to 32 x 32: 12 and 12 at K = 256, 2-3 and 3 at 1024, 1 and 1.5 at 4096
+// (8192 x 1024 -> 10: 5.5 -> 4.1 us, 65536 x 1024 -> 10: 28.7 -> 15.0, 512 x 256 -> 1000: 14.5 -> 5.9 against one and
+// two per SM throughout).  K is cut into as many slices as it has 256-bit steps, up to 8; column groups
+// fill the block up to 8 warps where K is too short for that.  (Long K on few tiles: 16 slices.)
 int run_gemm_small(const GemmArgs& g, int sms, cudaStream_t st) {
     const int steps = (g.K + 255) / 256;
     auto tiles = [&](int rows, int cols) { return (long long)((g.M + rows - 1) / rows) * ((g.N + cols - 1) / cols); };
@@ -201,9 +205,10 @@ int run_gemm_small(const GemmArgs& g, int sms, cudaStream_t st) {
     if (steps >= 64 && tiles(16, 8) * 8 <= 16LL * sms) KW = 16;
     const int NWmax = 8 / KW > 1 ? 8 / KW : 1;
     auto groups = [&](int cols) { int nw = 1; while (nw < NWmax && nw * cols < g.N) nw *= 2; return nw; };
-    if (g.M <= 16 || tiles(32, 16) < sms) return launch_gemm_small<1, 1>(g, KW, groups(8), st);
+    const double per_sm = 12.0 / steps;
+    if (g.M <= 16 || tiles(32, 16) < (per_sm > 1.0 ? per_sm : 1.0) * sms) return launch_gemm_small<1, 1>(g, KW, groups(8), st);
     if (KW > 8) KW = 8;
-    if (tiles(32, 32) < 2LL * sms) return launch_gemm_small<2, 2>(g, KW, groups(16), st);
+    if (g.N <= 16 || tiles(32, 32) < (per_sm > 1.5 ? per_sm : 1.5) * sms) return launch_gemm_small<2, 2>(g, KW, groups(16), st);
     return launch_gemm_small<2, 4>(g, KW, groups(32), st);
 }
 

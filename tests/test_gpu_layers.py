@@ -69,6 +69,13 @@ def test_bgemm_fc_out(cuda, M, N, K, split):
     np.testing.assert_allclose(out, ref, rtol=1e-5, atol=1e-5)
 
 
+# around the sizes where the small GEMM goes to a larger tile (148 SMs): K = 250, 1000, 4100, ragged
+@pytest.mark.parametrize("M,N,K", [(513, 1000, 250), (2060, 1001, 250), (8200, 10, 1000), (14300, 13, 1000), (8300, 70, 1000),
+                                   (1000, 70, 4100), (2080, 99, 4100)])
+def test_small_gemm_tiles(cuda, M, N, K):
+    test_bgemm_fc_out(cuda, M, N, K, False)
+
+
 UMMA_GEMM_CASES = [
     # M, N, K, pair, splits: large enough for the tcgen05 GEMM (M*N*K >= 2^30, less with a forced
     # plan), ragged on purpose.
