@@ -81,12 +81,19 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
                    size_t workspace_bytes, void* stream);
 /* The same with operands in the tcgen05 GEMM's own form ("units": +-1 4-bit values in 4 KB blocks), for
  * chains of FC layers.  tcbnn_fc_units_bytes(M, N, K, rows) is the size of `rows` rows of K for a layer of
- * that shape, 0 where the layer does not run on that kernel.  w_units: the layer's weight, expanded once
- * by tcbnn_fc_expand_weight; a_units: its input, written by the producer; next_units: the output
+ * that shape, 0 where the layer does not run on that kernel.  w_units: the layer's weight as
+ * tcbnn_fc_expand_weight or tcbnn_pack_rows_w last expanded it -- a weight written to since has to be expanded
+ * again; a_units: its input, written by the producer; next_units: the output
  * bits also go there, as the next layer's a_units (K = N here).  tcbnn_pack_rows_x writes the first
- * layer's.  Buffers are 256-byte aligned and zeroed by the caller once; A, W and out are as above, and are
+ * layer's; tcbnn_pack_rows_w also expands weights in the same launch, so that a pass over a chain can
+ * follow its weights at next to no cost.  Buffers are 256-byte aligned and zeroed by the caller once; A, W and out are as above, and are
  * what a call uses whose shape takes another kernel.  Any of the three may be NULL.  No reference
  * counterpart. */
+typedef struct tcbnn_fc_weight {
+    const uint32_t* W;      /* [N][ldw] packed rows of K */
+    int N, K, ldw;
+    void* units;            /* tcbnn_fc_units_bytes(M, N, K, N) */
+} tcbnn_fc_weight;
 size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows);
 int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units, void* stream);
 int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
@@ -94,6 +101,8 @@ int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int
                      const void* a_units, const void* w_units, void* next_units, void* stream);
 int tcbnn_pack_rows_x(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
                       void* stream);
+int tcbnn_pack_rows_w(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
+                      const tcbnn_fc_weight* weights, int n_weights, void* stream);
 /* Output layer: out[m][n] = fma((float)(K - 2*popc), scale[n], bias[n]), fp32 [M][ldo].
  * Out128LayerFMT, kernel.cuh:230-280. */
 int tcbnn_out_layer(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,

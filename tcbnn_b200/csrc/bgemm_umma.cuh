@@ -76,12 +76,43 @@ __device__ __forceinline__ void store_unit_chunk(uint4* units, int KB, int r, in
     units[((size_t)(r >> 7) * KB + (c >> 1)) * 256 + (c & 1) * 128 + (r & 127)] = e;
 }
 
-// packed bits [rows][ld words] (bit k of a row at bit 31 - k%32 of word k/32) -> units; one launch
-// expands both operands.  A task is (128-row tile, group of four k-blocks): 256 threads, two per
-// row, each reading the 16 bytes (four 32-bit chunks) of its row that fall into its half of the
-// group -- a whole 32-byte sector per row -- and writing four 16-byte slots; for a given chunk the
-// threads of a warp write two runs of 256 contiguous bytes.  Tasks [0, RT_a * KG) belong to A, the
-// rest to W (KG = groups per row tile).  lda / ldw are even, so the 8-byte loads are aligned.
+// packed bits [rows][ld words] (bit k of a row at bit 31 - k%32 of word k/32) -> units.  A task is
+// (128-row tile, group of four k-blocks): 256 threads, two per row, each reading the 16 bytes (four
+// 32-bit chunks) of its row that fall into its half of the group -- a whole 32-byte sector per row -- and
+// writing four 16-byte slots; for a given chunk the threads of a warp write two runs of 256 contiguous
+// bytes.  ld is even, so the 8-byte loads are aligned.  W's rows go in the order of the accumulator's columns.
+__device__ __forceinline__ void expand_rows_task(const uint32_t* bits, int rows, int ld, int K, int KB, int tk, bool isw, uint4* out) {
+    const int KG = (KB + 3) >> 2;
+    const int t = threadIdx.x, row = t >> 1, half = t & 1;
+    const int rt = tk / KG, kg = tk - rt * KG;
+    out += (size_t)rt * KB * 256;                                        // 256 slots of 16 bytes per unit
+    const int r = rt * 128 + (isw ? (row & ~31) + f4_channel_of_column(row & 31) : row);
+    const int w0 = kg * 8 + half * 4;                                    // first 32-bit chunk of this thread
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (r < rows) {
+        const uint32_t* src = bits + (size_t)r * ld + w0;
+        if (w0 + 1 < ld) { const uint2 q = __ldg(reinterpret_cast<const uint2*>(src)); w[0] = q.x; w[1] = q.y; }
+        else if (w0 < ld) w[0] = __ldg(src);
+        if (w0 + 3 < ld) { const uint2 q = __ldg(reinterpret_cast<const uint2*>(src + 2)); w[2] = q.x; w[3] = q.y; }
+        else if (w0 + 2 < ld) w[2] = __ldg(src + 2);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int c = w0 + j, kb = c >> 1;                               // chunk -> k-block
+        if (kb >= KB) break;
+        const int k0 = c * 32;
+        uint4 e = make_uint4(0u, 0u, 0u, 0u);
+        if (r < rows && k0 < K) {
+            e = expand32_f4(w[j]);
+            const int valid = K - k0;                                    // elements of this chunk that exist
+            if (valid < 32) e = keep32_f4(e, 0xFFFFFFFFu << (32 - valid));   // the rest is padding: 0, not -1
+        }
+        out[(size_t)kb * 256 + (c & 1) * 128 + row] = e;
+    }
+}
+
+// Both operands of a GEMM in one launch: tasks [0, RT_a * KG) belong to A, the rest to W (KG = groups per
+// row tile).
 __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_rows, int a_ld, int RT_a,
                                                  const uint32_t* w_bits, int w_rows, int w_ld, int RT_w,
                                                  int K, int KB, uint4* out_a, uint4* out_w) {
@@ -91,37 +122,27 @@ __device__ __forceinline__ void expand_rows_pair(const uint32_t* a_bits, int a_r
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int KG = (KB + 3) >> 2;
     const int tasks = (RT_a + RT_w) * KG;
-    const int t = threadIdx.x, row = t >> 1, half = t & 1;
     for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
         const bool isw = task >= RT_a * KG;
-        const int tk = isw ? task - RT_a * KG : task;
-        const int rt = tk / KG, kg = tk - rt * KG;
-        const uint32_t* bits = isw ? w_bits : a_bits;
-        const int rows = isw ? w_rows : a_rows, ld = isw ? w_ld : a_ld;
-        uint4* out = (isw ? out_w : out_a) + (size_t)rt * KB * 256;      // 256 slots of 16 bytes per unit
-        const int r = rt * 128 + (isw ? (row & ~31) + f4_channel_of_column(row & 31) : row);
-        const int w0 = kg * 8 + half * 4;                                // first 32-bit chunk of this thread
-        uint32_t w[4] = {0u, 0u, 0u, 0u};
-        if (r < rows) {
-            const uint32_t* src = bits + (size_t)r * ld + w0;
-            if (w0 + 1 < ld) { const uint2 q = __ldg(reinterpret_cast<const uint2*>(src)); w[0] = q.x; w[1] = q.y; }
-            else if (w0 < ld) w[0] = __ldg(src);
-            if (w0 + 3 < ld) { const uint2 q = __ldg(reinterpret_cast<const uint2*>(src + 2)); w[2] = q.x; w[3] = q.y; }
-            else if (w0 + 2 < ld) w[2] = __ldg(src + 2);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int c = w0 + j, kb = c >> 1;                           // chunk -> k-block
-            if (kb >= KB) break;
-            const int k0 = c * 32;
-            uint4 e = make_uint4(0u, 0u, 0u, 0u);
-            if (r < rows && k0 < K) {
-                e = expand32_f4(w[j]);
-                const int valid = K - k0;                                // elements of this chunk that exist
-                if (valid < 32) e = keep32_f4(e, 0xFFFFFFFFu << (32 - valid));   // the rest is padding: 0, not -1
-            }
-            out[(size_t)kb * 256 + (c & 1) * 128 + row] = e;
-        }
+        expand_rows_task(isw ? w_bits : a_bits, isw ? w_rows : a_rows, isw ? w_ld : a_ld, K, KB, isw ? task - RT_a * KG : task, isw,
+                         isw ? out_w : out_a);
+    }
+}
+
+// Weights that a pass over a chain of FC layers expands beside the packing of its input rows
+// (tcbnn_pack_rows_w): tasks are those of expand_rows_task, weight i's from first[i] on.
+constexpr int kMaxPassWeights = 8;
+struct PassWeights {
+    int n, first[kMaxPassWeights + 1];
+    const uint32_t* bits[kMaxPassWeights];
+    uint4* units[kMaxPassWeights];
+    int rows[kMaxPassWeights], ld[kMaxPassWeights], K[kMaxPassWeights];
+};
+__device__ __forceinline__ void expand_pass_weights(const PassWeights& p, int block, int blocks) {
+    for (int task = block; task < p.first[p.n]; task += blocks) {
+        int i = 0;
+        while (task >= p.first[i + 1]) i++;
+        expand_rows_task(p.bits[i], p.rows[i], p.ld[i], p.K[i], (p.K[i] + 63) >> 6, task - p.first[i], true, p.units[i]);
     }
 }
 

@@ -486,15 +486,17 @@ __device__ __forceinline__ uint32_t spread4(uint32_t b) {
 // used -- with 48 warps per SM that keeps up to 192 KB in flight.  Four ballots give one bit per
 // (lane, component); lane L interleaves eight lanes' four bits into word L & 3 of block L >> 2.
 // rows * ceil(blocks / 8) must fit in 31 bits (the caller checks).
-// also(row, chunk, word): what else becomes of each word that holds columns.
+// also(row, chunk, word): what else becomes of each word that holds columns.  The grid's first `skip`
+// blocks take no part.
 template <class F>
 __device__ __forceinline__ void pack_rows_vec(const float* x, int rows, int cols, int ld_words,
-                                              uint32_t* out, F&& also) {
+                                              uint32_t* out, int skip, F&& also) {
     constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const unsigned blocks = (unsigned)ld_words >> 2, chunks = (blocks + U - 1) / U;
-    const unsigned total = (unsigned)rows * chunks, step = (unsigned)grid_warps();
-    for (unsigned task = (unsigned)grid_warp(); task < total; task += step) {
+    const unsigned none = (unsigned)skip * (blockDim.x >> 5);
+    const unsigned total = (unsigned)rows * chunks, step = (unsigned)grid_warps() - none;
+    for (unsigned task = (unsigned)grid_warp() - none; task < total; task += step) {
         const unsigned row = task / chunks, blk0 = (task - row * chunks) * U;
         const float* xr = x + (size_t)row * cols;
         float4 f[U];

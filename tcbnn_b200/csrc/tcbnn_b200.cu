@@ -111,14 +111,24 @@ k_pack_rows(const float* x, int rows, int cols, int ld, uint32_t* out) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the consumer waits before it reads
     pack_rows(x, rows, cols, ld, out);
 }
-// UNITS: the FC layer behind takes its operand expanded too (bgemm_umma.cuh).  Six CTAs per SM: 8192 x 784
+// CHAIN: of a chain of FC layers.  The layer behind takes its operand expanded too (units, bgemm_umma.cuh), and
+// the grid's first blocks expand the weights of the layers to come.  Six CTAs per SM: 8192 x 784
 // 8.5 -> 5.8 us against eight, which left 32 registers for a task of eight 16-byte loads (80 bytes spilled).
-template <bool UNITS>
+template <bool CHAIN>
 __global__ void __launch_bounds__(kThreads, 6)
-k_pack_rows_vec(const float* x, int rows, int cols, int ld, uint32_t* out, uint4* units) {
+k_pack_rows_vec(const float* x, int rows, int cols, int ld, uint32_t* out, uint4* units, int weight_blocks,
+                const __grid_constant__ umma::PassWeights weights) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the consumer waits before it reads
-    pack_rows_vec(x, rows, cols, ld, out, [&](int row, int c, uint32_t word) {
-        if constexpr (UNITS) umma::store_unit_chunk(units, (cols + 63) >> 6, row, c, word, cols - c * 32);
+    if constexpr (CHAIN) {
+        if ((int)blockIdx.x < weight_blocks) {
+            umma::expand_pass_weights(weights, blockIdx.x, weight_blocks);
+            return;
+        }
+    }
+    pack_rows_vec(x, rows, cols, ld, out, CHAIN ? weight_blocks : 0, [&](int row, int c, uint32_t word) {
+        if constexpr (CHAIN) {
+            if (units) umma::store_unit_chunk(units, (cols + 63) >> 6, row, c, word, cols - c * 32);
+        }
     });
 }
 __global__ void k_unpack_rows(const uint32_t* in, int rows, int cols, int ld, float* out) {
@@ -291,6 +301,13 @@ int expand_units(const uint32_t* a_bits, int M, int lda, void* a_units, const ui
     if (e != cudaSuccess) return fail("gemm (operand expansion): %s", cudaGetErrorString(e));
     return 0;
 }
+
+int check_fc_weight(const tcbnn_fc_weight& w) {
+    if (w.N <= 0 || w.K <= 0 || (w.ldw & 1) || w.ldw * 32 < w.K || !w.W || ((uintptr_t)w.W & 7)) return fail("fc weight: bad sizes or alignment");
+    if (!w.units || ((uintptr_t)w.units & 255)) return fail("fc weight: units must be 256-byte aligned");
+    return 0;
+}
+long long fc_weight_tasks(const tcbnn_fc_weight& w) { return (long long)((w.N + 127) / 128) * (((w.K + 63) / 64 + 3) / 4); }
 
 int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, const GemmUnits& u, int sms, cudaStream_t st) {
     static bool configured[64] = {false};
@@ -1136,28 +1153,52 @@ int tcbnn_pack_rows(const float* x, int rows, int cols, int ld_words, uint32_t* 
 }
 
 int tcbnn_pack_rows_x(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units, void* stream) {
+    return tcbnn_pack_rows_w(x, rows, cols, ld_words, out, units, nullptr, 0, stream);
+}
+
+int tcbnn_pack_rows_w(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
+                      const tcbnn_fc_weight* weights, int n_weights, void* stream) {
     if ((uintptr_t)units & 255) return fail("pack_rows: units must be 256-byte aligned");
     if (rows <= 0 || cols <= 0) return fail("pack_rows: empty input");
     if ((ld_words & 3) || ld_words * 32 < cols) return fail("pack_rows: ld_words must be a multiple of 4 and cover cols");
     if ((uintptr_t)out & 15) return fail("pack_rows: output must be 16-byte aligned");
+    if (n_weights < 0 || (n_weights > 0 && !weights)) return fail("pack_rows: no weights given");
+    for (int i = 0; i < n_weights; i++)
+        if (check_fc_weight(weights[i])) return 1;
     int sms;
     if (sm_count(&sms)) return 1;
+    cudaStream_t st = (cudaStream_t)stream;
     const long long tasks = (long long)rows * (ld_words / 4);
     const long long vtasks = (long long)rows * ((ld_words / 4 + 7) / 8);
+    int taken = 0;                                       // weights this launch expands itself
     if ((cols & 3) == 0 && ((uintptr_t)x & 15) == 0 && vtasks < (1LL << 31)) {   // 16-byte loads, eight blocks per task
-        // memory-bound: all the CTAs an SM holds
-        long long ctas = (vtasks + kThreads / 32 - 1) / (kThreads / 32);
+        umma::PassWeights p = {};
+        while (taken < n_weights && taken < umma::kMaxPassWeights) {
+            const tcbnn_fc_weight& w = weights[taken];
+            const long long end = p.first[taken] + fc_weight_tasks(w);
+            if (end >= (1LL << 31)) break;
+            p.bits[taken] = w.W; p.units[taken] = (uint4*)w.units; p.rows[taken] = w.N; p.ld[taken] = w.ldw; p.K[taken] = w.K;
+            p.first[++taken] = (int)end;
+        }
+        p.n = taken;
+        // memory-bound: all the CTAs an SM holds, of which the weights (of which there is little) get a sixth at most
         const long long cap = 6LL * sms;
-        if (ctas > cap) ctas = cap;
-        if (units)
-            k_pack_rows_vec<true><<<(int)ctas, kThreads, 0, (cudaStream_t)stream>>>(x, rows, cols, ld_words, out, (uint4*)units);
+        const int wb = (int)(p.first[taken] < sms ? p.first[taken] : sms);
+        long long ctas = (vtasks + kThreads / 32 - 1) / (kThreads / 32);
+        if (ctas > cap - wb) ctas = cap - wb;
+        if (units || wb)
+            k_pack_rows_vec<true><<<(int)ctas + wb, kThreads, 0, st>>>(x, rows, cols, ld_words, out, (uint4*)units, wb, p);
         else
-            k_pack_rows_vec<false><<<(int)ctas, kThreads, 0, (cudaStream_t)stream>>>(x, rows, cols, ld_words, out, nullptr);
-        return launch_check("pack_rows");
-    } else
-        k_pack_rows<<<warp_grid(tasks, sms), kThreads, 0, (cudaStream_t)stream>>>(x, rows, cols, ld_words, out);
-    if (launch_check("pack_rows")) return 1;
-    return units ? expand_units(out, rows, ld_words, units, nullptr, 0, 0, nullptr, cols, sms, (cudaStream_t)stream) : 0;
+            k_pack_rows_vec<false><<<(int)ctas, kThreads, 0, st>>>(x, rows, cols, ld_words, out, nullptr, 0, p);
+        if (launch_check("pack_rows")) return 1;
+    } else {
+        k_pack_rows<<<warp_grid(tasks, sms), kThreads, 0, st>>>(x, rows, cols, ld_words, out);
+        if (launch_check("pack_rows")) return 1;
+        if (units && expand_units(out, rows, ld_words, units, nullptr, 0, 0, nullptr, cols, sms, st)) return 1;
+    }
+    for (int i = taken; i < n_weights; i++)
+        if (expand_units(nullptr, 0, 0, nullptr, weights[i].W, weights[i].N, weights[i].ldw, weights[i].units, weights[i].K, sms, st)) return 1;
+    return 0;
 }
 
 int tcbnn_unpack_rows(const uint32_t* in, int rows, int cols, int ld_words, float* out, void* stream) {
@@ -1260,8 +1301,8 @@ size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows) {
 }
 
 int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units, void* stream) {
-    if (N <= 0 || K <= 0 || (ldw & 1) || ldw * 32 < K || ((uintptr_t)W & 7)) return fail("fc_expand_weight: bad sizes or alignment");
-    if (!units || ((uintptr_t)units & 255)) return fail("fc_expand_weight: units must be 256-byte aligned");
+    const tcbnn_fc_weight w{W, N, K, ldw, units};
+    if (check_fc_weight(w)) return 1;
     int sms;
     if (sm_count(&sms)) return 1;
     return expand_units(nullptr, 0, 0, nullptr, W, N, ldw, units, K, sms, (cudaStream_t)stream);

@@ -17,6 +17,11 @@ class ConvDesc(C.Structure):
                  "pad_h", "pad_w", "OH", "OW")]
 
 
+class FcWeight(C.Structure):
+    """struct tcbnn_fc_weight of include/tcbnn_b200.h."""
+    _fields_ = [("W", C.c_void_p), ("N", C.c_int), ("K", C.c_int), ("ldw", C.c_int), ("units", C.c_void_p)]
+
+
 _P = C.c_void_p
 _I = C.c_int
 _LL = C.c_longlong
@@ -41,6 +46,7 @@ SIGNATURES = {
     "tcbnn_fc_expand_weight": (_I, [_P, _I, _I, _I, _P, _P]),
     "tcbnn_fc_layer_x": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P, _P, _P]),
     "tcbnn_pack_rows_x": (_I, [_P, _I, _I, _I, _P, _P, _P]),
+    "tcbnn_pack_rows_w": (_I, [_P, _I, _I, _I, _P, _P, C.POINTER(FcWeight), _I, _P]),
     "tcbnn_out_layer": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
     "tcbnn_conv_shape": (_I, [C.POINTER(ConvDesc)]),
     "tcbnn_conv_prepared_bytes": (_SZ, [C.POINTER(ConvDesc)]),

@@ -289,29 +289,35 @@ class Network:
             cons.input_planes = planes
 
     def _wire_units(self):
-        """FC layers on the tcgen05 GEMM: the weight is expanded once, and a producer that packs bits
-        (the input layer, another FC layer) writes the expanded input too."""
+        """FC layers on the tcgen05 GEMM: a producer that packs bits (the input layer, another FC layer) also
+        writes them expanded, and where the network starts with an input layer, its launch expands the
+        weights.  Both are done anew in every pass."""
         for prod, cons in zip(self.layers, self.layers[1:]):
             if type(cons).__name__ != "Fc128LayerParam":
                 continue
             M, K, N, dev = cons.input_height, cons.input_width, cons.weight_width, cons.weight_gpu.device
-            cons.weight_units = ops.fc_units(M, N, K, N, dev)
-            if cons.weight_units is None:
-                continue
-            ops.fc_expand_weight(cons.weight_gpu, K, cons.weight_units)
             if type(prod).__name__ in ("In128LayerParam", "Fc128LayerParam"):
                 cons.units_room = ops.fc_units(M, N, K, M, dev)
-            cons.units_versions = cons.versions()
+            if type(self.layers[0]).__name__ == "In128LayerParam":
+                cons.weight_room = ops.fc_units(M, N, K, N, dev)
         self._use_units()
 
     def _use_units(self):
-        """Producers write expanded inputs while the live batch has their consumer on the kernel that
-        reads them."""
+        """Expanded operands are written while the live batch has the layer on the kernel that reads
+        them."""
+        expands = []
         for prod, cons in zip(self.layers, self.layers[1:]):
-            room = getattr(cons, "units_room", None)
-            if room is not None:
-                used = ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0
-                cons.input_units = prod.next_units = room if used else None
+            if type(cons).__name__ != "Fc128LayerParam" or (cons.units_room is None and cons.weight_room is None):
+                continue
+            used = ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0
+            if cons.units_room is not None:
+                cons.producer = prod
+                cons.input_units = prod.next_units = cons.units_room if used else None
+            cons.weight_units = cons.weight_room if used else None
+            if cons.weight_units is not None:
+                expands.append(cons)
+        if type(self.layers[0]).__name__ == "In128LayerParam":
+            self.layers[0].expands = tuple(expands)
 
     def _wire_residual_layouts(self):
         """An int16 residual tensor is kept in the chunk-major layout (TCBNN_RES_INT16_CHUNKED)
@@ -370,7 +376,7 @@ class Network:
         seen, graph = 0, None
         if p is not None and p[1] == lib.settings_generation and p[2] == device and not torch.cuda.is_current_stream_capturing():
             for l, c in zip(self.layers, p[0]):
-                if c is not l.__dict__.get("_call") or not l._call_valid(c):
+                if c is not l._calls[True] or not l._call_valid(c):
                     break
             else:
                 graph, seen = p[3], p[4]
@@ -381,8 +387,8 @@ class Network:
             graph.replay()
             return self.layers[-1].get_output_gpu()
         for l in self.layers:
-            l.forward()
-        self._pass = ([l.__dict__.get("_call") for l in self.layers], lib.settings_generation, device, None, seen + 1)
+            l.forward(in_pass=True)
+        self._pass = ([l._calls[True] for l in self.layers], lib.settings_generation, device, None, seen + 1)
         return self.layers[-1].get_output_gpu()
 
     def _record(self):
@@ -398,7 +404,7 @@ class Network:
                 graph.capture_begin(capture_error_mode="thread_local")
                 try:
                     for l in self.layers:
-                        l.forward()
+                        l.forward(in_pass=True)
                 finally:
                     graph.capture_end()
         except RuntimeError:
@@ -417,7 +423,7 @@ class Network:
         g = graphs.get(key)
         if g is None:
             for l in self.layers:
-                l.forward()
+                l.forward(in_pass=True)
             torch.cuda.synchronize()
             g = self._record()
             if g is None:

@@ -76,22 +76,32 @@ def _dev():
 
 
 class _Layer:
-    """What the layer classes share: forward() makes one call of the C ABI whose arguments are worked
-    out once (_call_args) and kept until an attribute of the object is set -- a buffer, the live batch,
-    a hand-over -- so that a pass over a network of small layers is not spent on preparing arguments."""
+    """What the layer classes share.  A layer's call of the C ABI is prepared once (_call_args) and kept
+    until an attribute of the object is set -- a buffer, the live batch, a hand-over -- so that a pass
+    over a network of small layers is not spent on preparing arguments.
+
+    There are two such calls.  forward() runs the layer by itself, on the bits in input_gpu.
+    forward(in_pass=True) is a layer's turn in a pass over a whole network (models.Network): the layer in
+    front has just run, and what it handed over besides its bits (expanded operands) is used."""
 
     def __setattr__(self, name, value):
-        self.__dict__[name] = value
-        self.__dict__["_call"] = None
+        d = self.__dict__
+        d[name] = value
+        d["_calls"] = [None, None]
 
-    def forward(self):
-        c = self.__dict__.get("_call")
-        if c is None or not self._call_valid(c):
-            name, *rest = self._call_args()
-            # after the arguments: tensors and descriptors they point into, what _call_valid looks at
-            c = self.__dict__["_call"] = (ops._l.bound(name), *rest)
+    def forward(self, in_pass=False):
+        c = self.call(in_pass)
         if c[0](*c[1], ops._stream()) != 0:
             raise ops._l.TcbnnError(ops._l.load().tcbnn_last_error().decode())
+
+    def call(self, in_pass):
+        """The prepared call: (entry point, its arguments without the stream, the tensors and descriptors
+        they point into)."""
+        c = self._calls[in_pass]
+        if c is None or not self._call_valid(c):
+            name, *rest = self._call_args(in_pass)
+            c = self._calls[in_pass] = (ops._l.bound(name), *rest)
+        return c
 
     def _call_valid(self, c):
         return True
@@ -105,7 +115,6 @@ class _Layer:
             c.desc.B = n
         else:
             c.live = n
-        c._call = None
         return c
 
 
@@ -138,12 +147,21 @@ class In128LayerParam(_Layer):
         src = src.reshape(-1, self.input_width)
         self.input_gpu[:src.shape[0]].copy_(src, non_blocking=True)
 
-    next_units = None      # the FC layer behind takes its input expanded (Fc128LayerParam.input_units)
+    # wired by models.Network: room for the input of the FC layer behind in expanded form
+    # (Fc128LayerParam.input_units), and the FC layers whose weights the pass expands in this launch
+    next_units = None
+    expands = ()
 
-    def _call_args(self):
-        x, out, nxt = self.input_gpu, self.output_gpu, self.next_units
-        return "tcbnn_pack_rows_x", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out),
-                                     ops._ptr(nxt)), (x, out, nxt)
+    def _call_args(self, in_pass):
+        x, out, nxt = self.input_gpu, self.output_gpu, self.next_units if in_pass else None
+        layers = self.expands if in_pass else ()
+        weights = (ops._l.FcWeight * len(layers))(*(l.fc_weight() for l in layers))
+        return "tcbnn_pack_rows_w", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out),
+                                     ops._ptr(nxt), weights, len(layers)), (x, out, nxt, [l.weight_gpu for l in layers])
+
+    def _call_valid(self, c):
+        # the weights it expands are those the FC layers have now
+        return all(l.weight_gpu is w for l, w in zip(self.expands, c[2][3]))
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -191,25 +209,26 @@ class Fc128LayerParam(_Layer):
             raise ValueError("%s: input rows of %d words do not cover K=%d" % (self.name, t.shape[1], K))
         self.input_gpu = t
 
-    # Operands in the GEMM kernel's own form (tcbnn_fc_layer_x), wired by models.Network: this layer's
-    # weight, its input as the producer writes it (units_room; input_units while the live batch takes that
-    # kernel), and the next FC layer's input.  They follow the packed operands: another input or weight
-    # tensor, or one written to since, drops them.
-    units_room = input_units = weight_units = next_units = units_versions = None
+    # Operands in the GEMM kernel's own form (tcbnn_fc_layer_x), wired by models.Network for its passes: this
+    # layer's input as its producer writes it (units_room; input_units while the live batch takes that
+    # kernel), the next FC layer's input, and room for this layer's weight where the first layer of
+    # every pass expands it (weight_units).  None of them outlives a pass: whoever writes the packed
+    # rows between two passes, by whatever means, is followed.
+    units_room = input_units = next_units = weight_room = weight_units = None
+    producer = None
 
     def __setattr__(self, name, value):
         super().__setattr__(name, value)
         if name == "input_gpu":
             self.units_room = self.input_units = None
-        elif name == "weight_gpu":
-            self.weight_units = None
 
-    def versions(self):
-        """Changes when torch writes to the packed operands (tensors of inference mode do not say)."""
-        return tuple(0 if t.is_inference() else t._version for t in (self.input_gpu, self.weight_gpu))
+    def fc_weight(self):
+        w = self.weight_gpu
+        ops._need_cuda(w)
+        return ops._l.FcWeight(w.data_ptr(), w.shape[0], self.input_width, w.shape[1], self.weight_units.data_ptr())
 
     def _call_valid(self, c):
-        return c[3] == self.versions()
+        return c[2][6] is (self.producer.output_gpu if self.producer is not None else None)
 
     def kernel_launches(self):
         # the operand expansion is not launched where both operands come expanded; where a finishing
@@ -217,16 +236,15 @@ class Fc128LayerParam(_Layer):
         return (self.launches - int(self.input_units is not None and self.weight_units is not None)
                 + int(self.next_units is not None and self.launches == 3))
 
-    def _call_args(self):
+    def _call_args(self, in_pass):
         a, w, thr, out, ws = self.input_gpu, self.weight_gpu, self.bn_gpu, self.output_gpu, self.workspace
         ops._need_cuda(a, w, thr)
-        versions = self.versions()
-        if self.units_versions is not None and self.units_versions != versions:
-            self.units_room = self.input_units = self.weight_units = None
-        u = (self.input_units, self.weight_units, self.next_units)
+        made = self.producer.output_gpu if self.producer is not None else None
+        u = (self.input_units if made is not None and made.data_ptr() == a.data_ptr() else None,
+             self.weight_units, self.next_units) if in_pass else (None, None, None)
         return "tcbnn_fc_layer_x", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
                                     a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws),
-                                    *(ops._ptr(t) for t in u)), (a, w, thr, out, ws, u), versions
+                                    *(ops._ptr(t) for t in u)), (a, w, thr, out, ws, u, made)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -272,7 +290,7 @@ class Out128LayerParam(_Layer):
     def kernel_launches(self):
         return self.launches
 
-    def _call_args(self):
+    def _call_args(self, in_pass):
         a, w, out, ws = self.input_gpu, self.weight_gpu, self.output_gpu, self.workspace
         scale, bias = self.bn_scale_gpu, self.bn_bias_gpu
         ops._need_cuda(a, w, scale, bias)
@@ -381,7 +399,7 @@ class InConv128LayerParam(_Layer):
         src = src.reshape((-1,) + tuple(self.input_gpu.shape[1:]))
         self.input_gpu[:src.shape[0]].copy_(src, non_blocking=True)
 
-    def _call_args(self):
+    def _call_args(self, in_pass):
         d, x, f, thr, lut = self.desc, self.input_gpu, self.filter_gpu, self.bn_gpu, self.input_lut_gpu
         out, res, spec = self.output_gpu, self.output_residual_gpu, self.specialized
         nxt = self.next_layer if spec is not None else None
@@ -470,7 +488,7 @@ class Conv128LayerParam(_Layer):
         if n != self.desc.B and self.input_planes is not None:
             self.input_planes.zero_()
         self.desc.B = n
-        self._call = None                # the scratch a call needs depends on the batch
+        self.desc = self.desc            # (prepares the call again: the scratch it needs depends on the batch)
 
     def set_input_gpu(self, t):
         d = self.desc
@@ -518,7 +536,7 @@ class Conv128LayerParam(_Layer):
         pools_output = self.desc.pool != 1 and has_ws          # tcgen05 on the pre-pool grid + OR-pooling pass
         return 1 + int(own_expand) + int(pools_output)
 
-    def _call_args(self):
+    def _call_args(self, in_pass):
         d, x, prep, thr = self.desc, self.input_gpu, self.prepared, self.bn_gpu
         res_in = self.input_residual_gpu if self.inject_residual else None
         out, res_out, planes, nxt = self.output_gpu, self.output_residual_gpu, self.input_planes, self.next_layer

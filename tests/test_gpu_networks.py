@@ -4,7 +4,8 @@ import pytest
 import torch
 
 import networks as onet
-from tcbnn_b200 import models
+import util
+from tcbnn_b200 import models, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -60,6 +61,80 @@ def test_fc_layers_hand_their_operands_over_expanded(cuda, batch, widths):
     plain = models.Network(spec, w, x, handover=False)
     plain.layers[2].weight_gpu.zero_()
     assert torch.equal(changed, plain.forward()) and not torch.equal(changed, want)
+
+
+def _write(how, t, new):
+    """`new` into tensor `t`, by a torch operation, past torch's version counter, or by this library."""
+    if how == "copy_":
+        t.copy_(new)
+    elif how == "data":
+        t.data.copy_(new)
+    else:
+        ops.fc_layer(new, torch.zeros((t.shape[1] * 32, 4), dtype=torch.int32, device=t.device),
+                     torch.zeros(t.shape[1] * 32, device=t.device), 128, out=t)
+
+
+def _fc_chain(batch=1100):
+    """Two FC layers on the tcgen05 GEMM between an input layer and the output layer, and other weights."""
+    spec = models.mlp_spec(batch)
+    w = models.synthetic_weights(spec, 31)
+    return spec, w, models.synthetic_input(spec, 32), models.synthetic_weights(spec, 33)
+
+
+@pytest.mark.parametrize("path", ["forward", "forward_graph", "feeder", "feeder_parts"])
+@pytest.mark.parametrize("how", ["copy_", "data", "library", "inference"])
+def test_fc_weights_written_between_passes_count(cuda, how, path):
+    """Whatever writes a packed weight between two passes is followed by the next one: on the call paths of
+    a network, its replayed passes and the feeder's, whole batches and parts."""
+    spec, w, x, other = _fc_chain(2200 if path == "feeder_parts" else 1100)      # (parts of 1100)
+    with torch.inference_mode(how == "inference"):
+        net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+        assert all(l.weight_units is not None for l in net.layers[2:4])
+        host = torch.from_numpy(x).pin_memory()
+        feeder = models.HostFeeder(net)
+        if path == "feeder_parts":
+            feeder.PART_BYTES = x.nbytes // 2
+        def run():
+            if path.startswith("feeder"):
+                got = []
+                feeder.run([host], lambda out: got.append(out.clone()))
+                return got[0]
+            return getattr(net, path)().clone()
+        want = plain.forward().clone()
+        for _ in range(4):                           # (forward() replays a graph by then)
+            assert torch.equal(run(), want)
+        g = util.rng(34)
+        for i in (2, 3):
+            t = net.layers[i].weight_gpu
+            if how == "library":                     # bits of an FC layer, N = K of the weight's rows
+                src = torch.from_numpy(util.rand_words(g, (t.shape[0], 4)).view(np.int32)).to(cuda)
+                _write(how, t, src)
+            else:
+                new = ops.pack_fc_weight(torch.from_numpy(other[2 * i - 2].reshape(1024, 1024)).to(cuda))
+                _write("copy_" if how == "inference" else how, t, new)
+            plain.layers[i].weight_gpu.copy_(t)
+        changed = plain.forward().clone()
+        assert not torch.equal(changed, want)
+        for _ in range(3):
+            assert torch.equal(run(), changed)
+
+
+@pytest.mark.parametrize("how", ["copy_", "data", "library"])
+def test_layer_called_by_itself_reads_its_input_rows(cuda, how):
+    """A layer object's own forward() computes from the packed rows in input_gpu, whoever wrote them last."""
+    spec, w, x, _ = _fc_chain()
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    net.forward()
+    before = net.layers[2].get_output_gpu().clone()
+    rows = net.layers[1].get_output_gpu()
+    g = util.rng(35)
+    words = 4 if how == "library" else rows.shape[1]
+    _write(how, rows, torch.from_numpy(util.rand_words(g, (rows.shape[0], words)).view(np.int32)).to(cuda))
+    plain.layers[1].get_output_gpu().copy_(rows)
+    net.layers[2].forward()
+    plain.layers[2].forward()
+    assert torch.equal(net.layers[2].get_output_gpu(), plain.layers[2].get_output_gpu())
+    assert not torch.equal(net.layers[2].get_output_gpu(), before)
 
 
 def test_vgg_cifar(cuda):
