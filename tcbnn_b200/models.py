@@ -287,6 +287,8 @@ class Network:
                 continue
             prod.next_layer = (cons.desc, planes)
             cons.input_planes = planes
+            if kind == "Conv128LayerParam" and prod.desc.pool != 1:
+                cons.pooling_producer = prod
 
     def _wire_units(self):
         """FC layers on the tcgen05 GEMM: a producer that packs bits (the input layer, another FC layer) also
@@ -348,6 +350,8 @@ class Network:
             if getattr(cons, "input_planes", None) is not None:
                 cons.input_planes = ops.new_planes(cons.desc, cons.input_gpu.device)
                 prod.next_layer = (cons.desc, cons.input_planes)
+                if cons.pooling_producer is not None:
+                    cons.pooling_producer = prod
         p._use_units()
         return p
 

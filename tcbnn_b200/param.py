@@ -80,9 +80,10 @@ class _Layer:
     until an attribute of the object is set -- a buffer, the live batch, a hand-over -- so that a pass
     over a network of small layers is not spent on preparing arguments.
 
-    There are two such calls.  forward() runs the layer by itself, on the bits in input_gpu.
-    forward(in_pass=True) is a layer's turn in a pass over a whole network (models.Network): the layer in
-    front has just run, and what it handed over besides its bits (expanded operands) is used."""
+    There are two such calls.  forward() runs the layer by itself, on the bits in input_gpu (or on the
+    planes it was wired to, Conv128LayerParam.input_planes).  forward(in_pass=True) is a layer's turn in a
+    pass over a whole network (models.Network): the layer in front has just run, and what it handed over
+    besides its bits (expanded operands) is used."""
 
     def __setattr__(self, name, value):
         d = self.__dict__
@@ -504,6 +505,9 @@ class Conv128LayerParam(_Layer):
     # layer's planes when its producer fills them.
     next_layer = None
     input_planes = None
+    # A producer that pools writes planes for passes over the network only: called by itself the layer
+    # expands the bits in input_gpu.
+    pooling_producer = None
     # chunk-major int16 residual tensors (TCBNN_RES_INT16_CHUNKED), wired by models.Network
     residual_chunked = False            # this layer's saved residual
     input_residual_chunked = False      # the injected one
@@ -543,16 +547,20 @@ class Conv128LayerParam(_Layer):
         ops._need_cuda(x, prep, thr, res_in)
         # planes that a producer fills, or the scratch shared by the layers that bring none
         ws = planes if planes is not None else ops.conv_workspace(d, x.device)
+        made = self.pooling_producer.output_gpu if self.pooling_producer is not None else x
+        ready = planes is not None and (made is x or (in_pass and made.data_ptr() == x.data_ptr()))
         name, args = ops.conv_call(d, x, prep, thr, res_in, self.residual_channels, self.residual_pool, out,
-                                   self.out_image_stride, res_out, None, ws, planes is not None, nxt,
+                                   self.out_image_stride, res_out, None, ws, ready, nxt,
                                    self.input_residual_chunked and self.inject_residual, self.residual_chunked,
                                    # int16 was chosen from the bound fan-in + bound of the injected residual
                                    self.residual_bound is not None and self.residual_bound <= 32767)
-        return name, args, (ws, d, x, prep, thr, res_in, out, res_out, nxt)
+        return name, args, (ws, d, x, prep, thr, res_in, out, res_out, nxt, made)
 
     def _call_valid(self, c):
         # the shared scratch is replaced when a larger layer asks for it
-        ws = c[2][0]
+        ws, made = c[2][0], c[2][9]
+        if self.pooling_producer is not None and made is not self.pooling_producer.output_gpu:
+            return False
         return ws is None or ws is self.__dict__.get("input_planes") or ws is ops.shared_scratch(ws.device)
 
     def get_output_gpu(self):

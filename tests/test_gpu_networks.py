@@ -137,6 +137,28 @@ def test_layer_called_by_itself_reads_its_input_rows(cuda, how):
     assert not torch.equal(net.layers[2].get_output_gpu(), before)
 
 
+@pytest.mark.parametrize("replaced", [False, True])
+def test_conv_behind_pooling_layer_follows_its_input_rows(cuda, replaced):
+    """A convolution behind a pooling layer, called by itself after its input rows were written to; and in a
+    pass after the producer was given another output tensor (the consumer keeps reading its own)."""
+    spec = models.vgg_cifar_spec(3)
+    w, x = models.synthetic_weights(spec, 36), models.synthetic_input(spec, 37)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    i = 1 + next(k for k, l in enumerate(net.layers) if type(l).__name__ == "Conv128LayerParam" and l.desc.pool == 2)
+    assert net.layers[i].input_planes is not None
+    net.forward()
+    before = net.layers[i].get_output_gpu().clone()
+    rows = net.layers[i - 1].get_output_gpu()
+    new = torch.from_numpy(util.rand_words(util.rng(38), tuple(rows.shape)).view(np.int32)).to(cuda)
+    for n in (net, plain):
+        if replaced:
+            n.layers[i - 1].output_gpu = torch.zeros_like(rows)
+        n.layers[i].input_gpu.copy_(new.reshape(n.layers[i].input_gpu.shape))
+        n.forward() if replaced else n.layers[i].forward()
+    assert torch.equal(net.layers[i].get_output_gpu(), plain.layers[i].get_output_gpu())
+    assert not torch.equal(net.layers[i].get_output_gpu(), before)
+
+
 def test_vgg_cifar(cuda):
     _compare(models.vgg_cifar_spec(8), 10, cuda)
 
