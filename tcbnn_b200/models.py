@@ -219,6 +219,77 @@ def synthetic_input_u8(spec, seed, batch=None):
     return u8, lut.astype(np.float32)
 
 
+_FACTS = (torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride)
+
+
+class _Pass:
+    """The prepared calls of one pass over a network's layers, which it makes at once, and the graph recorded
+    of them.  They serve while nothing they were prepared from has changed: an attribute of a layer, a descriptor, a
+    process-wide setting, the place or shape of a tensor (t.data = ... changes these in place).  The tensors
+    are kept alive but for the input, which is compared by its facts."""
+
+    def __init__(self, layers):
+        device = layers[0].output_gpu.device
+        while True:
+            scratch = ops.shared_scratch(device)
+            prepared = [l._call_args(True) for l in layers]
+            if scratch is ops.shared_scratch(device):                        # (else replaced by a larger one on the way)
+                break
+        self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
+        self.run()
+        # (noted behind the first launches: the GPU is busy meanwhile)
+        self.input = self._input_facts(layers)
+        self.kept = [t for _, _, keep in prepared for t in keep if t is not layers[0].input_gpu]
+        self.tensors = list({id(t): t for t in self.kept if torch.is_tensor(t)}.values())
+        self.facts = [list(map(f, self.tensors)) for f in _FACTS]
+        self.descs = list({id(d): d for d in self.kept if isinstance(d, lib.ConvDesc)}.values())
+        self.desc_facts = list(map(bytes, self.descs))
+        self.scratch = next((t for t in self.tensors if t is scratch), None)     # replaced when a larger layer asks for it
+        self.layers = list(layers)
+        self.generations = [l.generation for l in layers]
+        self.settings, self.device = lib.settings_generation, torch._C._cuda_getDevice()
+        self.seen, self.graph = 1, None
+
+    @staticmethod
+    def _input_facts(layers):
+        t = layers[0].input_gpu
+        return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
+
+    def holds(self, layers):
+        """Whether the layers would make the same calls now."""
+        return (self.layers == layers and [l.generation for l in layers] == self.generations and
+                self.input == self._input_facts(layers) and
+                all(list(map(f, self.tensors)) == g for f, g in zip(_FACTS, self.facts)) and
+                list(map(bytes, self.descs)) == self.desc_facts and
+                self.settings == lib.settings_generation and self.device == torch._C._cuda_getDevice() and
+                (self.scratch is None or self.scratch is ops.shared_scratch(self.scratch.device)))
+
+    def run(self):
+        stream = ops._stream()
+        for f, args in self.calls:
+            if f(*args, stream) != 0:
+                lib.check(1)
+
+    def record(self):
+        """The calls as a graph, or None where they cannot be recorded (another capture mode of the
+        caller's, say): they then go on being made one by one."""
+        graph = torch.cuda.CUDAGraph()
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                # thread_local: only this thread's calls are checked during the capture; another
+                # thread (e.g. a communicator's watchdog polling its events) is left alone.  (Not
+                # torch.cuda.graph: it collects garbage and empties the allocator's cache first, 50 to
+                # 100 ms per graph, and the launches allocate nothing.)
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    self.run()
+                finally:
+                    graph.capture_end()
+        except RuntimeError:
+            return None
+        return graph
+
+
 class Network:
     """Chain of layer objects built from a spec, the way the reference drivers build theirs
     (new XLayerParam(...) ; initialize(config, prev->get_output_gpu(), residual))."""
@@ -367,7 +438,7 @@ class Network:
         self._use_units()
         self.live_batch = n
 
-    _pass = None           # (layers' calls, settings, device, graph or None, passes seen) of the last pass
+    _pass = None           # of the last call of forward()
 
     def forward(self):
         """One pass over the layers on the current stream.  A pass that repeats the one before -- the
@@ -376,44 +447,19 @@ class Network:
         us one by one).  Anything that changes a layer's call (a buffer, the live batch, a
         process-wide setting) starts over."""
         p = self._pass
-        device = torch._C._cuda_getDevice()
-        seen, graph = 0, None
-        if p is not None and p[1] == lib.settings_generation and p[2] == device and not torch.cuda.is_current_stream_capturing():
-            for l, c in zip(self.layers, p[0]):
-                if c is not l._calls[True] or not l._call_valid(c):
-                    break
-            else:
-                graph, seen = p[3], p[4]
-        if graph is None and seen == 2:
-            graph = self._record()
-            self._pass = (p[0], p[1], device, graph, 3)
-        if graph is not None:
-            graph.replay()
+        if p is None or not p.holds(self.layers):
+            self._pass = _Pass(self.layers)
             return self.layers[-1].get_output_gpu()
-        for l in self.layers:
-            l.forward(in_pass=True)
-        self._pass = ([l._calls[True] for l in self.layers], lib.settings_generation, device, None, seen + 1)
+        capturing = torch.cuda.is_current_stream_capturing()
+        if not capturing:
+            if p.seen == 2:
+                p.graph = p.record()
+            p.seen += p.seen < 3
+        if p.graph is None or capturing:
+            p.run()
+        else:
+            p.graph.replay()
         return self.layers[-1].get_output_gpu()
-
-    def _record(self):
-        """The layers' launches as a graph, or None where they cannot be recorded (another capture mode
-        of the caller's, say): they then go on being made one by one."""
-        graph = torch.cuda.CUDAGraph()
-        try:
-            with torch.cuda.stream(torch.cuda.Stream()):
-                # thread_local: only this thread's calls are checked during the capture; another
-                # thread (e.g. a communicator's watchdog polling its events) is left alone.  (Not
-                # torch.cuda.graph: it collects garbage and empties the allocator's cache first, 50 to
-                # 100 ms per graph, and the launches allocate nothing.)
-                graph.capture_begin(capture_error_mode="thread_local")
-                try:
-                    for l in self.layers:
-                        l.forward(in_pass=True)
-                finally:
-                    graph.capture_end()
-        except RuntimeError:
-            return None
-        return graph
 
     def forward_graph(self):
         """forward() replayed from a CUDA graph: the layer launches (every entry point takes the
@@ -424,16 +470,15 @@ class Network:
         first = self.layers[0]
         key = (first.input_gpu.data_ptr(), getattr(self, "live_batch", None))
         graphs = self.__dict__.setdefault("_graphs", {})
-        g = graphs.get(key)
-        if g is None:
-            for l in self.layers:
-                l.forward(in_pass=True)
+        p = graphs.get(key)
+        if p is None:
+            p = _Pass(self.layers)
             torch.cuda.synchronize()
-            g = self._record()
-            if g is None:
+            p.graph = p.record()
+            if p.graph is None:
                 raise lib.TcbnnError("the layers' launches could not be recorded as a graph on this stream")
-            graphs[key] = g
-        g.replay()
+            graphs[key] = p
+        p.graph.replay()
         return self.layers[-1].get_output_gpu()
 
 

@@ -76,36 +76,24 @@ def _dev():
 
 
 class _Layer:
-    """What the layer classes share.  A layer's call of the C ABI is prepared once (_call_args) and kept
-    until an attribute of the object is set -- a buffer, the live batch, a hand-over -- so that a pass
-    over a network of small layers is not spent on preparing arguments.
+    """What the layer classes share.  forward() runs the layer by itself, on the bits in input_gpu (or on the
+    planes it was wired to, Conv128LayerParam.input_planes): one call of the C ABI, prepared (_call_args)
+    each time.  models.Network prepares the calls of a whole pass with in_pass=True -- the layer in front
+    has just run, and what it handed over besides its bits (expanded operands) is used -- and keeps them
+    while no layer's generation changes and no tensor moves."""
 
-    There are two such calls.  forward() runs the layer by itself, on the bits in input_gpu (or on the
-    planes it was wired to, Conv128LayerParam.input_planes).  forward(in_pass=True) is a layer's turn in a
-    pass over a whole network (models.Network): the layer in front has just run, and what it handed over
-    besides its bits (expanded operands) is used."""
+    # what a caller replaces from pass to pass: not a change of the layer
+    _PER_PASS = ()
 
     def __setattr__(self, name, value):
         d = self.__dict__
         d[name] = value
-        d["_calls"] = [None, None]
+        if name not in self._PER_PASS:
+            d["generation"] = d.get("generation", 0) + 1
 
-    def forward(self, in_pass=False):
-        c = self.call(in_pass)
-        if c[0](*c[1], ops._stream()) != 0:
-            raise ops._l.TcbnnError(ops._l.load().tcbnn_last_error().decode())
-
-    def call(self, in_pass):
-        """The prepared call: (entry point, its arguments without the stream, the tensors and descriptors
-        they point into)."""
-        c = self._calls[in_pass]
-        if c is None or not self._call_valid(c):
-            name, *rest = self._call_args(in_pass)
-            c = self._calls[in_pass] = (ops._l.bound(name), *rest)
-        return c
-
-    def _call_valid(self, c):
-        return True
+    def forward(self):
+        name, args, _ = self._call_args(False)
+        ops._l.call(name, *args, ops._stream())
 
     def part(self, first, n):
         """A layer object with this one's weights for n images of the batch, its activations in this
@@ -121,6 +109,8 @@ class _Layer:
 
 class In128LayerParam(_Layer):
     """param.h:115-222.  fp32 [input_height][input_width] -> bit rows."""
+
+    _PER_PASS = ("input_gpu",)
 
     def __init__(self, name, input_height, input_width):
         self.name = name
@@ -158,11 +148,7 @@ class In128LayerParam(_Layer):
         layers = self.expands if in_pass else ()
         weights = (ops._l.FcWeight * len(layers))(*(l.fc_weight() for l in layers))
         return "tcbnn_pack_rows_w", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out),
-                                     ops._ptr(nxt), weights, len(layers)), (x, out, nxt, [l.weight_gpu for l in layers])
-
-    def _call_valid(self, c):
-        # the weights it expands are those the FC layers have now
-        return all(l.weight_gpu is w for l, w in zip(self.expands, c[2][3]))
+                                     ops._ptr(nxt), weights, len(layers)), (x, out, nxt)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -228,9 +214,6 @@ class Fc128LayerParam(_Layer):
         ops._need_cuda(w)
         return ops._l.FcWeight(w.data_ptr(), w.shape[0], self.input_width, w.shape[1], self.weight_units.data_ptr())
 
-    def _call_valid(self, c):
-        return c[2][6] is (self.producer.output_gpu if self.producer is not None else None)
-
     def kernel_launches(self):
         # the operand expansion is not launched where both operands come expanded; where a finishing
         # launch computes the bits (launches == 3), the next layer's input is expanded from them
@@ -245,7 +228,7 @@ class Fc128LayerParam(_Layer):
              self.weight_units, self.next_units) if in_pass else (None, None, None)
         return "tcbnn_fc_layer_x", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
                                     a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws),
-                                    *(ops._ptr(t) for t in u)), (a, w, thr, out, ws, u, made)
+                                    *(ops._ptr(t) for t in u)), (a, w, thr, out, ws, *u)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -308,6 +291,8 @@ class Out128LayerParam(_Layer):
 
 class InConv128LayerParam(_Layer):
     """param.h:701-870.  First conv layer on fp32 NCHW images."""
+
+    _PER_PASS = ("input_gpu",)
 
     def __init__(self, name, input_height, input_width, filter_height, filter_width,
                  input_channels, output_channels, batch, stride_height=1, stride_width=1,
@@ -409,7 +394,7 @@ class InConv128LayerParam(_Layer):
             raise ops._l.TcbnnError("%s: uint8 images need a lut, fp32 images must not have one" % self.name)
         name, args = ops.inconv_call(d, x, f, thr, out, d.OH * d.OW * ((d.O + 31) // 32), res, None, lut, spec, nxt,
                                      self.residual_chunked)
-        return name, args, (d, x, f, thr, lut, out, res, spec, nxt)
+        return name, args, (d, x, f, thr, lut, out, res, spec, *(nxt or ()))
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -489,7 +474,6 @@ class Conv128LayerParam(_Layer):
         if n != self.desc.B and self.input_planes is not None:
             self.input_planes.zero_()
         self.desc.B = n
-        self.desc = self.desc            # (prepares the call again: the scratch it needs depends on the batch)
 
     def set_input_gpu(self, t):
         d = self.desc
@@ -554,14 +538,7 @@ class Conv128LayerParam(_Layer):
                                    self.input_residual_chunked and self.inject_residual, self.residual_chunked,
                                    # int16 was chosen from the bound fan-in + bound of the injected residual
                                    self.residual_bound is not None and self.residual_bound <= 32767)
-        return name, args, (ws, d, x, prep, thr, res_in, out, res_out, nxt, made)
-
-    def _call_valid(self, c):
-        # the shared scratch is replaced when a larger layer asks for it
-        ws, made = c[2][0], c[2][9]
-        if self.pooling_producer is not None and made is not self.pooling_producer.output_gpu:
-            return False
-        return ws is None or ws is self.__dict__.get("input_planes") or ws is ops.shared_scratch(ws.device)
+        return name, args, (ws, d, x, prep, thr, res_in, out, res_out, *(nxt or ()))
 
     def get_output_gpu(self):
         return self.output_gpu

@@ -5,7 +5,7 @@ import torch
 
 import networks as onet
 import util
-from tcbnn_b200 import models, ops
+from tcbnn_b200 import lib, models, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -135,6 +135,39 @@ def test_layer_called_by_itself_reads_its_input_rows(cuda, how):
     plain.layers[2].forward()
     assert torch.equal(net.layers[2].get_output_gpu(), plain.layers[2].get_output_gpu())
     assert not torch.equal(net.layers[2].get_output_gpu(), before)
+
+
+@pytest.mark.parametrize("which", ["mlp", "resnet18"])
+def test_tensor_given_another_storage_in_place_counts(cuda, which):
+    """layer.tensor.data = other moves a tensor under its layer: the next pass uses the new storage, replayed
+    passes and single calls alike.  (The old storage is kept alive throughout.)"""
+    spec = models.mlp_spec(8) if which == "mlp" else models.resnet18_spec(2, image=64, classes=100)
+    w, x = models.synthetic_weights(spec, 40), models.synthetic_input(spec, 41)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    for _ in range(4):
+        want = net.forward().clone()
+    old = []
+    for i in ((1, 3) if which == "mlp" else (4, len(spec["layers"]) - 2)):
+        for n in (net, plain):
+            t = n.layers[i].bn_gpu
+            old.append(t.detach())
+            t.data = t + 9.0
+    changed = plain.forward().clone()
+    assert not torch.equal(changed, want)
+    for _ in range(4):
+        assert torch.equal(net.forward(), changed)
+    i = 3 if which == "mlp" else 4
+    for n in (net, plain):
+        t = n.layers[i].bn_gpu
+        old.append(t.detach())
+        t.data = t - 20.0
+        n.layers[i].forward()
+    assert torch.equal(net.layers[i].get_output_gpu(), plain.layers[i].get_output_gpu())
+    fc = next(l for l in net.layers if type(l).__name__ == "Fc128LayerParam")
+    assert fc.weight_gpu.shape[0] > 4
+    fc.weight_gpu.t_()
+    with pytest.raises(lib.TcbnnError):              # refused as it always was: rows are no longer contiguous
+        net.forward()
 
 
 @pytest.mark.parametrize("replaced", [False, True])
