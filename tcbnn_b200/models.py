@@ -461,22 +461,28 @@ class Network:
             p.graph.replay()
         return self.layers[-1].get_output_gpu()
 
+    MAX_GRAPHS = 16
+
     def forward_graph(self):
         """forward() replayed from a CUDA graph: the layer launches (every entry point takes the
         stream and none allocates or synchronises) are captured once per input buffer, after one
         eager pass that lets the first layer compile its kernel variants, and replayed as one
         submission on the current stream.  Same launches, same results; the host's per-launch
-        work and the gaps between the launches go away."""
+        work and the gaps between the launches go away.  A graph serves while its pass holds (_Pass) and
+        keeps the buffers it points into alive; the last MAX_GRAPHS are kept."""
         first = self.layers[0]
         key = (first.input_gpu.data_ptr(), getattr(self, "live_batch", None))
         graphs = self.__dict__.setdefault("_graphs", {})
         p = graphs.get(key)
-        if p is None:
+        if p is None or not p.holds(self.layers):
             p = _Pass(self.layers)
             torch.cuda.synchronize()
             p.graph = p.record()
             if p.graph is None:
                 raise lib.TcbnnError("the layers' launches could not be recorded as a graph on this stream")
+            graphs.pop(key, None)
+            while len(graphs) >= self.MAX_GRAPHS:
+                graphs.pop(next(iter(graphs)))
             graphs[key] = p
         p.graph.replay()
         return self.layers[-1].get_output_gpu()

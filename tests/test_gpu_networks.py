@@ -170,6 +170,55 @@ def test_tensor_given_another_storage_in_place_counts(cuda, which):
         net.forward()
 
 
+def test_graph_is_recorded_again_when_its_pass_has_changed(cuda):
+    """forward_graph() after a layer's tensor was replaced, after a process-wide setting changed and for live
+    batches that come back: the results of a network without graphs.  The graphs kept are bounded."""
+    spec = models.mlp_spec(40)
+    w, x = models.synthetic_weights(spec, 42), models.synthetic_input(spec, 43)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    want = net.forward_graph().clone()
+    kept = [t for n in (net, plain) for t in (n.layers[2].bn_gpu, n.layers[3].weight_gpu)]     # (whoever reads these is caught)
+    for n in (net, plain):
+        n.layers[2].bn_gpu = n.layers[2].bn_gpu + 9.0
+        n.layers[3].weight_gpu = n.layers[3].weight_gpu.flip(0).contiguous()
+    changed = plain.forward().clone()
+    assert torch.equal(net.forward_graph(), changed) and not torch.equal(changed, want) and len(kept) == 4
+    net.MAX_GRAPHS = 3
+    for live in (40, 33, 7, 12, 40, 33):
+        net.set_batch(live)
+        assert torch.equal(net.forward_graph()[:live], changed[:live])
+        assert len(net._graphs) <= 3
+    held = net._graphs[next(reversed(net._graphs))]
+    ops.set_conv_path(6)
+    try:
+        assert torch.equal(net.forward_graph()[:33], changed[:33])
+        assert net._graphs[next(reversed(net._graphs))] is not held
+    finally:
+        ops.set_conv_path(0)
+
+
+def test_graph_keeps_off_scratch_that_was_replaced(cuda):
+    """The scratch shared by layers without planes grows for a larger layer: a graph recorded before that must
+    not write to the old one's memory, which by then belongs to somebody else."""
+    spec = models.vgg_cifar_spec(2)
+    w, x = models.synthetic_weights(spec, 44), models.synthetic_input(spec, 45)
+    torch.cuda.synchronize()
+    ops._scratch.clear()
+    torch.cuda.empty_cache()
+    net = models.Network(spec, w, x, handover=False)
+    net.set_batch(2)
+    want = net.forward_graph().clone()
+    size = ops.shared_scratch(cuda if cuda.index is not None else torch.device("cuda", 0)).numel()
+    d = ops.conv_desc(64, 32, 32, 128, 128, 3, 3, 1, 1)
+    assert ops.conv_workspace(d, torch.device("cuda", 0)).numel() > size
+    net.set_batch(1)                                # drops the layers' own hold on the old scratch
+    net.set_batch(2)
+    others = [torch.full((size,), 7, dtype=torch.uint8, device=cuda) for _ in range(3)]
+    for _ in range(2):
+        assert torch.equal(net.forward_graph(), want)
+    assert all(bool((t == 7).all()) for t in others)
+
+
 @pytest.mark.parametrize("replaced", [False, True])
 def test_conv_behind_pooling_layer_follows_its_input_rows(cuda, replaced):
     """A convolution behind a pooling layer, called by itself after its input rows were written to; and in a
