@@ -299,7 +299,7 @@ class Network:
         is provably small and is stored as int16 instead of int32.
         input_lut: images arrive as uint8 with this [3][256] table of their fp32 values.
         handover: producers write the pre-expanded input of the conv layers that follow them."""
-        self.spec = spec
+        self.spec, self.live_batch = spec, None
         B = spec["batch"]
         cfg = weights if hasattr(weights, "read") else param.ArrayConfig(weights)
         self.layers = []
@@ -408,18 +408,22 @@ class Network:
                 for c in cons:
                     c.input_residual_chunked = True
 
-    def part(self, first, n):
+    def part(self, first, n, planes=None):
         """A Network over images [first, first + n) of the live batch: this one's weights, input images and
         logits rows; the activations in between share this one's buffers, and what a producer lays out
-        for its consumer (planes) has room of its own, because that layout depends on the batch."""
+        for its consumer (planes) has room of its own, because that layout depends on the batch.
+        planes: a dict that parts of the same n which run one after another share theirs through."""
         p = Network.__new__(Network)
         p.spec, p.live_batch = self.spec, n
         p.layers = [l.part(first, n) for l in self.layers]
         p.layers[0].input_gpu = self.layers[0].input_gpu[first:first + n]
         p.layers[-1].output_gpu = self.layers[-1].output_gpu[first:first + n]
-        for prod, cons in zip(p.layers, p.layers[1:]):
+        for i, (prod, cons) in enumerate(zip(p.layers, p.layers[1:])):
             if getattr(cons, "input_planes", None) is not None:
-                cons.input_planes = ops.new_planes(cons.desc, cons.input_gpu.device)
+                room = None if planes is None else planes.get(i)
+                cons.input_planes = ops.new_planes(cons.desc, cons.input_gpu.device) if room is None else room
+                if planes is not None:
+                    planes[i] = cons.input_planes
                 prod.next_layer = (cons.desc, cons.input_planes)
                 if cons.pooling_producer is not None:
                     cons.pooling_producer = prod
@@ -471,7 +475,7 @@ class Network:
         work and the gaps between the launches go away.  A graph serves while its pass holds (_Pass) and
         keeps the buffers it points into alive; the last MAX_GRAPHS are kept."""
         first = self.layers[0]
-        key = (first.input_gpu.data_ptr(), getattr(self, "live_batch", None))
+        key = (first.input_gpu.data_ptr(), self.live_batch)
         graphs = self.__dict__.setdefault("_graphs", {})
         p = graphs.get(key)
         if p is None or not p.holds(self.layers):
@@ -518,11 +522,14 @@ class HostFeeder:
         self.n = 0
         self.pending = None
         self.part_copied = [[torch.cuda.Event() for _ in range(self.MAX_PARTS)] for _ in range(2)]
-        self.parts = {}                                  # (first, n) -> Network.part
+        self.cuts = [None, None]                         # how each slot's batch was copied
+        # the parts of the network as it is now: (first, n) -> Network.part, and the planes of parts of n
+        # images, which run one after another
+        self.parts, self.planes, self.parts_of = {}, {}, None
 
     def _cuts(self):
         """[(first, n)] of the live batch's parts."""
-        live = getattr(self.net, "live_batch", None) or self.net.spec["batch"]
+        live = self.net.live_batch or self.net.spec["batch"]
         b = self.bufs[0]
         k = max(1, min(self.MAX_PARTS, live * b[0].numel() * b.element_size() // self.PART_BYTES, live))
         size = (live + k - 1) // k
@@ -531,7 +538,7 @@ class HostFeeder:
     def _enqueue_copy(self, slot, x_host):
         buf = self.bufs[slot]
         x = x_host.reshape(buf.shape)
-        cuts = self._cuts()
+        cuts = self.cuts[slot] = self._cuts()
         with torch.cuda.stream(self.copy_stream):
             self.copy_stream.wait_event(self.free[slot])
             for i, (first, n) in enumerate(cuts):
@@ -541,11 +548,20 @@ class HostFeeder:
                     self.part_copied[slot][i].record(self.copy_stream)
             self.copied[slot].record(self.copy_stream)
 
+    def _network(self):
+        """What a part takes over from the network when it is made."""
+        layers = self.net.layers
+        return (self.net.live_batch, layers[-1].output_gpu.data_ptr(), [(l, l.generation) for l in layers],
+                [bytes(l.desc) for l in layers if hasattr(l, "desc")])
+
     def _run_parts(self, main, slot, cuts):
+        now = self._network()
+        if now != self.parts_of:
+            self.parts, self.planes, self.parts_of = {}, {}, now
         for i, (first, n) in enumerate(cuts):
             p = self.parts.get((first, n))
             if p is None:
-                p = self.parts[(first, n)] = self.net.part(first, n)
+                p = self.parts[(first, n)] = self.net.part(first, n, self.planes.setdefault(n, {}))
             main.wait_event(self.part_copied[slot][i])
             p.layers[0].input_gpu = self.bufs[slot][first:first + n]
             p.forward_graph() if self.graph else p.forward()
@@ -572,10 +588,10 @@ class HostFeeder:
                 slot ^= 1
                 self._enqueue_copy(slot, nxt)
             self.first.input_gpu = self.bufs[cur_slot]
-            cuts = self._cuts()
-            if len(cuts) > 1:
+            cuts = self.cuts[cur_slot]
+            if len(cuts) > 1 and cuts == self._cuts():
                 out = self._run_parts(main, cur_slot, cuts)
-            else:
+            else:                                        # (or the live batch has changed since it was copied)
                 main.wait_event(self.copied[cur_slot])
                 out = self.net.forward_graph() if self.graph else self.net.forward()
             self.free[cur_slot].record(main)
@@ -584,9 +600,9 @@ class HostFeeder:
             if result_host is not None:
                 # (two staging buffers: waiting for the read itself, which shares PCIe with the input
                 # copies, held the next pass back by 65 us at batch 256)
+                main.wait_event(self.stage_free[stage])      # (before its memory can go, too)
                 if self.staged[stage] is None or self.staged[stage].shape != out.shape:
                     self.staged[stage] = torch.empty_like(out)
-                main.wait_event(self.stage_free[stage])
                 self.staged[stage].copy_(out)
                 self.computed.record(main)
                 with torch.cuda.stream(self.read_stream):

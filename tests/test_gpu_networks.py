@@ -383,6 +383,55 @@ def test_host_feeder_computes_large_batches_in_parts(cuda, which, parts, graph):
         assert np.array_equal(last.numpy(), expect[-1])
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_host_feeder_parts_follow_the_network(cuda, graph):
+    """Between two runs a layer is given other thresholds, the logits tensor another storage, and from a
+    batch's callback, with the next batch copied in parts already, the live batch changes.  Parts of
+    the same size share their planes, and none is kept of a network that has changed."""
+    spec = models.resnet18_spec(6, image=64, classes=100)
+    w, bound = models.synthetic_weights(spec, 46), models.SYNTHETIC_IMAGE_ABS_BOUND
+    xs = [np.ascontiguousarray(models.synthetic_input(spec, 47 + i)) for i in range(4)]
+    net, plain = (models.Network(spec, w, xs[0], input_abs_bound=bound, handover=h) for h in (True, False))
+    feeder = models.HostFeeder(net, graph=graph)
+    feeder.PART_BYTES = xs[0].nbytes // 3                                   # 2, 2, 2
+    host = [torch.from_numpy(x).pin_memory() for x in xs]
+
+    def expect(live=6):
+        got = []
+        plain.set_batch(live)
+        for x in xs:
+            plain.set_input(x[:live])
+            got.append(plain.forward()[:live].clone())
+        return got
+
+    def run(on_result=lambda i: None):
+        got = []
+        def result(out):
+            got.append(out.clone())
+            on_result(len(got))
+        feeder.run(host, result)
+        return got
+
+    assert len(feeder._cuts()) == 3
+    first = expect()
+    assert all(torch.equal(a, b) for a, b in zip(run(), first))
+    old = [n.layers[5].bn_gpu for n in (net, plain)] + [net.layers[-1].output_gpu.detach()]
+    for n in (net, plain):
+        n.layers[5].bn_gpu = n.layers[5].bn_gpu + 9.0
+    net.layers[-1].output_gpu.data = torch.zeros_like(net.layers[-1].output_gpu)
+    second = expect()
+    assert not torch.equal(first[0], second[0]) and len(old) == 3
+    assert all(torch.equal(a, b) for a, b in zip(run(), second))
+    four = expect(4)
+    got = run(lambda i: net.set_batch(4) if i == 2 else None)
+    assert all(torch.equal(a, b) for a, b in zip(got[:2], second[:2]))
+    assert all(torch.equal(a[:4], b) for a, b in zip(got[2:], four[2:]))
+    net.set_batch(6)
+    assert all(torch.equal(a, b) for a, b in zip(run(), second)) and len(feeder.parts) == 3
+    planes = [[l.input_planes for l in p.layers if getattr(l, "input_planes", None) is not None] for p in feeder.parts.values()]
+    assert len(planes) == 3 and planes[0] and all(a is b for p in planes[1:] for a, b in zip(planes[0], p))
+
+
 @pytest.mark.parametrize("which", ["resnet18", "vgg_cifar", "mlp"])
 def test_set_batch_runs_ragged_batches_on_the_same_objects(cuda, which):
     """Layer objects built for 8 images process 5, then 8, then 3 images (Network.set_batch)
