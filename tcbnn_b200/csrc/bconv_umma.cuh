@@ -352,11 +352,11 @@ __device__ __forceinline__ int f4_acc_to_int(int raw) { return f4_acc_to_biased(
 // Four consecutive residual channels (element index i, a multiple of 4) widened to int32.
 __device__ __forceinline__ int4 ld_res4(const void* p, int bytes, size_t i) {
     if (bytes == 2) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2*>(reinterpret_cast<const short*>(p) + i));
+        const uint2 q = ld_dep(reinterpret_cast<const uint2*>(reinterpret_cast<const short*>(p) + i));
         return make_int4((int)(short)(q.x & 0xFFFFu), (int)(short)(q.x >> 16),
                          (int)(short)(q.y & 0xFFFFu), (int)(short)(q.y >> 16));
     }
-    return __ldg(reinterpret_cast<const int4*>(reinterpret_cast<const int*>(p) + i));
+    return ld_dep(reinterpret_cast<const int4*>(reinterpret_cast<const int*>(p) + i));
 }
 __device__ __forceinline__ int4 max4(int4 a, int4 b) {
     return make_int4(max(a.x, b.x), max(a.y, b.y), max(a.z, b.z), max(a.w, b.w));

@@ -82,7 +82,7 @@ __device__ __forceinline__ void expand_raster(const ConvWsArgs& a, uint4* planes
             const int n = fastdiv(vy, a.vh_mul, a.vh_sh), vr = vy - n * a.VH;
             const int iy = nplane == 4 ? 2 * vr + (pl >> 1) : vr, ix = nplane == 4 ? 2 * vx + (pl & 1) : vx;
             if (vr < a.OHg && vx < a.OWg && iy < a.H && ix < a.W) {
-                const uint2 b = ldg64(a.in + ((size_t)(n * a.H + iy) * a.W + ix) * Cw + cb * 2);
+                const uint2 b = ld_dep(reinterpret_cast<const uint2*>(a.in + ((size_t)(n * a.H + iy) * a.W + ix) * Cw + cb * 2));
                 e0 = expand32_f4(b.x); e1 = expand32_f4(b.y);
             }
         }
@@ -248,7 +248,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             float tf = __int_as_float(0x7FC00000);       // NaN: never "less", the bit is always set
             const int o = obase + (i & ~31) + f4_channel_of_column(i & 31);      // column i's channel
             if (o < a.O) {
-                const float t = __ldg(a.thr + o);
+                const float t = ld_dep(a.thr + o);
                 tf = t;
                 if (t == t) it = t >= 2147483520.0f ? INT_MAX : t <= -2147483648.0f ? INT_MIN : (int)ceilf(t);
             }
@@ -519,13 +519,13 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (live && o0 + oc < lim) {
                         const uint4* q = rin + (size_t)(oc >> 3) * a.res_in_npix;
                         if (a.residual_pool) {
-                            const uint4 w0 = __ldg(q + i00), w1 = __ldg(q + i00 + 1), w2 = __ldg(q + i00 + rw), w3 = __ldg(q + i00 + rw + 1);
+                            const uint4 w0 = ld_dep(q + i00), w1 = ld_dep(q + i00 + 1), w2 = ld_dep(q + i00 + rw), w3 = ld_dep(q + i00 + rw + 1);
                             r[j].x = __vmaxs2(__vmaxs2(w0.x, w1.x), __vmaxs2(w2.x, w3.x));
                             r[j].y = __vmaxs2(__vmaxs2(w0.y, w1.y), __vmaxs2(w2.y, w3.y));
                             r[j].z = __vmaxs2(__vmaxs2(w0.z, w1.z), __vmaxs2(w2.z, w3.z));
                             r[j].w = __vmaxs2(__vmaxs2(w0.w, w1.w), __vmaxs2(w2.w, w3.w));
                         } else {
-                            r[j] = __ldg(q + opix);
+                            r[j] = ld_dep(q + opix);
                         }
                     }
                 }
@@ -745,7 +745,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                             uint2 w = make_uint2(0u, 0u);
                             if (on) {
                                 const short* src = reinterpret_cast<const short*>(a.res_in) + (size_t)rpix * in_ps + in_off(o);
-                                auto ld = [&](size_t off) { return __ldg(reinterpret_cast<const uint2*>(src + off)); };
+                                auto ld = [&](size_t off) { return ld_dep(reinterpret_cast<const uint2*>(src + off)); };
                                 w = ld(0);
                                 if (a.residual_pool) {     // 2x2 max (kernel.cuh:773-783)
                                     const size_t dn = (size_t)2 * a.OWg * in_ps;

@@ -15,13 +15,6 @@ namespace tcbnn {
 
 constexpr int kSmallMaxWarps = 16;
 
-// A plain load: what the launch in front wrote does not come through the read-only path
-__device__ __forceinline__ uint2 ld64_dep(const uint32_t* p) {
-    uint2 v;
-    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-    return v;
-}
-
 template <int MT, int NTL>
 __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int NW, int* red) {
     constexpr int R = 16 * MT, C = 8 * NTL, CP = C + 2;    // rows, columns, padded row of the exchange buffer
@@ -63,9 +56,9 @@ __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int 
                 const int kp = kb + u * KW * 4 + t;
                 const bool ok = kp < KP;
 #pragma unroll
-                for (int i = 0; i < 2 * MT; i++) a[u][i] = ok ? ld64_dep(ap[i] + 2 * kp) : make_uint2(0u, 0u);
+                for (int i = 0; i < 2 * MT; i++) a[u][i] = ok ? ld_dep(reinterpret_cast<const uint2*>(ap[i] + 2 * kp)) : make_uint2(0u, 0u);
 #pragma unroll
-                for (int j = 0; j < NTL; j++) b[u][j] = ok ? ld64_dep(wp[j] + 2 * kp) : make_uint2(0u, 0u);
+                for (int j = 0; j < NTL; j++) b[u][j] = ok ? ld_dep(reinterpret_cast<const uint2*>(wp[j] + 2 * kp)) : make_uint2(0u, 0u);
             }
 #pragma unroll
             for (int u = 0; u < U; u++) {
@@ -110,14 +103,14 @@ __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int 
             for (int k = 0; k < KW; k++) v += red[(size_t)(w * KW + k) * R * CP + r * CP + c];
         if (g.mode == GEMM_FC_BITS) {
             // (float)K - 2*(float)c >= thr[n]  (kernel.cuh:210-213)
-            const bool bit = in && col < g.N && (float)v >= __ldg(g.p0 + col);
+            const bool bit = in && col < g.N && (float)v >= ld_dep(g.p0 + col);
             const uint32_t bits = __ballot_sync(0xffffffffu, bit) >> (lane & 24);
             if (in && (lane & 7) == 0)                     // column `col` at bit 31 - col % 32 of its word
                 reinterpret_cast<unsigned char*>((uint32_t*)g.out + (size_t)row * g.ldo + (col >> 5))[3 - ((col & 31) >> 3)] =
                     (unsigned char)(__brev(bits & 0xFFu) >> 24);
         } else if (in) {
             if (g.mode == GEMM_INT32) ((int32_t*)g.out)[(size_t)row * g.ldo + col] = v;
-            else ((float*)g.out)[(size_t)row * g.ldo + col] = __fmaf_rn((float)v, __ldg(g.p0 + col), __ldg(g.p1 + col));
+            else ((float*)g.out)[(size_t)row * g.ldo + col] = __fmaf_rn((float)v, ld_dep(g.p0 + col), ld_dep(g.p1 + col));
         }
     }
 }

@@ -91,10 +91,10 @@ __device__ __forceinline__ void expand_rows_task(const uint32_t* bits, int rows,
     uint32_t w[4] = {0u, 0u, 0u, 0u};
     if (r < rows) {
         const uint32_t* src = bits + (size_t)r * ld + w0;
-        if (w0 + 1 < ld) { const uint2 q = __ldg(reinterpret_cast<const uint2*>(src)); w[0] = q.x; w[1] = q.y; }
-        else if (w0 < ld) w[0] = __ldg(src);
-        if (w0 + 3 < ld) { const uint2 q = __ldg(reinterpret_cast<const uint2*>(src + 2)); w[2] = q.x; w[3] = q.y; }
-        else if (w0 + 2 < ld) w[2] = __ldg(src + 2);
+        if (w0 + 1 < ld) { const uint2 q = ld_dep(reinterpret_cast<const uint2*>(src)); w[0] = q.x; w[1] = q.y; }
+        else if (w0 < ld) w[0] = ld_dep(src);
+        if (w0 + 3 < ld) { const uint2 q = ld_dep(reinterpret_cast<const uint2*>(src + 2)); w[2] = q.x; w[3] = q.y; }
+        else if (w0 + 2 < ld) w[2] = ld_dep(src + 2);
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -472,11 +472,16 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             // per tile).  NaN behind the last column: never reached.
             float* const thr = sThr + warp * 128;
             if (g.splits == 1 && g.mode == GEMM_FC_BITS) {
-                __syncwarp();
-                for (int nb = nb0; nb < nb1; nb++) {
-                    const int n = tn * 128 + nb * 32 + f4_channel_of_column(lane);
-                    thr[nb * 32 + lane] = n < g.N ? __ldg(g.p0 + n) : __int_as_float(0x7FC00000);
+                constexpr int NB = PAIR ? 4 : 2;
+                float tv[NB];
+#pragma unroll
+                for (int i = 0; i < NB; i++) {           // (all on their way before the first is stored)
+                    const int n = tn * 128 + (nb0 + i) * 32 + f4_channel_of_column(lane);
+                    tv[i] = n < g.N ? ld_dep(g.p0 + n) : __int_as_float(0x7FC00000);
                 }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < NB; i++) thr[(nb0 + i) * 32 + lane] = tv[i];
                 __syncwarp();
             }
             const long long e0 = clock64();
@@ -527,10 +532,10 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
 #pragma unroll
                             for (int gg = 0; gg < 2; gg++) {
                                 const int n = n0 + 16 * gg;
-                                sc[gg] = make_float4(n < g.N ? __ldg(g.p0 + n) : 0.f, n + 1 < g.N ? __ldg(g.p0 + n + 1) : 0.f,
-                                                     n + 2 < g.N ? __ldg(g.p0 + n + 2) : 0.f, n + 3 < g.N ? __ldg(g.p0 + n + 3) : 0.f);
-                                bi[gg] = make_float4(n < g.N ? __ldg(g.p1 + n) : 0.f, n + 1 < g.N ? __ldg(g.p1 + n + 1) : 0.f,
-                                                     n + 2 < g.N ? __ldg(g.p1 + n + 2) : 0.f, n + 3 < g.N ? __ldg(g.p1 + n + 3) : 0.f);
+                                sc[gg] = make_float4(n < g.N ? ld_dep(g.p0 + n) : 0.f, n + 1 < g.N ? ld_dep(g.p0 + n + 1) : 0.f,
+                                                     n + 2 < g.N ? ld_dep(g.p0 + n + 2) : 0.f, n + 3 < g.N ? ld_dep(g.p0 + n + 3) : 0.f);
+                                bi[gg] = make_float4(n < g.N ? ld_dep(g.p1 + n) : 0.f, n + 1 < g.N ? ld_dep(g.p1 + n + 1) : 0.f,
+                                                     n + 2 < g.N ? ld_dep(g.p1 + n + 2) : 0.f, n + 3 < g.N ? ld_dep(g.p1 + n + 3) : 0.f);
                             }
                         }
 #pragma unroll

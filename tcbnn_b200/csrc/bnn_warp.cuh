@@ -28,6 +28,36 @@ __device__ __forceinline__ void mma_b1_and(int (&c)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ uint2 ldg64(const uint32_t* p) {
     return __ldg(reinterpret_cast<const uint2*>(p));
 }
+// A load of what an earlier launch wrote, in a kernel that may have been set up while that launch was
+// still running (griddepcontrol): not through the read-only path, whose data has to stay the same for as
+// long as the kernel lives -- a line of a buffer that is used again may be in L1 from before.
+// (volatile keeps it behind the wait; without a memory clobber it may still be issued ahead of stores: as plain
+// loads, ResNet-18 at batch 1024 1937 -> 2012 us.)
+__device__ __forceinline__ uint32_t ld_dep(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_dep(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_dep(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_dep(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int4 ld_dep(const int4* p) {
+    int4 v;
+    asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 
 __device__ __forceinline__ int quad_sum(int v) {   // sum over the 4 lanes sharing g
     v += __shfl_xor_sync(0xffffffffu, v, 1);

@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(256) k_pool_bits(const uint32_t* in, uint32_t*
         const long long n = row / (unsigned)P;
         const uint32_t* s0 = in + ((n * 2 * P + 2 * y) * 2 * Q + 2 * x) * Ow + w;
         const uint32_t* s1 = s0 + (long long)2 * Q * Ow;
-        const uint32_t v = __ldg(s0) | __ldg(s0 + Ow) | __ldg(s1) | __ldg(s1 + Ow);
+        const uint32_t v = ld_dep(s0) | ld_dep(s0 + Ow) | ld_dep(s1) | ld_dep(s1 + Ow);
         out[n * out_image_stride + ((long long)y * Q + x) * Ow + w] = v;
         if (nx.planes) {
             const bool par = nx.nplane == 4;               // stride-2 consumer: one plane per row / column parity

@@ -197,6 +197,25 @@ def test_graph_is_recorded_again_when_its_pass_has_changed(cuda):
         ops.set_conv_path(0)
 
 
+def test_passes_back_to_back_on_shared_scratch(cuda):
+    """Passes queued one behind the other on changing images, every layer expanding its input and pooling its
+    output through the one scratch: each pass's logits are those of a pass with nothing around it."""
+    spec = models.vgg_cifar_spec(37)
+    net = models.Network(spec, models.synthetic_weights(spec, 52), models.synthetic_input(spec, 53), handover=False)
+    xs = [torch.from_numpy(models.synthetic_input(spec, 54 + i)).to(cuda) for i in range(3)]
+    alone = []
+    for x in xs:
+        net.set_input(x)
+        alone.append(net.forward().clone())
+        torch.cuda.synchronize()
+    assert not torch.equal(alone[0], alone[1])
+    got = []
+    for i in range(60):
+        net.set_input(xs[i % 3])
+        got.append((net.forward_graph() if i >= 30 else net.forward()).clone())
+    assert all(torch.equal(g, alone[i % 3]) for i, g in enumerate(got))
+
+
 def test_graph_keeps_off_scratch_that_was_replaced(cuda):
     """The scratch shared by layers without planes grows for a larger layer: a graph recorded before that must
     not write to the old one's memory, which by then belongs to somebody else."""
