@@ -13,10 +13,9 @@
 //                         scale + bias straight from the accumulator) or store int32 partial sums for
 //                         gemm_splitk_finish.  128 x 128 tiles alternate between two accumulators, so
 //                         that a tile is finished while the next one is computed
-//   warp  8    loader A : one lane, one bulk copy per stage (a stage holds up to
+//   warp  8    loader A : one lane, one bulk copy (tensor copy in a pair) per stage (a stage holds up to
 //                         kGemmKU consecutive k-blocks, contiguous in the expanded operand)
-//   warp  9    MMA      : converged warp, elected lane: one MMA per k-block (in the second CTA of a pair
-//                         the relay that tells the first that a stage has arrived)
+//   warp  9    MMA      : converged warp, elected lane: one MMA per k-block (the leader's, in a pair)
 //   warp  10   loader W : one lane, one bulk copy per stage
 //
 // A 128 x 128 tile reads 8 KB of operands per k-block and has 8 KB copied in, which fills the
@@ -36,6 +35,7 @@
 // copies and one issuing warp per operand.
 #pragma once
 #include "bconv_umma_pre.cuh"
+#include <cuda.h>
 
 namespace tcbnn {
 namespace umma {
@@ -148,27 +148,45 @@ __device__ __forceinline__ void expand_pass_weights(const PassWeights& p, int bl
 
 // ---- a pair of CTAs on one 256 x 256 tile (cta_group::2) ------------------------------------------
 // Each CTA holds its 128 rows of A, half of W's 256 rows and its 128 x 256 accumulator; the leader (even
-// rank) issues MMAs that read both shared memories.  A bulk copy completes on a barrier of the CTA it
-// writes to, so the second CTA relays: its warp 9 waits for a stage and arrives on the leader's barrier.
+// rank) issues MMAs that read both shared memories.  The copies of both complete on the leader's barrier,
+// which only a tensor copy of a pair may do (cta_group::2; no multicast): a thread of the second CTA that passed its
+// CTA's completion on would have to do so with an arrival of cluster scope, 1400 clocks each, one at a
+// time (8192 x 8192 x 8192 with threshold bits 174 us, 219 with three warps taking turns at it).
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Arrives on the leader's copy of a barrier.  (The relay has written nothing itself; with .release.cluster
-// each arrival took about 1400 clocks, and a k-block 360 instead of 135.)
+__device__ __forceinline__ uint32_t leader_address(uint32_t shared) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(shared));
+    return r;
+}
+// The accumulator goes back to the leader's MMAs: tensor memory is ordered by the tcgen05 fences around
+// the arrival and the wait, for which the arrival itself can be relaxed.
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
-    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\t"
-                 "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_address(bar)) : "memory");
+}
+// One stage of an operand, kGemmKU units: rows of 1 KB of the expanded operand from `row` on.  (A stage
+// that holds fewer k-blocks is followed by others' units or, behind the last, by zeros, which no MMA reads.)
+__device__ __forceinline__ void tensor_g2s_pair(uint32_t dst, const CUtensorMap* map, int row, uint32_t leader_bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(0), "r"(row), "r"(leader_bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_test_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
 }
 // WsWait with the bound in clocks, about a second, as a CTA waits for its partner too.  Polls rather than
-// suspends: a stage passes through three barriers on its way (360 clocks per k-block with try_wait).
+// suspends (360 clocks per k-block with try_wait).
 struct GemmPairWait {
     volatile int* abort;
     int* err;
     __device__ __forceinline__ bool poll(uint32_t bar, uint32_t parity, bool sleep) const {
-        if (mbar_test_wait(bar, parity)) return true;
+        if (mbar_test_cluster(bar, parity)) return true;
         const long long t0 = clock64();
         for (int i = 0; i < (1 << 28); i++) {
-            if (mbar_test_wait(bar, parity)) return true;
+            if (mbar_test_cluster(bar, parity)) return true;
             if (sleep) __nanosleep(64);
             if ((i & 63) == 63 && (*abort || clock64() - t0 > (1LL << 31))) break;
         }
@@ -197,8 +215,8 @@ struct GemmPairWait {
     "setp.ne.b32 pl, %1, 0;\n\tsetp.ne.b32 pq, %7, 0;\n\tsetp.eq.b32 pt, %1, %1;\n\t"              \
     "mov.u32 xa, %2;\n\tmov.u32 xb, %4;\n\t"
 #define TCBNN_F4_PAIR_TEST                                                                           \
-    "mbarrier.test_wait.parity.shared::cta.b64 p0, [%11], %12;\n\t"                                 \
-    "mbarrier.test_wait.parity.shared::cta.b64 p1, [%13], %14;\n\tsetp.ne.and.b32 pc, %16, 0, pl;\n\tmov.b16 both, 3;\n\t"
+    "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p0, [%11], %12;\n\t"                 \
+    "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p1, [%13], %14;\n\tsetp.ne.and.b32 pc, %16, 0, pl;\n\tmov.b16 both, 3;\n\t"
 #define TCBNN_F4_PAIR_TAIL                                                                           \
     "@pl tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%15], both;\n\t" \
     "@pc tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%16], both;\n\t" \
@@ -233,7 +251,7 @@ __device__ __forceinline__ uint32_t mma_f4_pair_end(uint32_t leader, uint32_t d_
 #undef TCBNN_F4_PAIR_IN
 
 template <bool PAIR>
-__device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned char* smem) {
+__device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, const CUtensorMap* map_a, const CUtensorMap* map_w, unsigned char* smem) {
     constexpr int STAGE = kGemmStageBytes, NST = kGemmStages;
     constexpr int NACC = PAIR ? 1 : 2;                  // accumulators of 256 / 128 columns
     constexpr uint32_t TM_COLS = 512, SF_COL = TM_COLS - 32;
@@ -271,7 +289,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
     };
 
     if (tid == 0) {
-        for (int s = 0; s < NST; s++) { mbar_init(BAR_FULL(s), PAIR && rank == 0 ? 3 : 2); mbar_init(BAR_EMPTY(s), 1); }
+        for (int s = 0; s < NST; s++) { mbar_init(BAR_FULL(s), 2); mbar_init(BAR_EMPTY(s), 1); }
         for (int b = 0; b < NACC; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), PAIR ? 16 : 8); }
         mbar_init(BAR_DRAIN, 1);
         *sAbort = 0;
@@ -320,11 +338,16 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
                     const uint32_t bytes = (uint32_t)min(kGemmKU, q.kb1 - kb) * kGemmUnit;
                     ok = tr ? wait.timed(BAR_EMPTY(s), ph ^ 1, tr_w) : wait(BAR_EMPTY(s), ph ^ 1);
                     if (!ok) break;
-                    if (!PAIR || exists) {
+                    if constexpr (PAIR) {
+                        constexpr uint32_t kStage = kGemmKU * kGemmUnit;
+                        if (rank == 0)                   // (the leader's tile always exists)
+                            mbar_expect_tx(BAR_FULL(s), tile128 + 1 < (isw ? g.NT : g.MT) ? 2 * kStage : kStage);
+                        if (exists)
+                            tensor_g2s_pair(smem_u32(smem + (size_t)s * STAGE) + (isw ? OFF_W : 0u), isw ? map_w : map_a,
+                                            (tile128 * g.KB + kb) * (kGemmUnit / 1024), leader_address(BAR_FULL(s)));
+                    } else {
                         mbar_expect_tx(BAR_FULL(s), bytes);
                         bulk_g2s(smem_u32(smem + (size_t)s * STAGE) + (isw ? OFF_W : 0u), src + (size_t)kb * kGemmUnit, bytes, BAR_FULL(s));
-                    } else {
-                        mbar_arrive(BAR_FULL(s));
                     }
                     issued++;
                     if (++s == NST) { s = 0; ph ^= 1; }
@@ -334,32 +357,20 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             if (!ok) {
                 // giving up: wait (bounded) for the copies still in flight before the CTA exits.  A
                 // stage's barrier completes once both loaders' copies have landed; if the other
-                // loader never got that far the polls run out, which takes longer than any copy.
+                // loader never got that far the polls run out, which takes longer than any copy.  (A pair's
+                // second CTA cannot poll the leader's barriers: it lets that time pass.)
                 for (int s2 = 0; s2 < NST; s2++) {
                     const bool this_pass = s2 < s;
                     if (!this_pass && issued < (uint32_t)NST) continue;
                     for (int i = 0; i < (PAIR ? 1 << 16 : 1 << 20); i++)
-                        if (PAIR ? mbar_test_wait(BAR_FULL(s2), this_pass ? ph : ph ^ 1) : mbar_try_wait(BAR_FULL(s2), this_pass ? ph : ph ^ 1)) break;
+                        if (PAIR ? rank == 0 && mbar_test_cluster(BAR_FULL(s2), this_pass ? ph : ph ^ 1) : mbar_try_wait(BAR_FULL(s2), this_pass ? ph : ph ^ 1)) break;
+                        else if (PAIR) __nanosleep(20);
                 }
             }
         }
         __syncwarp();
     } else if (PAIR && warp == 9 && rank == 1) {
-        // =============================== relay: this CTA's stage is there ===================
-        if (lane == 0) {
-            uint32_t s = 0, ph = 0;
-            bool ok = true;
-            for (int t = t_first; t < ntiles && ok; t += t_step) {
-                const Tile q = tile(t);
-                for (int kb = q.kb0; kb < q.kb1; kb += kGemmKU) {
-                    ok = wait.spin(BAR_FULL(s), ph);
-                    if (!ok) break;
-                    mbar_arrive_leader(BAR_FULL(s));
-                    if (++s == (uint32_t)NST) { s = 0; ph ^= 1; }
-                }
-            }
-        }
-        __syncwarp();
+        __syncwarp();                                   // (the leader issues for both)
     } else if (warp == 9) {
         // =============================== MMA issuer =========================================
         // (what the next stage needs is worked out and asked for while this one's MMAs are queued: the
@@ -452,7 +463,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, unsigned ch
             else
                 mma_commit(BAR_DRAIN);
             for (int i = 0; i < (1 << 20); i++)
-                if (PAIR ? mbar_test_wait(BAR_DRAIN, 0) : mbar_try_wait(BAR_DRAIN, 0)) break;
+                if (PAIR ? mbar_test_cluster(BAR_DRAIN, 0) : mbar_try_wait(BAR_DRAIN, 0)) break;
         }
         __syncwarp();
     } else if (warp < 8) {

@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstring>
 #include <atomic>
+#include <cuda.h>
 #include <mutex>
 #include <utility>
 #include <vector>
@@ -234,11 +235,32 @@ __global__ void __launch_bounds__(256) k_expand_rows(const uint32_t* a_bits, int
 }
 __global__ void __launch_bounds__(umma::kGemmThreads, 1) k_gemm_umma(umma::GemmUmmaArgs g) {
     extern __shared__ __align__(128) unsigned char dyn_smem_gemm[];
-    umma::gemm_umma_cta<false>(g, dyn_smem_gemm);
+    umma::gemm_umma_cta<false>(g, nullptr, nullptr, dyn_smem_gemm);
 }
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(umma::kGemmThreads, 1) k_gemm_umma_pair(umma::GemmUmmaArgs g) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(umma::kGemmThreads, 1)
+k_gemm_umma_pair(umma::GemmUmmaArgs g, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w) {
     extern __shared__ __align__(128) unsigned char dyn_smem_gemm[];
-    umma::gemm_umma_cta<true>(g, dyn_smem_gemm);
+    umma::gemm_umma_cta<true>(g, &map_a, &map_w, dyn_smem_gemm);
+}
+
+// Expanded operand of `units` units as rows of 1 KB, copied kGemmKU units at a time
+int unit_map(CUtensorMap* map, const void* base, long long units) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &r) == cudaSuccess && r == cudaDriverEntryPointSuccess
+                   ? (Encode)f : (Encode)nullptr;
+    }();
+    if (!encode) return fail("gemm (tcgen05): the driver has no cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {256, (cuuint64_t)units * (umma::kGemmUnit / 1024)}, strides[1] = {1024};
+    const cuuint32_t box[2] = {256, umma::kGemmKU * (umma::kGemmUnit / 1024)}, steps[2] = {1, 1};
+    const CUresult e = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, steps,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (e != CUDA_SUCCESS) return fail("gemm (tcgen05): tensor map of %lld units: error %d", units, (int)e);
+    return 0;
 }
 
 struct GemmUmmaPlan {
@@ -347,8 +369,14 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, con
         const long long tiles = (p.pair ? (long long)((p.MT + 1) / 2) * ((p.NT + 1) / 2) : (long long)p.MT * p.NT) * p.splits;
         const long long slots = p.pair ? sms / 2 : sms;
         const unsigned grid = (unsigned)(tiles < slots ? tiles : slots) * (p.pair ? 2u : 1u);
-        const cudaError_t e = launch_dependent(p.pair ? k_gemm_umma_pair : k_gemm_umma, grid, umma::kGemmThreads,
-                                               umma::kGemmSmem, st, a);
+        cudaError_t e;
+        if (p.pair) {
+            CUtensorMap map_a, map_w;
+            if (unit_map(&map_a, a.ea, (long long)p.MT * p.KB) || unit_map(&map_w, a.ew, (long long)p.NT * p.KB)) return 1;
+            e = launch_dependent(k_gemm_umma_pair, grid, umma::kGemmThreads, umma::kGemmSmem, st, a, map_a, map_w);
+        } else {
+            e = launch_dependent(k_gemm_umma, grid, umma::kGemmThreads, umma::kGemmSmem, st, a);
+        }
         if (e != cudaSuccess) return fail("gemm (tcgen05): %s", cudaGetErrorString(e));
     }
     if (launch_check("gemm (tcgen05)")) return 1;

@@ -79,7 +79,7 @@ def test_small_gemm_tiles(cuda, M, N, K):
 UMMA_GEMM_CASES = [
     # M, N, K, pair, splits: large enough for the tcgen05 GEMM (M*N*K >= 2^30, less with a forced
     # plan), ragged on purpose.
-    # pair / splits force the tile shape (1: 256 x 128, 0: 128 x 128) and the number of K slices
+    # pair / splits force the tile shape (1: 256 x 256 on two SMs, 0: 128 x 128) and the number of K slices
     # (1: the GEMM's own epilogue finishes the layer; more: partial sums and a finishing pass);
     # -1 leaves the choice to the library's cost model.
     (300, 200, 40010, -1, -1),      # partial row tiles, K not a multiple of 32
@@ -104,6 +104,30 @@ UMMA_GEMM_CASES = [
     (1000, 520, 576, 0, 1),         # K = 9 k-blocks: stages of 4, 4 and 1
     (1000, 520, 576, 1, 2),         # splits of 5 and 4 k-blocks
 ]
+
+
+# one wave of pairs, several waves (one accumulator handed back from tile to tile), an odd tile in M and N, and
+# a last stage of one k-block
+@pytest.mark.parametrize("M,N,K", [(1024, 1024, 16384), (4096, 4096, 2048), (2200, 2700, 4160), (300, 5000, 2112)])
+def test_pairs_of_ctas_agree_with_single_ones_on_changing_operands(cuda, M, N, K):
+    """Calls back to back, each on operands the one before has not seen, at the same addresses: an operand read
+    before it arrived, or an accumulator overwritten before it was read, would show as a difference."""
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(M + N + K)
+    ld = orc.step128_words(K)
+    A, W = (torch.empty((r, ld), dtype=torch.int32, device=cuda) for r in (M, N))
+    got = {}
+    try:
+        for i in range(25):
+            for t in (A, W):
+                t.copy_(torch.randint(-2 ** 31, 2 ** 31, t.shape, dtype=torch.int64, device=cuda, generator=gen))
+            for pair in (1, 0):
+                ops.set_gemm_plan(pair, 1)
+                got[pair] = ops.bgemm(A, W, K, workspace=ops.gemm_workspace(M, N, K, cuda))
+            assert torch.equal(got[0], got[1]), i
+        assert ops.gemm_status() == 0
+    finally:
+        ops.set_gemm_plan(-1, -1)
 
 
 @pytest.mark.parametrize("M,N,K,pair,splits", UMMA_GEMM_CASES)
