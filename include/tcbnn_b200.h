@@ -194,8 +194,12 @@ int tcbnn_conv_layer_w(const tcbnn_conv_desc* d, const uint32_t* in, const void*
  *    written.  out_image_stride must be dense.  Kernels that cannot write the planes themselves
  *    are followed by the expansion pass, so the result is the same for every layer.
  *  - workspace_ready != 0: `workspace` already holds this layer's input planes (its producer was
- *    called with next = this layer); the expansion pass is skipped.
+ *    called with next = this layer); the expansion pass is skipped.  The value
+ *    TCBNN_PLANES_AND_FILTER_READY says more: no kernel of the caller's has written `prepared` since
+ *    the call in front on this stream, or ever (tcbnn_conv_prepare's writes do not count).  The filter is
+ *    then fetched while the launch in front still runs.
  * No reference counterpart. */
+#define TCBNN_PLANES_AND_FILTER_READY 0x46520101
 int tcbnn_conv_layer_x(const tcbnn_conv_desc* d, const uint32_t* in, const void* prepared,
                        const float* thr, const void* res_in, int res_in_bytes, int res_in_ch,
                        int residual_channels, int residual_pool, uint32_t* out,

@@ -64,9 +64,10 @@ __host__ __device__ constexpr size_t pre_res_ring_bytes(int nt, int epiw) {
 // raster position (vr, vx) of the OUTPUT grid, so that a filter tap is again a fixed offset.
 __device__ __forceinline__ void expand_raster(const ConvWsArgs& a, uint4* planes, long long plane_positions,
                                               long long front) {
-    // a programmatic dependent of the bits' producer; the convolution that follows is one of this pass
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // a programmatic dependent of the bits' producer; the convolution that follows is one of this pass,
+    // and is let in only when all that came before this pass is complete (ConvWsArgs::filter_settled)
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int NCB = a.C >> 6, Cw = a.C >> 5;
     const int nplane = a.stride == 2 ? 4 : 1;
     const long long total = plane_positions * NCB * nplane;
@@ -184,7 +185,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     const int obase = nt * NT;
 
     // Launched as a programmatic dependent: everything up to griddepcontrol.wait may run while the
-    // launch in front is still running, so it touches nothing but this CTA's own memory and the filter.
+    // launch in front is still running, so it touches nothing but this CTA's own memory and a settled filter.
     if (tid == 0) {
         for (int s = 0; s < 8; s++) { mbar_init(BAR_AFULL(s), 1); mbar_init(BAR_AEMPTY(s), 1); }
         for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), WPG); }
@@ -221,9 +222,9 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     tc_fence_after();
     constexpr int kIssueLanes = 8;
     if (warp == LOAD_WARP) {
-        // The filter block, in eight pieces (a multiple of 16 bytes each).  Before the wait: the blob is
-        // written by tcbnn_conv_prepare alone, whose last operation is no kernel, so that nothing behind
-        // it starts before the blob is complete.
+        // The filter block, in eight pieces (a multiple of 16 bytes each).  Where the caller's filter is
+        // settled (ConvWsArgs::filter_settled) before the wait, under the launch in front.
+        if (!a.filter_settled) asm volatile("griddepcontrol.wait;" ::: "memory");
         const uint32_t nB = (uint32_t)(RS * (a.C >> 5) * NT), part = (nB + kIssueLanes - 1) / kIssueLanes;
         if (lane == 0) mbar_expect_tx(BAR_FILTER, nB * 16u);
         __syncwarp();

@@ -53,6 +53,10 @@ struct ConvWsArgs {
     // (bconv_umma_pre.cuh layout over THAT layer's raster; dead slots stay as the caller zeroed them)
     uint4* nxt; long long nxt_positions, nxt_front; int nxt_PW, nxt_VH;
     int nxt_nplane;           // 1, or 4 when that layer has stride 2 (one plane per row / column parity)
+    // The filter blob is complete before the launch in front of this one can start: whoever wrote it was
+    // waited for by that launch, which does not write it itself.  So where the call launches its own
+    // expansion pass, which lets the convolution in only behind its wait; elsewhere the caller says so.
+    int filter_settled;
     const void* res_in; int res_in_bytes, res_in_ch, residual_channels, residual_pool;
     // int16 residual tensors may be laid out by 8-channel chunk, [ch/8][pixels][8], instead of NHWC
     // (bconv_umma_pre.cuh only): npix = pixels of the whole tensor

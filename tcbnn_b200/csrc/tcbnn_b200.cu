@@ -1404,8 +1404,8 @@ int tcbnn_conv_prepare(const tcbnn_conv_desc* d, const uint32_t* filter_bits, vo
             filter_bits, d->O, d->R * d->S, d->C, umma::kAsNT, (uint4*)(p + L.off_wi8_as));
         if (launch_check("conv_prepare (int8 filter, 128-channel tiles)")) return 1;
     }
-    // last, and no kernel: the convolutions read the blob ahead of their place in the stream (programmatic
-    // launches), which a memset in front of them rules out until the blob is complete
+    // last, and no kernel: a convolution whose caller calls its filter settled reads the blob ahead of its place
+    // in the stream (programmatic launches), which a memset in front of it rules out until the blob is complete
     CUDA_TRY(cudaMemsetAsync(p + L.off_err, 0, 256, (cudaStream_t)stream));
     return 0;
 }
@@ -1552,6 +1552,7 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
         a.err_flag = (int*)(p + L.off_err);
         a.trace = g_conv_trace;
         a.pre = nullptr; a.pre_positions = 0; a.pre_front = 0;
+        a.filter_settled = !workspace_ready || workspace_ready == TCBNN_PLANES_AND_FILTER_READY;
         a.pre_stages = 0; a.pre_cbs = 1;
         a.nxt = nullptr; a.nxt_positions = 0; a.nxt_front = 0; a.nxt_PW = 0; a.nxt_VH = 0; a.nxt_nplane = 1;
         if (nx && !use_as && !pooled) {     // (a pooled layer's kernel sees the pre-pool grid)

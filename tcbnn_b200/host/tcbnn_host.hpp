@@ -539,7 +539,8 @@ public:
                                            inject_residual ? input_residual_gpu : NULL, input_residual_bytes,
                                            input_residual_channels,
                                            residual_channels, residual_pool ? 1 : 0, output_gpu, out_image_stride,
-                                           output_residual_gpu, residual_bytes, NULL, ws, wsb, input_planes.p ? 1 : 0, next,
+                                           output_residual_gpu, residual_bytes, NULL, ws, wsb,
+                                           input_planes.p ? TCBNN_PLANES_AND_FILTER_READY : 0, next,      // (prepared_gpu: initialize() alone writes it)
                                            next_planes ? next_planes->ptr : NULL, next_planes ? next_planes->bytes : 0,
                                            stream));
     }

@@ -226,9 +226,14 @@ def conv_layer(d, x, prepared, thr, res_in=None, residual_channels=0, residual_p
     return out, res_out, acc_out
 
 
+PLANES_AND_FILTER_READY = 0x46520101         # TCBNN_PLANES_AND_FILTER_READY
+
+
 def conv_call(d, x, prepared, thr, res_in, residual_channels, residual_pool, out, stride, res_out, acc_out,
-              workspace, workspace_ready, next_layer, res_in_chunked, res_out_chunked, res_out_proven):
-    """(entry point, its arguments without the stream) of a conv_layer call on these tensors."""
+              workspace, workspace_ready, next_layer, res_in_chunked, res_out_chunked, res_out_proven, filter_ready=False):
+    """(entry point, its arguments without the stream) of a conv_layer call on these tensors.
+    filter_ready: the call in front on the stream is this library's, and nothing has written `prepared`
+    since that began."""
     res_in_ch = res_in.shape[-1] if res_in is not None else 0
     args = (C.byref(d), _ptr(x), _ptr(prepared), _ptr(thr), _ptr(res_in),
             _residual_code(res_in, res_in_chunked),
@@ -237,7 +242,8 @@ def conv_call(d, x, prepared, thr, res_in, residual_channels, residual_pool, out
     if next_layer is not None or workspace_ready:
         nd, npl = next_layer if next_layer is not None else (None, None)
         return "tcbnn_conv_layer_x", args + (
-            _ptr(workspace), workspace.numel() if workspace is not None else 0, int(bool(workspace_ready)),
+            _ptr(workspace), workspace.numel() if workspace is not None else 0,
+            PLANES_AND_FILTER_READY if workspace_ready and filter_ready else int(bool(workspace_ready)),
             C.byref(nd) if nd is not None else None, _ptr(npl), npl.numel() if npl is not None else 0)
     if workspace is not None:
         return "tcbnn_conv_layer_w", args + (_ptr(workspace), workspace.numel())

@@ -537,7 +537,9 @@ class Conv128LayerParam(_Layer):
                                    self.out_image_stride, res_out, None, ws, ready, nxt,
                                    self.input_residual_chunked and self.inject_residual, self.residual_chunked,
                                    # int16 was chosen from the bound fan-in + bound of the injected residual
-                                   self.residual_bound is not None and self.residual_bound <= 32767)
+                                   self.residual_bound is not None and self.residual_bound <= 32767,
+                                   # a pass starts with a launch that waits for all before it
+                                   filter_ready=in_pass)
         return name, args, (ws, d, x, prep, thr, res_in, out, res_out, *(nxt or ()))
 
     def get_output_gpu(self):

@@ -6,7 +6,7 @@ import torch
 
 import oracle as orc
 import util
-from tcbnn_b200 import ops
+from tcbnn_b200 import lib, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -673,6 +673,46 @@ def test_conv_layer_reports_int16_overflow_on_tile_epilogue(cuda):
                    residual_dtype=torch.int16, res_in_chunked=True, res_out_chunked=True)
     assert ops.conv_status(d, prep) == 2
     assert ops.conv_status(d, prep) == 0          # reading clears it
+
+
+@pytest.mark.parametrize("ready", [False, True])
+def test_conv_layer_follows_a_filter_written_right_in_front(cuda, ready):
+    """The prepared filter is written by a kernel that lets the next launch in at once (the packing kernel, the
+    blob being the last of many rows), directly in front of the convolution: the new filter counts, with
+    and without an expansion pass between."""
+    B, H, C, O = 6, 16, 128, 128
+    g = util.rng(77)
+    x = dev(util.rand_words(g, (B, H, H, C // 32)), cuda)
+    thr = dev((g.standard_normal(O) * np.sqrt(C * 9) * 0.5).astype(np.float32), cuda)
+    d = ops.conv_desc(B, H, H, C, O, 3, 3, 1, 1)
+    preps = [ops.conv_prepare(d, dev(util.rand_words(g, (O, 9, C // 32)), cuda)) for _ in range(2)]
+    blobs = [p.view(torch.int32).reshape(1, -1) for p in preps]
+    assert blobs[0].shape[1] % 4 == 0
+    want = [ops.conv_layer(d, x, p, thr)[0] for p in preps]
+    assert not torch.equal(*want)
+    cols = blobs[0].shape[1] * 32
+    rows = 1 + (160 << 20) // (4 * cols)
+    values = [torch.cat([torch.zeros((rows - 1, cols), device=cuda), ops.unpack_rows(b, cols)]) for b in blobs]
+    planes = ops.new_planes(d, cuda)
+    ops.conv_layer(d, x, preps[0], thr, workspace=planes)
+    room = torch.zeros((rows, cols // 32), dtype=torch.int32, device=cuda)
+    blob = room[-1].view(torch.uint8)
+    assert blob.numel() == preps[0].numel() and blob.data_ptr() % 256 == 0
+    out = torch.empty((B, H * H * O // 32), dtype=torch.int32, device=cuda)
+
+    def pair(i):
+        lib.call("tcbnn_pack_rows", ops._ptr(values[i]), rows, cols, cols // 32, ops._ptr(room), ops._stream())
+        ops.conv_layer(d, x, blob, thr, out=out, workspace=planes, workspace_ready=ready)
+
+    graphs = [torch.cuda.CUDAGraph() for _ in range(2)]         # (launches right behind each other)
+    for i in range(2):
+        pair(i)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graphs[i]):
+            pair(i)
+    for i in range(12):
+        graphs[i & 1].replay()
+        assert torch.equal(out.reshape(want[0].shape), want[i & 1]), i
 
 
 @pytest.mark.parametrize("C,O,stride,mode", [(64, 32, 1, "plain"), (64, 64, 1, "pool"), (128, 128, 2, "none"), (128, 256, 1, "pool")])
