@@ -267,7 +267,7 @@ struct GemmUmmaPlan {
     bool use;
     bool pair;            // 256 x 256 tiles on pairs of SMs instead of 128 x 128 on one
     int MT, NT, KB, splits, per;
-    size_t off_ea, off_ew, off_partial, bytes;
+    size_t off_ew, off_partial, bytes;    // of the scratch: expanded A, expanded W, partial sums
 };
 
 // Tile shape and split count of the tcgen05 path from a clock model of its launches, calibrated
@@ -276,7 +276,9 @@ struct GemmUmmaPlan {
 // tiles 150; set-up, first loads and the last epilogue are paid once per CTA, the pair's epilogue (one
 // accumulator) once per tile; more than one split adds the finishing launch and the partial sums'
 // round trip.
-GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
+// Among the plans that fit `room` bytes of scratch: fewer rows can want more slices of K and with them more
+// scratch than the caller sized for his largest batch.  An operand that comes expanded needs none.
+GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms, size_t room = SIZE_MAX, bool have_a = false, bool have_w = false) {
     GemmUmmaPlan p = {};
     // below 2^30 multiply-adds the single launch of the warp-level kernel wins (measured; a plan
     // forced through tcbnn_set_gemm_plan waives that); the fp32 accumulators hold K exactly up to 2^22
@@ -284,6 +286,8 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
     p.use = M >= 128 && N >= 64 && K >= 512 && K < (1 << 22) && ((long long)M * N * K >= (1LL << 30) || forced);
     if (!p.use) return p;
     p.MT = (M + 127) / 128; p.NT = (N + 127) / 128; p.KB = (K + 63) / 64;
+    p.off_ew = have_a ? 0 : (size_t)p.MT * p.KB * umma::kGemmUnit;
+    p.off_partial = p.off_ew + (have_w ? 0 : (size_t)p.NT * p.KB * umma::kGemmUnit);
     double best = 1e30;
     for (int pair = 0; pair < 2; pair++) {
         if (g_gemm_force_pair >= 0 && pair != g_gemm_force_pair) continue;
@@ -298,15 +302,11 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms) {
             const long long waves = (tiles * splits + slots - 1) / slots;
             double clk = pair ? (double)waves * (per * 150.0 + 3000.0) + 6000.0 : (double)waves * per * 140.0 + 7000.0;
             if (splits > 1) clk += 12000.0 + 6.0 * splits * (double)M * N * 4.0 / 3000.0;
-            if (clk < best) { best = clk; p.pair = pair != 0; p.splits = splits; p.per = per; }
+            const size_t bytes = p.off_partial + (splits > 1 ? (size_t)splits * M * N * sizeof(int32_t) : 0);
+            if (clk < best && bytes <= room) { best = clk; p.pair = pair != 0; p.splits = splits; p.per = per; p.bytes = bytes; }
         }
     }
-    if (p.splits < 1) { p.use = false; return p; }      // a forced plan no slicing of K gives
-    size_t o = 0;
-    p.off_ea = o;      o += (size_t)p.MT * p.KB * umma::kGemmUnit;  o = (o + 255) & ~(size_t)255;
-    p.off_ew = o;      o += (size_t)p.NT * p.KB * umma::kGemmUnit;  o = (o + 255) & ~(size_t)255;
-    p.off_partial = o; o += p.splits > 1 ? (size_t)p.splits * M * N * sizeof(int32_t) : 0;
-    p.bytes = o;
+    if (p.splits < 1) p.use = false;      // nothing fits, or a forced plan no slicing of K gives
     return p;
 }
 
@@ -340,10 +340,10 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, con
         }))
         return 1;
     char* w = (char*)workspace;
-    if ((!u.a || !u.w) && expand_units(g.A, g.M, g.lda, u.a ? nullptr : w + p.off_ea, g.W, g.N, g.ldw, u.w ? nullptr : w + p.off_ew, g.K, sms, st))
+    if ((!u.a || !u.w) && expand_units(g.A, g.M, g.lda, u.a ? nullptr : w, g.W, g.N, g.ldw, u.w ? nullptr : w + p.off_ew, g.K, sms, st))
         return 1;
     umma::GemmUmmaArgs a;
-    a.ea = (const unsigned char*)(u.a ? u.a : w + p.off_ea); a.ew = (const unsigned char*)(u.w ? u.w : w + p.off_ew);
+    a.ea = (const unsigned char*)(u.a ? u.a : w); a.ew = (const unsigned char*)(u.w ? u.w : w + p.off_ew);
     a.nxt = (uint4*)u.next; a.nxt_KB = (g.N + 63) / 64;
     a.M = g.M; a.N = g.N; a.KB = p.KB; a.MT = p.MT; a.NT = p.NT; a.splits = p.splits; a.per = p.per;
     a.partial = p.splits > 1 ? (int32_t*)(w + p.off_partial) : nullptr;
@@ -400,8 +400,8 @@ int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t s
     if (((uintptr_t)g.A & 7) || ((uintptr_t)g.W & 7)) return fail("gemm: operands must be 8-byte aligned");
     int sms;
     if (sm_count(&sms)) return 1;
-    const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms);
-    if (plan.use && g_gemm_path != 1 && workspace && workspace_bytes >= plan.bytes && ((uintptr_t)workspace & 255) == 0) {
+    const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0, u.a, u.w);
+    if (plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0) {
         // (the epilogue writes the next operand where it finishes the layer itself)
         const GemmUnits mine{u.a, u.w, plan.splits == 1 ? u.next : nullptr};
         if (run_gemm_umma(g, plan, workspace, mine, sms, st)) return 1;
@@ -1277,8 +1277,8 @@ size_t tcbnn_gemm_workspace_bytes(int M, int N, int K) {
 int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes) {
     int sms;
     if (M <= 0 || N <= 0 || K <= 0 || sm_count(&sms)) return 0;
-    const GemmUmmaPlan plan = gemm_umma_plan(M, N, K, sms);
-    if (plan.use && g_gemm_path != 1 && workspace_bytes >= plan.bytes) return plan.splits > 1 ? 3 : 2;   // expansion, GEMM, finish
+    const GemmUmmaPlan plan = gemm_umma_plan(M, N, K, sms, workspace_bytes);
+    if (plan.use && g_gemm_path != 1) return plan.splits > 1 ? 3 : 2;   // expansion, GEMM, finish
     return gemm_use_splits(M, N, K, sms, workspace_bytes) > 1 ? 2 : 1;
 }
 

@@ -106,6 +106,28 @@ UMMA_GEMM_CASES = [
 ]
 
 
+@pytest.mark.parametrize("M,live,N,K", [(256, 128, 4096, 25088), (1024, 130, 1024, 25088), (4096, 300, 256, 65536)])
+def test_fewer_rows_stay_on_tcgen05_in_the_workspace_of_the_full_batch(cuda, M, live, N, K):
+    """Scratch sized for a batch serves every smaller one that takes the tcgen05 GEMM with scratch of its own
+    (fewer rows may want more slices of K), with the b1 kernel's results."""
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(M + live)
+    ld = orc.step128_words(K)
+    A, W = (torch.randint(-2 ** 31, 2 ** 31, (r, ld), dtype=torch.int64, device=cuda, generator=gen).to(torch.int32) for r in (live, N))
+    ws = ops.gemm_workspace(M, N, K, cuda)
+    for rows in range(128, M + 1, 61):
+        own = ops.gemm_workspace(rows, N, K, cuda)
+        assert (ops.gemm_launches(rows, N, K, ws) > 1) == (ops.gemm_launches(rows, N, K, own) > 1), rows
+    assert ops.gemm_launches(live, N, K, ws) > 1
+    got = ops.bgemm(A, W, K, workspace=ws)
+    try:
+        ops.set_gemm_path(1)
+        assert torch.equal(got, ops.bgemm(A, W, K))
+    finally:
+        ops.set_gemm_path(0)
+    assert ops.gemm_status() == 0
+
+
 # one wave of pairs, several waves (one accumulator handed back from tile to tile), an odd tile in M and N, and
 # a last stage of one k-block
 @pytest.mark.parametrize("M,N,K", [(1024, 1024, 16384), (4096, 4096, 2048), (2200, 2700, 4160), (300, 5000, 2112)])
