@@ -428,8 +428,8 @@ def test_conv_layer_tcgen05_and_b1_paths_agree_with_oracle(cuda, case):
     try:
         # 5x5 filters over 256 channels do not fit the filter-stationary kernel's shared memory
         # ... and 200-pixel rows do not fit its patch
-        # path 5: automatic choice with the int16 residual rows staged in shared memory wherever possible
-        for path in ((2, 5, 1) if ((R == 5 and C >= 256) or W >= 160) else (2, 5, 3, 1)):
+        # paths 6 and 9: the loader-fed kernel as one CTA of 16 epilogue warps per SM, and with one 64-channel block per stage
+        for path in ((2, 6, 9, 1) if ((R == 5 and C >= 256) or W >= 160) else (2, 6, 9, 3, 1)):
             ops.set_conv_path(path)
             go, gr, ga = ops.conv_layer(d, dev(x, cuda), prep, dev(thr, cuda),
                                         res_in=dev(res_in, cuda) if res_in is not None else None,
@@ -615,8 +615,8 @@ CHUNKED_CASES = [
 @pytest.mark.parametrize("case", CHUNKED_CASES)
 def test_conv_layer_chunked_int16_residuals(cuda, case):
     """int16 residual tensors laid out by 8-channel chunk (TCBNN_RES_INT16_CHUNKED) in and out of
-    the loader-fed kernel -- its tile-per-group epilogue (one or two CTAs per SM) and, with an
-    NHWC tensor on the other side or path 7, the all-warps-per-tile epilogues: same values as the
+    the loader-fed kernel -- its thread-per-pixel epilogues in all three forms of CTA and, with an
+    NHWC tensor on the other side, the epilogue by row pieces: same values as the
     oracle's NHWC tensors; calls that cannot honour the layout fail instead of misreading it."""
     B, H, W, C, O, mode = case
     g = util.rng(sum(case[:5]) + 5)
@@ -640,7 +640,8 @@ def test_conv_layer_chunked_int16_residuals(cuda, case):
     r16 = ops.nhwc_to_chunked(dev(res_in.astype(np.int16), cuda)) if res_in is not None else None
     dx, dthr = dev(x, cuda), dev(thr, cuda)
     try:
-        for path in (0, 6, 8, 7, 9, 10):
+        # as chosen; 16 epilogue warps, one CTA per SM; no single-group CTAs; one block per stage; even shares
+        for path in (0, 6, 7, 9, 10):
             ops.set_conv_path(path)
             for out_chunked in (True, False):
                 for proven in (False, True):

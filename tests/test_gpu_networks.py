@@ -170,6 +170,59 @@ def test_tensor_given_another_storage_in_place_counts(cuda, which):
         net.forward()
 
 
+@pytest.mark.parametrize("which", ["mlp", "resnet18", "vgg_cifar"])
+def test_forward_replays_follow_inputs_and_every_change(cuda, which):
+    """forward() replays a recorded graph from its third call on: on new images each time, and after each of
+    the things that end a replay, its logits are those of the layers called one by one."""
+    spec = {"mlp": models.mlp_spec(1100), "resnet18": models.resnet18_spec(3, image=64, classes=100),
+            "vgg_cifar": models.vgg_cifar_spec(5)}[which]
+    w, bound = models.synthetic_weights(spec, 60), models.SYNTHETIC_IMAGE_ABS_BOUND if which == "resnet18" else None
+    net = models.Network(spec, w, models.synthetic_input(spec, 61), input_abs_bound=bound)
+    xs = [torch.from_numpy(models.synthetic_input(spec, 62 + i)).to(cuda) for i in range(5)]
+    B = spec["batch"]
+
+    def check(live=B):
+        seen = set()
+        for x in xs:
+            net.set_input(x[:live])
+            got = net.forward()[:live].clone()
+            replays = net._pass.graph is not None
+            for l in net.layers:
+                l.forward()
+            want = net.layers[-1].get_output_gpu()[:live]
+            assert torch.equal(got, want)
+            seen.add(bytes(want.cpu().numpy()))
+        assert replays and len(seen) == len(xs)             # the last of them at least was a replay
+
+    try:
+        check()
+        for change in ("weight", "thresholds", "settings", "plan", "live", "input", "scratch"):
+            if change == "weight":
+                net.layers[-1].weight_gpu.copy_(net.layers[-1].weight_gpu.flip(0))
+            elif change == "thresholds":
+                net.layers[2].bn_gpu = net.layers[2].bn_gpu - 3.0
+            elif change == "settings":
+                ops.set_conv_path(6)
+                check()
+                ops.set_conv_path(0)
+            elif change == "plan":
+                ops.set_gemm_plan(1, 1)
+                check()
+                ops.set_gemm_plan(-1, -1)
+            elif change == "live":
+                net.set_batch(B - 1)
+                check(B - 1)
+                net.set_batch(B)
+            elif change == "input":
+                net.layers[0].input_gpu = torch.empty_like(net.layers[0].input_gpu)
+            elif ops.shared_scratch(net.layers[0].output_gpu.device) is not None:
+                ops.conv_workspace(ops.conv_desc(96, 32, 32, 128, 128, 3, 3, 1, 1, pool=2), net.layers[0].output_gpu.device)
+            check()
+    finally:
+        ops.set_conv_path(0)
+        ops.set_gemm_plan(-1, -1)
+
+
 def test_graph_is_recorded_again_when_its_pass_has_changed(cuda):
     """forward_graph() after a layer's tensor was replaced, after a process-wide setting changed and for live
     batches that come back: the results of a network without graphs.  The graphs kept are bounded."""
