@@ -1,4 +1,4 @@
-// tcgen05 binary convolution fed from a pre-expanded input (stride 1, C <= 512), 4-bit operands:
+// tcgen05 binary convolution fed from a pre-expanded input (strides 1 and 2, C <= 512), 4-bit operands:
 // tcgen05.mma kind::mxf4 on +-1.0 as e2m1 with unit block scales (bconv_umma.cuh), 128 x NT x 64
 // per instruction -- one MMA per filter tap and 64-channel block.
 //
@@ -9,17 +9,16 @@
 // occupancy, HBM-bound, 8 bytes in and 32 out per pixel and 64-channel block) -- which writes it
 // as +-1 nibbles straight in the layout the MMA wants: for every 32-channel chunk a plane
 // [raster position][16 bytes] over the zero-padded virtual raster of bconv_umma.cuh, zeros on the
-// dead bands.  A tile's patch is then two contiguous runs per 64-channel block, which one thread
-// fetches with bulk asynchronous copies (cp.async.bulk + mbarrier complete_tx).  With half a byte
+// dead bands.  A tile's patch is then two contiguous runs per 64-channel block (and input parity, at
+// stride 2), fetched with bulk asynchronous copies (cp.async.bulk + mbarrier complete_tx).  With half a byte
 // per channel the filter block of 128 output channels stays resident up to 256 input channels
 // (64 output channels at 512), so the wide layers run filter-stationary too.  The CTA becomes
 //
-//   warps 0-15  epilogue   : warp w reads TMEM lanes 32*(w%4).., columns (w/4) * NT/4 ..
-//   warp  16    loader     : one lane, bulk copies of the patch planes into the stage ring
-//   warp  17    MMA issuer : one lane, as in bconv_umma_ws.cuh
+//   warps 0-15  epilogue   : groups of four warps (eight at an n-tile of 128), each on a tile of its own
+//   warp  16    loader     : up to eight lanes, bulk copies of the patch planes into the stage ring
+//   warp  17    MMA issuer : converged, one elected lane
 //
-// i.e. twice the epilogue threads on every accumulator, each holding a quarter of its columns.
-// The scratch planes come from the caller (tcbnn_conv_workspace_bytes).
+// (or 8 or 4 epilogue warps, see EPIW).  The planes come from the caller (tcbnn_conv_workspace_bytes).
 #pragma once
 #include "bconv_umma_as.cuh"
 
@@ -30,14 +29,14 @@ namespace umma {
 // faster: an mbarrier wait names its phase by parity only, so a waiter must see every phase of a
 // barrier; with two consumers alternating on the same ring slot the one that runs ahead finds the
 // parity of the phase before last already complete and reads a slot that has not been refilled.)
-constexpr int kPreMmaWarps = 1;
+//
 // EPIW, the kernel's third template argument, is the number of epilogue warps: 16 (one CTA per SM,
 // all of tensor memory), a single group of 4 or 8 (launches with one tile per CTA, where only latency
-// counts: registers for all of a tile's residual at once, and the epilogue rehearsed) or 8 (n-tile 64 only: each thread then takes 32 columns instead of 16, the
-// CTA allocates half of tensor memory and two CTAs share an SM -- twice the independent
+// counts: registers for all of a tile's residual at once, and the epilogue rehearsed) or 8 at an n-tile of
+// 64 (two groups; the CTA allocates half of tensor memory and two CTAs share an SM -- twice the independent
 // loader / issuer / epilogue pipelines, so that one CTA's barrier round trips and epilogue
-// latency are covered by the other's work, and half the per-thread bookkeeping per output).
-__host__ __device__ constexpr int pre_threads(int epiw) { return epiw * 32 + 32 + 32 * kPreMmaWarps; }
+// latency are covered by the other's work).
+__host__ __device__ constexpr int pre_threads(int epiw) { return epiw * 32 + 64; }
 constexpr int kPreMaxStages = 8;           // patch ring depth is chosen by the host from the shared memory left
 
 // positions of zero padding in front of the planes (a tile's patch starts up to back_y*PW+back_x
@@ -310,15 +309,13 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             }
         }
         __syncwarp();
-    } else if (warp >= MMA_WARP && warp < MMA_WARP + kPreMmaWarps) {
+    } else if (warp > LOAD_WARP) {
         // =============================== MMA issuer =========================================
         // The whole warp runs the control flow converged and polls the barriers, and one elected
         // lane issues: what the issuing thread executes between two MMAs is time the tensor pipe
         // idles, and a lone lane in a diverged warp pays far more per branch and per wait.
-        constexpr bool converged = true;
-        const bool elected = elect_one();
-        if (converged || lane == 0) {
-            const bool leader = converged ? elected : true;
+        {
+            const bool leader = elect_one();
             const uint32_t lboA = (uint32_t)a.NPOS * 16u, lboB = NT * 16u;
             const uint64_t descA0 = smem_desc(smem_u32(sAraw), lboA, 128u);
             const uint64_t descB0 = smem_desc(smem_u32(sB), lboB, 128u);
@@ -339,7 +336,6 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             // the next stage needs is worked out behind the stage's first MMAs, while these keep the
             // pipe busy: between the last MMA of a stage and the first of the next only a branch on
             // the outcome of tests made earlier is left.
-            static_assert(kPreMmaWarps == 1, "the counters below assume one issuing warp");
             const uint32_t spt = (uint32_t)(NCB / CBS);    // stages per tile
             const uint32_t nit = mfirst < mtiles ? (uint32_t)((mtiles - mfirst + mstep - 1) / mstep) * spt : 0u;
             uint32_t s = 0, b = 0, sph = 0, bph = 0, left = spt;      // left: stages of this tile still to issue
