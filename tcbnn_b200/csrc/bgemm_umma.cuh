@@ -21,8 +21,8 @@
 // A 128 x 128 tile reads 8 KB of operands per k-block and has 8 KB copied in, which fills the
 // shared-memory port for 128 clocks (136 measured) where its MMA takes 64.  A pair does four times the work on
 // twice the SMs: each reads its 128 rows of A and half of W, 4 + 4 KB, and receives as much, for an MMA that
-// takes 128 (131-152 measured).  8192 x 8192 x 8192 with threshold bits 204 -> 186 us against 256 x 128
-// tiles on one SM (28 KB and 220 clocks per k-block), the kernel itself 0.79 of the MMA rate.
+// takes 128 (133-153 measured).  8192 x 8192 x 8192 with threshold bits 204 -> 186 us against 256 x 128
+// tiles on one SM (28 KB and 220 clocks per k-block); 174 by graph replay, the kernel 145 of it, 0.85 of the MMA rate.
 //
 // Loaders and issuer run ahead across tile boundaries, so set-up, first loads and epilogue of all
 // but a CTA's last tile are hidden: as one CTA per tile (two per SM) the MLP's hidden layer, 8192 x 1024
