@@ -16,6 +16,8 @@ Topologies follow the reference drivers, not the textbook networks:
   * alexnet, vgg16_imagenet : alexnet.cu:141-178, imagenet_vgg.cu:217-280 (11x11 / 5x5 filters,
                  192 / 384 channels, pooled layers at 224 x 224).
 """
+import weakref
+
 import numpy as np
 import torch
 
@@ -222,47 +224,60 @@ def synthetic_input_u8(spec, seed, batch=None):
 _FACTS = (torch.Tensor.data_ptr, torch.Tensor.size, torch.Tensor.stride)
 
 
-class _Pass:
-    """The prepared calls of one pass over a network's layers, which it makes at once, and the graph recorded
-    of them.  They serve while nothing they were prepared from has changed: an attribute of a layer, a descriptor, a
-    process-wide setting, the place or shape of a tensor (t.data = ... changes these in place).  The tensors
-    are kept alive but for the input, which is compared by its facts."""
+def _input_facts(layers):
+    t = layers[0].input_gpu
+    return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
+
+
+class _Calls:
+    """A network's layers' calls, prepared.  Once noted they serve while nothing but the input has changed of what
+    they were prepared from: an attribute of a layer, its live batch, a descriptor, a process-wide
+    setting, the place or shape of a tensor (t.data = ... changes these in place).  The tensors, but for the
+    input, are kept alive."""
+
+    noted = False
 
     def __init__(self, layers):
         device = layers[0].output_gpu.device
         while True:
-            scratch = ops.shared_scratch(device)
+            self.scratch = ops.shared_scratch(device)
             prepared = [l._call_args(True) for l in layers]
-            if scratch is ops.shared_scratch(device):                        # (else replaced by a larger one on the way)
+            if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
-        self.run()
-        # (noted behind the first launches: the GPU is busy meanwhile)
-        self.input = self._input_facts(layers)
         self.kept = [t for _, _, keep in prepared for t in keep if t is not layers[0].input_gpu]
+
+    def note(self, layers):
         self.tensors = list({id(t): t for t in self.kept if torch.is_tensor(t)}.values())
         self.facts = [list(map(f, self.tensors)) for f in _FACTS]
+        self.scratch = next((t for t in self.tensors if t is self.scratch), None)    # replaced when a larger layer asks for it
         self.descs = list({id(d): d for d in self.kept if isinstance(d, lib.ConvDesc)}.values())
         self.desc_facts = list(map(bytes, self.descs))
-        self.scratch = next((t for t in self.tensors if t is scratch), None)     # replaced when a larger layer asks for it
         self.layers = list(layers)
-        self.generations = [l.generation for l in layers]
+        self.states = [l.state() for l in layers]
         self.settings, self.device = lib.settings_generation, torch._C._cuda_getDevice()
-        self.seen, self.graph = 1, None
+        self.noted = True
 
-    @staticmethod
-    def _input_facts(layers):
-        t = layers[0].input_gpu
-        return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
-
-    def holds(self, layers):
-        """Whether the layers would make the same calls now."""
-        return (self.layers == layers and [l.generation for l in layers] == self.generations and
-                self.input == self._input_facts(layers) and
+    def hold(self, layers):
+        """Whether the layers would make the same calls now, whatever their input."""
+        return (self.noted and self.layers == layers and [l.state() for l in layers] == self.states and
                 all(list(map(f, self.tensors)) == g for f, g in zip(_FACTS, self.facts)) and
                 list(map(bytes, self.descs)) == self.desc_facts and
                 self.settings == lib.settings_generation and self.device == torch._C._cuda_getDevice() and
                 (self.scratch is None or self.scratch is ops.shared_scratch(self.scratch.device)))
+
+
+class _Pass:
+    """_Calls on one input tensor, and the graph recorded of them."""
+
+    def __init__(self, calls, layers, fresh=True):
+        """fresh: the calls have just been prepared, on this input."""
+        self.common, self.calls = calls, list(calls.calls)
+        if not fresh:
+            name, args, _ = layers[0]._call_args(True)
+            self.calls[0] = lib.bound(name), args
+        self.input = _input_facts(layers)
+        self.seen, self.graph = 0, None
 
     def run(self):
         stream = ops._stream()
@@ -384,7 +399,7 @@ class Network:
                 continue
             used = ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0
             if cons.units_room is not None:
-                cons.producer = prod
+                cons.producer = weakref.ref(prod)         # (prod may hold cons: In128LayerParam.expands)
                 cons.input_units = prod.next_units = cons.units_room if used else None
             cons.weight_units = cons.weight_room if used else None
             if cons.weight_units is not None:
@@ -450,10 +465,17 @@ class Network:
         then on: the same launches, submitted at once (the MLP's five layers at batch 8 cost the host 21
         us one by one).  Anything that changes a layer's call (a buffer, the live batch, a
         process-wide setting) starts over."""
-        p = self._pass
-        if p is None or not p.holds(self.layers):
-            self._pass = _Pass(self.layers)
+        last = self._pass
+        if last is None or not last.common.hold(self.layers):
+            p = self._pass = _Pass(_Calls(self.layers), self.layers)
+            p.run()
+            if last is not None:                         # (behind the launches: the GPU is busy meanwhile)
+                p.common.note(self.layers)
+            p.seen = 2 if last is not None and not last.common.noted and last.input == p.input else 1
             return self.layers[-1].get_output_gpu()
+        p = last
+        if p.input != _input_facts(self.layers):
+            p = self._pass = _Pass(last.common, self.layers, fresh=False)
         capturing = torch.cuda.is_current_stream_capturing()
         if not capturing:
             if p.seen == 2:
@@ -469,17 +491,18 @@ class Network:
 
     def forward_graph(self):
         """forward() replayed from a CUDA graph: the layer launches (every entry point takes the
-        stream and none allocates or synchronises) are captured once per input buffer, after one
+        stream and none allocates or synchronises) are captured once per input buffer and live batch, after one
         eager pass that lets the first layer compile its kernel variants, and replayed as one
         submission on the current stream.  Same launches, same results; the host's per-launch
-        work and the gaps between the launches go away.  A graph serves while its pass holds (_Pass) and
-        keeps the buffers it points into alive; the last MAX_GRAPHS are kept."""
-        first = self.layers[0]
-        key = (first.input_gpu.data_ptr(), self.live_batch)
+        work and the gaps between the launches go away.  A graph serves while its calls hold (_Calls) and
+        keeps the buffers they point into alive; the last MAX_GRAPHS are kept."""
+        key = (self.layers[0].input_gpu.data_ptr(), self.live_batch)
         graphs = self.__dict__.setdefault("_graphs", {})
         p = graphs.get(key)
-        if p is None or not p.holds(self.layers):
-            p = _Pass(self.layers)
+        if p is None or p.input != _input_facts(self.layers) or not p.common.hold(self.layers):
+            p = _Pass(_Calls(self.layers), self.layers)
+            p.run()
+            p.common.note(self.layers)
             torch.cuda.synchronize()
             p.graph = p.record()
             if p.graph is None:
@@ -551,7 +574,7 @@ class HostFeeder:
     def _network(self):
         """What a part takes over from the network when it is made."""
         layers = self.net.layers
-        return (self.net.live_batch, layers[-1].output_gpu.data_ptr(), [(l, l.generation) for l in layers],
+        return (self.net.live_batch, layers[-1].output_gpu.data_ptr(), [(l, l.state()) for l in layers],
                 [bytes(l.desc) for l in layers if hasattr(l, "desc")])
 
     def _run_parts(self, main, slot, cuts):

@@ -80,16 +80,21 @@ class _Layer:
     planes it was wired to, Conv128LayerParam.input_planes): one call of the C ABI, prepared (_call_args)
     each time.  models.Network prepares the calls of a whole pass with in_pass=True -- the layer in front
     has just run, and what it handed over besides its bits (expanded operands) is used -- and keeps them
-    while no layer's generation changes and no tensor moves."""
+    while no layer's state changes and no tensor moves."""
 
-    # what a caller replaces from pass to pass: not a change of the layer
-    _PER_PASS = ()
+    # The live batch and what follows from it come and go (set_batch); the first layer's input is the caller's.
+    _NO_CHANGE = ("live", "input_units", "next_units", "weight_units", "expands")
+    live = None
 
     def __setattr__(self, name, value):
         d = self.__dict__
         d[name] = value
-        if name not in self._PER_PASS:
+        if name not in self._NO_CHANGE:
             d["generation"] = d.get("generation", 0) + 1
+
+    def state(self):
+        """Changes with every attribute that is set, except that a live batch that comes back is the same."""
+        return self.generation, self.live
 
     def forward(self):
         name, args, _ = self._call_args(False)
@@ -110,7 +115,7 @@ class _Layer:
 class In128LayerParam(_Layer):
     """param.h:115-222.  fp32 [input_height][input_width] -> bit rows."""
 
-    _PER_PASS = ("input_gpu",)
+    _NO_CHANGE = _Layer._NO_CHANGE + ("input_gpu",)
 
     def __init__(self, name, input_height, input_width):
         self.name = name
@@ -202,7 +207,7 @@ class Fc128LayerParam(_Layer):
     # every pass expands it (weight_units).  None of them outlives a pass: whoever writes the packed
     # rows between two passes, by whatever means, is followed.
     units_room = input_units = next_units = weight_room = weight_units = None
-    producer = None
+    producer = None        # weak reference to the layer that writes the input
 
     def __setattr__(self, name, value):
         super().__setattr__(name, value)
@@ -223,8 +228,8 @@ class Fc128LayerParam(_Layer):
     def _call_args(self, in_pass):
         a, w, thr, out, ws = self.input_gpu, self.weight_gpu, self.bn_gpu, self.output_gpu, self.workspace
         ops._need_cuda(a, w, thr)
-        made = self.producer.output_gpu if self.producer is not None else None
-        u = (self.input_units if made is not None and made.data_ptr() == a.data_ptr() else None,
+        prod = self.producer() if self.producer is not None else None
+        u = (self.input_units if prod is not None and prod.output_gpu.data_ptr() == a.data_ptr() else None,
              self.weight_units, self.next_units) if in_pass else (None, None, None)
         return "tcbnn_fc_layer_x", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
                                     a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws),
@@ -292,7 +297,7 @@ class Out128LayerParam(_Layer):
 class InConv128LayerParam(_Layer):
     """param.h:701-870.  First conv layer on fp32 NCHW images."""
 
-    _PER_PASS = ("input_gpu",)
+    _NO_CHANGE = _Layer._NO_CHANGE + ("input_gpu",)
 
     def __init__(self, name, input_height, input_width, filter_height, filter_width,
                  input_channels, output_channels, batch, stride_height=1, stride_width=1,

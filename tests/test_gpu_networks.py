@@ -1,4 +1,7 @@
 """GPU parity of whole networks, layer by layer, against the CPU oracle."""
+import gc
+import weakref
+
 import numpy as np
 import pytest
 import torch
@@ -168,6 +171,42 @@ def test_tensor_given_another_storage_in_place_counts(cuda, which):
     fc.weight_gpu.t_()
     with pytest.raises(lib.TcbnnError):              # refused as it always was: rows are no longer contiguous
         net.forward()
+
+
+@pytest.mark.parametrize("which", ["mlp", "vgg_cifar"])
+def test_network_gives_its_memory_back_when_dropped(cuda, which):
+    """Layers, buffers and recorded passes form no reference cycle: what a network holds is free as soon as the
+    last reference to it goes, not when the garbage collector gets to it."""
+    spec = models.mlp_spec(1100) if which == "mlp" else models.vgg_cifar_spec(4)
+    w, x = models.synthetic_weights(spec, 70), models.synthetic_input(spec, 71)
+    gc.collect()
+    gc.disable()
+    try:
+        net = models.Network(spec, w, x)
+        feeder = models.HostFeeder(net)
+        feeder.PART_BYTES = x.nbytes // 2
+        for _ in range(4):
+            net.forward()
+        net.forward_graph()
+        feeder.run([torch.from_numpy(np.ascontiguousarray(x)).pin_memory()])
+        torch.cuda.synchronize()
+        gone = [weakref.ref(l) for l in net.layers] + [weakref.ref(p) for p in feeder.parts.values()]
+        del net, feeder
+        assert all(r() is None for r in gone)
+    finally:
+        gc.enable()
+
+
+def test_live_batches_that_come_back_replay_their_graphs(cuda):
+    spec = models.vgg_cifar_spec(6)
+    net = models.Network(spec, models.synthetic_weights(spec, 72), models.synthetic_input(spec, 73))
+    want = net.forward().clone()
+    kept = {}
+    for live in (6, 5, 6, 5, 6):
+        net.set_batch(live)
+        assert torch.equal(net.forward_graph()[:live], want[:live])
+        p = net._graphs[(net.layers[0].input_gpu.data_ptr(), live)]
+        assert kept.setdefault(live, p) is p
 
 
 @pytest.mark.parametrize("which", ["mlp", "resnet18", "vgg_cifar"])
