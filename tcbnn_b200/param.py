@@ -75,6 +75,9 @@ def _dev():
     return torch.device("cuda", torch.cuda.current_device())
 
 
+changes = 0            # attributes set on any layer so far: while it stands, no layer has changed
+
+
 class _Layer:
     """What the layer classes share.  forward() runs the layer by itself, on the bits in input_gpu (or on the
     planes it was wired to, Conv128LayerParam.input_planes): one call of the C ABI, prepared (_call_args)
@@ -91,6 +94,9 @@ class _Layer:
         d[name] = value
         if name not in self._NO_CHANGE:
             d["generation"] = d.get("generation", 0) + 1
+        if name != "input_gpu" or name not in self._NO_CHANGE:
+            global changes
+            changes += 1
 
     def state(self):
         """Changes with every attribute that is set, except that a live batch that comes back is the same."""
