@@ -804,27 +804,41 @@ struct NextPlanes { uint4* planes; long long positions, front; int PW, VH, nplan
 // pools by OR-ing the window's bits): the tcgen05 kernels compute a pooled layer on its pre-pool
 // grid, this pass reduces it.
 // With `nx` (planes set) it also writes the pooled output as the next layer's pre-expanded input, which
-// saves that layer's own pass over it.
+// saves that layer's own pass over it.  A thread takes V words of a pixel (V divides Ow): four loads of up to 16
+// bytes at once.
+template <int V>
 __global__ void __launch_bounds__(256) k_pool_bits(const uint32_t* in, uint32_t* out, int B, int P, int Q, int Ow,
                                                   long long out_image_stride, NextPlanes nx) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a programmatic dependent, like what follows it
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const long long total = (long long)B * P * Q * Ow;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long q = total < (1LL << 32) ? (unsigned)i / (unsigned)Ow : (unsigned long long)i / Ow;
-        const int w = (int)(i - (long long)q * Ow);
-        const unsigned pix = (unsigned)q, row = pix / (unsigned)Q;       // (fewer than 2^31 pixels: conv_check)
-        const int x = (int)(pix - row * Q), y = (int)(row % (unsigned)P);
-        const long long n = row / (unsigned)P;
-        const uint32_t* s0 = in + ((n * 2 * P + 2 * y) * 2 * Q + 2 * x) * Ow + w;
-        const uint32_t* s1 = s0 + (long long)2 * Q * Ow;
-        const uint32_t v = ld_dep(s0) | ld_dep(s0 + Ow) | ld_dep(s1) | ld_dep(s1 + Ow);
-        out[n * out_image_stride + ((long long)y * Q + x) * Ow + w] = v;
+    using Words = typename std::conditional<V == 4, uint4, typename std::conditional<V == 2, uint2, uint32_t>::type>::type;
+    const unsigned G = (unsigned)Ow / V;
+    const unsigned long long total = (unsigned long long)B * P * Q * G;
+    const int step = Ow * 2 * Q;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (unsigned)gridDim.x * blockDim.x) {
+        const unsigned pix = total < (1ULL << 32) ? (unsigned)i / G : (unsigned)(i / G);       // (fewer than 2^31 pixels: conv_check)
+        const unsigned row = pix / (unsigned)Q, n = row / (unsigned)P;
+        const int x = (int)(pix - row * Q), y = (int)(row - n * P), w = (int)((unsigned)i - pix * G) * V;
+        const uint32_t* s0 = in + (((long long)n * 2 * P + 2 * y) * 2 * Q + 2 * x) * Ow + w;
+        const Words q[4] = {ld_dep((const Words*)s0), ld_dep((const Words*)(s0 + Ow)), ld_dep((const Words*)(s0 + step)),
+                            ld_dep((const Words*)(s0 + step + Ow))};
+        uint32_t v[V];
+        const uint32_t* e = reinterpret_cast<const uint32_t*>(q);
+#pragma unroll
+        for (int i = 0; i < V; i++) v[i] = e[i] | e[V + i] | e[2 * V + i] | e[3 * V + i];
+        uint32_t* dst = out + (long long)n * out_image_stride + ((long long)y * Q + x) * Ow + w;
+        if (((uintptr_t)dst & (sizeof(Words) - 1)) == 0) {
+            *reinterpret_cast<Words*>(dst) = *reinterpret_cast<const Words*>(v);
+        } else {
+#pragma unroll
+            for (int i = 0; i < V; i++) dst[i] = v[i];
+        }
         if (nx.planes) {
             const bool par = nx.nplane == 4;               // stride-2 consumer: one plane per row / column parity
             const int pl = par ? (y & 1) * 2 + (x & 1) : 0, py = par ? y >> 1 : y, px = par ? x >> 1 : x;
-            nx.planes[((size_t)w * nx.nplane + pl) * nx.positions + nx.front + (n * nx.VH + py) * nx.PW + px] = umma::expand32_f4(v);
+            uint4* at = nx.planes + ((size_t)w * nx.nplane + pl) * nx.positions + nx.front + ((long long)n * nx.VH + py) * nx.PW + px;
+#pragma unroll
+            for (int i = 0; i < V; i++) at[(size_t)i * nx.nplane * nx.positions] = umma::expand32_f4(v[i]);
         }
     }
 }
@@ -950,6 +964,18 @@ __global__ void __launch_bounds__(128) k_umma_peak_mxf4(int iters, long long* cy
     umma::tc_fence_before();
     __syncthreads();
     umma::tc_fence_after();
+// (the pre-pool bits are 256-byte aligned scratch)
+cudaError_t launch_pool_bits(const uint32_t* prepool, uint32_t* out, const tcbnn_conv_desc* d, int Ow, long long out_image_stride,
+                             const NextPlanes& nx, int sms, cudaStream_t st) {
+    // as many words per thread as leaves every SM four blocks: fewer threads each with more to store are slower
+    // (14 x 14 x 512 at batch 32, pooled layer: 33.7 us a word at a time, 35.8 four; 32 x 32 x 128 at batch 1024:
+    // 63.3 and 58.2)
+    const long long words = (long long)d->B * d->OH * d->OW * Ow, enough = 4LL * sms * 256;
+    const int V = Ow % 4 == 0 && words >= 4 * enough ? 4 : Ow % 2 == 0 && words >= 2 * enough ? 2 : 1;
+    return launch_dependent(V == 4 ? k_pool_bits<4> : V == 2 ? k_pool_bits<2> : k_pool_bits<1>,
+                            (unsigned)elementwise_grid((long long)d->B * d->OH * d->OW * (Ow / V), sms), 256, 0, st, prepool, out, d->B, d->OH,
+                            d->OW, Ow, out_image_stride, nx);
+}
     if (threadIdx.x == 0) {
         // K-major, no swizzle: a 16-byte row of a core matrix holds 32 elements; K = 64 is two core
         // matrices `lbo` apart
@@ -1615,8 +1641,7 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
       };
       if (launch_tc()) return 1;
       if (pooled) {
-          const cudaError_t e = launch_dependent(k_pool_bits, (unsigned)elementwise_grid((long long)d->B * d->OH * d->OW * Ow, sms), 256,
-                                                 0, st, prepool, out, d->B, d->OH, d->OW, Ow, out_image_stride, nx ? *nx : NextPlanes{});
+          const cudaError_t e = launch_pool_bits(prepool, out, d, Ow, out_image_stride, nx ? *nx : NextPlanes{}, sms, st);
           if (nx) *fed = true;
           if (e != cudaSuccess) return fail("conv_layer (OR pooling): %s", cudaGetErrorString(e));
       }
