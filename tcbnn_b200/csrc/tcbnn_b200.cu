@@ -638,7 +638,22 @@ __global__ void __launch_bounds__(umma::pre_threads(EPIW), EPIW == 8 && NT == 64
 }
 __global__ void __launch_bounds__(256) k_expand_raster(umma::ConvWsArgs a, uint4* planes, long long positions,
                                                        long long front) {
-    umma::expand_raster(a, planes, positions, front);
+    umma::expand_raster<V>(a, planes, positions, front);
+}
+cudaError_t launch_expand_raster(const umma::ConvWsArgs& a, uint4* planes, long long positions, long long front, int sms, cudaStream_t st) {
+    const int V = a.C % 128 == 0 && ((uintptr_t)a.in & 15) == 0 ? 4 : 2;
+    const unsigned rows = (unsigned)(a.C / 32 / V * (a.stride == 2 ? 4 : 1));
+    const long long want = (positions + 255) / 256, most = (8LL * sms + rows - 1) / rows;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(want < most ? want : most), rows);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, V == 4 ? k_expand_raster<4> : k_expand_raster<2>, a, planes, positions, front);
 }
 
 template <int NT, int EPI, int EPIW>
@@ -737,13 +752,12 @@ int launch_conv_umma_pre_ring(umma::ConvWsArgs& a, int sms, cudaStream_t st, boo
 template <int NT>
 int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st, bool expand) {
     if (expand) {
-        const long long units = a.pre_positions * (a.C >> 6) * (a.stride == 2 ? 4 : 1);
-        const cudaError_t e = launch_dependent(k_expand_raster, (unsigned)elementwise_grid(units, sms), 256, 0, st, a,
-                                               const_cast<uint4*>(a.pre), a.pre_positions, a.pre_front);
+        const cudaError_t e = launch_expand_raster(a, const_cast<uint4*>(a.pre), a.pre_positions, a.pre_front, sms, st);
         if (e != cudaSuccess) return fail("conv_layer (input expansion): %s", cudaGetErrorString(e));
     }
     const bool plain = !a.res_in && !a.res_out && !a.acc_out;
     const bool chunked = !a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked);
+template <int V>
     // A tile per CTA and none to spare: the form for latency (one image through ResNet-18: 135 -> 115 us)
     constexpr int kSingle = NT == 128 ? 8 : 4;
     if (g_conv_single && (plain || chunked) && (a.NV + 127) / 128 * (a.O / NT) <= sms)
@@ -1494,8 +1508,7 @@ static int expand_for_next(const tcbnn_conv_desc* next, const uint32_t* bits, co
     umma::fastdiv_setup(a.VH, &a.vh_mul, &a.vh_sh);
     int sms;
     if (sm_count(&sms)) return 1;
-    const cudaError_t e = launch_dependent(k_expand_raster, (unsigned)elementwise_grid(nx.positions * (next->C >> 6) * nx.nplane, sms),
-                                           256, 0, st, a, nx.planes, nx.positions, nx.front);
+    const cudaError_t e = launch_expand_raster(a, nx.planes, nx.positions, nx.front, sms, st);
     if (e != cudaSuccess) return fail("expansion for the next layer: %s", cudaGetErrorString(e));
     return 0;
 }

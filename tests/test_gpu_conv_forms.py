@@ -1,0 +1,49 @@
+"""Forms that a convolution's launches take by size and alignment, at their edges, against the CPU oracle (bits,
+integers and fp32 sums are exact)."""
+import numpy as np
+import pytest
+import torch
+
+import oracle as orc
+import util
+from tcbnn_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a, cuda):
+    return torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).to(cuda)
+
+
+def _u32(t):
+    return t.cpu().numpy().view(np.uint32)
+
+
+# B, H, W, C, O, stride, pool; words in front of the input (the expansion pass takes four words of a pixel where they are
+# 16-byte aligned, two otherwise; the pooling pass one, two or four words of a pixel by their number)
+FORMS = [
+    (2, 7, 9, 64, 64, 1, 1, 0), (2, 7, 9, 128, 64, 1, 1, 0), (2, 7, 9, 128, 64, 1, 1, 2), (3, 8, 6, 192, 64, 1, 1, 0),
+    (3, 8, 6, 256, 32, 2, 1, 0), (3, 8, 6, 256, 32, 2, 1, 2), (1, 1, 1, 128, 128, 1, 1, 0),
+    (2, 10, 6, 64, 32, 1, 2, 0), (2, 10, 6, 64, 96, 1, 2, 0), (2, 10, 6, 64, 128, 1, 2, 0), (40, 160, 160, 64, 64, 1, 2, 0),
+    (160, 64, 64, 64, 128, 1, 2, 0),
+]
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_expansion_and_pooling_passes(cuda, form):
+    B, H, W, C, O, st, pool, front = form
+    g = util.rng(sum(form))
+    x = util.rand_words(g, (B, H, W, C // 32))
+    f = util.rand_words(g, (O, 9, C // 32))
+    thr = (g.standard_normal(O) * np.sqrt(C * 9) * 0.5).astype(np.float32)
+    d = ops.conv_desc(B, H, W, C, O, 3, 3, st, st, True, pool)
+    room = torch.zeros((x.size + front,), dtype=torch.int32, device=cuda)
+    dx = room[front:].view(x.shape)
+    dx.copy_(_dev(x, cuda))
+    prep = ops.conv_prepare(d, _dev(f, cuda))
+    go, _, _ = ops.conv_layer(d, dx, prep, _dev(thr, cuda))
+    assert ops.conv_status(d, prep) == 0
+    n = min(B, 3)                                        # (the oracle on the first and the last images)
+    for part in {(0, n), (B - n, B)}:
+        eo, _, _ = orc.conv_layer(x[part[0]:part[1]], f, thr, C, 3, 3, st, st, True, pool)
+        assert np.array_equal(_u32(go)[part[0]:part[1]].reshape(eo.shape), eo), part
