@@ -132,7 +132,28 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
          " const float* img = c.x + (size_t)n * 3 * plane;\n"
          " const unsigned char* img8 = c.x8 + (size_t)n * 3 * plane;\n";
     s += " float ";
-    for (int o = 0; o < O; o++) emit(s, "a%d = 0.f%s", o, o + 1 < O ? ", " : ";\n");
+    for (int o = 0; o < O; o++) emit(s, "a%d%s", o, o + 1 < O ? ", " : ";\n");
+    // The first two taps make the sums.  0 + v + w is v + w but for the sign of a zero, which only a stored
+    // accumulator shows (it gets its zero there); a channel whose first term is a -v sums the
+    // negatives of everything and is turned round at the end; and channels that agree in both terms share
+    // their sum until the third (28 different ones of 64 are usual): 136 adds less of 640 for 64 channels of a
+    // 3 x 3 filter, 3 % of a 7 x 7 one.
+    auto minus = [&](int tap, int o) { return codes[(size_t)tap * Oall + OB + o] < 4; };       // pattern k is minus pattern 7 - k
+    auto mag = [&](int tap, int o) { const int k = codes[(size_t)tap * Oall + OB + o]; return k >= 4 ? k : 7 - k; };
+    std::vector<int> shared(O, 0);                       // the channel's sum of two taps
+    s += " float u4, u5, u6, u7;\n";
+    if (RS > 1) {
+        std::vector<int> seen;
+        for (int o = 0; o < O; o++) {
+            const int key = mag(0, o) * 16 + mag(1, o) * 2 + (minus(0, o) != minus(1, o));
+            size_t i = 0;
+            while (i < seen.size() && seen[i] != key) i++;
+            if (i == seen.size()) seen.push_back(key);
+            shared[o] = (int)i;
+        }
+        s += " float ";
+        for (size_t i = 0; i < seen.size(); i++) emit(s, "b%d%s", (int)i, i + 1 < seen.size() ? ", " : ";\n");
+    }
     for (int r = 0; r < h.R; r++) {
         s += " {\n";
         emit(s, "  float g0[%d], g1[%d], g2[%d];\n", 4 * NQ4, 4 * NQ4, 4 * NQ4);
@@ -174,16 +195,24 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
             // free: they are emitted grouped by the magnitude they add, consecutive instructions then
             // share a source register and the assembler can serve it from the operand reuse cache
             // instead of the register file (fewer bank conflicts next to the accumulator reads).
-            for (int mag = 4; mag < 8; mag++)
+            if (t == 0) s += "   u4 = v4; u5 = v5; u6 = v6; u7 = v7;\n";
+            std::vector<char> done(O, 0);
+            for (int m = 4; m < 8 && t > 0; m++)
                 for (int o = 0; o < O; o++) {
-                    const int k = codes[(size_t)t * Oall + OB + o];
-                    if ((k >= 4 ? k : 7 - k) != mag) continue;
-                    if (k >= 4) emit(s, "   a%d = __fadd_rn(a%d, v%d);\n", o, o, k);
-                    else emit(s, "   a%d = __fadd_rn(a%d, -v%d);\n", o, o, 7 - k);     // pattern k is minus pattern 7-k
+                    if (mag(t, o) != m) continue;
+                    const char* sign = minus(t, o) == minus(0, o) ? "" : "-";
+                    if (t > 2) emit(s, "   a%d = __fadd_rn(a%d, %sv%d);\n", o, o, sign, m);
+                    else if (t == 2) emit(s, "   a%d = __fadd_rn(b%d, %sv%d);\n", o, shared[o], sign, m);
+                    else if (!done[shared[o]]++) emit(s, "   b%d = __fadd_rn(u%d, %sv%d);\n", shared[o], mag(0, o), sign, m);
                 }
             s += "  }\n";
         }
         s += " }\n";
+    }
+    for (int o = 0; o < O; o++) {
+        if (RS == 1) emit(s, " a%d = u%d;\n", o, mag(0, o));
+        if (RS == 2) emit(s, " a%d = b%d;\n", o, shared[o]);
+        if (minus(0, o)) emit(s, " a%d = -a%d;\n", o, o);
     }
     // threshold (kernel.cuh:655), pack, pool
     s += " uint32_t w0 = 0, w1 = 0;\n";
@@ -256,7 +285,7 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
     }
     if (want_acc) {
         emit(s, " float* q = c.acc_out + opix * %d + OBASE;\n", Oall);
-        for (int o = 0; o < O; o++) emit(s, " q[%d] = a%d;\n", o, o);
+        for (int o = 0; o < O; o++) emit(s, " q[%d] = a%d + 0.f;\n", o, o);
     }
     s += "}\n";
     }   // channel groups

@@ -47,3 +47,28 @@ def test_expansion_and_pooling_passes(cuda, form):
     for part in {(0, n), (B - n, B)}:
         eo, _, _ = orc.conv_layer(x[part[0]:part[1]], f, thr, C, 3, 3, st, st, True, pool)
         assert np.array_equal(_u32(go)[part[0]:part[1]].reshape(eo.shape), eo), part
+
+
+# R, S, O: one tap, two, three; channels that share their first two terms, and a filter all of whose channels do
+@pytest.mark.parametrize("R,S,O,same", [(1, 1, 40, False), (1, 2, 64, False), (2, 1, 5, False), (1, 3, 70, False), (3, 3, 64, True), (3, 3, 96, False)])
+def test_first_layer_sums_of_few_taps(cuda, R, S, O, same):
+    """The compiled first layer makes its sums from the first two taps, shared between channels that agree in them:
+    sums, residuals and bits of the oracle, with zeros among the pixels (a sum of -0 is stored as 0)."""
+    g = util.rng(R * 100 + S * 10 + O)
+    B, H, W = 3, 13, 11
+    x = g.standard_normal((B, 3, H, W)).astype(np.float32)
+    x[:, :, :4] = 0.0
+    F = g.standard_normal((R * S, 3, O)).astype(np.float32)
+    if same:
+        F[:2] = F[:2, :, :1]
+    thr = (g.standard_normal(O) * 2).astype(np.float32)
+    thr[0] = 0.0
+    eo, er, ea = orc.inconv_layer(x, F, thr, R, S, 1, 1, True, 1, save_residual=True, want_acc=True)
+    d = ops.conv_desc(B, H, W, 3, O, R, S, 1, 1, True, 1)
+    fb = ops.pack_inconv_filter(_dev(F, cuda))
+    spec = ops.inconv_specialize(d, fb, _dev(thr, cuda))
+    go, gr, ga = ops.inconv_layer(d, _dev(x, cuda), fb, _dev(thr, cuda), save_residual=True, want_acc=True, specialized=spec)
+    assert np.array_equal(ga.cpu().numpy().view(np.uint32), ea.view(np.uint32))        # (the sign of a zero too)
+    assert np.array_equal(gr.cpu().numpy(), er)
+    assert np.array_equal(_u32(go), eo)
+    spec.release()
