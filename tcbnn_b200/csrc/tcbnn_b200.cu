@@ -1382,7 +1382,7 @@ int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int
     if (ldo * 32 < N) return fail("fc_layer: ldo too small");
     if (((uintptr_t)a_units | (uintptr_t)w_units | (uintptr_t)next_units) & 255) return fail("fc_layer: units must be 256-byte aligned");
     if (next_units && (ldo & 1)) return fail("fc_layer: next_units needs an even ldo");
-    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr};
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr, settled};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream, GemmUnits{a_units, w_units, next_units});
 }
 
@@ -1390,7 +1390,7 @@ int tcbnn_out_layer(const uint32_t* A, const uint32_t* W, const float* scale, co
                     int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
                     size_t workspace_bytes, void* stream) {
     if (ldo < N) return fail("out_layer: ldo < N");
-    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_OUT_AFFINE, out, ldo, scale, bias, 1, nullptr};
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_OUT_AFFINE, out, ldo, scale, bias, 1, nullptr, settled};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -1519,6 +1519,12 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
                            long long out_image_stride, void* res_out, int res_out_bytes,
                            int32_t* acc_out, void* workspace, size_t workspace_bytes, int workspace_ready,
                            const NextPlanes* nx, bool* fed, void* stream) {
+    return tcbnn_fc_layer_p(A, W, thr, M, K, N, lda, ldw, out, ldo, workspace, workspace_bytes, a_units, w_units, next_units, 0, stream);
+}
+
+int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N, int lda, int ldw, uint32_t* out,
+                     int ldo, void* workspace, size_t workspace_bytes, const void* a_units, const void* w_units, void* next_units,
+                     int settled, void* stream) {
     *fed = false;
     if (conv_check(d, true)) return 1;
     const int Ow = (d->O + 31) / 32;
@@ -1529,6 +1535,12 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
     if (res_in && !residual_format(res_in_bytes, &res_in_bytes, &res_in_chunked))
         return fail("conv_layer: res_in_bytes must be 2, 4 or TCBNN_RES_INT16_CHUNKED");
     if (res_out && !residual_format(res_out_bytes, &res_out_bytes, &res_out_chunked, &res_out_proven))
+    return tcbnn_out_layer_p(A, W, scale, bias, M, K, N, lda, ldw, out, ldo, workspace, workspace_bytes, 0, stream);
+}
+
+int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,
+                      int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
+                      size_t workspace_bytes, int settled, void* stream) {
         return fail("conv_layer: res_out_bytes must be 2, 4 or TCBNN_RES_INT16_CHUNKED");
     if (!res_in) res_in_chunked = 0;
     if (!res_out) res_out_chunked = 0;

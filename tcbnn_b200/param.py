@@ -237,9 +237,10 @@ class Fc128LayerParam(_Layer):
         prod = self.producer() if self.producer is not None else None
         u = (self.input_units if prod is not None and prod.output_gpu.data_ptr() == a.data_ptr() else None,
              self.weight_units, self.next_units) if in_pass else (None, None, None)
-        return "tcbnn_fc_layer_x", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
+        # (a pass starts with a launch that waits for all before it: its weights are settled)
+        return "tcbnn_fc_layer_p", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
                                     a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws),
-                                    *(ops._ptr(t) for t in u)), (a, w, thr, out, ws, *u)
+                                    *(ops._ptr(t) for t in u), int(in_pass)), (a, w, thr, out, ws, *u)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -289,9 +290,9 @@ class Out128LayerParam(_Layer):
         a, w, out, ws = self.input_gpu, self.weight_gpu, self.output_gpu, self.workspace
         scale, bias = self.bn_scale_gpu, self.bn_bias_gpu
         ops._need_cuda(a, w, scale, bias)
-        return "tcbnn_out_layer", (ops._ptr(a), ops._ptr(w), ops._ptr(scale), ops._ptr(bias), self.live, self.input_width,
-                                   w.shape[0], a.shape[1], w.shape[1], ops._ptr(out), out.shape[1],
-                                   *ops._ws(ws)), (a, w, scale, bias, out, ws)
+        return "tcbnn_out_layer_p", (ops._ptr(a), ops._ptr(w), ops._ptr(scale), ops._ptr(bias), self.live, self.input_width,
+                                     w.shape[0], a.shape[1], w.shape[1], ops._ptr(out), out.shape[1],
+                                     *ops._ws(ws), int(in_pass)), (a, w, scale, bias, out, ws)
 
     def get_output_gpu(self):
         return self.output_gpu
