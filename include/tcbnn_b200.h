@@ -99,6 +99,15 @@ int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units
 int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
                      int lda, int ldw, uint32_t* out, int ldo, void* workspace, size_t workspace_bytes,
                      const void* a_units, const void* w_units, void* next_units, void* stream);
+/* The same within a pass: settled != 0 says that the weight and the thresholds (scale, bias) were complete before the
+ * launch in front of this one could start, e.g. because an ordinary launch came between whatever wrote them
+ * and it; they are then read ahead of the wait for that launch. */
+int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
+                     int lda, int ldw, uint32_t* out, int ldo, void* workspace, size_t workspace_bytes,
+                     const void* a_units, const void* w_units, void* next_units, int settled, void* stream);
+int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,
+                      int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
+                      size_t workspace_bytes, int settled, void* stream);
 int tcbnn_pack_rows_x(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
                       void* stream);
 int tcbnn_pack_rows_w(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
@@ -114,15 +123,6 @@ typedef struct tcbnn_conv_desc {
     int B, H, W, C, O, R, S;
     int stride_h, stride_w;
     int padding;            /* 1: "same"-style padding with the reference's arithmetic */
-/* The same within a pass: settled != 0 says that the weight and the thresholds (scale, bias) were complete before the
- * launch in front of this one could start, e.g. because an ordinary launch came between whatever wrote them
- * and it; they are then read ahead of the wait for that launch. */
-int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
-                     int lda, int ldw, uint32_t* out, int ldo, void* workspace, size_t workspace_bytes,
-                     const void* a_units, const void* w_units, void* next_units, int settled, void* stream);
-int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,
-                      int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
-                      size_t workspace_bytes, int settled, void* stream);
     int pool;               /* 1 or 2 (non-overlapping pool x pool OR-pooling) */
     /* derived */
     int pad_h, pad_w, OH, OW;

@@ -256,9 +256,9 @@ __device__ __forceinline__ void mma_f4_split(uint32_t d_tmem, uint32_t a_lo, uin
 //                   Bit 0 / 1 of the result: phase par0 / par1 of barrier bar0 / bar1 is complete.
 // Measured on groups of nine with one wait and one commit per group: 61.8 -> 48.0 clocks per MMA at
 // N = 64, 70.7 -> 64.0 at N = 128, the pipe's own rate.
-#define TCBNN_F4_MMA(AOFF, PRED)                                                                     \
+#define TCBNN_F4_MMA(G, AOFF, PRED)                                                                  \
     "add.u32 xa, %1, " AOFF ";\n\tmov.b64 da, {xa, %2};\n\tmov.b64 db, {xb, %4};\n\t"                \
-    "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%5], da, db, %6, [%8], [%9], " PRED ";\n\t" \
+    "@pl tcgen05.mma.cta_group::" G ".kind::mxf4.block_scale.block32 [%5], da, db, %6, [%8], [%9], " PRED ";\n\t" \
     "add.u32 xb, xb, %10;\n\t"
 #define TCBNN_F4_HEAD                                                                                \
     ".reg .pred pq, pt, pl;\n\t.reg .b64 da, db;\n\t.reg .b32 xa, xb;\n\t"                           \
@@ -266,49 +266,64 @@ __device__ __forceinline__ void mma_f4_split(uint32_t d_tmem, uint32_t a_lo, uin
 #define TCBNN_F4_IN                                                                                  \
     "r"(leader), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(d_tmem), "r"(idesc), "r"(acc), "r"(sfa), \
         "r"(sfb), "r"(step_b)
-template <int K>
+#define TCBNN_F4_RUN(G)                                                                              \
+    if constexpr (K == 9)                                                                            \
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA(G, "%11", "pq") TCBNN_F4_MMA(G, "%12", "pt") TCBNN_F4_MMA(G, "%13", "pt") \
+                     TCBNN_F4_MMA(G, "%14", "pt") TCBNN_F4_MMA(G, "%15", "pt") TCBNN_F4_MMA(G, "%16", "pt") \
+                     TCBNN_F4_MMA(G, "%17", "pt") TCBNN_F4_MMA(G, "%18", "pt") TCBNN_F4_MMA(G, "%19", "pt") "}" \
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]), \
+                       "r"(t[7]), "r"(t[8]) : "memory");                                             \
+    else if constexpr (K == 5)                                                                       \
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA(G, "%11", "pq") TCBNN_F4_MMA(G, "%12", "pt") TCBNN_F4_MMA(G, "%13", "pt") \
+                     TCBNN_F4_MMA(G, "%14", "pt") TCBNN_F4_MMA(G, "%15", "pt") "}"                   \
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]) : "memory"); \
+    else if constexpr (K == 4)                                                                       \
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA(G, "%11", "pq") TCBNN_F4_MMA(G, "%12", "pt") TCBNN_F4_MMA(G, "%13", "pt") \
+                     TCBNN_F4_MMA(G, "%14", "pt") "}"                                                \
+                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");          \
+    else                                                                                             \
+        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA(G, "%11", "pq") "}" ::TCBNN_F4_IN, "r"(t[0]) : "memory")
+template <int K, bool PAIR = false>
 __device__ __forceinline__ void mma_f4_run(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                            uint32_t b_lo, uint32_t b_hi, uint32_t step_b, const uint32_t* t,
                                            uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb) {
     static_assert(K == 1 || K == 4 || K == 5 || K == 9, "run lengths in use");
-    if constexpr (K == 9)
-        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
-                     TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") TCBNN_F4_MMA("%16", "pt")
-                     TCBNN_F4_MMA("%17", "pt") TCBNN_F4_MMA("%18", "pt") TCBNN_F4_MMA("%19", "pt") "}"
-                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]),
-                       "r"(t[7]), "r"(t[8]) : "memory");
-    else if constexpr (K == 5)
-        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
-                     TCBNN_F4_MMA("%14", "pt") TCBNN_F4_MMA("%15", "pt") "}"
-                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]) : "memory");
-    else if constexpr (K == 4)
-        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") TCBNN_F4_MMA("%12", "pt") TCBNN_F4_MMA("%13", "pt")
-                     TCBNN_F4_MMA("%14", "pt") "}"
-                     ::TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
-    else
-        asm volatile("{\n\t" TCBNN_F4_HEAD TCBNN_F4_MMA("%11", "pq") "}" ::TCBNN_F4_IN, "r"(t[0]) : "memory");
+    if constexpr (PAIR) { TCBNN_F4_RUN("2"); } else { TCBNN_F4_RUN("1"); }
 }
+#undef TCBNN_F4_RUN
 #undef TCBNN_F4_MMA
 #undef TCBNN_F4_HEAD
 #undef TCBNN_F4_IN
-#define TCBNN_F4_MMA(AOFF, PRED)                                                                     \
+#define TCBNN_F4_MMA(G, AOFF, PRED)                                                                  \
     "add.u32 xa, %2, " AOFF ";\n\tmov.b64 da, {xa, %3};\n\tmov.b64 db, {xb, %5};\n\t"                \
-    "@pl tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%6], da, db, %7, [%9], [%10], " PRED ";\n\t" \
+    "@pl tcgen05.mma.cta_group::" G ".kind::mxf4.block_scale.block32 [%6], da, db, %7, [%9], [%10], " PRED ";\n\t" \
     "add.u32 xb, xb, %11;\n\t"
-#define TCBNN_F4_HEAD                                                                                \
-    "{\n\t.reg .pred p0, p1, pq, pt, pl, pc;\n\t.reg .b64 da, db;\n\t.reg .b32 xa, xb, r1;\n\t"       \
-    "mbarrier.test_wait.parity.shared::cta.b64 p0, [%12], %13;\n\t"                                 \
-    "mbarrier.test_wait.parity.shared::cta.b64 p1, [%14], %15;\n\t"                                 \
+#define TCBNN_F4_HEAD(Q)                                                                             \
+    "{\n\t.reg .b16 both;\n\tmov.b16 both, 3;\n\t.reg .pred p0, p1, pq, pt, pl, pc;\n\t.reg .b64 da, db;\n\t.reg .b32 xa, xb, r1;\n\t"       \
+    "mbarrier.test_wait.parity" Q ".shared::cta.b64 p0, [%12], %13;\n\t"                            \
+    "mbarrier.test_wait.parity" Q ".shared::cta.b64 p1, [%14], %15;\n\t"                            \
     "setp.ne.b32 pl, %1, 0;\n\tsetp.ne.b32 pq, %8, 0;\n\tsetp.eq.b32 pt, %1, %1;\n\tmov.u32 xb, %4;\n\t" \
     "setp.ne.and.b32 pc, %17, 0, pl;\n\t"
-#define TCBNN_F4_TAIL                                                                                \
-    "@pl tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%16];\n\t"           \
-    "@pc tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%17];\n\t"           \
+#define TCBNN_F4_TAIL(G, W, M)                                                                       \
+    "@pl tcgen05.commit.cta_group::" G ".mbarrier::arrive::one.shared::cluster" W ".b64 [%16]" M ";\n\t" \
+    "@pc tcgen05.commit.cta_group::" G ".mbarrier::arrive::one.shared::cluster" W ".b64 [%17]" M ";\n\t" \
     "selp.u32 %0, 1, 0, p0;\n\tselp.u32 r1, 2, 0, p1;\n\tor.b32 %0, %0, r1;\n\t}"
 #define TCBNN_F4_IN                                                                                  \
     "r"(leader), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(d_tmem), "r"(idesc), "r"(acc), "r"(sfa), \
         "r"(sfb), "r"(step_b), "r"(bar0), "r"(par0), "r"(bar1), "r"(par1), "r"(bar_e), "r"(bar_c)
-template <int K>
+#define TCBNN_F4_END(G, Q, W, M)                                                                     \
+    if constexpr (K == 4)                                                                            \
+        asm volatile(TCBNN_F4_HEAD(Q) TCBNN_F4_MMA(G, "%18", "pq") TCBNN_F4_MMA(G, "%19", "pt") TCBNN_F4_MMA(G, "%20", "pt") \
+                     TCBNN_F4_MMA(G, "%21", "pt") TCBNN_F4_TAIL(G, W, M)                             \
+                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory"); \
+    else if constexpr (K == 3)                                                                       \
+        asm volatile(TCBNN_F4_HEAD(Q) TCBNN_F4_MMA(G, "%18", "pq") TCBNN_F4_MMA(G, "%19", "pt") TCBNN_F4_MMA(G, "%20", "pt") TCBNN_F4_TAIL(G, W, M) \
+                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]) : "memory");         \
+    else                                                                                             \
+        asm volatile(TCBNN_F4_HEAD(Q) TCBNN_F4_MMA(G, "%18", "pq") TCBNN_F4_TAIL(G, W, M)            \
+                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]) : "memory")
+// (PAIR: the MMAs of a pair of CTAs, barriers of cluster scope, the commits arrive in both)
+template <int K, bool PAIR = false>
 __device__ __forceinline__ uint32_t mma_f4_end(uint32_t leader, uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi,
                                                uint32_t b_lo, uint32_t b_hi, uint32_t step_b, const uint32_t* t,
                                                uint32_t idesc, uint32_t acc, uint32_t sfa, uint32_t sfb,
@@ -316,18 +331,10 @@ __device__ __forceinline__ uint32_t mma_f4_end(uint32_t leader, uint32_t d_tmem,
                                                uint32_t bar_e, uint32_t bar_c) {
     static_assert(K == 1 || K == 3 || K == 4, "run lengths in use");
     uint32_t ok;
-    if constexpr (K == 4)
-        asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_MMA("%19", "pt") TCBNN_F4_MMA("%20", "pt")
-                     TCBNN_F4_MMA("%21", "pt") TCBNN_F4_TAIL
-                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]) : "memory");
-    else if constexpr (K == 3)
-        asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_MMA("%19", "pt") TCBNN_F4_MMA("%20", "pt") TCBNN_F4_TAIL
-                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]), "r"(t[1]), "r"(t[2]) : "memory");
-    else
-        asm volatile(TCBNN_F4_HEAD TCBNN_F4_MMA("%18", "pq") TCBNN_F4_TAIL
-                     : "=&r"(ok) : TCBNN_F4_IN, "r"(t[0]) : "memory");
+    if constexpr (PAIR) { TCBNN_F4_END("2", ".acquire.cluster", ".multicast::cluster", ", both"); } else { TCBNN_F4_END("1", "", "", ""); }
     return ok;
 }
+#undef TCBNN_F4_END
 #undef TCBNN_F4_MMA
 #undef TCBNN_F4_HEAD
 #undef TCBNN_F4_TAIL

@@ -21,6 +21,8 @@
 // (or 8 or 4 epilogue warps, see EPIW).  The planes come from the caller (tcbnn_conv_workspace_bytes).
 #pragma once
 #include "bconv_umma_as.cuh"
+#include <cuda.h>
+#include <type_traits>
 
 namespace tcbnn {
 namespace umma {
@@ -36,8 +38,71 @@ namespace umma {
 // 64 (two groups; the CTA allocates half of tensor memory and two CTAs share an SM -- twice the independent
 // loader / issuer / epilogue pipelines, so that one CTA's barrier round trips and epilogue
 // latency are covered by the other's work).
+//
+// PAIR, the fourth: a pair of CTAs shares an n-tile of 128 whose filter block neither could hold (more than 256 input
+// channels) -- each holds half of its rows and the patch of its own tile; the leader issues MMAs of 256 x 128 x 64 that
+// read both shared memories (cta_group::2), and each finishes its own 128 rows.
 __host__ __device__ constexpr int pre_threads(int epiw) { return epiw * 32 + 64; }
 constexpr int kPreMaxStages = 8;           // patch ring depth is chosen by the host from the shared memory left
+
+// ---- a pair of CTAs on one tile (cta_group::2) ----------------------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t leader_address(uint32_t shared) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(shared));
+    return r;
+}
+// The accumulator goes back to the leader's MMAs: tensor memory is ordered by the tcgen05 fences around
+// the arrival and the wait, for which the arrival itself can be relaxed.
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_address(bar)) : "memory");
+}
+__device__ __forceinline__ bool mbar_test_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// WsWait with the bound in clocks, about a second, as a CTA waits for its partner too.  Polls rather than
+// suspends (360 clocks per k-block with try_wait).
+struct PairWait {
+    volatile int* abort;
+    int* err;
+    __device__ __forceinline__ bool poll(uint32_t bar, uint32_t parity, bool sleep) const {
+        if (mbar_test_cluster(bar, parity)) return true;
+        const long long t0 = clock64();
+        for (int i = 0; i < (1 << 28); i++) {
+            if (mbar_test_cluster(bar, parity)) return true;
+            if (sleep) __nanosleep(64);
+            if ((i & 63) == 63 && (*abort || clock64() - t0 > (1LL << 31))) break;
+        }
+        *abort = 1;
+        atomicExch(err, 1);
+        return false;
+    }
+    __device__ __forceinline__ bool operator()(uint32_t bar, uint32_t parity) const { return poll(bar, parity, false); }
+    __device__ __forceinline__ bool spin(uint32_t bar, uint32_t parity) const { return poll(bar, parity, false); }
+    __device__ __forceinline__ bool relaxed(uint32_t bar, uint32_t parity) const { return poll(bar, parity, true); }
+    __device__ __forceinline__ bool timed(uint32_t bar, uint32_t parity, long long& acc) const {
+        const long long t0 = clock64();
+        const bool ok = poll(bar, parity, false);
+        acc += clock64() - t0;
+        return ok;
+    }
+    __device__ __forceinline__ bool relaxed_timed(uint32_t bar, uint32_t parity, uint32_t& acc) const {
+        const uint32_t t0 = (uint32_t)clock64();
+        const bool ok = poll(bar, parity, true);
+        acc += (uint32_t)clock64() - t0;
+        return ok;
+    }
+};
+// A run of a plane, in elements of 8 bytes, to the calling CTA, completing on the leader's barrier.
+__device__ __forceinline__ void tensor_g2s_pair_1d(uint32_t dst, const CUtensorMap* map, int at, uint32_t leader_bar) {
+    asm volatile("cp.async.bulk.tensor.1d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2}], [%3];"
+                 ::"r"(dst), "l"(map), "r"(at), "r"(leader_bar) : "memory");
+}
 
 // positions of zero padding in front of the planes (a tile's patch starts up to back_y*PW+back_x
 // positions before its first output position) and the rounded-up plane length
@@ -48,8 +113,9 @@ __host__ __device__ inline long long pre_plane_positions(long long NV, int npos,
     return ((front + ((NV + 127) / 128) * 128 + npos + 7) & ~7LL);
 }
 // nplane: 1 for stride 1, 4 for stride 2 (the input's four row / column parity planes)
-__host__ __device__ inline size_t pre_smem_bytes(int npos, int C, int RS, int nt, int stages, int nplane) {
-    return (size_t)stages * nplane * 2 * npos * 16 + (size_t)RS * C * nt / 2 + nt * 8 + RS * 8 + 44 * 8 + 64;
+// rows: of the filter block that the CTA holds (half the n-tile in a pair)
+__host__ __device__ inline size_t pre_smem_bytes(int npos, int C, int RS, int nt, int stages, int nplane, int rows = 0) {
+    return (size_t)stages * nplane * 2 * npos * 16 + (size_t)RS * C * (rows ? rows : nt) / 2 + nt * 8 + RS * 8 + 44 * 8 + 64;
 }
 // kEpiTileRes: one buffer per epilogue group for the injected residual of its next tile, [chunk][128
 // pixels][16 B]
@@ -128,8 +194,9 @@ __device__ __forceinline__ void expand_raster(const ConvWsArgs& a, uint4* planes
 //                 requested before the one in front is computed.  Measured on 56 x 56 x 128 -> 128, batch
 //                 256, int32 result saved (411 MB): 251 us with a thread per pixel.
 constexpr int kEpiTile = 0, kEpiTileRes = 1, kEpiRows2 = 2, kEpiRows4 = 3, kEpiTilePool = 4;
-template <int NT, int EPI, int EPIW>
-__device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
+template <int NT, int EPI, int EPIW, bool PAIR = false>
+__device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem, const CUtensorMap* map_head = nullptr,
+                                  const CUtensorMap* map_tail = nullptr) {
     constexpr int kEpiThreads = EPIW * 32, kThreadsCta = pre_threads(EPIW);
     constexpr bool ROWS = EPI == kEpiRows2 || EPI == kEpiRows4;
     constexpr int CPT = NT < 64 ? NT : 64;            // columns of a tile per thread
@@ -137,6 +204,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     constexpr int NG = EPIW / WPG;                    // groups, each on a tile of its own
     constexpr bool SINGLE = NG == 1;
     static_assert(EPIW == 16 || (EPIW == 8 && NT == 64) || (SINGLE && !ROWS), "forms in use");
+    static_assert(!PAIR || (EPIW == 16 && NT == 128), "forms in use");
+    constexpr int NB = PAIR ? NT / 2 : NT;             // filter rows (output channels) that this CTA holds
     // Tensor memory: accumulators (7 at NT = 64) below column 480, the unit block scales of the
     // 4-bit MMA above it; the patch ring is as deep as shared memory allows, so that no role waits
     // on another's latency.
@@ -156,7 +225,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
 
     unsigned char* sAraw = smem;
     uint4* sB = reinterpret_cast<uint4*>(smem + (size_t)NSTAGE * stage_bytes);
-    int* sThr = reinterpret_cast<int*>(sB + (size_t)RS * (a.C >> 5) * NT);
+    int* sThr = reinterpret_cast<int*>(sB + (size_t)RS * (a.C >> 5) * NB);
     float* sThrF = reinterpret_cast<float*>(sThr + NT);       // the thresholds as given (fp32)
     uint32_t* sTapK = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(sThrF + NT) + 7) & ~(uintptr_t)7);
     uint64_t* sBar = reinterpret_cast<uint64_t*>(sTapK + 2 * RS);
@@ -167,6 +236,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     const uint32_t BAR_DRAIN = bar0 + 8u * 32;         // MMAs still in flight when the issuer gives up
     volatile int* sP0 = reinterpret_cast<volatile int*>(sTmem + 2);      // first pixel in each group's residual buffer
     const uint32_t BAR_FILTER = bar0 + 8u * 41;        // the filter block has landed
+    const uint32_t BAR_BOTH = bar0 + 8u * 42;          // (pair) ... the second CTA's, too
     unsigned char* sRes = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(sTmem + 6) + 127) & ~(uintptr_t)127);
     auto BAR_AFULL = [&](int s) { return bar0 + 8u * s; };
     auto BAR_AEMPTY = [&](int s) { return bar0 + 8u * (8 + s); };
@@ -177,7 +247,11 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     // share of the grid; where only the first n-tiles carry the epilogue's expensive part (a pooled
     // residual injected into the first channels) the host gives those more CTAs each.
     int nt, mfirst, mstep;
-    if (a.nt_heavy > 0) {
+    const int rank = PAIR ? (int)(blockIdx.x & 1u) : 0;
+    if constexpr (PAIR) {
+        const int pair = (int)(blockIdx.x >> 1);
+        nt = pair % a.ntiles_n; mfirst = 2 * (pair / a.ntiles_n) + rank; mstep = 2 * ((int)(gridDim.x >> 1) / a.ntiles_n);
+    } else if (a.nt_heavy > 0) {
         const int nh = a.nt_heavy * a.per_heavy;
         if ((int)blockIdx.x < nh) {
             nt = blockIdx.x % a.nt_heavy; mfirst = blockIdx.x / a.nt_heavy; mstep = a.per_heavy;
@@ -190,20 +264,31 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     }
     const int NV = (int)a.NV;
     const int mtiles = (NV + 127) / 128;
+    // (a pair goes on while its first CTA has a tile: the second one's last may lie behind the batch, sums that
+    // nobody stores)
+    const int mend = PAIR ? ((mtiles + 1) & ~1) : mtiles;
     const int obase = nt * NT;
 
     // Launched as a programmatic dependent: everything up to griddepcontrol.wait may run while the
     // launch in front is still running, so it touches nothing but this CTA's own memory and a settled filter.
     if (tid == 0) {
         for (int s = 0; s < 8; s++) { mbar_init(BAR_AFULL(s), 1); mbar_init(BAR_AEMPTY(s), 1); }
-        for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), WPG); }
+        for (int b = 0; b < 8; b++) { mbar_init(BAR_CFULL(b), 1); mbar_init(BAR_CEMPTY(b), PAIR ? 2 * WPG : WPG); }
         mbar_init(BAR_DRAIN, 1);
         mbar_init(BAR_FILTER, 1);
+        if constexpr (PAIR) mbar_init(BAR_BOTH, 1);
         for (int g = 0; g < NG; g++) { mbar_init(bar0 + 8u * (33 + g), WPG); mbar_init(bar0 + 8u * (37 + g), WPG); }
         *sAbort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == MMA_WARP) tmem_alloc(smem_u32(sTmem), TM_COLS);
+    if (warp == MMA_WARP) {
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(sTmem)), "r"(TM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            tmem_alloc(smem_u32(sTmem), TM_COLS);
+        }
+    }
     for (int t = tid; t < RS; t += kThreadsCta) {
         // offset of the tap's operand inside a stage, in 16-byte units
         const int r = t / a.S, sx = t % a.S;
@@ -227,18 +312,19 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     if (warp < 4) tmem_fill_unit_scales(tmem, SF_COL);
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_sync();                // the partner's barriers and scales are set up as well
     tc_fence_after();
     constexpr int kIssueLanes = 8;
     if (warp == LOAD_WARP) {
         // The filter block, in eight pieces (a multiple of 16 bytes each).  Where the caller's filter is
         // settled (ConvWsArgs::filter_settled) before the wait, under the launch in front.
         if (!a.filter_settled) asm volatile("griddepcontrol.wait;" ::: "memory");
-        const uint32_t nB = (uint32_t)(RS * (a.C >> 5) * NT), part = (nB + kIssueLanes - 1) / kIssueLanes;
+        const uint32_t nB = (uint32_t)(RS * (a.C >> 5) * NB), part = (nB + kIssueLanes - 1) / kIssueLanes;
         if (lane == 0) mbar_expect_tx(BAR_FILTER, nB * 16u);
         __syncwarp();
         const uint32_t first = (uint32_t)lane * part;
         if (lane < kIssueLanes && first < nB)
-            bulk_g2s(smem_u32(sB + first), a.wf4 + (size_t)nt * nB + first, min(part, nB - first) * 16u, BAR_FILTER);
+            bulk_g2s(smem_u32(sB + first), a.wf4 + (size_t)(PAIR ? 2 * nt + rank : nt) * nB + first, min(part, nB - first) * 16u, BAR_FILTER);
     }
     // Rehearsal (single-group CTAs): the epilogue runs its loop once without effect (nothing read from or
     // written to global memory, no barrier touched) before it waits for the launch in front.  Its code
@@ -267,7 +353,9 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         }
         asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
     };
-    const WsWait wait{sAbort, a.err_flag};
+    // an epilogue warp is done with accumulator b
+    auto release = [&](int b) { if constexpr (PAIR) mbar_arrive_leader(BAR_CEMPTY(b)); else mbar_arrive(BAR_CEMPTY(b)); };
+    const typename std::conditional<PAIR, PairWait, WsWait>::type wait{sAbort, a.err_flag};
 
     if (warp == LOAD_WARP) {
         // =============================== patch loader =======================================
@@ -282,7 +370,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             uint32_t it = 0, sph = 0;
             int s = 0;
             bool ok = true;
-            for (int m = mfirst; m < mtiles && ok; m += mstep) {
+            for (int m = mfirst; m - rank < mend && ok; m += mstep) {
                 const long long slot0 = (long long)m * 128 - back + a.pre_front;
                 for (int cb = 0; cb < NCB; cb += CBS, it++) {
                     // the ring is several tiles deep: lane 0 mostly waits for a slot, and sleeps
@@ -290,9 +378,26 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (lane == 0) ok = wait.relaxed(BAR_AEMPTY(s), sph ^ 1);
                     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                     if (!ok) break;
+                    const uint32_t dst = smem_u32(sAraw + (size_t)s * stage_bytes);
+                    if constexpr (PAIR) {
+                        // Both CTAs' copies complete on the leader's barrier, which only a tensor copy of a pair may do:
+                        // a plane's run as up to 128 positions and what is left.
+                        if (lane == 0 && rank == 0) mbar_expect_tx(BAR_AFULL(s), m + 1 < mtiles ? 2 * stage_bytes : stage_bytes);
+                        __syncwarp();
+                        if (m < mtiles && lane < kIssueLanes) {
+                            for (int i = lane; i < 2 * ncopy; i += kIssueLanes) {
+                                const int tail = i & 1, c = (i >> 1) & 1, sub = i >> 2;
+                                const long long at = (long long)((cb + sub) * 2 + c) * a.pre_positions + slot0 + 128 * tail;
+                                tensor_g2s_pair_1d(dst + (uint32_t)sub * block_bytes + (uint32_t)c * (uint32_t)a.NPOS * 16u + 2048u * tail,
+                                                   tail ? map_tail : map_head, (int)(2 * at), leader_address(BAR_AFULL(s)));
+                            }
+                        }
+                        __syncwarp();
+                        if (++s == NSTAGE) { s = 0; sph ^= 1; }
+                        continue;
+                    }
                     if (lane == 0) mbar_expect_tx(BAR_AFULL(s), stage_bytes);
                     __syncwarp();
-                    const uint32_t dst = smem_u32(sAraw + (size_t)s * stage_bytes);
                     if (lane < kIssueLanes) {
                         for (int i = lane; i < ncopy; i += kIssueLanes) {
                             const int c = i & 1, pl = (i >> 1) % NPLANE, sub = (i >> 1) / NPLANE;
@@ -304,7 +409,11 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (++s == NSTAGE) { s = 0; sph ^= 1; }
                 }
             }
-            if (!ok && lane == 0) {
+            if (PAIR && !ok && lane == 0) {
+                // giving up: the time of any copy passes (the second CTA's complete on the leader's barrier)
+                for (int i = 0; i < (1 << 17); i++) __nanosleep(20);
+            }
+            if (!PAIR && !ok && lane == 0) {
                 for (int i = 0; i < (1 << 20); i++)
                     if (mbar_try_wait(BAR_FILTER, 0)) break;
                 // giving up: wait (bounded) for the copies still in flight before the CTA exits;
@@ -318,6 +427,12 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             }
         }
         __syncwarp();
+    } else if (PAIR && warp > LOAD_WARP && rank == 1) {
+        // (the leader issues for both; it must know that this CTA's half of the filter is there)
+        const bool landed = wait(BAR_FILTER, 0);
+        if (landed && lane == 0)
+            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_address(BAR_BOTH)) : "memory");
+        __syncwarp();
     } else if (warp > LOAD_WARP) {
         // =============================== MMA issuer =========================================
         // The whole warp runs the control flow converged and polls the barriers, and one elected
@@ -325,14 +440,14 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         // idles, and a lone lane in a diverged warp pays far more per branch and per wait.
         {
             const bool leader = elect_one();
-            const uint32_t lboA = (uint32_t)a.NPOS * 16u, lboB = NT * 16u;
+            const uint32_t lboA = (uint32_t)a.NPOS * 16u, lboB = NB * 16u;
             const uint64_t descA0 = smem_desc(smem_u32(sAraw), lboA, 128u);
             const uint64_t descB0 = smem_desc(smem_u32(sB), lboB, 128u);
             const uint32_t aHi = (uint32_t)(descA0 >> 32), bHi = (uint32_t)(descB0 >> 32);
             const uint32_t aLo0 = (uint32_t)descA0, bLo0 = (uint32_t)descB0;
             const uint32_t stepB = (2u * lboB) >> 4, stepStage = stage_bytes >> 4;   // one tap = two chunks of B
             const uint32_t stepBlock = block_bytes >> 4;
-            constexpr uint32_t IDESC = idesc_f4(NT);
+            constexpr uint32_t IDESC = idesc_f4(NT) + (PAIR ? (128u >> 4) << 24 : 0u);       // (a pair: M = 256)
             const uint32_t sfa = tmem + SF_COL, sfb = tmem + SF_COL + 16;
             uint32_t tapk[9];                              // 3x3 filters: the tap offsets in registers
 #pragma unroll
@@ -346,7 +461,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             // pipe busy: between the last MMA of a stage and the first of the next only a branch on
             // the outcome of tests made earlier is left.
             const uint32_t spt = (uint32_t)(NCB / CBS);    // stages per tile
-            const uint32_t nit = mfirst < mtiles ? (uint32_t)((mtiles - mfirst + mstep - 1) / mstep) * spt : 0u;
+            const uint32_t nit = mfirst < mend ? (uint32_t)((mend - mfirst + mstep - 1) / mstep) * spt : 0u;
             uint32_t s = 0, b = 0, sph = 0, bph = 0, left = spt;      // left: stages of this tile still to issue
             uint32_t acc = 0, bLo = bLo0, d = tmem, aLo = aLo0;
             // ready: bit 0 = this stage is known to be full, bit 1 = this tile's accumulator to be free,
@@ -354,6 +469,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             uint32_t ready = 0, need = 3u;
             const uint32_t tap_end = sTapK[RS - 1];
             ok = wait(BAR_FILTER, 0);
+            if (PAIR && ok) ok = wait(BAR_BOTH, 0);
             for (uint32_t it = 0; it < nit && ok; it++) {
                 if ((ready & need) != need) {
                     if ((need & 2u) && !(ready & 2u)) {
@@ -366,14 +482,14 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     }
                 }
                 tc_fence_after();
-                if (RS == 9) {
+                if (PAIR || RS == 9) {
                     for (int sub = 0; sub + 1 < CBS; sub++) {
-                        mma_f4_run<9>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk, IDESC, acc, sfa, sfb);
+                        mma_f4_run<9, PAIR>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk, IDESC, acc, sfa, sfb);
                         bLo += 9 * stepB;
                         aLo += stepBlock;
                         acc = 1;
                     }
-                    mma_f4_run<5>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk, IDESC, acc, sfa, sfb);
+                    mma_f4_run<5, PAIR>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk, IDESC, acc, sfa, sfb);
                     bLo += 5 * stepB;
                 } else {
                     // other filters: taps in runs of five while they last, then one by one; the last is left
@@ -421,8 +537,8 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                 acc = last ? 0u : 1u;
                 asm volatile("" : "+r"(bar_a), "+r"(bar_b), "+r"(par_b), "+r"(bar_e), "+r"(bar_c), "+r"(aLon), "+r"(dn),
                                   "+r"(bLon), "+r"(need), "+r"(b), "+r"(bph), "+r"(left), "+r"(s), "+r"(sph), "+r"(acc));
-                if (RS == 9) {
-                    ready = mma_f4_end<4>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk + 5, IDESC, acc_end, sfa, sfb,
+                if (PAIR || RS == 9) {
+                    ready = mma_f4_end<4, PAIR>(leader, d, aLo, aHi, bLo, bHi, stepB, tapk + 5, IDESC, acc_end, sfa, sfb,
                                           bar_a, sphn, bar_b, par_b, bar_e, bar_c);
                 } else {
                     ready = mma_f4_end<1>(leader, d, aLo, aHi, bLo, bHi, stepB, &tap_end, IDESC, acc_end, sfa, sfb,
@@ -434,7 +550,10 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             }
             if (!ok && leader) {
                 // giving up: the MMAs already issued must have finished before tensor memory is freed
-                mma_commit(BAR_DRAIN);
+                if constexpr (PAIR)
+                    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(BAR_DRAIN) : "memory");
+                else
+                    mma_commit(BAR_DRAIN);
                 for (int i = 0; i < (1 << 20); i++)
                     if (mbar_try_wait(BAR_DRAIN, 0)) break;
             }
@@ -498,7 +617,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
             if (ring && mfirst + grp * mstep < mtiles) request(mfirst + grp * mstep);
         }
 #pragma unroll 1
-        for (int m = mfirst + grp * mstep; (m < mtiles || dry) && ok; m += NG * mstep, b += NG) {
+        for (int m = mfirst + grp * mstep; (m - rank < mend || dry) && ok; m += NG * mstep, b += NG) {
             if (b >= NACC) { b -= NACC; bph ^= 1u; }
             // raster position -> output pixel
             const int p = m * 128 + row;
@@ -562,7 +681,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (k == PASSES - 1) {
                         tc_fence_before();                 // this warp is done with the accumulator
                         __syncwarp();
-                        if (lane == 0 && !dry) mbar_arrive(BAR_CEMPTY(b));
+                        if (lane == 0 && !dry) release(b);
                     }
                     // the reference's comparison as it stands, !((float)value < threshold)
                     // (kernel.cuh:795-796), on the fp32 accumulator
@@ -651,7 +770,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                     if (k == PASSES - 1) {
                         tc_fence_before();                 // this warp is done with the accumulator
                         __syncwarp();
-                        if (lane == 0 && !dry) mbar_arrive(BAR_CEMPTY(b));
+                        if (lane == 0 && !dry) release(b);
                     } else {
                         tmem_ld16(taddr + HSTEP * 32, v0);
                     }
@@ -706,7 +825,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
         int b = grp;
         uint32_t bph = 0;
         epilogue_start();
-        for (int m = mfirst + grp * mstep; m < mtiles && ok; m += NG * mstep, b += NG) {
+        for (int m = mfirst + grp * mstep; m - rank < mend && ok; m += NG * mstep, b += NG) {
             if (b >= NACC) { b -= NACC; bph ^= 1u; }
             const int p = m * 128 + row;
             bool live = false;
@@ -786,7 +905,7 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
                 if (u == NU - 1) {
                     tc_fence_before();                     // this warp is done with the accumulator
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(BAR_CEMPTY(b));
+                    if (lane == 0) release(b);
                 }
                 // values of row i of this unit, channel run g: four consecutive channels
                 int4 c[2][2];
@@ -878,7 +997,12 @@ __device__ void conv_umma_pre_cta(const ConvWsArgs& a, unsigned char* smem) {
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == MMA_WARP) tmem_dealloc(tmem, TM_COLS);
+    if constexpr (PAIR) {
+        cluster_sync();                                 // nothing of the partner's reaches into this CTA any more
+        if (warp == MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS) : "memory");
+    } else if (warp == MMA_WARP) {
+        tmem_dealloc(tmem, TM_COLS);
+    }
 }
 
 }  // namespace umma

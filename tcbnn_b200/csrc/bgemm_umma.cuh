@@ -35,7 +35,6 @@
 // copies and one issuing warp per operand.
 #pragma once
 #include "bconv_umma_pre.cuh"
-#include <cuda.h>
 
 namespace tcbnn {
 namespace umma {
@@ -152,58 +151,12 @@ __device__ __forceinline__ void expand_pass_weights(const PassWeights& p, int bl
 // which only a tensor copy of a pair may do (cta_group::2; no multicast): a thread of the second CTA that passed its
 // CTA's completion on would have to do so with an arrival of cluster scope, 1400 clocks each, one at a
 // time (8192 x 8192 x 8192 with threshold bits 174 us, 219 with three warps taking turns at it).
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t leader_address(uint32_t shared) {
-    uint32_t r;
-    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(shared));
-    return r;
-}
-// The accumulator goes back to the leader's MMAs: tensor memory is ordered by the tcgen05 fences around
-// the arrival and the wait, for which the arrival itself can be relaxed.
-__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
-    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_address(bar)) : "memory");
-}
 // One stage of an operand, kGemmKU units: rows of 1 KB of the expanded operand from `row` on.  (A stage
 // that holds fewer k-blocks is followed by others' units or, behind the last, by zeros, which no MMA reads.)
 __device__ __forceinline__ void tensor_g2s_pair(uint32_t dst, const CUtensorMap* map, int row, uint32_t leader_bar) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(0), "r"(row), "r"(leader_bar) : "memory");
 }
-__device__ __forceinline__ bool mbar_test_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// WsWait with the bound in clocks, about a second, as a CTA waits for its partner too.  Polls rather than
-// suspends (360 clocks per k-block with try_wait).
-struct GemmPairWait {
-    volatile int* abort;
-    int* err;
-    __device__ __forceinline__ bool poll(uint32_t bar, uint32_t parity, bool sleep) const {
-        if (mbar_test_cluster(bar, parity)) return true;
-        const long long t0 = clock64();
-        for (int i = 0; i < (1 << 28); i++) {
-            if (mbar_test_cluster(bar, parity)) return true;
-            if (sleep) __nanosleep(64);
-            if ((i & 63) == 63 && (*abort || clock64() - t0 > (1LL << 31))) break;
-        }
-        *abort = 1;
-        atomicExch(err, 1);
-        return false;
-    }
-    __device__ __forceinline__ bool operator()(uint32_t bar, uint32_t parity) const { return poll(bar, parity, false); }
-    __device__ __forceinline__ bool spin(uint32_t bar, uint32_t parity) const { return poll(bar, parity, false); }
-    __device__ __forceinline__ bool relaxed(uint32_t bar, uint32_t parity) const { return poll(bar, parity, true); }
-    __device__ __forceinline__ bool timed(uint32_t bar, uint32_t parity, long long& acc) const {
-        const long long t0 = clock64();
-        const bool ok = poll(bar, parity, false);
-        acc += clock64() - t0;
-        return ok;
-    }
-};
 // K MMAs of 256 x 256 x 64, A and W advancing by `step` alike; with END what mma_f4_end does (the commits
 // arrive in both CTAs).
 #define TCBNN_F4_PAIR_MMA(PRED)                                                                      \
@@ -314,7 +267,7 @@ __device__ __forceinline__ void gemm_umma_cta(const GemmUmmaArgs& g, const CUten
     __syncthreads();
     if constexpr (PAIR) cluster_sync();                 // the partner's barriers and scales are set up as well
     tc_fence_after();
-    const typename std::conditional<PAIR, GemmPairWait, WsWait>::type wait{sAbort, g.status};
+    const typename std::conditional<PAIR, PairWait, WsWait>::type wait{sAbort, g.status};
     // Launched as a programmatic dependent of the expansion pass, the CTA has come this far while
     // that pass was still running; its units are complete (and visible) once this returns.
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -244,23 +244,37 @@ k_gemm_umma_pair(umma::GemmUmmaArgs g, const __grid_constant__ CUtensorMap map_a
 }
 
 // Expanded operand of `units` units as rows of 1 KB, copied kGemmKU units at a time
-int unit_map(CUtensorMap* map, const void* base, long long units) {
-    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static const Encode encode = [] {
+using TensorEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+TensorEncode tensor_encode() {
+    static const TensorEncode encode = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult r;
         return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &r) == cudaSuccess && r == cudaDriverEntryPointSuccess
-                   ? (Encode)f : (Encode)nullptr;
+                   ? (TensorEncode)f : (TensorEncode)nullptr;
     }();
-    if (!encode) return fail("gemm (tcgen05): the driver has no cuTensorMapEncodeTiled");
-    const cuuint64_t dims[2] = {256, (cuuint64_t)units * (umma::kGemmUnit / 1024)}, strides[1] = {1024};
-    const cuuint32_t box[2] = {256, umma::kGemmKU * (umma::kGemmUnit / 1024)}, steps[2] = {1, 1};
-    const CUresult e = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, steps,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (e != CUDA_SUCCESS) return fail("gemm (tcgen05): tensor map of %lld units: error %d", units, (int)e);
+    return encode;
+}
+int encode_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+               const cuuint32_t* box) {
+    if (!tensor_encode()) return fail("tensor map: the driver has no cuTensorMapEncodeTiled");
+    const cuuint32_t steps[2] = {1, 1};
+    const CUresult e = tensor_encode()(map, type, rank, const_cast<void*>(base), dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (e != CUDA_SUCCESS) return fail("tensor map of %llu elements: error %d", (unsigned long long)dims[rank - 1], (int)e);
     return 0;
+}
+// expanded operands of the GEMM, in rows of 1 KB
+int unit_map(CUtensorMap* map, const void* base, long long units) {
+    const cuuint64_t dims[2] = {256, (cuuint64_t)units * (umma::kGemmUnit / 1024)}, strides[1] = {1024};
+    const cuuint32_t box[2] = {256, umma::kGemmKU * (umma::kGemmUnit / 1024)};
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, base, dims, strides, box);
+}
+// a convolution's input planes, runs of `box` elements of 8 bytes
+int run_map(CUtensorMap* map, const void* base, long long elements, int box) {
+    const cuuint64_t dims[1] = {(cuuint64_t)elements}, strides[1] = {0};
+    const cuuint32_t boxes[1] = {(cuuint32_t)box};
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 1, base, dims, strides, boxes);
 }
 
 struct GemmUmmaPlan {
@@ -331,6 +345,18 @@ int check_fc_weight(const tcbnn_fc_weight& w) {
 }
 long long fc_weight_tasks(const tcbnn_fc_weight& w) { return (long long)((w.N + 127) / 128) * (((w.K + 63) / 64 + 3) / 4); }
 
+// the device's status word of the tcgen05 GEMMs
+int gemm_status_address(int** out) {
+    static int* status_addr[64] = {nullptr};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(g_configure_mutex);
+    if (dev >= 0 && dev < 64 && status_addr[dev]) { *out = status_addr[dev]; return 0; }
+    CUDA_TRY(cudaGetSymbolAddress((void**)out, g_gemm_status));
+    if (dev >= 0 && dev < 64) status_addr[dev] = *out;
+    return 0;
+}
+
 int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, const GemmUnits& u, int sms, cudaStream_t st) {
     static bool configured[64] = {false};
     if (configure_once(configured, [] {
@@ -349,20 +375,7 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, con
     a.partial = p.splits > 1 ? (int32_t*)(w + p.off_partial) : nullptr;
     a.mode = g.mode; a.out = g.out; a.ldo = g.ldo; a.p0 = g.p0; a.p1 = g.p1;
     a.trace = g_conv_trace;
-    {
-        static int* status_addr[64] = {nullptr};
-        int dev = 0;
-        cudaGetDevice(&dev);
-        std::lock_guard<std::mutex> lock(g_configure_mutex);
-        if (dev < 0 || dev >= 64 || !status_addr[dev]) {
-            int* q = nullptr;
-            CUDA_TRY(cudaGetSymbolAddress((void**)&q, g_gemm_status));
-            if (dev >= 0 && dev < 64) status_addr[dev] = q;
-            a.status = q;
-        } else {
-            a.status = status_addr[dev];
-        }
-    }
+    if (gemm_status_address(&a.status)) return 1;
     {
         // a programmatic dependent of the expansion launch: set-up (barriers, tensor memory, unit
         // scales) overlaps the expansion pass, the kernel waits for it before its first copy
@@ -636,6 +649,7 @@ __global__ void __launch_bounds__(umma::pre_threads(EPIW), EPIW == 8 && NT == 64
     extern __shared__ __align__(128) unsigned char dyn_smem_pre[];
     umma::conv_umma_pre_cta<NT, EPI, EPIW>(a, dyn_smem_pre);
 }
+template <int V>
 __global__ void __launch_bounds__(256) k_expand_raster(umma::ConvWsArgs a, uint4* planes, long long positions,
                                                        long long front) {
     umma::expand_raster<V>(a, planes, positions, front);
@@ -750,14 +764,9 @@ int launch_conv_umma_pre_ring(umma::ConvWsArgs& a, int sms, cudaStream_t st, boo
 }
 
 template <int NT>
-int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st, bool expand) {
-    if (expand) {
-        const cudaError_t e = launch_expand_raster(a, const_cast<uint4*>(a.pre), a.pre_positions, a.pre_front, sms, st);
-        if (e != cudaSuccess) return fail("conv_layer (input expansion): %s", cudaGetErrorString(e));
-    }
+int launch_conv_umma_pre(umma::ConvWsArgs& a, size_t smem, int sms, cudaStream_t st) {
     const bool plain = !a.res_in && !a.res_out && !a.acc_out;
     const bool chunked = !a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked);
-template <int V>
     // A tile per CTA and none to spare: the form for latency (one image through ResNet-18: 135 -> 115 us)
     constexpr int kSingle = NT == 128 ? 8 : 4;
     if (g_conv_single && (plain || chunked) && (a.NV + 127) / 128 * (a.O / NT) <= sms)
@@ -775,6 +784,67 @@ template <int V>
     }
     if (a.res_in && a.res_in_bytes == 4) return launch_conv_umma_pre_epi<NT, umma::kEpiRows4>(a, smem, sms, st);
     return launch_conv_umma_pre_epi<NT, umma::kEpiRows2>(a, smem, sms, st);
+}
+
+// ---- loader-fed kernel on pairs of SMs ---------------------------------------------------------
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(umma::pre_threads(16), 1)
+k_conv_umma_pair(umma::ConvWsArgs a, const __grid_constant__ CUtensorMap map_head, const __grid_constant__ CUtensorMap map_tail) {
+    extern __shared__ __align__(128) unsigned char dyn_smem_pair[];
+    umma::conv_umma_pre_cta<128, EPI, 16, true>(a, dyn_smem_pair, &map_head, &map_tail);
+}
+
+template <int EPI>
+int launch_conv_umma_pair_epi(umma::ConvWsArgs& a, unsigned grid, size_t smem, const CUtensorMap& head, const CUtensorMap& tail, cudaStream_t st) {
+    static bool configured[64] = {false};
+    if (configure_once(configured, [] { return cudaFuncSetAttribute(k_conv_umma_pair<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); }))
+        return 1;
+    const cudaError_t e = launch_dependent(k_conv_umma_pair<EPI>, grid, umma::pre_threads(16), smem, st, a, head, tail);
+    if (e != cudaSuccess) return fail("conv_layer (tcgen05, pairs): %s", cudaGetErrorString(e));
+    return 0;
+}
+
+// 3x3 stride-1 layers whose filter block of 128 output channels does not fit beside a patch ring (more than 256
+// input channels) run 64 channels at a time, at 54 clocks per MMA where 32 are math: the operands' way out of
+// shared memory.  A pair of SMs shares a block of 128, half each, for 256 positions: 68 clocks per SM for twice the
+// work.  Taken where it has fewer clocks left, which leaves out launches of a tile or two per CTA: *use = the plan
+// applies.  7 x 7 x 512 at batch 1024 68.5 -> 43.9 us, with int16 residuals 73.1 -> 46.8; 8 x 8 x 512 pooled 85.9 -> 54.5;
+// 28 x 28 x 512 at batch 32 29.6 -> 21.5.  Not with a pooled int32 residual, where n-tiles get uneven shares of the GPU
+// (8 x 8 x 512 at batch 201: 31.4 us, 37.1 in pairs).
+int launch_conv_umma_pair(umma::ConvWsArgs& a, int sms, cudaStream_t st, bool* use) {
+    *use = false;
+    const long long mtiles = (a.NV + 127) / 128;
+    const int ntiles = a.O / 128, tail = 2 * a.NPOS - 256;                 // a plane's run: 256 elements of 8 bytes, and the rest
+    if ((a.res_in && a.residual_pool && a.res_in_bytes == 4) || a.O % 128 || a.R != 3 || a.S != 3 || a.stride != 1 || ntiles > sms / 2 || tail <= 0 || tail > 256) return 0;
+    const long long per = sms / 2 / ntiles, per64 = sms / (a.O / 64);
+    if (per64 < 1) return 0;
+    const double pairs = (double)(((mtiles + 1) / 2 + per - 1) / per) * 68.0, singles = (double)((mtiles + per64 - 1) / per64) * 54.0;
+    if (pairs >= singles) return 0;
+    const long long elements = a.pre_positions * (a.C / 32) * 2;
+    if (elements >= (1LL << 31)) return 0;
+    size_t smem = 0;
+    const int NCB = a.C / 64;
+    for (int cbs = 4; cbs >= 1 && !smem; cbs >>= 1) {
+        if (NCB % cbs) continue;
+        for (int stages = 6; stages >= 3 && !smem; stages--) {
+            const size_t need = umma::pre_smem_bytes(a.NPOS, a.C, 9, 128, stages, cbs, 64);
+            if (need <= 227 * 1024) { smem = need; a.pre_cbs = cbs; a.pre_stages = stages; }
+        }
+    }
+    if (!smem) return 0;
+    CUtensorMap head, rest;
+    if (run_map(&head, a.pre, elements, 256) || run_map(&rest, a.pre, elements, tail)) return 1;
+    *use = true;
+    a.ntiles_n = ntiles;
+    a.nt_heavy = 0; a.per_heavy = a.per_light = 0;
+    const long long want = (mtiles + 1) / 2;
+    const unsigned grid = (unsigned)((per < want ? per : want) * ntiles * 2);
+    const bool plain = !a.res_in && !a.res_out && !a.acc_out;
+    const bool chunked = !a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked);
+    if (plain) return launch_conv_umma_pair_epi<umma::kEpiTile>(a, grid, smem, head, rest, st);
+    if (chunked) return launch_conv_umma_pair_epi<umma::kEpiTilePool>(a, grid, smem, head, rest, st);
+    if (a.res_in && a.res_in_bytes == 4) return launch_conv_umma_pair_epi<umma::kEpiRows4>(a, grid, smem, head, rest, st);
+    return launch_conv_umma_pair_epi<umma::kEpiRows2>(a, grid, smem, head, rest, st);
 }
 
 // The *_bytes arguments of the conv entry points name the residual's element format: 4 = int32
@@ -855,6 +925,18 @@ __global__ void __launch_bounds__(256) k_pool_bits(const uint32_t* in, uint32_t*
             for (int i = 0; i < V; i++) at[(size_t)i * nx.nplane * nx.positions] = umma::expand32_f4(v[i]);
         }
     }
+}
+// (the pre-pool bits are 256-byte aligned scratch)
+cudaError_t launch_pool_bits(const uint32_t* prepool, uint32_t* out, const tcbnn_conv_desc* d, int Ow, long long out_image_stride,
+                             const NextPlanes& nx, int sms, cudaStream_t st) {
+    // as many words per thread as leaves every SM four blocks: fewer threads each with more to store are slower
+    // (14 x 14 x 512 at batch 32, pooled layer: 33.7 us a word at a time, 35.8 four; 32 x 32 x 128 at batch 1024:
+    // 63.3 and 58.2)
+    const long long words = (long long)d->B * d->OH * d->OW * Ow, enough = 4LL * sms * 256;
+    const int V = Ow % 4 == 0 && words >= 4 * enough ? 4 : Ow % 2 == 0 && words >= 2 * enough ? 2 : 1;
+    return launch_dependent(V == 4 ? k_pool_bits<4> : V == 2 ? k_pool_bits<2> : k_pool_bits<1>,
+                            (unsigned)elementwise_grid((long long)d->B * d->OH * d->OW * (Ow / V), sms), 256, 0, st, prepool, out, d->B, d->OH,
+                            d->OW, Ow, out_image_stride, nx);
 }
 
 __global__ void __launch_bounds__(umma::kAsThreads, 1) k_conv_umma_as(umma::ConvWsArgs a) {
@@ -978,18 +1060,6 @@ __global__ void __launch_bounds__(128) k_umma_peak_mxf4(int iters, long long* cy
     umma::tc_fence_before();
     __syncthreads();
     umma::tc_fence_after();
-// (the pre-pool bits are 256-byte aligned scratch)
-cudaError_t launch_pool_bits(const uint32_t* prepool, uint32_t* out, const tcbnn_conv_desc* d, int Ow, long long out_image_stride,
-                             const NextPlanes& nx, int sms, cudaStream_t st) {
-    // as many words per thread as leaves every SM four blocks: fewer threads each with more to store are slower
-    // (14 x 14 x 512 at batch 32, pooled layer: 33.7 us a word at a time, 35.8 four; 32 x 32 x 128 at batch 1024:
-    // 63.3 and 58.2)
-    const long long words = (long long)d->B * d->OH * d->OW * Ow, enough = 4LL * sms * 256;
-    const int V = Ow % 4 == 0 && words >= 4 * enough ? 4 : Ow % 2 == 0 && words >= 2 * enough ? 2 : 1;
-    return launch_dependent(V == 4 ? k_pool_bits<4> : V == 2 ? k_pool_bits<2> : k_pool_bits<1>,
-                            (unsigned)elementwise_grid((long long)d->B * d->OH * d->OW * (Ow / V), sms), 256, 0, st, prepool, out, d->B, d->OH,
-                            d->OW, Ow, out_image_stride, nx);
-}
     if (threadIdx.x == 0) {
         // K-major, no swizzle: a 16-byte row of a core matrix holds 32 elements; K = 64 is two core
         // matrices `lbo` apart
@@ -1379,6 +1449,12 @@ int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units
 int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N, int lda, int ldw, uint32_t* out,
                      int ldo, void* workspace, size_t workspace_bytes, const void* a_units, const void* w_units, void* next_units,
                      void* stream) {
+    return tcbnn_fc_layer_p(A, W, thr, M, K, N, lda, ldw, out, ldo, workspace, workspace_bytes, a_units, w_units, next_units, 0, stream);
+}
+
+int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N, int lda, int ldw, uint32_t* out,
+                     int ldo, void* workspace, size_t workspace_bytes, const void* a_units, const void* w_units, void* next_units,
+                     int settled, void* stream) {
     if (ldo * 32 < N) return fail("fc_layer: ldo too small");
     if (((uintptr_t)a_units | (uintptr_t)w_units | (uintptr_t)next_units) & 255) return fail("fc_layer: units must be 256-byte aligned");
     if (next_units && (ldo & 1)) return fail("fc_layer: next_units needs an even ldo");
@@ -1389,6 +1465,12 @@ int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int
 int tcbnn_out_layer(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,
                     int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
                     size_t workspace_bytes, void* stream) {
+    return tcbnn_out_layer_p(A, W, scale, bias, M, K, N, lda, ldw, out, ldo, workspace, workspace_bytes, 0, stream);
+}
+
+int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,
+                      int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
+                      size_t workspace_bytes, int settled, void* stream) {
     if (ldo < N) return fail("out_layer: ldo < N");
     GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_OUT_AFFINE, out, ldo, scale, bias, 1, nullptr, settled};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
@@ -1519,12 +1601,6 @@ static int conv_layer_impl(const tcbnn_conv_desc* d, const uint32_t* in, const v
                            long long out_image_stride, void* res_out, int res_out_bytes,
                            int32_t* acc_out, void* workspace, size_t workspace_bytes, int workspace_ready,
                            const NextPlanes* nx, bool* fed, void* stream) {
-    return tcbnn_fc_layer_p(A, W, thr, M, K, N, lda, ldw, out, ldo, workspace, workspace_bytes, a_units, w_units, next_units, 0, stream);
-}
-
-int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N, int lda, int ldw, uint32_t* out,
-                     int ldo, void* workspace, size_t workspace_bytes, const void* a_units, const void* w_units, void* next_units,
-                     int settled, void* stream) {
     *fed = false;
     if (conv_check(d, true)) return 1;
     const int Ow = (d->O + 31) / 32;
@@ -1535,12 +1611,6 @@ int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int
     if (res_in && !residual_format(res_in_bytes, &res_in_bytes, &res_in_chunked))
         return fail("conv_layer: res_in_bytes must be 2, 4 or TCBNN_RES_INT16_CHUNKED");
     if (res_out && !residual_format(res_out_bytes, &res_out_bytes, &res_out_chunked, &res_out_proven))
-    return tcbnn_out_layer_p(A, W, scale, bias, M, K, N, lda, ldw, out, ldo, workspace, workspace_bytes, 0, stream);
-}
-
-int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,
-                      int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
-                      size_t workspace_bytes, int settled, void* stream) {
         return fail("conv_layer: res_out_bytes must be 2, 4 or TCBNN_RES_INT16_CHUNKED");
     if (!res_in) res_in_chunked = 0;
     if (!res_out) res_out_chunked = 0;
@@ -1653,9 +1723,19 @@ int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, 
                     if (need <= 227 * 1024) { a.pre_cbs = 2; a.pre_stages = 2; pre_smem = need; }
                 }
             }
-            if (L.pre_nt == 32) return launch_conv_umma_pre<32>(a, pre_smem, sms, st, !workspace_ready);
-            if (L.pre_nt == 64) return launch_conv_umma_pre<64>(a, pre_smem, sms, st, !workspace_ready);
-            if (L.pre_nt == 128) return launch_conv_umma_pre<128>(a, pre_smem, sms, st, !workspace_ready);
+            if (!workspace_ready) {
+                const cudaError_t e = launch_expand_raster(a, (uint4*)workspace, a.pre_positions, a.pre_front, sms, st);
+                if (e != cudaSuccess) return fail("conv_layer (input expansion): %s", cudaGetErrorString(e));
+            }
+            if (L.pre_nt == 64) {
+                bool pairs;
+                umma::ConvWsArgs b = a;
+                if (launch_conv_umma_pair(b, sms, st, &pairs)) return 1;
+                if (pairs) return 0;
+            }
+            if (L.pre_nt == 32) return launch_conv_umma_pre<32>(a, pre_smem, sms, st);
+            if (L.pre_nt == 64) return launch_conv_umma_pre<64>(a, pre_smem, sms, st);
+            if (L.pre_nt == 128) return launch_conv_umma_pre<128>(a, pre_smem, sms, st);
         }
 #define TCBNN_WS_CASE(NN, SS) \
         if (L.umma_nt == NN && d->stride_h == SS) return launch_conv_umma_ws<NN, SS>(a, L.umma_smem, sms, st);

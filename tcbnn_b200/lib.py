@@ -45,6 +45,8 @@ SIGNATURES = {
     "tcbnn_fc_units_bytes": (_SZ, [_I, _I, _I, _I]),
     "tcbnn_fc_expand_weight": (_I, [_P, _I, _I, _I, _P, _P]),
     "tcbnn_fc_layer_x": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P, _P, _P]),
+    "tcbnn_fc_layer_p": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P, _P, _I, _P]),
+    "tcbnn_out_layer_p": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _I, _P]),
     "tcbnn_pack_rows_x": (_I, [_P, _I, _I, _I, _P, _P, _P]),
     "tcbnn_pack_rows_w": (_I, [_P, _I, _I, _I, _P, _P, C.POINTER(FcWeight), _I, _P]),
     "tcbnn_out_layer": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
@@ -53,8 +55,6 @@ SIGNATURES = {
     "tcbnn_conv_prepare": (_I, [C.POINTER(ConvDesc), _P, _P, _P]),
     "tcbnn_conv_layer": (_I, [C.POINTER(ConvDesc), _P, _P, _P, _P, _I, _I, _I, _I, _P, _LL, _P, _I, _P, _P]),
     "tcbnn_set_conv_path": (_I, [_I]),
-    "tcbnn_fc_layer_p": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P, _P, _I, _P]),
-    "tcbnn_out_layer_p": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _I, _P]),
     "tcbnn_conv_set_trace": (_I, [_P]),
     "tcbnn_set_gemm_plan": (_I, [_I, _I]),
     "tcbnn_mma_operand_probe": (_I, [_I, _I, _I, C.POINTER(C.c_double)]),

@@ -72,3 +72,51 @@ def test_first_layer_sums_of_few_taps(cuda, R, S, O, same):
     assert np.array_equal(gr.cpu().numpy(), er)
     assert np.array_equal(_u32(go), eo)
     spec.release()
+
+
+# B, H, W, C, O, residual in / out.  3x3 layers of more than 256 channels run on pairs of SMs from two tiles per CTA on; the
+# batches give an odd number of tiles (a pair whose second CTA has none), several tiles per pair, one block per stage.
+PAIR_FORMS = [
+    (29, 8, 8, 512, 512, None, None), (60, 7, 7, 512, 256, None, None), (121, 8, 8, 384, 128, None, None), (30, 8, 9, 448, 512, None, None),
+    (29, 8, 8, 512, 512, "int16", "int16"), (33, 8, 8, 512, 512, "int32", "int32"), (29, 8, 8, 512, 512, None, "int32"),
+    (31, 8, 8, 512, 512, "chunked", "chunked"), (31, 8, 8, 512, 512, None, "chunked"), (60, 6, 8, 512, 512, "pooled chunked", "chunked"),
+    (60, 6, 8, 512, 512, "pooled int32", "int32"), (29, 8, 8, 512, 512, "acc", None),
+]
+
+
+@pytest.mark.parametrize("form", PAIR_FORMS)
+def test_wide_layers_on_pairs_of_sms(cuda, form):
+    B, H, W, C, O, rin, rout = form
+    g = util.rng(B + H + W + C + O)
+    x = util.rand_words(g, (B, H, W, C // 32))
+    f = util.rand_words(g, (O, 9, C // 32))
+    thr = (g.standard_normal(O) * np.sqrt(C * 9) * 0.5).astype(np.float32)
+    pooled = rin is not None and rin.startswith("pooled")
+    kind = rin.replace("pooled ", "") if rin not in (None, "acc") else None
+    rc = 256 if pooled else O                            # a pooled residual goes into the first channels
+    res = None
+    if kind:
+        res = g.integers(-1500, 1501, size=(B, H * (2 if pooled else 1), W * (2 if pooled else 1), rc)).astype(np.int32)
+    eo, er, ea = orc.conv_layer(x, f, thr, C, 3, 3, 1, 1, True, 1, res_in=res, residual_channels=rc if kind else 0, residual_pool=pooled,
+                                save_residual=rout is not None, want_acc=rin == "acc")
+    d = ops.conv_desc(B, H, W, C, O, 3, 3)
+    prep = ops.conv_prepare(d, _dev(f, cuda))
+    dres = None
+    if kind:
+        dres = torch.from_numpy(res).to(cuda)
+        if kind != "int32":
+            dres = dres.to(torch.int16)
+        if kind == "chunked":
+            dres = ops.nhwc_to_chunked(dres)
+    for _ in range(3):
+        go, gr, ga = ops.conv_layer(d, _dev(x, cuda), prep, _dev(thr, cuda), res_in=dres, residual_channels=rc if kind else 0,
+                                    residual_pool=pooled, save_residual=rout is not None, want_acc=rin == "acc",
+                                    residual_dtype=torch.int32 if rout == "int32" else torch.int16,
+                                    res_in_chunked=kind == "chunked", res_out_chunked=rout == "chunked")
+        assert ops.conv_status(d, prep) == 0
+        assert np.array_equal(_u32(go).reshape(eo.shape), eo)
+        if rout is not None:
+            gr = ops.chunked_to_nhwc(gr) if rout == "chunked" else gr
+            assert np.array_equal(gr.cpu().numpy().astype(np.int32), er)
+        if rin == "acc":
+            assert np.array_equal(ga.cpu().numpy(), ea)
