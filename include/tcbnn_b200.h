@@ -60,9 +60,10 @@ int tcbnn_gemm_status(int* status);
  * tcbnn_gemm_workspace_bytes AFTER this call fits the forced plan.
  * Process-wide; for tests and measurements.  No reference counterpart. */
 int tcbnn_set_gemm_plan(int pair, int splits);
-/* How many kernels a GEMM-family call of this shape launches when given a workspace of that size
+/* How many kernels a GEMM-family call of this shape launches at most when given a workspace of that size
  * (warp-level kernel: 1, or 2 with split K; tcgen05 path: 2 = operand expansion and a GEMM that
- * finishes the layer, 3 with split K); for callers that account for their launches. */
+ * finishes the layer, 3 with split K); for callers that account for their launches.  Operands whose rows are
+ * 16-byte aligned may take a single launch that needs no workspace instead. */
 int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes);
 
 /* GEMM family (the next three entry points): the pad bits of every row of A and of B / W -- the

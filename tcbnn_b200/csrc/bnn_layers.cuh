@@ -47,10 +47,11 @@ struct GemmArgs {
     const float* p0;      // thresholds (FC) or scale (OUT)
     const float* p1;      // bias (OUT)
     int splits;           // >1: split K, partial sums go to `partial`
-    int32_t* partial;     // [splits][M][N] raw (-2*popc(a) - 2*popc(w) + 4*popc(a&w)) sums
     // W, p0 and p1 are complete before the launch in front of this one can start (an ordinary launch came in
     // between): a dependent launch may read them ahead of its wait
+    // (in the padding behind splits: eight bytes more of parameters cost the host 0.3 us a launch)
     int settled;
+    int32_t* partial;     // [splits][M][N] raw (-2*popc(a) - 2*popc(w) + 4*popc(a&w)) sums
 };
 
 // One warp computes a 32 x 32 tile: 2 m-tiles x 4 n-tiles of m16n8k256.

@@ -8,6 +8,7 @@
 #include "bconv_umma_as.cuh"
 #include "bconv_umma_pre.cuh"
 #include "bgemm_umma.cuh"
+#include "bgemm_bits.cuh"
 #include "inconv_spec.cuh"
 #include "inconv_tiled.cuh"
 #include <cstdio>
@@ -77,18 +78,25 @@ int configure_once(bool (&done)[64], F&& configure) {
 // be set up while that still runs, and it waits (griddepcontrol.wait) before it touches anything that
 // an earlier launch writes or reads.  Every kernel launched this way executes that wait.
 template <class... P, class... A>
-cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+cudaError_t launch_dependent_cluster(void (*kernel)(P...), unsigned grid, unsigned cluster, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 0 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+    return launch_dependent_cluster(kernel, grid, 0, block, smem, st, std::forward<A>(args)...);
 }
 
 constexpr int kThreads = 256;          // 8 warps per CTA
@@ -279,6 +287,7 @@ int run_map(CUtensorMap* map, const void* base, long long elements, int box) {
 
 struct GemmUmmaPlan {
     bool use;
+    double clocks;
     bool pair;            // 256 x 256 tiles on pairs of SMs instead of 128 x 128 on one
     int MT, NT, KB, splits, per;
     size_t off_ew, off_partial, bytes;    // of the scratch: expanded A, expanded W, partial sums
@@ -317,7 +326,7 @@ GemmUmmaPlan gemm_umma_plan(int M, int N, int K, int sms, size_t room = SIZE_MAX
             double clk = pair ? (double)waves * (per * 150.0 + 3000.0) + 6000.0 : (double)waves * per * 140.0 + 7000.0;
             if (splits > 1) clk += 12000.0 + 6.0 * splits * (double)M * N * 4.0 / 3000.0;
             const size_t bytes = p.off_partial + (splits > 1 ? (size_t)splits * M * N * sizeof(int32_t) : 0);
-            if (clk < best && bytes <= room) { best = clk; p.pair = pair != 0; p.splits = splits; p.per = per; p.bytes = bytes; }
+            if (clk < best && bytes <= room) { best = p.clocks = clk; p.pair = pair != 0; p.splits = splits; p.per = per; p.bytes = bytes; }
         }
     }
     if (p.splits < 1) p.use = false;      // nothing fits, or a forced plan no slicing of K gives
@@ -402,6 +411,82 @@ int run_gemm_umma(const GemmArgs& g, const GemmUmmaPlan& p, void* workspace, con
     return launch_check("gemm (tcgen05) finish");
 }
 
+// ---- tcgen05 bit GEMM fed from the packed bits (bgemm_bits.cuh) -----------------------------
+__global__ void __launch_bounds__(umma::kBitsThreads, 1) k_gemm_bits(umma::GemmBitsArgs g) {
+    extern __shared__ __align__(128) unsigned char dyn_smem_bits[];
+    umma::gemm_bits_cta<false>(g, dyn_smem_bits);
+}
+__global__ void __launch_bounds__(umma::kBitsThreads, 1) k_gemm_bits_cluster(umma::GemmBitsArgs g) {
+    extern __shared__ __align__(128) unsigned char dyn_smem_bits_cluster[];
+    umma::gemm_bits_cta<true>(g, dyn_smem_bits_cluster);
+}
+
+struct GemmBitsPlan {
+    int cols, splits, per;       // rows of A per tile; CTAs of a cluster that share K, stages of each; 0 columns: not a shape for it
+    double us;
+};
+// The plan with the least time, in us as measured with operands in L2: a stage of 512 bits costs a CTA 0.46 to 0.97 (W's way into
+// tensor memory, then the pipeline's two or three stages), a tile's epilogue by its columns, a cluster the exchange of
+// its sums, a launch 3.2.
+GemmBitsPlan gemm_bits_plan(int M, int N, int K, int mode, int sms) {
+    GemmBitsPlan p = {};
+    if (K >= (1 << 22)) return p;                        // the fp32 accumulators hold K exactly up to that
+    const int stages = (K + 511) / 512;
+    p.us = 1e30;
+    const int tiles_n = (N + 127) / 128;
+    for (int cols = 32; cols <= umma::kBitsMaxCols; cols += 32) {
+        const long long tiles = (long long)((M + cols - 1) / cols) * tiles_n;
+        const double stage = cols <= 64 ? 0.46 : cols <= 96 ? 0.55 : cols <= 128 ? 0.60 : 0.95;
+        const double epilogue = mode == GEMM_FC_BITS ? 0.45 + 0.0095 * cols : 0.8 + 0.022 * cols;
+        const double waves = tiles <= sms ? 1.0 : (double)((tiles + sms - 1) / sms);
+        double us = 3.2 + waves * (stages * stage + epilogue) - (tiles <= sms ? 0.5 : 0.0);
+        if (us < p.us) { p.us = us; p.cols = cols; p.splits = 1; p.per = stages; }
+        // (of clusters of eight fewer fit at once than SMs suggest: 16 took two waves)
+        for (int splits = 2; splits <= 8 && tiles * splits <= (splits == 8 ? sms * 3 / 4 : sms); splits *= 2) {
+            const int per = (stages + splits - 1) / splits;
+            if ((splits - 1) * per >= stages) break;
+            us = 3.2 + per * stage + epilogue + 1.1 + 0.015 * cols;
+            if (us < p.us) { p.us = us; p.cols = cols; p.splits = splits; p.per = per; }
+        }
+    }
+    return p;
+}
+
+// What the other kernels take, in us, to the same measure: a fifth off at most from 4 us on.  The expansion pass writes half a
+// byte per bit; the b1 kernel costs its MMAs (390 TOP/s at best), its outputs, and a round trip to L2 for every
+// eight steps of K.
+double gemm_umma_us(const GemmUmmaPlan& p, const GemmArgs& g, const GemmUnits& u) {
+    return p.clocks / 1965.0 + 1.0 + ((u.a ? 0.0 : (double)g.M) + (u.w ? 0.0 : (double)g.N)) * g.K * 0.625 / 5.0e6;
+}
+double gemm_small_us(const GemmArgs& g) {
+    const int steps = (g.K + 255) / 256;
+    const double outputs = (double)((g.M + 15) & ~15) * g.N;
+    return 1.9 + 6.0e-6 * outputs + 1.25 * 2.0 * outputs * steps * 256.0 / 390.0e6 + 0.5 * ((steps + 7) / 8);
+}
+
+int run_gemm_bits(const GemmArgs& g, const GemmBitsPlan& p, void* next, int sms, cudaStream_t st) {
+    static bool configured[64] = {false};
+    if (configure_once(configured, [] {
+            cudaError_t e = cudaFuncSetAttribute(k_gemm_bits_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            return e != cudaSuccess ? e : cudaFuncSetAttribute(k_gemm_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        }))
+        return 1;
+    umma::GemmBitsArgs a;
+    a.A = g.A; a.W = g.W; a.M = g.M; a.N = g.N; a.K = g.K; a.lda = g.lda; a.ldw = g.ldw;
+    a.cols = p.cols; a.tiles_m = (g.M + p.cols - 1) / p.cols; a.tiles_n = (g.N + 127) / 128;
+    a.stages = (g.K + 511) / 512; a.per = p.per;
+    a.mode = g.mode; a.out = g.out; a.ldo = g.ldo; a.p0 = g.p0; a.p1 = g.p1;
+    a.nxt = (uint4*)next; a.nxt_KB = (g.N + 63) / 64; a.settled = g.settled;
+    if (gemm_status_address(&a.status)) return 1;
+    const long long tiles = (long long)a.tiles_m * a.tiles_n;
+    const size_t smem = umma::bits_smem_bytes(p.cols, p.splits);
+    const cudaError_t e = p.splits > 1
+        ? launch_dependent_cluster(k_gemm_bits_cluster, (unsigned)(tiles * p.splits), (unsigned)p.splits, umma::kBitsThreads, smem, st, a)
+        : launch_dependent(k_gemm_bits, (unsigned)(tiles < sms ? tiles : sms), umma::kBitsThreads, smem, st, a);
+    if (e != cudaSuccess) return fail("gemm (tcgen05, packed operands): %s", cudaGetErrorString(e));
+    return 0;
+}
+
 int g_gemm_path = 0;     // 0 automatic, 1 warp-level b1 MMA only
 
 int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st, const GemmUnits& u = GemmUnits{}) {
@@ -414,7 +499,18 @@ int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t s
     int sms;
     if (sm_count(&sms)) return 1;
     const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0, u.a, u.w);
-    if (plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0) {
+    const bool umma_fits = plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0;
+    if (g_gemm_path == 0 && g_gemm_force_pair < 0 && g_gemm_force_splits <= 0 && ((g.lda | g.ldw) & 3) == 0 && (((uintptr_t)g.A | (uintptr_t)g.W) & 15) == 0) {
+        // The packed operands' kernel where the estimates say that it is clearly the faster one.  Of 83 shapes, most of them
+        // drawn at random (1..8192 x 10..8192 x 64..16384), it takes 27, 1.04 to 4.4 times faster but for one that stays
+        // the same; seven of the others would have gained 8 to 45 %.
+        const double other = umma_fits ? 0.85 * gemm_umma_us(plan, g, u) : 0.9 * gemm_small_us(g);
+        if (other > 3.9) {                               // (no plan takes less, and looking for one costs the host half a microsecond)
+            const GemmBitsPlan bits = gemm_bits_plan(g.M, g.N, g.K, g.mode, sms);
+            if (bits.cols && bits.us < other) return run_gemm_bits(g, bits, u.next, sms, st);
+        }
+    }
+    if (umma_fits) {
         // (the epilogue writes the next operand where it finishes the layer itself)
         const GemmUnits mine{u.a, u.w, plan.splits == 1 ? u.next : nullptr};
         if (run_gemm_umma(g, plan, workspace, mine, sms, st)) return 1;
@@ -1420,7 +1516,7 @@ int tcbnn_gemm_status(int* status) {
 int tcbnn_bgemm(const uint32_t* A, const uint32_t* B, int M, int N, int K, int lda, int ldb,
                 int32_t* C, int ldc, void* workspace, size_t workspace_bytes, void* stream) {
     if (ldc < N) return fail("bgemm: ldc < N");
-    GemmArgs g{A, B, M, N, K, lda, ldb, GEMM_INT32, C, ldc, nullptr, nullptr, 1, nullptr};
+    GemmArgs g{A, B, M, N, K, lda, ldb, GEMM_INT32, C, ldc, nullptr, nullptr, 1, 0, nullptr};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -1428,7 +1524,7 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
                    int lda, int ldw, uint32_t* out, int ldo, void* workspace,
                    size_t workspace_bytes, void* stream) {
     if (ldo * 32 < N) return fail("fc_layer: ldo too small");
-    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr};
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, 0, nullptr};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -1458,7 +1554,7 @@ int tcbnn_fc_layer_p(const uint32_t* A, const uint32_t* W, const float* thr, int
     if (ldo * 32 < N) return fail("fc_layer: ldo too small");
     if (((uintptr_t)a_units | (uintptr_t)w_units | (uintptr_t)next_units) & 255) return fail("fc_layer: units must be 256-byte aligned");
     if (next_units && (ldo & 1)) return fail("fc_layer: next_units needs an even ldo");
-    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr, settled};
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, settled, nullptr};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream, GemmUnits{a_units, w_units, next_units});
 }
 
@@ -1472,7 +1568,7 @@ int tcbnn_out_layer_p(const uint32_t* A, const uint32_t* W, const float* scale, 
                       int M, int K, int N, int lda, int ldw, float* out, int ldo, void* workspace,
                       size_t workspace_bytes, int settled, void* stream) {
     if (ldo < N) return fail("out_layer: ldo < N");
-    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_OUT_AFFINE, out, ldo, scale, bias, 1, nullptr, settled};
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_OUT_AFFINE, out, ldo, scale, bias, 1, settled, nullptr};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -2193,7 +2289,7 @@ int tcbnn_fc_layer_noalloc(const uint32_t* A, const uint32_t* W, const float* th
                     need, (size_t)kStaticScratchBytes);
     void* scratch = nullptr;
     if (static_scratch(&scratch)) return 1;
-    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, nullptr};
+    GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, 0, nullptr};
     return run_gemm(g, scratch, kStaticScratchBytes, (cudaStream_t)stream);
 }
 

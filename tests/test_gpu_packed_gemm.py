@@ -1,14 +1,64 @@
-"""GEMM-family layers and MLPs in the forms that a pass gives them, against the CPU oracle and the layers called one
-by one.  Integers and bits are exact; logits are one fp32 multiply-add on an exact integer (rounded once here, twice
-in the oracle: 2^-23 of the larger term)."""
+"""The bit GEMM that reads packed rows (one launch) and the MLP that takes one launch, at the edges of their
+tiles, against the CPU oracle and against the layers called one by one.  Integers and bits are exact; logits are
+one fp32 multiply-add on an exact integer (rounded once here, twice in the oracle: 2^-23 of the larger term)."""
 import numpy as np
 import pytest
 import torch
 
+import oracle as orc
 import util
 from tcbnn_b200 import models, ops
 
 pytestmark = pytest.mark.gpu
+
+
+def _dev(a, cuda):
+    return torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).to(cuda)
+
+
+def _rows(words, ld, offset, cuda):
+    """`words` on the GPU in rows of ld words that start `offset` words into an allocation."""
+    t = torch.zeros((words.shape[0] * ld + offset,), dtype=torch.int32, device=cuda)[offset:].view(words.shape[0], ld)
+    t[:, :words.shape[1]] = _dev(words, cuda)
+    return t
+
+
+# M, N, K; extra words per row, words in front of the first row (rows that are not 16-byte aligned go to another kernel)
+SHAPES = [
+    (1, 1, 1, 0, 0), (1, 10, 64, 0, 0), (31, 33, 65, 0, 0), (32, 128, 512, 0, 0), (33, 129, 513, 0, 0),       # a tile and one more
+    (129, 200, 1000, 0, 0), (256, 128, 511, 0, 0), (257, 300, 449, 0, 0),
+    (640, 4096, 200, 0, 0),            # short K, several tiles per CTA
+    (2000, 3000, 64, 0, 0),            # one 64-bit block
+    (5000, 1000, 1500, 0, 0),          # several tiles per CTA, stages of 512, 512 and 476 bits
+    (70, 130, 2112, 0, 0), (40, 4096, 9216, 0, 0), (3, 1000, 16384, 0, 0),        # K cut over a cluster
+    (33, 140, 700, 4, 0), (33, 140, 700, 2, 0), (33, 140, 700, 0, 2), (300, 1100, 4100, 2, 2),
+]
+
+
+@pytest.mark.parametrize("M,N,K,pad,offset", SHAPES)
+def test_gemm_family_on_packed_rows(cuda, M, N, K, pad, offset):
+    g = util.rng(M + 3 * N + 7 * K)
+    ld = orc.step128_words(K)
+    A, W = (util.mask_row_pad(util.rand_words(g, (r, ld)), K) for r in (M, N))
+    thr = (g.standard_normal(N) * np.sqrt(K)).astype(np.float32)
+    thr[0] = np.nan                                                  # no value reaches it
+    scale, bias = g.standard_normal(N).astype(np.float32), g.standard_normal(N).astype(np.float32)
+    a, w = _rows(A, ld + pad, offset, cuda), _rows(W, ld + pad, offset, cuda)
+    ref = orc.bgemm(A, W, K)
+    ws = ops.gemm_workspace(M, N, K, cuda)
+    got = ops.bgemm(a, w, K, workspace=ws)
+    assert np.array_equal(got.cpu().numpy(), ref)
+    assert torch.equal(got, ops.bgemm(a, w, K))                      # (and without scratch)
+    bits = torch.full((M, orc.step128_words(N)), -1, dtype=torch.int32, device=cuda)
+    ops.fc_layer(a, w, _dev(thr, cuda), K, out=bits, workspace=ws)
+    words = (N + 31) // 32
+    want = util.pm1_to_bits(np.where(ref >= thr, 1.0, -1.0))         # NaN: never
+    assert np.array_equal(bits.cpu().numpy().view(np.uint32)[:, :words], want)
+    assert (bits[:, words:] == -1).all()                             # nothing behind the last word is touched
+    out = ops.out_layer(a, w, _dev(scale, cuda), _dev(bias, cuda), K, workspace=ws).cpu().numpy()
+    exact = ref.astype(np.float64) * scale + bias
+    np.testing.assert_allclose(out, exact, rtol=2.0 ** -23, atol=2.0 ** -23 * float(np.abs(bias).max()))
+    assert ops.gemm_status() == 0
 
 
 @pytest.mark.parametrize("batch", [8, 100])
