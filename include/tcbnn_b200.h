@@ -95,6 +95,21 @@ typedef struct tcbnn_fc_weight {
     int N, K, ldw;
     void* units;            /* tcbnn_fc_units_bytes(M, N, K, N) */
 } tcbnn_fc_weight;
+/* An MLP in one launch: fp32 rows [M][K] packed to bits[M][ld_words] (tcbnn_pack_rows), hidden layers
+ * (tcbnn_fc_layer: p0 = thresholds, p1 unused, out = words) and, last, an output layer (tcbnn_out_layer: p0 = scale,
+ * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which.
+ * Results are those of the layers called one by one. */
+typedef struct tcbnn_chain_layer {
+    const uint32_t* W;      /* [N][ldw] packed weight, 16-byte aligned, ldw a multiple of 4 */
+    int ldw, K, N;
+    const float* p0;
+    const float* p1;
+    void* out;              /* [M][ldo] */
+    int ldo;
+} tcbnn_chain_layer;
+int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words);
+int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n,
+                   void* stream);
 size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows);
 int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units, void* stream);
 int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,

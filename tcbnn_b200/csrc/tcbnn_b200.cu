@@ -9,6 +9,7 @@
 #include "bconv_umma_pre.cuh"
 #include "bgemm_umma.cuh"
 #include "bgemm_bits.cuh"
+#include "fc_chain.cuh"
 #include "inconv_spec.cuh"
 #include "inconv_tiled.cuh"
 #include <cstdio>
@@ -487,7 +488,41 @@ int run_gemm_bits(const GemmArgs& g, const GemmBitsPlan& p, void* next, int sms,
     return 0;
 }
 
+// ---- an MLP on a few rows in one launch (fc_chain.cuh) ---------------------------------------
+__global__ void __launch_bounds__(umma::kChainThreads, 1) k_fc_chain(const __grid_constant__ umma::ChainArgs g) {
+    extern __shared__ __align__(128) unsigned char dyn_smem_chain[];
+    umma::fc_chain_cta(g, dyn_smem_chain);
+}
+
 int g_gemm_path = 0;     // 0 automatic, 1 warp-level b1 MMA only
+
+// Fills `a` with the layers and their places in tensor memory; false: not a chain that the kernel takes.
+bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, int sms, umma::ChainArgs* a) {
+    if (g_gemm_path == 1 || n < 1 || n > umma::kChainMaxLayers || M < 64 || K < 1 || ld < 1 || ld * 32 < K) return false;
+    // as many clusters as run at once (GPCs hold no whole number of them), the rows dealt out evenly
+    const int clusters = sms / umma::kChainCtas * 7 / 8;
+    a->rows = M <= 16 * clusters ? 16 : M <= 32 * clusters ? 32 : 64;
+    if (clusters < 1 || M > 64 * clusters) return false;
+    a->units = 0;
+    a->n = n;
+    int first[umma::kChainMaxLayers], end[umma::kChainMaxLayers], next = 0;
+    for (int l = 0; l < n; l++) {
+        const tcbnn_chain_layer& y = layers[l];
+        if (y.K != (l ? layers[l - 1].N : K) || y.N < 1 || y.N > 128 * umma::kChainCtas) return false;
+        if (!y.W || ((uintptr_t)y.W & 15) || (y.ldw & 3) || y.ldw * 32 < y.K || !y.p0 || !y.out) return false;
+        if (l + 1 == n ? !y.p1 || y.ldo < y.N : y.ldo * 32 < y.N) return false;
+        const int kb = (y.K + 63) / 64, columns = kb * 8;
+        if (columns > umma::chain_columns(a->rows)) return false;
+        if (kb > a->units) a->units = kb;
+        if (next + columns > umma::chain_columns(a->rows)) next = 0;
+        first[l] = next; end[l] = next += columns;
+        int after = -1;
+        for (int e = 0; e < l; e++)
+            if (first[e] < end[l] && first[l] < end[e]) after = e;
+        a->layer[l] = {y.W, y.ldw, y.K, y.N, y.p0, y.p1, y.out, y.ldo, first[l], after};
+    }
+    return umma::chain_smem_bytes(a->rows, a->units) <= 200 * 1024;
+}
 
 int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st, const GemmUnits& u = GemmUnits{}) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) return fail("gemm: M, N, K must be positive");
@@ -1526,6 +1561,38 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
     if (ldo * 32 < N) return fail("fc_layer: ldo too small");
     GemmArgs g{A, W, M, N, K, lda, ldw, GEMM_FC_BITS, out, ldo, thr, nullptr, 1, 0, nullptr};
     return run_gemm(g, workspace, workspace_bytes, (cudaStream_t)stream);
+}
+
+int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words) {
+    int sms;
+    umma::ChainArgs a;
+    if (!layers || sm_count(&sms)) return 0;
+    return chain_plan(layers, n, M, K, ld_words, sms, &a) ? 1 : 0;
+}
+
+int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n, void* stream) {
+    umma::ChainArgs a;
+    int sms;
+    if (sm_count(&sms)) return 1;
+    if (!x || !bits || !layers || !chain_plan(layers, n, M, K, ld_words, sms, &a)) return fail("fc_chain: not a chain that one launch takes (tcbnn_fc_chain_fits)");
+    static bool configured[64] = {false};
+    if (configure_once(configured, [] { return cudaFuncSetAttribute(k_fc_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); })) return 1;
+    a.x = x; a.M = M; a.K = K; a.ld = ld_words; a.bits = bits;
+    if (gemm_status_address(&a.status)) return 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((M + a.rows - 1) / a.rows * umma::kChainCtas));
+    cfg.blockDim = dim3(umma::kChainThreads);
+    cfg.dynamicSmemBytes = umma::chain_smem_bytes(a.rows, a.units);
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = umma::kChainCtas;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_fc_chain, a);       // (an ordinary launch: it waits for all before it)
+    if (e != cudaSuccess) return fail("fc_chain: %s", cudaGetErrorString(e));
+    return 0;
 }
 
 size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows) {

@@ -22,6 +22,12 @@ class FcWeight(C.Structure):
     _fields_ = [("W", C.c_void_p), ("N", C.c_int), ("K", C.c_int), ("ldw", C.c_int), ("units", C.c_void_p)]
 
 
+class ChainLayer(C.Structure):
+    """struct tcbnn_chain_layer of include/tcbnn_b200.h."""
+    _fields_ = [("W", C.c_void_p), ("ldw", C.c_int), ("K", C.c_int), ("N", C.c_int), ("p0", C.c_void_p), ("p1", C.c_void_p),
+                ("out", C.c_void_p), ("ldo", C.c_int)]
+
+
 _P = C.c_void_p
 _I = C.c_int
 _LL = C.c_longlong
@@ -42,6 +48,8 @@ SIGNATURES = {
     "tcbnn_gemm_status": (_I, [C.POINTER(C.c_int)]),
     "tcbnn_bgemm": (_I, [_P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
     "tcbnn_fc_layer": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
+    "tcbnn_fc_chain_fits": (_I, [C.POINTER(ChainLayer), _I, _I, _I, _I]),
+    "tcbnn_fc_chain": (_I, [_P, _I, _I, _I, _P, C.POINTER(ChainLayer), _I, _P]),
     "tcbnn_fc_units_bytes": (_SZ, [_I, _I, _I, _I]),
     "tcbnn_fc_expand_weight": (_I, [_P, _I, _I, _I, _P, _P]),
     "tcbnn_fc_layer_x": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P, _P, _P, _P]),

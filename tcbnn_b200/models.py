@@ -229,6 +229,37 @@ def _input_facts(layers):
     return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
 
 
+def _chain_call(layers):
+    """The one call that makes an MLP's whole pass (tcbnn_fc_chain), or None where it does not apply: other
+    layers, more rows or wider layers than it takes, or inputs that are not the layer in front's outputs."""
+    first, last = layers[0], layers[-1]
+    if (type(first).__name__ != "In128LayerParam" or type(last).__name__ != "Out128LayerParam" or
+            any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
+        return None
+    x, bits = first.input_gpu, first.output_gpu
+    keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
+    for i, (prev, l) in enumerate(zip(layers, layers[1:])):
+        w, out = l.weight_gpu, l.output_gpu
+        p0, p1 = (l.bn_scale_gpu, l.bn_bias_gpu) if l is last else (l.bn_gpu, None)
+        if (l.live != first.live or l.input_gpu.data_ptr() != prev.output_gpu.data_ptr() or l.input_gpu.shape[1] != prev.output_gpu.shape[1]
+                or l.input_width != prev.output_width):
+            return None
+        ops._need_cuda(w, p0, p1)
+        chain[i] = lib.ChainLayer(w.data_ptr(), w.shape[1], l.input_width, w.shape[0], p0.data_ptr(), p1.data_ptr() if p1 is not None else None,
+                                  out.data_ptr(), out.shape[1])
+        keep += [w, p0, p1, out]
+    shape = first.live, first.input_width, bits.shape[1]
+    if not lib.load().tcbnn_fc_chain_fits(chain, len(chain), *shape):
+        return None
+    return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
+
+
+def _pass_calls(layers):
+    """[(entry point, arguments, what they point to)] of one pass."""
+    chain = _chain_call(layers)
+    return [chain] if chain else [l._call_args(True) for l in layers]
+
+
 class _Calls:
     """A network's layers' calls, prepared.  Once noted they serve while nothing but the input has changed of what
     they were prepared from: an attribute of a layer, its live batch, a descriptor, a process-wide
@@ -245,7 +276,7 @@ class _Calls:
         device = layers[0].output_gpu.device
         while True:
             self.scratch = ops.shared_scratch(device)
-            prepared = [l._call_args(True) for l in layers]
+            prepared = _pass_calls(layers)
             if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
@@ -286,7 +317,7 @@ class _Pass:
         """fresh: the calls have just been prepared, on this input."""
         self.common, self.calls = calls, list(calls.calls)
         if not fresh:
-            name, args, _ = layers[0]._call_args(True)
+            name, args, _ = _chain_call(layers) or layers[0]._call_args(True)
             self.calls[0] = lib.bound(name), args
         self.input = _input_facts(layers)
         self.seen, self.graph = 0, None

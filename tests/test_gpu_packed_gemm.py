@@ -7,7 +7,7 @@ import torch
 
 import oracle as orc
 import util
-from tcbnn_b200 import models, ops
+from tcbnn_b200 import lib, models, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -59,6 +59,66 @@ def test_gemm_family_on_packed_rows(cuda, M, N, K, pad, offset):
     exact = ref.astype(np.float64) * scale + bias
     np.testing.assert_allclose(out, exact, rtol=2.0 ** -23, atol=2.0 ** -23 * float(np.abs(bias).max()))
     assert ops.gemm_status() == 0
+
+
+WIDTHS = [(784, 1024, 1024, 1024, 10), (100, 130, 1000, 64, 7), (1, 1, 1), (845, 1024, 928, 1000), (513, 40, 1024, 257, 1024),
+          (1500, 96, 33, 500)]
+
+
+@pytest.mark.parametrize("widths", WIDTHS)
+@pytest.mark.parametrize("batch", [64, 65, 241, 300, 700])
+def test_mlp_in_one_launch_is_its_layers_one_by_one(cuda, widths, batch):
+    """Every layer's packed output and the logits of a pass in one launch, for 16, 32 and 64 rows per cluster with
+    a ragged last one, against the same layers called by themselves."""
+    spec = models.mlp_spec(batch, widths[0], 1, widths[-1])
+    spec["layers"] = [spec["layers"][0]] + [dict(type="fc", name="Fc%d" % i, N=n) for i, n in enumerate(widths[1:-1])] + [spec["layers"][-1]]
+    w, x = models.synthetic_weights(spec, 41), models.synthetic_input(spec, 42)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    assert models._chain_call(net.layers) is not None
+    for l in plain.layers:
+        l.forward()
+    for _ in range(4):                                               # (a replayed graph by the last)
+        for l in net.layers:
+            l.output_gpu.fill_(0)
+        net.forward()
+        for l, p in zip(net.layers, plain.layers):
+            assert torch.equal(l.output_gpu, p.output_gpu), l.name
+    for fewer in (batch - 1, batch // 3):                            # in the same buffers; in one launch or, below 64 rows, in several
+        for l in net.layers:
+            l.output_gpu.fill_(0)
+        net.set_batch(fewer)
+        assert (models._chain_call(net.layers) is not None) == (fewer >= 64)
+        net.forward()
+        for l, p in zip(net.layers, plain.layers):
+            assert torch.equal(l.output_gpu[:fewer], p.output_gpu[:fewer]), l.name
+            assert not l.output_gpu[fewer:].any()
+    assert ops.gemm_status() == 0
+
+
+def test_mlp_with_another_layers_input_is_not_one_launch(cuda):
+    """A layer whose input is not the output of the one in front keeps its own launch, and its input counts."""
+    spec = models.mlp_spec(72)
+    w, x = models.synthetic_weights(spec, 43), models.synthetic_input(spec, 44)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    other = torch.randint(-2 ** 31, 2 ** 31, net.layers[2].input_gpu.shape, dtype=torch.int64, device=cuda).to(torch.int32)
+    want = net.forward().clone()
+    for n in (net, plain):
+        n.layers[2].set_input_gpu(other.clone())
+    assert models._chain_call(net.layers) is None
+    for l in plain.layers:
+        l.forward()
+    got = net.forward().clone()
+    assert torch.equal(got, plain.layers[-1].output_gpu) and not torch.equal(got, want)
+
+
+def test_mlp_entry_point_refuses_what_it_does_not_take(cuda):
+    spec = models.mlp_spec(80)
+    net = models.Network(spec, models.synthetic_weights(spec, 45), models.synthetic_input(spec, 46))
+    name, (x, M, K, ld, bits, chain, n), _ = models._chain_call(net.layers)
+    chain[1].N += 1                                                  # not the next layer's K
+    assert not lib.load().tcbnn_fc_chain_fits(chain, n, M, K, ld)
+    with pytest.raises(lib.TcbnnError):
+        lib.call(name, x, M, K, ld, bits, chain, n, ops._stream())
 
 
 @pytest.mark.parametrize("batch", [8, 100])
