@@ -65,6 +65,10 @@ int tcbnn_set_gemm_plan(int pair, int splits);
  * finishes the layer, 3 with split K); for callers that account for their launches.  Operands whose rows are
  * 16-byte aligned may take a single launch that needs no workspace instead. */
 int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes);
+/* How many the call launches: mode 0 = tcbnn_bgemm, 1 = tcbnn_fc_layer, 2 = tcbnn_out_layer, for operands whose first rows are
+ * 16-byte aligned; a_units, w_units: whether it is given expanded operands.  (next_units cost a launch more where K
+ * is split.) */
+int tcbnn_gemm_call_launches(int M, int N, int K, int mode, int lda, int ldw, size_t workspace_bytes, int a_units, int w_units);
 
 /* GEMM family (the next three entry points): the pad bits of every row of A and of B / W -- the
  * bits past element K up to the leading dimension -- must be zero, as tcbnn_pack_rows,

@@ -19,7 +19,13 @@
 // A stage is 512 bits of K, 64 bytes of a row, which four lanes fetch together (cp.async): what the loads cost is
 // the lines they touch, about two clocks each (a lane per row, 32 lines an instruction, took 1890 clocks per
 // 256 bits of a 256-column tile whose MMAs take 512).  Each expander keeps two tiles of 32 rows in flight or in
-// hand, in shared memory; through registers, one ahead, a stage took the latency of L2 whatever its size.
+// hand, in shared memory.  A stage costs 0.46 us at 32 and 64 columns, where an expander of W needs 1000 clocks for 112
+// logic operations and 16 KB into tensor memory, and 0.95 at 256 (1024 clocks of MMAs), where only two stages fit and
+// their hand-overs show.  Masking every word for the end of K, if-converted by the compiler, had doubled the expanders' time.
+//
+// Measured in one launch of a graph, before (expansion pass and GEMM, or the b1 kernel) and here: 1024 x 1024 x 4096
+// 10.2 -> 8.4 us, 1024 x 25088 -> 512 21.0 -> 16.0, 32 x 25088 -> 4096 25.9 -> 12.5, 1024 x 512 -> 1000 11.2 -> 5.0, 2000 x 3000 x 64
+// 41 -> 13, 4000 x 200 -> 8192 224 -> 23; 8192 x 8192 x 8192 173 -> 224, which is why large ones stay where they were.
 //
 // Where the tiles of M x N leave SMs idle, K is cut over a cluster's CTAs, whose sums meet in the first shared
 // memory that the loop no longer needs; each CTA then finishes its share of the columns.

@@ -524,6 +524,17 @@ bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, in
     return umma::chain_smem_bytes(a->rows, a->units) <= 200 * 1024;
 }
 
+// The packed operands' kernel where the estimates say that it is clearly the faster one.  Of 83 shapes, most of them
+// drawn at random (1..8192 x 10..8192 x 64..16384), it takes 27, 1.04 to 4.4 times faster but for one that stays
+// the same; seven of the others would have gained 8 to 45 %.
+bool gemm_takes_bits(const GemmArgs& g, const GemmUmmaPlan& plan, bool umma_fits, const GemmUnits& u, int sms, GemmBitsPlan* bits) {
+    if (g_gemm_path != 0 || g_gemm_force_pair >= 0 || g_gemm_force_splits > 0 || ((g.lda | g.ldw) & 3) || (((uintptr_t)g.A | (uintptr_t)g.W) & 15)) return false;
+    const double other = umma_fits ? 0.85 * gemm_umma_us(plan, g, u) : 0.9 * gemm_small_us(g);
+    if (other <= 3.9) return false;                      // (no plan takes less, and looking for one costs the host half a microsecond)
+    *bits = gemm_bits_plan(g.M, g.N, g.K, g.mode, sms);
+    return bits->cols && bits->us < other;
+}
+
 int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st, const GemmUnits& u = GemmUnits{}) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) return fail("gemm: M, N, K must be positive");
     if ((g.lda & 1) || (g.ldw & 1)) return fail("gemm: lda and ldw must be even (64-bit loads)");
@@ -535,16 +546,8 @@ int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t s
     if (sm_count(&sms)) return 1;
     const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0, u.a, u.w);
     const bool umma_fits = plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0;
-    if (g_gemm_path == 0 && g_gemm_force_pair < 0 && g_gemm_force_splits <= 0 && ((g.lda | g.ldw) & 3) == 0 && (((uintptr_t)g.A | (uintptr_t)g.W) & 15) == 0) {
-        // The packed operands' kernel where the estimates say that it is clearly the faster one.  Of 83 shapes, most of them
-        // drawn at random (1..8192 x 10..8192 x 64..16384), it takes 27, 1.04 to 4.4 times faster but for one that stays
-        // the same; seven of the others would have gained 8 to 45 %.
-        const double other = umma_fits ? 0.85 * gemm_umma_us(plan, g, u) : 0.9 * gemm_small_us(g);
-        if (other > 3.9) {                               // (no plan takes less, and looking for one costs the host half a microsecond)
-            const GemmBitsPlan bits = gemm_bits_plan(g.M, g.N, g.K, g.mode, sms);
-            if (bits.cols && bits.us < other) return run_gemm_bits(g, bits, u.next, sms, st);
-        }
-    }
+    GemmBitsPlan bits;
+    if (gemm_takes_bits(g, plan, umma_fits, u, sms, &bits)) return run_gemm_bits(g, bits, u.next, sms, st);
     if (umma_fits) {
         // (the epilogue writes the next operand where it finishes the layer itself)
         const GemmUnits mine{u.a, u.w, plan.splits == 1 ? u.next : nullptr};
@@ -1520,6 +1523,20 @@ int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes) {
     if (M <= 0 || N <= 0 || K <= 0 || sm_count(&sms)) return 0;
     const GemmUmmaPlan plan = gemm_umma_plan(M, N, K, sms, workspace_bytes);
     if (plan.use && g_gemm_path != 1) return plan.splits > 1 ? 3 : 2;   // expansion, GEMM, finish
+    return gemm_use_splits(M, N, K, sms, workspace_bytes) > 1 ? 2 : 1;
+}
+
+int tcbnn_gemm_call_launches(int M, int N, int K, int mode, int lda, int ldw, size_t workspace_bytes, int a_units, int w_units) {
+    int sms;
+    if (M <= 0 || N <= 0 || K <= 0 || mode < 0 || mode > 2 || sm_count(&sms)) return 0;
+    GemmArgs g = {};
+    g.M = M; g.N = N; g.K = K; g.mode = mode; g.lda = lda; g.ldw = ldw;
+    const GemmUnits u{a_units ? &g : nullptr, w_units ? &g : nullptr, nullptr};          // (only whether they are there counts)
+    const GemmUmmaPlan plan = gemm_umma_plan(M, N, K, sms, workspace_bytes, u.a, u.w);
+    const bool umma_fits = plan.use && g_gemm_path != 1;
+    GemmBitsPlan bits;
+    if (gemm_takes_bits(g, plan, umma_fits, u, sms, &bits)) return 1;
+    if (umma_fits) return (a_units && w_units ? 1 : 2) + (plan.splits > 1 ? 1 : 0);
     return gemm_use_splits(M, N, K, sms, workspace_bytes) > 1 ? 2 : 1;
 }
 

@@ -89,9 +89,18 @@ def gemm_workspace(M, N, K, device):
 
 
 def gemm_launches(M, N, K, workspace):
-    """Kernels a GEMM-family call of this shape launches with this workspace tensor."""
+    """Kernels a GEMM-family call of this shape launches at most with this workspace tensor."""
     nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
     return _l.load().tcbnn_gemm_launches(M, N, K, nbytes)
+
+
+GEMM_INT32, GEMM_BITS, GEMM_AFFINE = 0, 1, 2
+
+
+def gemm_call_launches(mode, M, A, W, K, workspace, a_units=False, w_units=False):
+    """Kernels the call launches on M rows of A and on W (tcbnn_gemm_call_launches)."""
+    nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
+    return _l.load().tcbnn_gemm_call_launches(M, W.shape[0], K, mode, A.shape[1], W.shape[1], nbytes, int(a_units), int(w_units))
 
 
 def fc_units(M, N, K, rows, device):

@@ -226,10 +226,10 @@ class Fc128LayerParam(_Layer):
         return ops._l.FcWeight(w.data_ptr(), w.shape[0], self.input_width, w.shape[1], self.weight_units.data_ptr())
 
     def kernel_launches(self):
-        # the operand expansion is not launched where both operands come expanded; where a finishing
-        # launch computes the bits (launches == 3), the next layer's input is expanded from them
-        return (self.launches - int(self.input_units is not None and self.weight_units is not None)
-                + int(self.next_units is not None and self.launches == 3))
+        # (where a finishing launch computes the bits, the next layer's input is expanded from them)
+        a, w = self.input_units is not None, self.weight_units is not None
+        n = ops.gemm_call_launches(ops.GEMM_BITS, self.live, self.input_gpu, self.weight_gpu, self.input_width, self.workspace, a, w)
+        return n + int(self.next_units is not None and n > (1 if a and w else 2))
 
     def _call_args(self, in_pass):
         a, w, thr, out, ws = self.input_gpu, self.weight_gpu, self.bn_gpu, self.output_gpu, self.workspace
@@ -284,7 +284,7 @@ class Out128LayerParam(_Layer):
         return self
 
     def kernel_launches(self):
-        return self.launches
+        return ops.gemm_call_launches(ops.GEMM_AFFINE, self.live, self.input_gpu, self.weight_gpu, self.input_width, self.workspace)
 
     def _call_args(self, in_pass):
         a, w, out, ws = self.input_gpu, self.weight_gpu, self.output_gpu, self.workspace

@@ -111,6 +111,25 @@ def test_mlp_with_another_layers_input_is_not_one_launch(cuda):
     assert torch.equal(got, plain.layers[-1].output_gpu) and not torch.equal(got, want)
 
 
+def test_launches_a_call_makes(cuda):
+    """What a layer says it launches, against the kernels the profiler sees."""
+    from torch.profiler import ProfilerActivity, profile
+    for M, N, K in [(32, 128, 256), (1024, 1000, 512), (2048, 4096, 9216), (200, 256, 200000)]:
+        ld = orc.step128_words(K)
+        a, w = (torch.zeros((r, ld), dtype=torch.int32, device=cuda) for r in (M, N))
+        thr, out = torch.zeros(N, device=cuda), torch.zeros((M, orc.step128_words(N)), dtype=torch.int32, device=cuda)
+        ws = ops.gemm_workspace(M, N, K, cuda)
+        for room in (ws, None):
+            ops.fc_layer(a, w, thr, K, out=out, workspace=room)
+            torch.cuda.synchronize()
+            with profile(activities=[ProfilerActivity.CUDA]) as p:
+                ops.fc_layer(a, w, thr, K, out=out, workspace=room)
+                torch.cuda.synchronize()
+            seen = sum(e.device_type == torch.autograd.DeviceType.CUDA and "k_" in e.name for e in p.events())
+            assert ops.gemm_call_launches(ops.GEMM_BITS, M, a, w, K, room) == seen, (M, N, K, room is None)
+            assert seen <= ops.gemm_launches(M, N, K, room)
+
+
 def test_mlp_entry_point_refuses_what_it_does_not_take(cuda):
     spec = models.mlp_spec(80)
     net = models.Network(spec, models.synthetic_weights(spec, 45), models.synthetic_input(spec, 46))
