@@ -239,15 +239,15 @@ def _chain_call(layers):
     x, bits = first.input_gpu, first.output_gpu
     keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
     for i, (prev, l) in enumerate(zip(layers, layers[1:])):
-        w, out = l.weight_gpu, l.output_gpu
+        a, w, out = l.input_gpu, l.weight_gpu, l.output_gpu
         p0, p1 = (l.bn_scale_gpu, l.bn_bias_gpu) if l is last else (l.bn_gpu, None)
-        if (l.live != first.live or l.input_gpu.data_ptr() != prev.output_gpu.data_ptr() or l.input_gpu.shape[1] != prev.output_gpu.shape[1]
+        if (l.live != first.live or a.data_ptr() != prev.output_gpu.data_ptr() or a.shape[1] != prev.output_gpu.shape[1]
                 or l.input_width != prev.output_width):
             return None
-        ops._need_cuda(w, p0, p1)
+        ops._need_cuda(a, w, p0, p1)
         chain[i] = lib.ChainLayer(w.data_ptr(), w.shape[1], l.input_width, w.shape[0], p0.data_ptr(), p1.data_ptr() if p1 is not None else None,
                                   out.data_ptr(), out.shape[1])
-        keep += [w, p0, p1, out]
+        keep += [a, w, p0, p1, out]
     shape = first.live, first.input_width, bits.shape[1]
     if not lib.load().tcbnn_fc_chain_fits(chain, len(chain), *shape):
         return None

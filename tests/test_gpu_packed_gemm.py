@@ -111,6 +111,26 @@ def test_mlp_with_another_layers_input_is_not_one_launch(cuda):
     assert torch.equal(got, plain.layers[-1].output_gpu) and not torch.equal(got, want)
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_mlp_in_one_launch_follows_a_layers_input_given_another_storage(cuda, graph):
+    """The rows of a layer's input tensor are exchanged in place, behind passes that are replayed by then."""
+    spec = models.mlp_spec(72)
+    w, x = models.synthetic_weights(spec, 47), models.synthetic_input(spec, 48)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    one_pass = net.forward_graph if graph else net.forward
+    net.layers[2].input_gpu = net.layers[1].output_gpu.view(72, -1)
+    for _ in range(4):
+        want = one_pass().clone()
+    assert models._chain_call(net.layers) is not None
+    other = torch.randint(-2 ** 31, 2 ** 31, net.layers[2].input_gpu.shape, dtype=torch.int64, device=cuda).to(torch.int32)
+    net.layers[2].input_gpu.data = other
+    plain.layers[2].set_input_gpu(other)
+    for l in plain.layers:
+        l.forward()
+    got = one_pass().clone()
+    assert torch.equal(got, plain.layers[-1].output_gpu) and not torch.equal(got, want)
+
+
 def test_launches_a_call_makes(cuda):
     """What a layer says it launches, against the kernels the profiler sees."""
     from torch.profiler import ProfilerActivity, profile

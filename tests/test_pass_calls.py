@@ -1,0 +1,77 @@
+"""What a network prepares for a pass, without a GPU: layer objects on CPU tensors, and a stand-in for the library that
+records what it is asked."""
+import ctypes as C
+
+import pytest
+import torch
+
+from tcbnn_b200 import lib, models, ops, param
+
+
+class _Library:
+    def __init__(self):
+        self.asked = []
+
+    def tcbnn_fc_chain_fits(self, layers, n, M, K, ld):
+        self.asked.append((None if layers is None else n, M))
+        return int(64 <= M <= 960)
+
+
+@pytest.fixture
+def library(monkeypatch):
+    def need(*ts):
+        for t in ts:
+            if t is not None and not t.is_contiguous():
+                raise lib.TcbnnError("contiguous")
+    fake = _Library()
+    monkeypatch.setattr(lib, "load", lambda: fake)
+    monkeypatch.setattr(lib, "bound", lambda name: name)
+    monkeypatch.setattr(ops, "_need_cuda", need)
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 0, raising=False)
+    return fake
+
+
+def _ints(*shape):
+    return torch.zeros(shape, dtype=torch.int32)
+
+
+def _mlp(batch, widths):
+    words = [ops.step128_words(n) for n in widths]
+    first = param.In128LayerParam("Fin", batch, widths[0])
+    first.input_gpu, first.output_gpu = torch.zeros((batch, widths[0])), _ints(batch, words[0])
+    layers = [first]
+    for i, (k, n) in enumerate(zip(widths, widths[1:])):
+        last = i + 2 == len(widths)
+        l = (param.Out128LayerParam if last else param.Fc128LayerParam)("L%d" % (i + 1), batch, k, n)
+        l.weight_gpu, l.input_gpu, l.workspace = _ints(n, words[i]), layers[-1].output_gpu, None
+        if last:
+            l.bn_scale_gpu, l.bn_bias_gpu, l.output_gpu = torch.zeros(n), torch.zeros(n), torch.zeros((batch, n))
+        else:
+            l.bn_gpu, l.output_gpu = torch.zeros(n), _ints(batch, words[i + 1])
+        layers.append(l)
+    return layers
+
+
+def _names(layers):
+    return [name for name, _, _ in models._pass_calls(layers)]
+
+
+WIDTHS = (784, 1024, 512, 1024, 10)
+
+
+def test_one_launch_follows_every_layers_input(library):
+    """A layer's own input tensor counts where the whole pass is one call: given another storage in place, and where
+    its rows do not lie one behind the other."""
+    layers = _mlp(100, WIDTHS)
+    assert _names(layers) == ["tcbnn_fc_chain"]
+    layers[2].input_gpu = layers[1].output_gpu.view(100, -1)           # (a tensor of its own on the same rows)
+    calls = models._Calls(layers)
+    calls.note(layers)
+    assert calls.hold(layers) and not calls.moved()
+    layers[2].input_gpu.data = layers[2].input_gpu.clone()
+    assert calls.moved() and "tcbnn_fc_chain" not in _names(layers)
+    layers = _mlp(100, WIDTHS)
+    wide = _ints(100, 2 * layers[1].output_gpu.shape[1])
+    layers[1].output_gpu = layers[2].input_gpu = wide[:, :wide.shape[1] // 2]
+    with pytest.raises(lib.TcbnnError):
+        models._pass_calls(layers)
