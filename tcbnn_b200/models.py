@@ -254,10 +254,36 @@ def _chain_call(layers):
     return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
 
 
-def _pass_calls(layers):
+def _span(t):
+    """[first, last) address of a tensor's elements."""
+    at = t.data_ptr()
+    if t.is_contiguous():
+        return at, at + t.nbytes
+    return at, at + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
+
+
+def _meets(t, spans):
+    lo, hi = _span(t)
+    return any(lo < end and start < hi for start, end in spans)
+
+
+def _written(layers):
+    """Where a pass writes: every layer's outputs."""
+    return [_span(t) for l in layers for t in (l.output_gpu, getattr(l, "output_residual_gpu", None)) if t is not None]
+
+
+def _reads_what_it_writes(layers):
+    """Whether a pass writes a weight or a parameter of its own (one layer's output as another's weight).  FC layers
+    read or expand theirs ahead of the layers in front; here all then run as they do when called by
+    themselves."""
+    written = _written(layers)
+    return any(_meets(t, written) for l in layers for t in l.read_ahead())
+
+
+def _pass_calls(layers, in_pass=True):
     """[(entry point, arguments, what they point to)] of one pass."""
-    chain = _chain_call(layers)
-    return [chain] if chain else [l._call_args(True) for l in layers]
+    chain = _chain_call(layers) if in_pass else None
+    return [chain] if chain else [l._call_args(in_pass) for l in layers]
 
 
 class _Calls:
@@ -274,9 +300,10 @@ class _Calls:
 
     def __init__(self, layers):
         device = layers[0].output_gpu.device
+        self.in_pass = not _reads_what_it_writes(layers)
         while True:
             self.scratch = ops.shared_scratch(device)
-            prepared = _pass_calls(layers)
+            prepared = _pass_calls(layers, self.in_pass)
             if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
@@ -317,7 +344,7 @@ class _Pass:
         """fresh: the calls have just been prepared, on this input."""
         self.common, self.calls = calls, list(calls.calls)
         if not fresh:
-            name, args, _ = _chain_call(layers) or layers[0]._call_args(True)
+            name, args, _ = _pass_calls(layers, calls.in_pass)[0]
             self.calls[0] = lib.bound(name), args
         self.input = _input_facts(layers)
         self.seen, self.graph = 0, None

@@ -102,6 +102,10 @@ class _Layer:
         """Changes with every attribute that is set, except that a live batch that comes back is the same."""
         return self.generation, self.live
 
+    def read_ahead(self):
+        """Tensors that a pass may read before the layers in front have run."""
+        return ()
+
     def forward(self):
         name, args, _ = self._call_args(False)
         ops._l.call(name, *args, ops._stream())
@@ -225,6 +229,9 @@ class Fc128LayerParam(_Layer):
         ops._need_cuda(w)
         return ops._l.FcWeight(w.data_ptr(), w.shape[0], self.input_width, w.shape[1], self.weight_units.data_ptr())
 
+    def read_ahead(self):
+        return self.weight_gpu, self.bn_gpu
+
     def kernel_launches(self):
         # (where a finishing launch computes the bits, the next layer's input is expanded from them)
         a, w = self.input_units is not None, self.weight_units is not None
@@ -282,6 +289,9 @@ class Out128LayerParam(_Layer):
         self.launches = ops.gemm_launches(self.input_height, N, K, self.workspace)
         self.input_gpu = prev_layer_gpu.reshape(self.input_height, -1)
         return self
+
+    def read_ahead(self):
+        return self.weight_gpu, self.bn_scale_gpu, self.bn_bias_gpu
 
     def kernel_launches(self):
         return ops.gemm_call_launches(ops.GEMM_AFFINE, self.live, self.input_gpu, self.weight_gpu, self.input_width, self.workspace)

@@ -186,3 +186,25 @@ def test_small_mlp_follows_weights_and_parameters_written_between_passes(cuda, b
         plain.layers[2].weight_gpu.copy_(net.layers[2].weight_gpu)
         assert torch.equal(got, plain.forward())
         src.bitwise_not_()
+
+
+@pytest.mark.parametrize("batch", [8, 100, 1024])
+def test_a_layers_output_as_the_next_ones_weight(cuda, batch):
+    """Rows of activations against one another: the weight is what the same pass has just computed, whichever launches
+    the pass would take otherwise."""
+    spec = models.mlp_spec(batch)
+    spec["layers"][2] = dict(type="fc", name="Fc2", N=batch)
+    w = models.synthetic_weights(spec, 51)
+    inputs = [torch.from_numpy(models.synthetic_input(spec, s)).to(cuda) for s in (52, 53)]
+    net, plain = (models.Network(spec, w, inputs[0], handover=h) for h in (True, False))
+    for n in (net, plain):
+        n.layers[2].weight_gpu = n.layers[1].output_gpu
+    for i in (0, 1, 0, 0, 0, 1):
+        net.layers[0].input_gpu = plain.layers[0].input_gpu = inputs[i]
+        for l in plain.layers:
+            l.forward()
+        got = net.forward()
+        for l, p in zip(net.layers, plain.layers):
+            assert torch.equal(l.output_gpu, p.output_gpu), l.name
+        assert torch.equal(got, plain.layers[-1].output_gpu)
+    assert ops.gemm_status() == 0

@@ -52,8 +52,12 @@ def _mlp(batch, widths):
     return layers
 
 
+def _calls(layers):
+    return models._Calls(layers).calls
+
+
 def _names(layers):
-    return [name for name, _, _ in models._pass_calls(layers)]
+    return [name for name, _ in _calls(layers)]
 
 
 WIDTHS = (784, 1024, 512, 1024, 10)
@@ -74,4 +78,41 @@ def test_one_launch_follows_every_layers_input(library):
     wide = _ints(100, 2 * layers[1].output_gpu.shape[1])
     layers[1].output_gpu = layers[2].input_gpu = wide[:, :wide.shape[1] // 2]
     with pytest.raises(lib.TcbnnError):
-        models._pass_calls(layers)
+        _calls(layers)
+
+
+def _settled(layers):
+    return [args[-1] for name, args in _calls(layers) if name in ("tcbnn_fc_layer_p", "tcbnn_out_layer_p")]
+
+
+@pytest.mark.parametrize("which", ["weight_gpu", "bn_gpu", "bn_scale_gpu", "first"])
+@pytest.mark.parametrize("batch", [8, 100, 2000])
+def test_parameters_that_the_pass_writes_are_not_read_ahead(library, batch, which):
+    """A layer whose weight or parameters lie in another layer's output has its launches one by one, and nothing is
+    read or expanded before the layers in front have run."""
+    widths = (256, 256, batch, 128, 10) if which == "weight_gpu" else (784, 1024, 512, 1024, 10)
+    layers = _mlp(batch, widths)
+    layers[0].expands = (layers[2],)
+    layers[2].weight_units = layers[2].input_units = layers[1].next_units = torch.zeros(256, dtype=torch.uint8)
+    before = _settled(layers)
+    assert before == ([] if batch == 100 else [1] * 4)
+    if which == "weight_gpu":                            # rows of activations against one another
+        layers[2].weight_gpu = layers[1].output_gpu
+    elif which == "bn_gpu":                              # (the last words of the buffer)
+        layers[2].bn_gpu = layers[1].output_gpu.view(-1)[-512:].view(torch.float32) if batch > 8 else layers[1].output_gpu.view(torch.float32).view(-1)
+    elif which == "bn_scale_gpu":
+        layers[-1].bn_scale_gpu = layers[2].output_gpu.view(torch.float32).view(-1)[3:13]
+    else:
+        layers[1].weight_gpu = layers[0].output_gpu[-8:]
+    assert _settled(layers) == [0] * 4
+    for name, args in _calls(layers):
+        if name == "tcbnn_pack_rows_w":
+            assert args[-1] == 0                         # weights expanded at the start of the pass
+        if name == "tcbnn_fc_layer_p":
+            assert args[-4:-1] == (None, None, None)     # expanded operands
+    layers = _mlp(batch, widths)                         # beside one another in one allocation is not within
+    room = _ints(2 * layers[1].output_gpu.numel() + layers[2].weight_gpu.numel())
+    n = layers[1].output_gpu.numel()
+    layers[1].output_gpu = layers[2].input_gpu = room[:n].view(layers[1].output_gpu.shape)
+    layers[2].weight_gpu = room[n:n + layers[2].weight_gpu.numel()].view(layers[2].weight_gpu.shape)
+    assert _settled(layers) == before
