@@ -273,11 +273,16 @@ def _written(layers):
 
 
 def _reads_what_it_writes(layers):
-    """Whether a pass writes a weight or a parameter of its own (one layer's output as another's weight).  FC layers
-    read or expand theirs ahead of the layers in front; here all then run as they do when called by
-    themselves."""
+    """Whether a pass writes a weight or a parameter of its own (one layer's output as another's weight)."""
     written = _written(layers)
     return any(_meets(t, written) for l in layers for t in l.read_ahead())
+
+
+def _settled(layers):
+    """Whether weights and parameters are complete once the pass's first launch runs, which is when layers behind it
+    may read or expand theirs: the pass begins with an input layer, and writes none of them itself.  Otherwise
+    its layers run as they do when called by themselves."""
+    return layers[0].settles and not _reads_what_it_writes(layers)
 
 
 def _pass_calls(layers, in_pass=True):
@@ -300,7 +305,7 @@ class _Calls:
 
     def __init__(self, layers):
         device = layers[0].output_gpu.device
-        self.in_pass = not _reads_what_it_writes(layers)
+        self.in_pass = _settled(layers)
         while True:
             self.scratch = ops.shared_scratch(device)
             prepared = _pass_calls(layers, self.in_pass)

@@ -85,6 +85,8 @@ class _Layer:
     has just run, and what it handed over besides its bits (expanded operands) is used -- and keeps them
     while no layer's state changes and no tensor moves."""
 
+    settles = False        # an input layer: its launch waits for all before it, whatever kernels those launches were
+
     # The live batch and what follows from it come and go (set_batch); the first layer's input is the caller's.
     _NO_CHANGE = ("live", "input_units", "next_units", "weight_units", "expands")
     live = None
@@ -125,6 +127,7 @@ class _Layer:
 class In128LayerParam(_Layer):
     """param.h:115-222.  fp32 [input_height][input_width] -> bit rows."""
 
+    settles = True
     _NO_CHANGE = _Layer._NO_CHANGE + ("input_gpu",)
 
     def __init__(self, name, input_height, input_width):
@@ -314,6 +317,7 @@ class Out128LayerParam(_Layer):
 class InConv128LayerParam(_Layer):
     """param.h:701-870.  First conv layer on fp32 NCHW images."""
 
+    settles = True
     _NO_CHANGE = _Layer._NO_CHANGE + ("input_gpu",)
 
     def __init__(self, name, input_height, input_width, filter_height, filter_width,

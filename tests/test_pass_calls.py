@@ -116,3 +116,15 @@ def test_parameters_that_the_pass_writes_are_not_read_ahead(library, batch, whic
     layers[1].output_gpu = layers[2].input_gpu = room[:n].view(layers[1].output_gpu.shape)
     layers[2].weight_gpu = room[n:n + layers[2].weight_gpu.numel()].view(layers[2].weight_gpu.shape)
     assert _settled(layers) == before
+
+
+@pytest.mark.parametrize("batch", [8, 2000])
+def test_nothing_is_settled_behind_a_launch_that_need_not_wait(library, batch):
+    """Only an input layer's launch waits for all before it: what a pass over later layers reads may still be written
+    when its second launch starts."""
+    layers = _mlp(batch, WIDTHS)
+    assert _settled(layers) == [1] * 4
+    assert _settled(layers[1:]) == [0] * 4
+    assert _settled(layers[2:]) == [0] * 3
+    layers[1].input_units = layers[1].weight_units = layers[2].weight_units = torch.zeros(256, dtype=torch.uint8)
+    assert all(args[-4:-1] == (None, None, None) for name, args in _calls(layers[1:]) if name == "tcbnn_fc_layer_p")
