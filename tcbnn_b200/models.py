@@ -229,9 +229,28 @@ def _input_facts(layers):
     return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
 
 
+def _span(t):
+    """[first, last) address of a tensor's elements."""
+    at = t.data_ptr()
+    if t.is_contiguous():
+        return at, at + t.nbytes
+    return at, at + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
+
+
+def _meets(t, spans):
+    lo, hi = _span(t)
+    return any(lo < end and start < hi for start, end in spans)
+
+
+def _written(layers):
+    """Where a pass writes: every layer's outputs."""
+    return [_span(t) for l in layers for t in (l.output_gpu, getattr(l, "output_residual_gpu", None)) if t is not None]
+
+
 def _chain_call(layers):
     """The one call that makes an MLP's whole pass (tcbnn_fc_chain), or None where it does not apply: other
-    layers, more rows or wider layers than it takes, or inputs that are not the layer in front's outputs."""
+    layers, more rows or wider layers than it takes, inputs that are not the layer in front's outputs, or buffers that
+    are not all apart (rows are not worked on at the same time)."""
     first, last = layers[0], layers[-1]
     if (type(first).__name__ != "In128LayerParam" or type(last).__name__ != "Out128LayerParam" or
             any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
@@ -251,25 +270,10 @@ def _chain_call(layers):
     shape = first.live, first.input_width, bits.shape[1]
     if not lib.load().tcbnn_fc_chain_fits(chain, len(chain), *shape):
         return None
+    written = _written(layers)
+    if _meets(x, written) or any(_meets(l.output_gpu, written[:i]) for i, l in enumerate(layers)):
+        return None
     return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
-
-
-def _span(t):
-    """[first, last) address of a tensor's elements."""
-    at = t.data_ptr()
-    if t.is_contiguous():
-        return at, at + t.nbytes
-    return at, at + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
-
-
-def _meets(t, spans):
-    lo, hi = _span(t)
-    return any(lo < end and start < hi for start, end in spans)
-
-
-def _written(layers):
-    """Where a pass writes: every layer's outputs."""
-    return [_span(t) for l in layers for t in (l.output_gpu, getattr(l, "output_residual_gpu", None)) if t is not None]
 
 
 def _reads_what_it_writes(layers):
@@ -312,6 +316,7 @@ class _Calls:
             if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
+        self.apart = _written(layers) if prepared[0][0] == "tcbnn_fc_chain" else ()      # from the input, see _chain_call
         self.kept = [t for _, _, keep in prepared for t in keep if t is not layers[0].input_gpu]
 
     def note(self, layers):
@@ -337,6 +342,10 @@ class _Calls:
         return (list(map(bytes, self.descs)) == self.desc_facts and
                 self.settings == lib.settings_generation and self.device == torch._C._cuda_getDevice() and
                 (self.scratch is None or self.scratch is ops.shared_scratch(self.scratch.device)))
+
+    def serves(self, x):
+        """Whether the calls can be made on another input tensor as they are."""
+        return not _meets(x, self.apart)
 
     def moved(self):
         return any(list(map(f, self.tensors)) != g for f, g in zip(_FACTS, self.facts))
@@ -543,9 +552,11 @@ class Network:
         p = last = self._pass
         capturing = torch.cuda.is_current_stream_capturing()
         done = last is not None and last.common.hold(self.layers) and not (capturing and last.common.moved())
-        if done:
-            if p.input != _input_facts(self.layers):
+        if done and p.input != _input_facts(self.layers):
+            done = last.common.serves(self.layers[0].input_gpu)
+            if done:
                 p = self._pass = _Pass(last.common, self.layers, fresh=False)
+        if done:
             if not capturing:
                 if p.seen == 2:
                     p.graph = p.record()

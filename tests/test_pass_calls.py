@@ -128,3 +128,32 @@ def test_nothing_is_settled_behind_a_launch_that_need_not_wait(library, batch):
     assert _settled(layers[2:]) == [0] * 3
     layers[1].input_units = layers[1].weight_units = layers[2].weight_units = torch.zeros(256, dtype=torch.uint8)
     assert all(args[-4:-1] == (None, None, None) for name, args in _calls(layers[1:]) if name == "tcbnn_fc_layer_p")
+
+
+def test_one_launch_only_on_buffers_of_their_own(library):
+    """Rows are worked on at different times in one launch: an input that lies in a buffer of the pass, or two layers'
+    outputs in one, need a launch after the other."""
+    def chained(change):
+        layers = _mlp(100, (512, 512, 512, 512, 512))
+        change(layers)
+        return _names(layers) == ["tcbnn_fc_chain"]
+
+    def shared_output(layers):
+        layers[3].output_gpu = layers[4].input_gpu = layers[1].output_gpu
+
+    def input_is_output(layers):
+        layers[0].input_gpu = layers[4].output_gpu
+
+    def input_in_bits(layers):
+        layers[0].input_gpu = torch.zeros(60000)[:51200].view(100, 512)
+        layers[2].output_gpu = layers[3].input_gpu = layers[0].input_gpu.view(-1)[700:2300].view(torch.int32).view(100, 16)
+
+    assert chained(lambda layers: None)
+    assert not any(chained(f) for f in (shared_output, input_is_output, input_in_bits))
+    # ... and an input that comes later
+    layers = _mlp(100, (512, 512, 512, 512, 512))
+    calls = models._Calls(layers)
+    assert calls.serves(torch.zeros(100, 512)) and not calls.serves(layers[4].output_gpu)
+    layers[0].input_gpu = layers[4].output_gpu
+    other = models._Calls(layers)
+    assert len(other.calls) == 5 and other.serves(layers[4].output_gpu)
