@@ -101,7 +101,8 @@ typedef struct tcbnn_fc_weight {
 } tcbnn_fc_weight;
 /* An MLP in one launch: fp32 rows [M][K] packed to bits[M][ld_words] (tcbnn_pack_rows), hidden layers
  * (tcbnn_fc_layer: p0 = thresholds, p1 unused, out = words) and, last, an output layer (tcbnn_out_layer: p0 = scale,
- * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which.
+ * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which (without
+ * layers: whether any n of them could be taken on so many rows of K).
  * Results are those of the layers called one by one.  Rows are worked on at different times: no buffer that is written
  * (bits, every out) may overlap another one or anything that is read. */
 typedef struct tcbnn_chain_layer {

@@ -496,13 +496,19 @@ __global__ void __launch_bounds__(umma::kChainThreads, 1) k_fc_chain(const __gri
 
 int g_gemm_path = 0;     // 0 automatic, 1 warp-level b1 MMA only
 
-// Fills `a` with the layers and their places in tensor memory; false: not a chain that the kernel takes.
-bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, int sms, umma::ChainArgs* a) {
-    if (g_gemm_path == 1 || n < 1 || n > umma::kChainMaxLayers || M < 64 || K < 1 || ld < 1 || ld * 32 < K) return false;
+// Rows per cluster of a chain of n layers on M rows of K, 0: none that the kernel takes, whatever the layers.
+int chain_rows(int n, int M, int K, int ld, int sms) {
+    if (g_gemm_path == 1 || n < 1 || n > umma::kChainMaxLayers || M < 64 || K < 1 || ld < 1 || ld * 32 < K) return 0;
     // as many clusters as run at once (GPCs hold no whole number of them), the rows dealt out evenly
     const int clusters = sms / umma::kChainCtas * 7 / 8;
-    a->rows = M <= 16 * clusters ? 16 : M <= 32 * clusters ? 32 : 64;
-    if (clusters < 1 || M > 64 * clusters) return false;
+    if (clusters < 1 || M > 64 * clusters) return 0;
+    return M <= 16 * clusters ? 16 : M <= 32 * clusters ? 32 : 64;
+}
+
+// Fills `a` with the layers and their places in tensor memory; false: not a chain that the kernel takes.
+bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, int sms, umma::ChainArgs* a) {
+    a->rows = chain_rows(n, M, K, ld, sms);
+    if (!a->rows) return false;
     a->units = 0;
     a->n = n;
     int first[umma::kChainMaxLayers], end[umma::kChainMaxLayers], next = 0;
@@ -1583,7 +1589,8 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
 int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words) {
     int sms;
     umma::ChainArgs a;
-    if (!layers || sm_count(&sms)) return 0;
+    if (sm_count(&sms)) return 0;
+    if (!layers) return chain_rows(n, M, K, ld_words, sms) ? 1 : 0;
     return chain_plan(layers, n, M, K, ld_words, sms, &a) ? 1 : 0;
 }
 

@@ -256,6 +256,10 @@ def _chain_call(layers):
             any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
         return None
     x, bits = first.input_gpu, first.output_gpu
+    shape = first.live, first.input_width, bits.shape[1]
+    fits = lib.load().tcbnn_fc_chain_fits
+    if not fits(None, len(layers) - 1, *shape):          # (asked first: the list below costs the host 25 us)
+        return None
     keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
     for i, (prev, l) in enumerate(zip(layers, layers[1:])):
         a, w, out = l.input_gpu, l.weight_gpu, l.output_gpu
@@ -267,8 +271,7 @@ def _chain_call(layers):
         chain[i] = lib.ChainLayer(w.data_ptr(), w.shape[1], l.input_width, w.shape[0], p0.data_ptr(), p1.data_ptr() if p1 is not None else None,
                                   out.data_ptr(), out.shape[1])
         keep += [a, w, p0, p1, out]
-    shape = first.live, first.input_width, bits.shape[1]
-    if not lib.load().tcbnn_fc_chain_fits(chain, len(chain), *shape):
+    if not fits(chain, len(chain), *shape):
         return None
     written = _written(layers)
     if _meets(x, written) or any(_meets(l.output_gpu, written[:i]) for i, l in enumerate(layers)):
@@ -316,7 +319,8 @@ class _Calls:
             if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
-        self.apart = _written(layers) if prepared[0][0] == "tcbnn_fc_chain" else ()      # from the input, see _chain_call
+        self.chain = prepared[0][0] == "tcbnn_fc_chain"
+        self.apart = _written(layers) if self.chain else ()                  # from the input, see _chain_call
         self.kept = [t for _, _, keep in prepared for t in keep if t is not layers[0].input_gpu]
 
     def note(self, layers):
@@ -347,6 +351,14 @@ class _Calls:
         """Whether the calls can be made on another input tensor as they are."""
         return not _meets(x, self.apart)
 
+    def first(self, layers):
+        """The first call, on the input that layers[0] now has."""
+        if self.chain:
+            f, args = self.calls[0]
+            return f, (ops._ptr(layers[0].input_gpu), *args[1:])
+        name, args, _ = layers[0]._call_args(self.in_pass)
+        return lib.bound(name), args
+
     def moved(self):
         return any(list(map(f, self.tensors)) != g for f, g in zip(_FACTS, self.facts))
 
@@ -358,8 +370,7 @@ class _Pass:
         """fresh: the calls have just been prepared, on this input."""
         self.common, self.calls = calls, list(calls.calls)
         if not fresh:
-            name, args, _ = _pass_calls(layers, calls.in_pass)[0]
-            self.calls[0] = lib.bound(name), args
+            self.calls[0] = calls.first(layers)
         self.input = _input_facts(layers)
         self.seen, self.graph = 0, None
 

@@ -157,3 +157,40 @@ def test_one_launch_only_on_buffers_of_their_own(library):
     layers[0].input_gpu = layers[4].output_gpu
     other = models._Calls(layers)
     assert len(other.calls) == 5 and other.serves(layers[4].output_gpu)
+
+
+class _Counted:
+    """A layer that counts how often it is looked at."""
+
+    def __init__(self, layer):
+        self.__dict__.update(layer=layer, looks=0)
+
+    def __getattr__(self, name):
+        self.__dict__["looks"] += 1
+        return getattr(self.layer, name)
+
+
+@pytest.mark.parametrize("batch", [8, 100, 2000])
+def test_another_input_tensor_costs_the_first_call_only(library, batch):
+    """A pass on a tensor not seen before exchanges the input's address; nothing is prepared again, and no other layer
+    looked at."""
+    layers = _mlp(batch, WIDTHS)
+    calls = models._Calls(layers)
+    calls.note(layers)
+    watched = layers[:1] + [_Counted(l) for l in layers[1:]]
+    library.asked.clear()
+    layers[0].input_gpu = x = torch.ones(batch, 784)
+    p = models._Pass(calls, watched, fresh=False)
+    assert not library.asked and not any(l.looks for l in watched[1:])
+    assert p.calls[0][1][0] == x.data_ptr() and p.calls[1:] == calls.calls[1:]
+    name, args = calls.calls[0]
+    assert p.calls[0][0] == name and p.calls[0][1][1:4] == args[1:4]
+
+
+def test_rows_are_asked_for_before_a_chain_is_built(library, monkeypatch):
+    """Batches that one launch does not take cost no list of layers."""
+    def build(*a):
+        raise AssertionError("built")
+    layers = _mlp(8, WIDTHS)
+    monkeypatch.setattr(lib, "ChainLayer", build)
+    assert models._chain_call(layers) is None and library.asked == [(None, 8)]
