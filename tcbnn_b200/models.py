@@ -237,9 +237,12 @@ def _span(t):
     return at, at + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
 
 
-def _meets(t, spans):
-    lo, hi = _span(t)
-    return any(lo < end and start < hi for start, end in spans)
+def _meets(span, spans):
+    lo, hi = span
+    for start, end in spans:
+        if lo < end and start < hi:
+            return True
+    return False
 
 
 def _written(layers):
@@ -247,7 +250,7 @@ def _written(layers):
     return [_span(t) for l in layers for t in (l.output_gpu, getattr(l, "output_residual_gpu", None)) if t is not None]
 
 
-def _chain_call(layers):
+def _chain_call(layers, written=None):
     """The one call that makes an MLP's whole pass (tcbnn_fc_chain), or None where it does not apply: other
     layers, more rows or wider layers than it takes, inputs that are not the layer in front's outputs, or buffers that
     are not all apart (rows are not worked on at the same time)."""
@@ -273,28 +276,22 @@ def _chain_call(layers):
         keep += [a, w, p0, p1, out]
     if not fits(chain, len(chain), *shape):
         return None
-    written = _written(layers)
-    if _meets(x, written) or any(_meets(l.output_gpu, written[:i]) for i, l in enumerate(layers)):
+    written = _written(layers) if written is None else written
+    if _meets(_span(x), written) or any(_meets(s, written[:i]) for i, s in enumerate(written)):
         return None
     return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
 
 
-def _reads_what_it_writes(layers):
-    """Whether a pass writes a weight or a parameter of its own (one layer's output as another's weight)."""
-    written = _written(layers)
-    return any(_meets(t, written) for l in layers for t in l.read_ahead())
-
-
-def _settled(layers):
+def _settled(layers, written):
     """Whether weights and parameters are complete once the pass's first launch runs, which is when layers behind it
-    may read or expand theirs: the pass begins with an input layer, and writes none of them itself.  Otherwise
-    its layers run as they do when called by themselves."""
-    return layers[0].settles and not _reads_what_it_writes(layers)
+    may read or expand theirs: the pass begins with an input layer, and writes none of them itself (one layer's
+    output as another's weight).  Otherwise its layers run as they do when called by themselves."""
+    return layers[0].settles and not any(_meets(_span(t), written) for l in layers for t in l.read_ahead())
 
 
-def _pass_calls(layers, in_pass=True):
+def _pass_calls(layers, in_pass, written):
     """[(entry point, arguments, what they point to)] of one pass."""
-    chain = _chain_call(layers) if in_pass else None
+    chain = _chain_call(layers, written) if in_pass else None
     return [chain] if chain else [l._call_args(in_pass) for l in layers]
 
 
@@ -312,15 +309,16 @@ class _Calls:
 
     def __init__(self, layers):
         device = layers[0].output_gpu.device
-        self.in_pass = _settled(layers)
+        written = _written(layers)
+        self.in_pass = _settled(layers, written)
         while True:
             self.scratch = ops.shared_scratch(device)
-            prepared = _pass_calls(layers, self.in_pass)
+            prepared = _pass_calls(layers, self.in_pass, written)
             if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
         self.chain = prepared[0][0] == "tcbnn_fc_chain"
-        self.apart = _written(layers) if self.chain else ()                  # from the input, see _chain_call
+        self.apart = written if self.chain else ()       # from the input, see _chain_call
         self.kept = [t for _, _, keep in prepared for t in keep if t is not layers[0].input_gpu]
 
     def note(self, layers):
@@ -349,7 +347,7 @@ class _Calls:
 
     def serves(self, x):
         """Whether the calls can be made on another input tensor as they are."""
-        return not _meets(x, self.apart)
+        return not self.apart or not _meets(_span(x), self.apart)
 
     def first(self, layers):
         """The first call, on the input that layers[0] now has."""
