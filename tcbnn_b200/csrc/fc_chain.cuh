@@ -267,6 +267,10 @@ __device__ __forceinline__ void fc_chain_cta(const ChainArgs& g, unsigned char* 
     }
     tc_fence_before();
     cluster_sync();                                                      // (no CTA ends while a peer may still store into it)
+    // The MMA warp has waited for all that peers send, unless this CTA gave up: the time of any store passes then.
+    if (*sAbort)
+        for (int i = 0; i < 5000; i++) __nanosleep(20);
+    __syncwarp();
     if (warp == 20) tmem_dealloc(tmem, TM_COLS);
 }
 
