@@ -1046,7 +1046,7 @@ __global__ void __launch_bounds__(256) k_pool_bits(const uint32_t* in, uint32_t*
         const uint32_t* s0 = in + (((long long)n * 2 * P + 2 * y) * 2 * Q + 2 * x) * Ow + w;
         const Words q[4] = {ld_dep((const Words*)s0), ld_dep((const Words*)(s0 + Ow)), ld_dep((const Words*)(s0 + step)),
                             ld_dep((const Words*)(s0 + step + Ow))};
-        uint32_t v[V];
+        alignas(sizeof(Words)) uint32_t v[V];
         const uint32_t* e = reinterpret_cast<const uint32_t*>(q);
 #pragma unroll
         for (int i = 0; i < V; i++) v[i] = e[i] | e[V + i] | e[2 * V + i] | e[3 * V + i];
