@@ -69,6 +69,10 @@ int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes);
  * 16-byte aligned; a_units, w_units: whether it is given expanded operands.  (next_units cost a launch more where K
  * is split.) */
 int tcbnn_gemm_call_launches(int M, int N, int K, int mode, int lda, int ldw, size_t workspace_bytes, int a_units, int w_units);
+/* Which kernels the call takes: 0 = warp-level b1 MMA, 1 = tcgen05 on expanded operands, 2 = tcgen05 on the packed rows
+ * (which has no use for a_units, w_units and the workspace); -1: sizes that no call takes. */
+int tcbnn_gemm_route(const uint32_t* A, const uint32_t* W, int M, int N, int K, int mode, int lda, int ldw, const void* workspace,
+                     size_t workspace_bytes, int a_units, int w_units);
 
 /* GEMM family (the next three entry points): the pad bits of every row of A and of B / W -- the
  * bits past element K up to the leading dimension -- must be zero, as tcbnn_pack_rows,

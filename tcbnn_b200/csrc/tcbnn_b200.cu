@@ -541,6 +541,16 @@ bool gemm_takes_bits(const GemmArgs& g, const GemmUmmaPlan& plan, bool umma_fits
     return bits->cols && bits->us < other;
 }
 
+enum { GEMM_ROUTE_B1 = 0, GEMM_ROUTE_EXPANDED = 1, GEMM_ROUTE_PACKED = 2 };
+struct GemmRoute { int kind; GemmUmmaPlan plan; GemmBitsPlan bits; };
+GemmRoute gemm_route(const GemmArgs& g, const void* workspace, size_t workspace_bytes, const GemmUnits& u, int sms) {
+    GemmRoute r;
+    r.plan = gemm_umma_plan(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0, u.a, u.w);
+    const bool umma_fits = r.plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0;
+    r.kind = gemm_takes_bits(g, r.plan, umma_fits, u, sms, &r.bits) ? GEMM_ROUTE_PACKED : umma_fits ? GEMM_ROUTE_EXPANDED : GEMM_ROUTE_B1;
+    return r;
+}
+
 int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st, const GemmUnits& u = GemmUnits{}) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0) return fail("gemm: M, N, K must be positive");
     if ((g.lda & 1) || (g.ldw & 1)) return fail("gemm: lda and ldw must be even (64-bit loads)");
@@ -550,14 +560,12 @@ int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t s
     if (((uintptr_t)g.A & 7) || ((uintptr_t)g.W & 7)) return fail("gemm: operands must be 8-byte aligned");
     int sms;
     if (sm_count(&sms)) return 1;
-    const GemmUmmaPlan plan = gemm_umma_plan(g.M, g.N, g.K, sms, workspace ? workspace_bytes : 0, u.a, u.w);
-    const bool umma_fits = plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0;
-    GemmBitsPlan bits;
-    if (gemm_takes_bits(g, plan, umma_fits, u, sms, &bits)) return run_gemm_bits(g, bits, u.next, sms, st);
-    if (umma_fits) {
+    const GemmRoute r = gemm_route(g, workspace, workspace_bytes, u, sms);
+    if (r.kind == GEMM_ROUTE_PACKED) return run_gemm_bits(g, r.bits, u.next, sms, st);
+    if (r.kind == GEMM_ROUTE_EXPANDED) {
         // (the epilogue writes the next operand where it finishes the layer itself)
-        const GemmUnits mine{u.a, u.w, plan.splits == 1 ? u.next : nullptr};
-        if (run_gemm_umma(g, plan, workspace, mine, sms, st)) return 1;
+        const GemmUnits mine{u.a, u.w, r.plan.splits == 1 ? u.next : nullptr};
+        if (run_gemm_umma(g, r.plan, workspace, mine, sms, st)) return 1;
         return u.next && !mine.next ? expand_units((const uint32_t*)g.out, g.M, g.ldo, u.next, nullptr, 0, 0, nullptr, g.N, sms, st) : 0;
     }
     if (u.next) {
@@ -1532,18 +1540,32 @@ int tcbnn_gemm_launches(int M, int N, int K, size_t workspace_bytes) {
     return gemm_use_splits(M, N, K, sms, workspace_bytes) > 1 ? 2 : 1;
 }
 
-int tcbnn_gemm_call_launches(int M, int N, int K, int mode, int lda, int ldw, size_t workspace_bytes, int a_units, int w_units) {
+static int call_route(const void* A, const void* W, int M, int N, int K, int mode, int lda, int ldw, const void* workspace,
+                      size_t workspace_bytes, int a_units, int w_units, GemmRoute* r) {
     int sms;
-    if (M <= 0 || N <= 0 || K <= 0 || mode < 0 || mode > 2 || sm_count(&sms)) return 0;
+    if (M <= 0 || N <= 0 || K <= 0 || mode < 0 || mode > 2 || sm_count(&sms)) return 1;
     GemmArgs g = {};
+    g.A = (const uint32_t*)A; g.W = (const uint32_t*)W;
     g.M = M; g.N = N; g.K = K; g.mode = mode; g.lda = lda; g.ldw = ldw;
     const GemmUnits u{a_units ? &g : nullptr, w_units ? &g : nullptr, nullptr};          // (only whether they are there counts)
-    const GemmUmmaPlan plan = gemm_umma_plan(M, N, K, sms, workspace_bytes, u.a, u.w);
-    const bool umma_fits = plan.use && g_gemm_path != 1;
-    GemmBitsPlan bits;
-    if (gemm_takes_bits(g, plan, umma_fits, u, sms, &bits)) return 1;
-    if (umma_fits) return (a_units && w_units ? 1 : 2) + (plan.splits > 1 ? 1 : 0);
+    *r = gemm_route(g, workspace, workspace_bytes, u, sms);
+    return 0;
+}
+
+int tcbnn_gemm_call_launches(int M, int N, int K, int mode, int lda, int ldw, size_t workspace_bytes, int a_units, int w_units) {
+    GemmRoute r;
+    const void* workspace = workspace_bytes ? (const void*)256 : nullptr;                 // (its alignment)
+    int sms;
+    if (call_route(nullptr, nullptr, M, N, K, mode, lda, ldw, workspace, workspace_bytes, a_units, w_units, &r) || sm_count(&sms)) return 0;
+    if (r.kind == GEMM_ROUTE_PACKED) return 1;
+    if (r.kind == GEMM_ROUTE_EXPANDED) return (a_units && w_units ? 1 : 2) + (r.plan.splits > 1 ? 1 : 0);
     return gemm_use_splits(M, N, K, sms, workspace_bytes) > 1 ? 2 : 1;
+}
+
+int tcbnn_gemm_route(const uint32_t* A, const uint32_t* W, int M, int N, int K, int mode, int lda, int ldw, const void* workspace,
+                     size_t workspace_bytes, int a_units, int w_units) {
+    GemmRoute r;
+    return call_route(A, W, M, N, K, mode, lda, ldw, workspace, workspace_bytes, a_units, w_units, &r) ? -1 : r.kind;
 }
 
 int tcbnn_set_gemm_path(int path) {

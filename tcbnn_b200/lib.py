@@ -45,6 +45,7 @@ SIGNATURES = {
     "tcbnn_gemm_workspace_bytes": (_SZ, [_I, _I, _I]),
     "tcbnn_gemm_launches": (_I, [_I, _I, _I, _SZ]),
     "tcbnn_gemm_call_launches": (_I, [_I, _I, _I, _I, _I, _I, _SZ, _I, _I]),
+    "tcbnn_gemm_route": (_I, [_P, _P, _I, _I, _I, _I, _I, _I, _P, _SZ, _I, _I]),
     "tcbnn_set_gemm_path": (_I, [_I]),
     "tcbnn_gemm_status": (_I, [C.POINTER(C.c_int)]),
     "tcbnn_bgemm": (_I, [_P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),

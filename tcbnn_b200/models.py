@@ -490,7 +490,9 @@ class Network:
         for prod, cons in zip(self.layers, self.layers[1:]):
             if type(cons).__name__ != "Fc128LayerParam" or (cons.units_room is None and cons.weight_room is None):
                 continue
-            used = ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0
+            used = (ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0 and
+                    ops.gemm_route(ops.GEMM_BITS, cons.live, cons.input_gpu, cons.weight_gpu, cons.input_width, cons.workspace,
+                                   cons.units_room is not None, cons.weight_room is not None) != ops.GEMM_ON_PACKED)
             if cons.units_room is not None:
                 cons.producer = weakref.ref(prod)         # (prod may hold cons: In128LayerParam.expands)
                 cons.input_units = prod.next_units = cons.units_room if used else None

@@ -103,6 +103,15 @@ def gemm_call_launches(mode, M, A, W, K, workspace, a_units=False, w_units=False
     return _l.load().tcbnn_gemm_call_launches(M, W.shape[0], K, mode, A.shape[1], W.shape[1], nbytes, int(a_units), int(w_units))
 
 
+GEMM_ON_B1, GEMM_ON_EXPANDED, GEMM_ON_PACKED = 0, 1, 2
+
+
+def gemm_route(mode, M, A, W, K, workspace, a_units=False, w_units=False):
+    """Which kernels the call takes on M rows of A and on W (tcbnn_gemm_route)."""
+    return _l.load().tcbnn_gemm_route(_ptr(A), _ptr(W), M, W.shape[0], K, mode, A.shape[1], W.shape[1], *_ws(workspace),
+                                      int(a_units), int(w_units))
+
+
 def fc_units(M, N, K, rows, device):
     """Zeroed room for `rows` expanded rows of K (tcbnn_fc_layer_x) of an FC layer of that shape, or None
     where the layer does not run on the kernel that takes them."""

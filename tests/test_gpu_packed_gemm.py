@@ -208,3 +208,23 @@ def test_a_layers_output_as_the_next_ones_weight(cuda, batch):
             assert torch.equal(l.output_gpu, p.output_gpu), l.name
         assert torch.equal(got, plain.layers[-1].output_gpu)
     assert ops.gemm_status() == 0
+
+
+@pytest.mark.parametrize("batch,live", [(1100, 1100), (1400, 1100), (1400, 1400)])
+def test_operands_are_expanded_for_layers_that_read_them(cuda, batch, live):
+    """In a pass, a layer's operands are laid out expanded where its call takes the kernel that reads them so, and
+    nowhere else."""
+    spec = models.mlp_spec(batch)
+    w, x = models.synthetic_weights(spec, 61), models.synthetic_input(spec, 62)
+    net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
+    net.set_batch(live)
+    for prod, l in zip(net.layers, net.layers[1:-1]):
+        route = ops.gemm_route(ops.GEMM_BITS, live, l.input_gpu, l.weight_gpu, l.input_width, l.workspace, True, True)
+        assert route == (ops.GEMM_ON_PACKED if live == 1100 else ops.GEMM_ON_EXPANDED)
+        expanded = route == ops.GEMM_ON_EXPANDED
+        assert all((u is not None) == expanded for u in (l.input_units, l.weight_units, prod.next_units)), l.name
+        assert (l in net.layers[0].expands) == expanded
+    for l in plain.layers:
+        l.forward()
+    for _ in range(4):
+        assert torch.equal(net.forward()[:live], plain.layers[-1].output_gpu[:live])
