@@ -552,6 +552,12 @@ class Network:
         self._use_units()
         self.live_batch = n
 
+    def kernel_launches(self):
+        """Kernels one pass launches."""
+        if _Calls(self.layers).chain:
+            return 1
+        return sum(l.kernel_launches() if hasattr(l, "kernel_launches") else 1 for l in self.layers)
+
     _pass = None           # of the last call of forward()
 
     def forward(self):
