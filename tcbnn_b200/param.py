@@ -203,7 +203,6 @@ class Fc128LayerParam(_Layer):
         self.bn_gpu = torch.from_numpy(self.bn).to(dev)
         self.output_gpu = torch.zeros((self.input_height, ops.step128_words(N)), dtype=torch.int32, device=dev)
         self.workspace = ops.gemm_workspace(self.input_height, N, K, dev)
-        self.launches = ops.gemm_launches(self.input_height, N, K, self.workspace)
         self.set_input_gpu(prev_layer_gpu)
         return self
 
@@ -289,7 +288,6 @@ class Out128LayerParam(_Layer):
         self.bn_bias_gpu = torch.from_numpy(self.bn_bias).to(dev)
         self.output_gpu = torch.zeros((self.input_height, N), dtype=torch.float32, device=dev)
         self.workspace = ops.gemm_workspace(self.input_height, N, K, dev)
-        self.launches = ops.gemm_launches(self.input_height, N, K, self.workspace)
         self.input_gpu = prev_layer_gpu.reshape(self.input_height, -1)
         return self
 
