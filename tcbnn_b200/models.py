@@ -484,20 +484,21 @@ class Network:
         self._use_units()
 
     def _use_units(self):
-        """Expanded operands are written while the live batch has the layer on the kernel that reads
-        them."""
+        """Expanded operands are written where the live batch has a layer's call on the kernel that reads them so:
+        from 1024 to about 1190 rows, say, a layer of 1024 x 1024 reads packed rows whatever it is given."""
         expands = []
         for prod, cons in zip(self.layers, self.layers[1:]):
             if type(cons).__name__ != "Fc128LayerParam" or (cons.units_room is None and cons.weight_room is None):
                 continue
-            used = (ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0 and
-                    ops.gemm_route(ops.GEMM_BITS, cons.live, cons.input_gpu, cons.weight_gpu, cons.input_width, cons.workspace,
-                                   cons.units_room is not None, cons.weight_room is not None) != ops.GEMM_ON_PACKED)
+            some = ops.fc_units_bytes(cons.live, cons.weight_width, cons.input_width, cons.live) > 0
+            cons.reads_units = some and ops.gemm_route(
+                ops.GEMM_BITS, cons.live, cons.input_gpu, cons.weight_gpu, cons.input_width, cons.workspace,
+                cons.units_room is not None, cons.weight_room is not None) != ops.GEMM_ON_PACKED
             if cons.units_room is not None:
                 cons.producer = weakref.ref(prod)         # (prod may hold cons: In128LayerParam.expands)
-                cons.input_units = prod.next_units = cons.units_room if used else None
-            cons.weight_units = cons.weight_room if used else None
-            if cons.weight_units is not None:
+                cons.input_units = prod.next_units = cons.units_room if cons.reads_units else None
+            cons.weight_units = cons.weight_room if some else None
+            if cons.weight_units is not None and cons.reads_units:
                 expands.append(cons)
         if type(self.layers[0]).__name__ == "In128LayerParam":
             self.layers[0].expands = tuple(expands)

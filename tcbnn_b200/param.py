@@ -88,7 +88,7 @@ class _Layer:
     settles = False        # an input layer: its launch waits for all before it, whatever kernels those launches were
 
     # The live batch and what follows from it come and go (set_batch); the first layer's input is the caller's.
-    _NO_CHANGE = ("live", "input_units", "next_units", "weight_units", "expands")
+    _NO_CHANGE = ("live", "input_units", "next_units", "weight_units", "reads_units", "expands")
     live = None
 
     def __setattr__(self, name, value):
@@ -216,9 +216,10 @@ class Fc128LayerParam(_Layer):
     # Operands in the GEMM kernel's own form (tcbnn_fc_layer_x), wired by models.Network for its passes: this
     # layer's input as its producer writes it (units_room; input_units while the live batch takes that
     # kernel), the next FC layer's input, and room for this layer's weight where the first layer of
-    # every pass expands it (weight_units).  None of them outlives a pass: whoever writes the packed
-    # rows between two passes, by whatever means, is followed.
+    # every pass expands it (weight_units; both only where the call reads them, reads_units).  None of them outlives a
+    # pass: whoever writes the packed rows between two passes, by whatever means, is followed.
     units_room = input_units = next_units = weight_room = weight_units = None
+    reads_units = True
     producer = None        # weak reference to the layer that writes the input
 
     def __setattr__(self, name, value):
@@ -236,7 +237,7 @@ class Fc128LayerParam(_Layer):
 
     def kernel_launches(self):
         # (where a finishing launch computes the bits, the next layer's input is expanded from them)
-        a, w = self.input_units is not None, self.weight_units is not None
+        a, w = self.input_units is not None, self.reads_units and self.weight_units is not None
         n = ops.gemm_call_launches(ops.GEMM_BITS, self.live, self.input_gpu, self.weight_gpu, self.input_width, self.workspace, a, w)
         return n + int(self.next_units is not None and n > (1 if a and w else 2))
 
@@ -245,7 +246,7 @@ class Fc128LayerParam(_Layer):
         ops._need_cuda(a, w, thr)
         prod = self.producer() if self.producer is not None else None
         u = (self.input_units if prod is not None and prod.output_gpu.data_ptr() == a.data_ptr() else None,
-             self.weight_units, self.next_units) if in_pass else (None, None, None)
+             self.weight_units if self.reads_units else None, self.next_units) if in_pass else (None, None, None)
         # (a pass starts with a launch that waits for all before it: its weights are settled)
         return "tcbnn_fc_layer_p", (ops._ptr(a), ops._ptr(w), ops._ptr(thr), self.live, self.input_width, w.shape[0],
                                     a.shape[1], w.shape[1], ops._ptr(out), out.shape[1], *ops._ws(ws),

@@ -77,7 +77,7 @@ def _write(how, t, new):
                      torch.zeros(t.shape[1] * 32, device=t.device), 128, out=t)
 
 
-def _fc_chain(batch=1100):
+def _fc_chain(batch=1400):
     """Two FC layers on the tcgen05 GEMM between an input layer and the output layer, and other weights."""
     spec = models.mlp_spec(batch)
     w = models.synthetic_weights(spec, 31)
@@ -89,10 +89,10 @@ def _fc_chain(batch=1100):
 def test_fc_weights_written_between_passes_count(cuda, how, path):
     """Whatever writes a packed weight between two passes is followed by the next one: on the call paths of
     a network, its replayed passes and the feeder's, whole batches and parts."""
-    spec, w, x, other = _fc_chain(2200 if path == "feeder_parts" else 1100)      # (parts of 1100)
+    spec, w, x, other = _fc_chain(2800 if path == "feeder_parts" else 1400)      # (parts of 1400)
     with torch.inference_mode(how == "inference"):
         net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
-        assert all(l.weight_units is not None for l in net.layers[2:4])
+        assert all(l.weight_units is not None and l.reads_units for l in net.layers[2:4])
         host = torch.from_numpy(x).pin_memory()
         feeder = models.HostFeeder(net)
         if path == "feeder_parts":
