@@ -46,7 +46,8 @@ int tcbnn_pack_inconv_filter(const float* F, int RS, int O, uint32_t* out, void*
  * Passing NULL / 0 is always allowed (warp-level b1 MMA kernel, no split); the buffer must be
  * 256-byte aligned for the tcgen05 kernel to be taken. */
 size_t tcbnn_gemm_workspace_bytes(int M, int N, int K);
-/* Which kernel the GEMM family uses: 0 = automatic, 1 = always the warp-level b1 MMA kernel.
+/* Which kernel the GEMM family uses: 0 = automatic, 1 = always the warp-level b1 MMA kernel, 2 = the tcgen05 kernel that reads
+ * the packed rows wherever it can (16-byte aligned rows, K < 2^22, a plan that applies), 3 = automatic without that one.
  * Process-wide; for tests and measurements.  tcbnn_gemm_status reads the tcgen05 GEMM kernel's
  * device-side status word (synchronises): 0 = fine, 1 = a bounded wait inside it gave up and the
  * results since the last reading are not valid; reading a non-zero status clears it.  No reference
@@ -60,6 +61,9 @@ int tcbnn_gemm_status(int* status);
  * tcbnn_gemm_workspace_bytes AFTER this call fits the forced plan.
  * Process-wide; for tests and measurements.  No reference counterpart. */
 int tcbnn_set_gemm_plan(int pair, int splits);
+/* The same for the kernel on packed rows: `cols` rows of A per tile (32 to 256 in steps of 32), K cut over clusters of
+ * `splits` CTAs (1, 2, 4 or 8; a forced count that leaves a CTA without 512 bits of K does not apply); 0 = automatic. */
+int tcbnn_set_gemm_bits_plan(int cols, int splits);
 /* How many kernels a GEMM-family call of this shape launches at most when given a workspace of that size
  * (warp-level kernel: 1, or 2 with split K; tcgen05 path: 2 = operand expansion and a GEMM that
  * finishes the layer, 3 with split K); for callers that account for their launches.  Operands whose rows are

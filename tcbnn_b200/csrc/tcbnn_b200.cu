@@ -422,6 +422,9 @@ __global__ void __launch_bounds__(umma::kBitsThreads, 1) k_gemm_bits_cluster(umm
     umma::gemm_bits_cta<true>(g, dyn_smem_bits_cluster);
 }
 
+int g_gemm_path = 0;     // tcbnn_set_gemm_path
+int g_gemm_bits_cols = 0, g_gemm_bits_splits = 0;     // tcbnn_set_gemm_bits_plan: 0 = from the model
+
 struct GemmBitsPlan {
     int cols, splits, per;       // rows of A per tile; CTAs of a cluster that share K, stages of each; 0 columns: not a shape for it
     double us;
@@ -436,16 +439,18 @@ GemmBitsPlan gemm_bits_plan(int M, int N, int K, int mode, int sms) {
     p.us = 1e30;
     const int tiles_n = (N + 127) / 128;
     for (int cols = 32; cols <= umma::kBitsMaxCols; cols += 32) {
+        if (g_gemm_bits_cols && cols != g_gemm_bits_cols) continue;
         const long long tiles = (long long)((M + cols - 1) / cols) * tiles_n;
         const double stage = cols <= 64 ? 0.46 : cols <= 96 ? 0.55 : cols <= 128 ? 0.60 : 0.95;
         const double epilogue = mode == GEMM_FC_BITS ? 0.45 + 0.0095 * cols : 0.8 + 0.022 * cols;
         const double waves = tiles <= sms ? 1.0 : (double)((tiles + sms - 1) / sms);
         double us = 3.2 + waves * (stages * stage + epilogue) - (tiles <= sms ? 0.5 : 0.0);
-        if (us < p.us) { p.us = us; p.cols = cols; p.splits = 1; p.per = stages; }
+        if (us < p.us && g_gemm_bits_splits <= 1) { p.us = us; p.cols = cols; p.splits = 1; p.per = stages; }
         // (of clusters of eight fewer fit at once than SMs suggest: 16 took two waves)
-        for (int splits = 2; splits <= 8 && tiles * splits <= (splits == 8 ? sms * 3 / 4 : sms); splits *= 2) {
+        for (int splits = 2; splits <= 8; splits *= 2) {
             const int per = (stages + splits - 1) / splits;
-            if ((splits - 1) * per >= stages) break;
+            if (g_gemm_bits_splits ? g_gemm_bits_splits != splits : tiles * splits > (splits == 8 ? sms * 3 / 4 : sms)) continue;
+            if ((splits - 1) * per >= stages) break;     // (every CTA has a stage)
             us = 3.2 + per * stage + epilogue + 1.1 + 0.015 * cols;
             if (us < p.us) { p.us = us; p.cols = cols; p.splits = splits; p.per = per; }
         }
@@ -494,8 +499,6 @@ __global__ void __launch_bounds__(umma::kChainThreads, 1) k_fc_chain(const __gri
     umma::fc_chain_cta(g, dyn_smem_chain);
 }
 
-int g_gemm_path = 0;     // 0 automatic, 1 warp-level b1 MMA only
-
 // Rows per cluster of a chain of n layers on M rows of K, 0: none that the kernel takes, whatever the layers.
 int chain_rows(int n, int M, int K, int ld, int sms) {
     if (g_gemm_path == 1 || n < 1 || n > umma::kChainMaxLayers || M < 64 || K < 1 || ld < 1 || ld * 32 < K) return 0;
@@ -534,7 +537,9 @@ bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, in
 // drawn at random (1..8192 x 10..8192 x 64..16384), it takes 27, 1.04 to 4.4 times faster but for one that stays
 // the same; seven of the others would have gained 8 to 45 %.
 bool gemm_takes_bits(const GemmArgs& g, const GemmUmmaPlan& plan, bool umma_fits, const GemmUnits& u, int sms, GemmBitsPlan* bits) {
-    if (g_gemm_path != 0 || g_gemm_force_pair >= 0 || g_gemm_force_splits > 0 || ((g.lda | g.ldw) & 3) || (((uintptr_t)g.A | (uintptr_t)g.W) & 15)) return false;
+    if (((g.lda | g.ldw) & 3) || (((uintptr_t)g.A | (uintptr_t)g.W) & 15)) return false;
+    if (g_gemm_path == 2) return *bits = gemm_bits_plan(g.M, g.N, g.K, g.mode, sms), bits->cols > 0;
+    if (g_gemm_path != 0 || g_gemm_force_pair >= 0 || g_gemm_force_splits > 0) return false;
     const double other = umma_fits ? 0.85 * gemm_umma_us(plan, g, u) : 0.9 * gemm_small_us(g);
     if (other <= 3.9) return false;                      // (no plan takes less, and looking for one costs the host half a microsecond)
     *bits = gemm_bits_plan(g.M, g.N, g.K, g.mode, sms);
@@ -1569,8 +1574,17 @@ int tcbnn_gemm_route(const uint32_t* A, const uint32_t* W, int M, int N, int K, 
 }
 
 int tcbnn_set_gemm_path(int path) {
-    if (path < 0 || path > 1) return fail("set_gemm_path: 0 = automatic, 1 = warp-level b1 MMA only");
+    if (path < 0 || path > 3)
+        return fail("set_gemm_path: 0 = automatic, 1 = warp-level b1 MMA only, 2 = packed rows wherever they can be taken, 3 = never");
     g_gemm_path = path;
+    return 0;
+}
+
+int tcbnn_set_gemm_bits_plan(int cols, int splits) {
+    if (cols < 0 || cols > umma::kBitsMaxCols || cols % 32 || splits < 0 || splits > 8 || (splits & (splits - 1)))
+        return fail("set_gemm_bits_plan: cols is 0 or a multiple of 32 up to 256, splits is 0, 1, 2, 4 or 8");
+    g_gemm_bits_cols = cols;
+    g_gemm_bits_splits = splits;
     return 0;
 }
 

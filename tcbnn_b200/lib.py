@@ -66,6 +66,7 @@ SIGNATURES = {
     "tcbnn_conv_layer": (_I, [C.POINTER(ConvDesc), _P, _P, _P, _P, _I, _I, _I, _I, _P, _LL, _P, _I, _P, _P]),
     "tcbnn_set_conv_path": (_I, [_I]),
     "tcbnn_conv_set_trace": (_I, [_P]),
+    "tcbnn_set_gemm_bits_plan": (_I, [_I, _I]),
     "tcbnn_set_gemm_plan": (_I, [_I, _I]),
     "tcbnn_mma_operand_probe": (_I, [_I, _I, _I, C.POINTER(C.c_double)]),
     "tcbnn_bulk_copy_rate": (_I, [_I, _I, _I, _I, _I, C.POINTER(C.c_double), C.POINTER(C.c_double)]),
@@ -134,7 +135,7 @@ def bound(name):
 
 
 # process-wide settings: what is recorded of earlier calls (models.Network) does not outlive a change
-_SETTINGS = {"tcbnn_set_conv_path", "tcbnn_set_gemm_path", "tcbnn_set_gemm_plan", "tcbnn_conv_set_trace"}
+_SETTINGS = {"tcbnn_set_conv_path", "tcbnn_set_gemm_path", "tcbnn_set_gemm_plan", "tcbnn_set_gemm_bits_plan", "tcbnn_conv_set_trace"}
 settings_generation = 0
 
 

@@ -81,7 +81,9 @@ def main():
     ap.add_argument("--chunked", action="store_true",
                     help="conv --residual: int16 residuals in the chunk-major layout (TCBNN_RES_INT16_CHUNKED)")
     ap.add_argument("--mnk", default="1024,1024,4096", help="c1: M,N,K of the bit GEMM")
-    ap.add_argument("--gemm-path", type=int, default=0, help="c1: 0 automatic, 1 warp-level b1 MMA only")
+    ap.add_argument("--gemm-path", type=int, default=0,
+                    help="c1: 0 automatic, 1 warp-level b1 MMA only, 2 packed rows wherever they can be taken, 3 never")
+    ap.add_argument("--gemm-bits-plan", default="0,0", help="c1: cols,splits forced on the GEMM from packed rows (0 automatic)")
     ap.add_argument("--gemm-plan", default="-1,-1", help="c1: pair,splits forced on the tcgen05 GEMM (-1 automatic)")
     ap.add_argument("--trace", action="store_true", help="c1: print the kernel's cycle counters")
     ap.add_argument("--gemm-mode", default="int32", choices=["int32", "fc", "out"],
@@ -139,6 +141,8 @@ def main():
         ops.set_gemm_plan(*(int(v) for v in a.gemm_plan.split(",")))
         ws = ops.gemm_workspace(M, N, K, dev)
         ops.set_gemm_path(a.gemm_path)
+        ops.set_gemm_bits_plan(*(int(v) for v in a.gemm_bits_plan.split(",")))
+        launches = ops.gemm_call_launches(["int32", "fc", "out"].index(a.gemm_mode), M, A, B, K, ws)
         if a.gemm_mode == "int32":
             out = torch.empty((M, N), dtype=torch.int32, device=dev)
             fn = lambda: ops.bgemm(A, B, K, out=out, workspace=ws)
@@ -163,9 +167,9 @@ def main():
             print(json.dumps({"trace": {"loader_wait_free": t[10], "mma_total": t[11], "mma_wait_full": t[12],
                                         "epilogue_wait": t[13], "kblocks": t[14], "epilogue": t[15], "cta_total": t[9]}}))
         ops.set_gemm_path(0)
+        ops.set_gemm_bits_plan()
         work = 2.0 * M * N * K
-        desc = "bit GEMM %dx%dx%d (%s, %d launches)" % (M, N, K, a.gemm_mode,
-                                                       1 if a.gemm_path else ops.gemm_launches(M, N, K, ws))
+        desc = "bit GEMM %dx%dx%d (%s, %d launches)" % (M, N, K, a.gemm_mode, launches)
     elif a.case == "stem":
         Bn = a.batch
         d = ops.conv_desc(Bn, 224, 224, 3, 64, 7, 7, 4, 4)

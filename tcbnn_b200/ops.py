@@ -387,13 +387,18 @@ def mma_peak(kind, warps_per_sm=32, iters=4000):
 
 
 def set_gemm_path(path):
-    """0 = automatic, 1 = warp-level b1 MMA kernel only."""
+    """0 = automatic, 1 = warp-level b1 MMA kernel only, 2 = packed rows wherever they can be taken, 3 = automatic without those."""
     _l.call("tcbnn_set_gemm_path", int(path))
 
 
 def set_gemm_plan(pair=-1, splits=-1):
     """Force the tcgen05 GEMM's tile shape (1: 256 x 256 on two SMs, 0: 128 x 128) and split count; -1 = automatic."""
     _l.call("tcbnn_set_gemm_plan", int(pair), int(splits))
+
+
+def set_gemm_bits_plan(cols=0, splits=0):
+    """Force the tile width and the split of K of the GEMM on packed rows; 0 = automatic."""
+    _l.call("tcbnn_set_gemm_bits_plan", int(cols), int(splits))
 
 
 def gemm_status():

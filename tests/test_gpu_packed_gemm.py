@@ -23,14 +23,16 @@ def _rows(words, ld, offset, cuda):
     return t
 
 
-# M, N, K; extra words per row, words in front of the first row (rows that are not 16-byte aligned go to another kernel)
+# M, N, K; extra words per row, words in front of the first row.  As the library routes them: most of the small ones to the
+# warp-level kernel.
 SHAPES = [
-    (1, 1, 1, 0, 0), (1, 10, 64, 0, 0), (31, 33, 65, 0, 0), (32, 128, 512, 0, 0), (33, 129, 513, 0, 0),       # a tile and one more
+    (1, 1, 1, 0, 0), (1, 10, 64, 0, 0), (31, 33, 65, 0, 0), (32, 128, 512, 0, 0), (33, 129, 513, 0, 0),
     (129, 200, 1000, 0, 0), (256, 128, 511, 0, 0), (257, 300, 449, 0, 0),
-    (640, 4096, 200, 0, 0),            # short K, several tiles per CTA
-    (2000, 3000, 64, 0, 0),            # one 64-bit block
-    (5000, 1000, 1500, 0, 0),          # several tiles per CTA, stages of 512, 512 and 476 bits
-    (70, 130, 2112, 0, 0), (40, 4096, 9216, 0, 0), (3, 1000, 16384, 0, 0),        # K cut over a cluster
+    (640, 4096, 200, 0, 0),            # packed rows: short K, several tiles per CTA
+    (2000, 3000, 64, 0, 0),            # packed rows: one 64-bit block
+    (5000, 1000, 1500, 0, 0),          # packed rows without scratch, integers
+    (70, 130, 2112, 0, 0), (3, 1000, 16384, 0, 0),
+    (40, 4096, 9216, 0, 0),            # packed rows: K cut over clusters
     (33, 140, 700, 4, 0), (33, 140, 700, 2, 0), (33, 140, 700, 0, 2), (300, 1100, 4100, 2, 2),
 ]
 
@@ -59,6 +61,98 @@ def test_gemm_family_on_packed_rows(cuda, M, N, K, pad, offset):
     exact = ref.astype(np.float64) * scale + bias
     np.testing.assert_allclose(out, exact, rtol=2.0 ** -23, atol=2.0 ** -23 * float(np.abs(bias).max()))
     assert ops.gemm_status() == 0
+
+
+# Around one tile of every width, several tiles per CTA, and K of one bit, of one 64-bit block and one bit more, of whole
+# stages of 512 bits and one bit less and more; then K cut over clusters: 8 stages of which the last is short, 16 of which
+# the last has 20 bits, 18, which eight CTAs cannot share, 32.
+TILES = [(1, 1, 1), (31, 33, 65), (32, 128, 512), (33, 129, 513), (97, 40, 64), (129, 200, 1000), (256, 128, 511), (257, 300, 449),
+         (640, 4096, 200), (2000, 3000, 64), (2500, 1000, 1500), (70, 130, 4090), (300, 200, 7700), (40, 1100, 9216), (3, 1000, 16384)]
+
+
+@pytest.mark.parametrize("M,N,K", TILES)
+def test_every_tile_width_and_cluster_on_packed_rows(cuda, M, N, K):
+    """The kernel on packed rows at every tile width and cluster size that K allows, in all three forms, its weight settled
+    or not, and the next layer's expanded operand: against the oracle, and each time on this kernel."""
+    g = util.rng(M + 3 * N + 7 * K + 1)
+    ld = orc.step128_words(K)
+    A, W = (util.mask_row_pad(util.rand_words(g, (r, ld)), K) for r in (M, N))
+    thr = (g.standard_normal(N) * np.sqrt(K)).astype(np.float32)
+    scale, bias = g.standard_normal(N).astype(np.float32), g.standard_normal(N).astype(np.float32)
+    a, w, dthr, dscale, dbias = (_dev(t, cuda) for t in (A, W, thr, scale, bias))
+    ref = orc.bgemm(A, W, K)
+    exact = ref.astype(np.float64) * scale + bias
+    close = dict(rtol=2.0 ** -23, atol=2.0 ** -23 * float(np.abs(bias).max()))
+    words = orc.step128_words(N)
+    signs = np.where(ref >= thr, 1.0, -1.0).astype(np.float32)
+    want = torch.zeros((M, words), dtype=torch.int32, device=cuda)
+    want[:, :(N + 31) // 32] = _dev(util.pm1_to_bits(signs), cuda)
+    ref = torch.from_numpy(ref).to(cuda)
+    # the next layer's operand, as the input layer lays it out
+    units, packed = torch.zeros((-(-M // 128) * -(-N // 64) * 4096,), dtype=torch.uint8, device=cuda), torch.zeros_like(want)
+    x = _dev(signs, cuda)
+    lib.call("tcbnn_pack_rows_x", x.data_ptr(), M, N, words, packed.data_ptr(), units.data_ptr(), ops._stream())
+    assert torch.equal(packed, want)
+    stages, seen = -(-K // 512), set()
+    try:
+        ops.set_gemm_path(2)
+        for cols in range(32, 257, 32):
+            for splits in (1, 2, 4, 8):
+                ops.set_gemm_bits_plan(cols, splits)
+                fits = (splits - 1) * -(-stages // splits) < stages
+                assert (ops.gemm_route(ops.GEMM_INT32, M, a, w, K, None) == ops.GEMM_ON_PACKED) == fits, (cols, splits)
+                if not fits:
+                    continue
+                seen.add(splits)
+                assert torch.equal(ops.bgemm(a, w, K), ref), (cols, splits)
+                for settled in (0, 1):
+                    bits, nxt = torch.zeros_like(want), torch.zeros_like(units)
+                    lib.call("tcbnn_fc_layer_p", a.data_ptr(), w.data_ptr(), dthr.data_ptr(), M, K, N, ld, ld, bits.data_ptr(), words,
+                             None, 0, None, None, nxt.data_ptr(), settled, ops._stream())
+                    assert torch.equal(bits, want) and torch.equal(nxt, units), (cols, splits, settled)
+                    out = torch.zeros((M, N), device=cuda)
+                    lib.call("tcbnn_out_layer_p", a.data_ptr(), w.data_ptr(), dscale.data_ptr(), dbias.data_ptr(), M, K, N, ld, ld,
+                             out.data_ptr(), N, None, 0, settled, ops._stream())
+                    np.testing.assert_allclose(out.cpu().numpy(), exact, err_msg=str((cols, splits, settled)), **close)
+        assert ops.gemm_status() == 0
+        assert seen == {s for s in (1, 2, 4, 8) if (s - 1) * -(-stages // s) < stages}
+    finally:
+        ops.set_gemm_path(0)
+        ops.set_gemm_bits_plan()
+
+
+# extra words per row, words in front of the first row
+@pytest.mark.parametrize("pad,offset,packed", [(0, 0, True), (4, 0, True), (0, 4, True), (2, 0, False), (0, 2, False), (2, 2, False)])
+def test_rows_that_are_not_aligned_are_not_taken_packed(cuda, pad, offset, packed):
+    """A shape that the library takes packed goes to another kernel where a row does not start on 16 bytes, also where packed
+    rows are asked for: of either operand, with the same results."""
+    M, N, K = 640, 2048, 200
+    g = util.rng(5)
+    ld = orc.step128_words(K)
+    A, W = (util.mask_row_pad(util.rand_words(g, (r, ld)), K) for r in (M, N))
+    ref = orc.bgemm(A, W, K)
+    try:
+        for path in (0, 2):
+            ops.set_gemm_path(path)
+            for which in (0, 1):
+                a, w = (_rows(t, ld + (pad if i == which else 0), offset if i == which else 0, cuda) for i, t in enumerate((A, W)))
+                assert (ops.gemm_route(ops.GEMM_INT32, M, a, w, K, None) == ops.GEMM_ON_PACKED) == packed
+                assert np.array_equal(ops.bgemm(a, w, K).cpu().numpy(), ref)
+    finally:
+        ops.set_gemm_path(0)
+    assert ops.gemm_status() == 0
+
+
+def test_shapes_taken_packed_by_estimate(cuda):
+    """Which of some shapes the library takes packed, so that a changed estimate shows."""
+    for M, N, K, mode, room, route in [(640, 4096, 200, ops.GEMM_BITS, True, ops.GEMM_ON_PACKED), (2000, 3000, 64, ops.GEMM_INT32, True, ops.GEMM_ON_PACKED),
+                                       (40, 4096, 9216, ops.GEMM_BITS, True, ops.GEMM_ON_PACKED), (1024, 1024, 4096, ops.GEMM_INT32, True, ops.GEMM_ON_PACKED),
+                                       (1024, 512, 25088, ops.GEMM_BITS, True, ops.GEMM_ON_PACKED), (5000, 1000, 1500, ops.GEMM_INT32, False, ops.GEMM_ON_PACKED),
+                                       (8, 1024, 1024, ops.GEMM_BITS, True, ops.GEMM_ON_B1), (33, 129, 513, ops.GEMM_BITS, True, ops.GEMM_ON_B1),
+                                       (8192, 8192, 8192, ops.GEMM_INT32, True, ops.GEMM_ON_EXPANDED), (2048, 4096, 9216, ops.GEMM_BITS, True, ops.GEMM_ON_EXPANDED)]:
+        ld = orc.step128_words(K)
+        a, w = (torch.empty((r, ld), dtype=torch.int32, device=cuda) for r in (M, N))
+        assert ops.gemm_route(mode, M, a, w, K, ops.gemm_workspace(M, N, K, cuda) if room else None) == route, (M, N, K)
 
 
 WIDTHS = [(784, 1024, 1024, 1024, 10), (100, 130, 1000, 64, 7), (1, 1, 1), (845, 1024, 928, 1000), (513, 40, 1024, 257, 1024),
