@@ -74,6 +74,11 @@ def test_bgemm_fc_out(cuda, M, N, K, split):
                                    (1000, 70, 4100), (2080, 99, 4100)])
 def test_small_gemm_tiles(cuda, M, N, K):
     test_bgemm_fc_out(cuda, M, N, K, False)
+    try:
+        ops.set_gemm_path(1)                                             # (without it some go to the kernel on packed rows)
+        test_bgemm_fc_out(cuda, M, N, K, False)
+    finally:
+        ops.set_gemm_path(0)
 
 
 UMMA_GEMM_CASES = [
@@ -122,7 +127,12 @@ def test_fewer_rows_stay_on_tcgen05_in_the_workspace_of_the_full_batch(cuda, M, 
     got = ops.bgemm(A, W, K, workspace=ws)
     try:
         ops.set_gemm_path(1)
-        assert torch.equal(got, ops.bgemm(A, W, K))
+        want = ops.bgemm(A, W, K)
+        assert torch.equal(got, want)
+        ops.set_gemm_path(3)                                             # (packed rows, which some take, need no scratch)
+        assert ops.gemm_route(ops.GEMM_INT32, live, A, W, K, ws) == ops.GEMM_ON_EXPANDED
+        ws.fill_(-1)
+        assert torch.equal(ops.bgemm(A, W, K, workspace=ws), want)
     finally:
         ops.set_gemm_path(0)
     assert ops.gemm_status() == 0
@@ -171,8 +181,10 @@ def test_gemm_family_on_tcgen05_matches_oracle_and_b1_kernel(cuda, M, N, K, pair
         assert launches in (2, 3)                                        # i.e. the tcgen05 path
         if splits > 0:
             assert launches == (2 if splits == 1 else 3)
-        for path in (0, 1):
+        for path in (0, 3, 1):                                           # 3: without the kernel on packed rows
             ops.set_gemm_path(path)
+            if path == 3:
+                assert all(ops.gemm_route(m, M, dA, dW, K, ws) == ops.GEMM_ON_EXPANDED for m in range(3))
             assert np.array_equal(ops.bgemm(dA, dW, K, workspace=ws).cpu().numpy(), ref), path
             bits = ops.fc_layer(dA, dW, dev(thr, cuda), K, workspace=ws)
             assert np.array_equal(host_u32(bits), orc.fc_layer(A, W, thr, K)), path
