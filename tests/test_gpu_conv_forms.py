@@ -74,18 +74,18 @@ def test_first_layer_sums_of_few_taps(cuda, R, S, O, same):
     spec.release()
 
 
-# B, H, W, C, O, residual in / out.  3x3 layers of more than 256 channels run on pairs of SMs from two tiles per CTA on; the
-# batches give an odd number of tiles (a pair whose second CTA has none), several tiles per pair, one block per stage.
-PAIR_FORMS = [
-    (29, 8, 8, 512, 512, None, None), (60, 7, 7, 512, 256, None, None), (121, 8, 8, 384, 128, None, None), (30, 8, 9, 448, 512, None, None),
-    (29, 8, 8, 512, 512, "int16", "int16"), (33, 8, 8, 512, 512, "int32", "int32"), (29, 8, 8, 512, 512, None, "int32"),
-    (31, 8, 8, 512, 512, "chunked", "chunked"), (31, 8, 8, 512, 512, None, "chunked"), (60, 6, 8, 512, 512, "pooled chunked", "chunked"),
-    (60, 6, 8, 512, 512, "pooled int32", "int32"), (29, 8, 8, 512, 512, "acc", None),
-]
+def _kernels(call):
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
 
 
-@pytest.mark.parametrize("form", PAIR_FORMS)
-def test_wide_layers_on_pairs_of_sms(cuda, form):
+def _check_pairs(cuda, form, images, pairs=True):
+    """A layer three times in a row, compared with the oracle on ranges of its images; pairs: whether it runs on pairs
+    of SMs."""
     B, H, W, C, O, rin, rout = form
     g = util.rng(B + H + W + C + O)
     x = util.rand_words(g, (B, H, W, C // 32))
@@ -94,29 +94,68 @@ def test_wide_layers_on_pairs_of_sms(cuda, form):
     pooled = rin is not None and rin.startswith("pooled")
     kind = rin.replace("pooled ", "") if rin not in (None, "acc") else None
     rc = 256 if pooled else O                            # a pooled residual goes into the first channels
-    res = None
+    res = dres = None
     if kind:
         res = g.integers(-1500, 1501, size=(B, H * (2 if pooled else 1), W * (2 if pooled else 1), rc)).astype(np.int32)
-    eo, er, ea = orc.conv_layer(x, f, thr, C, 3, 3, 1, 1, True, 1, res_in=res, residual_channels=rc if kind else 0, residual_pool=pooled,
-                                save_residual=rout is not None, want_acc=rin == "acc")
-    d = ops.conv_desc(B, H, W, C, O, 3, 3)
-    prep = ops.conv_prepare(d, _dev(f, cuda))
-    dres = None
-    if kind:
         dres = torch.from_numpy(res).to(cuda)
         if kind != "int32":
             dres = dres.to(torch.int16)
         if kind == "chunked":
             dres = ops.nhwc_to_chunked(dres)
+    d = ops.conv_desc(B, H, W, C, O, 3, 3)
+    prep = ops.conv_prepare(d, _dev(f, cuda))
+    dx, dthr = _dev(x, cuda), _dev(thr, cuda)
+
+    def call():
+        return ops.conv_layer(d, dx, prep, dthr, res_in=dres, residual_channels=rc if kind else 0, residual_pool=pooled,
+                              save_residual=rout is not None, want_acc=rin == "acc",
+                              residual_dtype=torch.int32 if rout == "int32" else torch.int16,
+                              res_in_chunked=kind == "chunked", res_out_chunked=rout == "chunked")
+
+    expect = {(lo, hi): orc.conv_layer(x[lo:hi], f, thr, C, 3, 3, 1, 1, True, 1, res_in=None if res is None else res[lo:hi],
+                                       residual_channels=rc if kind else 0, residual_pool=pooled, save_residual=rout is not None,
+                                       want_acc=rin == "acc") for lo, hi in images}
     for _ in range(3):
-        go, gr, ga = ops.conv_layer(d, _dev(x, cuda), prep, _dev(thr, cuda), res_in=dres, residual_channels=rc if kind else 0,
-                                    residual_pool=pooled, save_residual=rout is not None, want_acc=rin == "acc",
-                                    residual_dtype=torch.int32 if rout == "int32" else torch.int16,
-                                    res_in_chunked=kind == "chunked", res_out_chunked=rout == "chunked")
+        go, gr, ga = call()
         assert ops.conv_status(d, prep) == 0
-        assert np.array_equal(_u32(go).reshape(eo.shape), eo)
-        if rout is not None:
-            gr = ops.chunked_to_nhwc(gr) if rout == "chunked" else gr
-            assert np.array_equal(gr.cpu().numpy().astype(np.int32), er)
-        if rin == "acc":
-            assert np.array_equal(ga.cpu().numpy(), ea)
+        if rout == "chunked":
+            gr = ops.chunked_to_nhwc(gr)
+        for (lo, hi), (eo, er, ea) in expect.items():
+            assert np.array_equal(_u32(go[lo:hi]).reshape(eo.shape), eo), (lo, hi)
+            if rout is not None:
+                assert np.array_equal(gr[lo:hi].cpu().numpy().astype(np.int32), er), (lo, hi)
+            if rin == "acc":
+                assert np.array_equal(ga[lo:hi].cpu().numpy(), ea), (lo, hi)
+    assert any("k_conv_umma_pair" in name for name in _kernels(call)) == pairs
+
+
+# B, H, W, C, O, residual in / out.  3x3 layers of more than 256 channels run on pairs of SMs from two tiles per CTA on.  Here
+# a pair has one tile or none: odd numbers of tiles (a pair whose second CTA has none), one block per stage.
+PAIR_FORMS = [
+    (29, 8, 8, 512, 512, None, None), (121, 7, 7, 512, 256, None, None), (121, 8, 8, 384, 128, None, None), (30, 8, 9, 448, 512, None, None),
+    (29, 8, 8, 512, 512, "int16", "int16"), (33, 8, 8, 512, 512, "int32", "int32"), (29, 8, 8, 512, 512, None, "int32"),
+    (31, 8, 8, 512, 512, "chunked", "chunked"), (31, 8, 8, 512, 512, None, "chunked"), (60, 6, 8, 512, 512, "pooled chunked", "chunked"),
+    (60, 6, 8, 512, 512, "pooled int32", "int32"), (29, 8, 8, 512, 512, "acc", None),
+]
+
+
+@pytest.mark.parametrize("form", PAIR_FORMS)
+def test_wide_layers_on_pairs_of_sms(cuda, form):
+    _check_pairs(cuda, form, [(0, form[0])], pairs=form[5] != "pooled int32")
+
+
+# Four or five tiles per pair and an odd number in all (159, 633, 635): both epilogue groups, accumulators handed back to the
+# leader and used again, for each form of epilogue.  Images of 56 pixels a row have the longest second copy (NPOS 248).
+PAIR_RUNS = [
+    (251, 8, 8, 512, 512, None, None), (1000, 8, 8, 384, 128, None, None), (25, 56, 56, 384, 128, None, None),
+    (251, 8, 8, 512, 512, "int16", "int16"), (251, 8, 8, 512, 512, "int32", "int32"), (251, 8, 8, 512, 512, None, "int16"),
+    (251, 8, 8, 512, 512, None, "int32"), (251, 8, 8, 512, 512, "chunked", "chunked"), (251, 8, 8, 512, 512, None, "chunked"),
+    (323, 6, 8, 512, 512, "pooled chunked", "chunked"), (251, 8, 8, 512, 512, "acc", None),
+]
+
+
+@pytest.mark.parametrize("form", PAIR_RUNS)
+def test_wide_layers_with_several_tiles_per_pair(cuda, form):
+    B = form[0]
+    n = 1 if B < 50 else 4
+    _check_pairs(cuda, form, [(0, n), (B // 3, B // 3 + n), (B // 2, B // 2 + n), (B - n, B)])
