@@ -429,6 +429,55 @@ struct GemmBitsPlan {
     int cols, splits, per;       // rows of A per tile; CTAs of a cluster that share K, stages of each; 0 columns: not a shape for it
     double us;
 };
+int configure_gemm_bits() {
+    static bool configured[64] = {false};
+    return configure_once(configured, [] {
+        cudaError_t e = cudaFuncSetAttribute(k_gemm_bits_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(k_gemm_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    });
+}
+
+// Clusters of two, four and eight CTAs, one per SM, that the device runs at once ([1], [2], [3]): fewer than its SMs suggest, as
+// no cluster spans two GPCs and a GPC need not hold a whole number of them (33 of four and 15 of eight on 148 SMs).
+struct ResidentClusters { int of[4]; };
+ResidentClusters resident_clusters(int sms) {
+    ResidentClusters r = {};
+    for (int i = 1; i < 4; i++) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(sms >> i << i));
+        cfg.blockDim = dim3(umma::kBitsThreads);
+        cfg.dynamicSmemBytes = umma::bits_smem_bytes(umma::kBitsMaxCols, 1 << i);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << i;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (configure_gemm_bits() || cudaOccupancyMaxActiveClusters(&r.of[i], k_gemm_bits_cluster, &cfg) != cudaSuccess || r.of[i] < 1) {
+            cudaGetLastError();
+            r.of[i] = sms * 3 / 4 >> i;
+        }
+    }
+    return r;
+}
+const ResidentClusters& gemm_bits_clusters(int sms) {
+    static ResidentClusters cache[64];
+    static std::atomic<bool> known[64];
+    static std::mutex mutex;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev &= 63;
+    if (!known[dev].load(std::memory_order_acquire)) {
+        const ResidentClusters r = resident_clusters(sms);
+        std::lock_guard<std::mutex> lock(mutex);
+        if (!known[dev].load(std::memory_order_relaxed)) {
+            cache[dev] = r;
+            known[dev].store(true, std::memory_order_release);
+        }
+    }
+    return cache[dev];
+}
+
 // The plan with the least time, in us as measured with operands in L2: a stage of 512 bits costs a CTA 0.46 to 0.97 (W's way into
 // tensor memory, then the pipeline's two or three stages), a tile's epilogue by its columns, a cluster the exchange of
 // its sums, a launch 3.2.
@@ -438,6 +487,7 @@ GemmBitsPlan gemm_bits_plan(int M, int N, int K, int mode, int sms) {
     const int stages = (K + 511) / 512;
     p.us = 1e30;
     const int tiles_n = (N + 127) / 128;
+    const ResidentClusters* most = nullptr;
     for (int cols = 32; cols <= umma::kBitsMaxCols; cols += 32) {
         if (g_gemm_bits_cols && cols != g_gemm_bits_cols) continue;
         const long long tiles = (long long)((M + cols - 1) / cols) * tiles_n;
@@ -446,11 +496,17 @@ GemmBitsPlan gemm_bits_plan(int M, int N, int K, int mode, int sms) {
         const double waves = tiles <= sms ? 1.0 : (double)((tiles + sms - 1) / sms);
         double us = 3.2 + waves * (stages * stage + epilogue) - (tiles <= sms ? 0.5 : 0.0);
         if (us < p.us && g_gemm_bits_splits <= 1) { p.us = us; p.cols = cols; p.splits = 1; p.per = stages; }
-        // (of clusters of eight fewer fit at once than SMs suggest: 16 took two waves)
-        for (int splits = 2; splits <= 8; splits *= 2) {
-            const int per = (stages + splits - 1) / splits;
-            if (g_gemm_bits_splits ? g_gemm_bits_splits != splits : tiles * splits > (splits == 8 ? sms * 3 / 4 : sms)) continue;
+        for (int i = 1; i < 4; i++) {
+            const int splits = 1 << i, per = (stages + splits - 1) / splits;
             if ((splits - 1) * per >= stages) break;     // (every CTA has a stage)
+            if (g_gemm_bits_splits) {
+                if (splits != g_gemm_bits_splits) continue;
+            } else {
+                // no second wave of a few: 34 clusters of four take 13.6 us where 33 take 8.1
+                if (tiles * splits > (splits == 8 ? sms * 3 / 4 : sms)) break;
+                if (!most) most = &gemm_bits_clusters(sms);
+                if (tiles > most->of[i]) continue;
+            }
             us = 3.2 + per * stage + epilogue + 1.1 + 0.015 * cols;
             if (us < p.us) { p.us = us; p.cols = cols; p.splits = splits; p.per = per; }
         }
@@ -471,12 +527,7 @@ double gemm_small_us(const GemmArgs& g) {
 }
 
 int run_gemm_bits(const GemmArgs& g, const GemmBitsPlan& p, void* next, int sms, cudaStream_t st) {
-    static bool configured[64] = {false};
-    if (configure_once(configured, [] {
-            cudaError_t e = cudaFuncSetAttribute(k_gemm_bits_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-            return e != cudaSuccess ? e : cudaFuncSetAttribute(k_gemm_bits, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        }))
-        return 1;
+    if (configure_gemm_bits()) return 1;
     umma::GemmBitsArgs a;
     a.A = g.A; a.W = g.W; a.M = g.M; a.N = g.N; a.K = g.K; a.lda = g.lda; a.ldw = g.ldw;
     a.cols = p.cols; a.tiles_m = (g.M + p.cols - 1) / p.cols; a.tiles_n = (g.N + 127) / 128;

@@ -155,6 +155,44 @@ def test_shapes_taken_packed_by_estimate(cuda):
         assert ops.gemm_route(mode, M, a, w, K, ops.gemm_workspace(M, N, K, cuda) if room else None) == route, (M, N, K)
 
 
+def _graph_us(call, n=20):
+    call()
+    torch.cuda.synchronize()
+    graph, best = torch.cuda.CUDAGraph(), 1e9
+    with torch.cuda.stream(torch.cuda.Stream()):
+        graph.capture_begin(capture_error_mode="thread_local")
+        for _ in range(n):
+            call()
+        graph.capture_end()
+    for _ in range(8):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        graph.replay()
+        end.record()
+        end.synchronize()
+        best = min(best, start.elapsed_time(end) * 1e3 / n)
+    return best
+
+
+def test_no_more_clusters_than_run_at_once(cuda):
+    """K is cut over clusters only while all of them run at once: a second wave of a few (34 to 37 of four CTAs) doubled the
+    call's time, 13.7 us where the kernel without clusters takes 9.8.  Within a quarter of that one now."""
+    M, K = 18, 7364
+    ld = orc.step128_words(K)
+    for tiles in range(31, 38):
+        N = 128 * tiles - 1
+        a, w = (torch.zeros((r, ld), dtype=torch.int32, device=cuda) for r in (M, N))
+        thr, out = torch.zeros(N, device=cuda), torch.zeros((M, orc.step128_words(N)), dtype=torch.int32, device=cuda)
+        took = {}
+        try:
+            for path in (0, 3):
+                ops.set_gemm_path(path)
+                took[path] = _graph_us(lambda: ops.fc_layer(a, w, thr, K, out=out))
+        finally:
+            ops.set_gemm_path(0)
+        assert took[0] < 1.25 * took[3], (tiles, took)
+
+
 WIDTHS = [(784, 1024, 1024, 1024, 10), (100, 130, 1000, 64, 7), (1, 1, 1), (845, 1024, 928, 1000), (513, 40, 1024, 257, 1024),
           (1500, 96, 33, 500)]
 
