@@ -229,14 +229,6 @@ def _input_facts(layers):
     return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
 
 
-def _span(t):
-    """[first, last) address of a tensor's elements."""
-    at = t.data_ptr()
-    if t.is_contiguous():
-        return at, at + t.nbytes
-    return at, at + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
-
-
 def _meets(span, spans):
     lo, hi = span
     for start, end in spans:
@@ -245,12 +237,7 @@ def _meets(span, spans):
     return False
 
 
-def _written(layers):
-    """Where a pass writes: every layer's outputs."""
-    return [_span(t) for l in layers for t in (l.output_gpu, getattr(l, "output_residual_gpu", None)) if t is not None]
-
-
-def _chain_call(layers, written=None):
+def _chain_call(layers):
     """The one call that makes an MLP's whole pass (tcbnn_fc_chain), or None where it does not apply: other
     layers, more rows or wider layers than it takes, inputs that are not the layer in front's outputs, or buffers that
     are not all apart (rows are not worked on at the same time)."""
@@ -259,40 +246,48 @@ def _chain_call(layers, written=None):
             any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
         return None
     x, bits = first.input_gpu, first.output_gpu
-    shape = first.live, first.input_width, bits.shape[1]
+    M, K, ld = shape = first.live, first.input_width, bits.shape[1]
     fits = lib.load().tcbnn_fc_chain_fits
     if not fits(None, len(layers) - 1, *shape):          # (asked first: the list below costs the host 25 us)
         return None
     keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
+    at, end = bits.data_ptr(), x.data_ptr()
+    read, written = [(end, end + 4 * M * K)], [(at, at + 4 * M * ld)]
     for i, (prev, l) in enumerate(zip(layers, layers[1:])):
         a, w, out = l.input_gpu, l.weight_gpu, l.output_gpu
         p0, p1 = (l.bn_scale_gpu, l.bn_bias_gpu) if l is last else (l.bn_gpu, None)
-        if (l.live != first.live or a.data_ptr() != prev.output_gpu.data_ptr() or a.shape[1] != prev.output_gpu.shape[1]
-                or l.input_width != prev.output_width):
+        if (l.live != M or a.data_ptr() != at or a.shape[1] != prev.output_gpu.shape[1] or l.input_width != prev.output_width):
             return None
         ops._need_cuda(a, w, p0, p1)
-        chain[i] = lib.ChainLayer(w.data_ptr(), w.shape[1], l.input_width, w.shape[0], p0.data_ptr(), p1.data_ptr() if p1 is not None else None,
-                                  out.data_ptr(), out.shape[1])
+        (N, ldw), ldo = w.shape, out.shape[1]
+        at = out.data_ptr()
+        y = w.data_ptr(), ldw, l.input_width, N, p0.data_ptr(), p1.data_ptr() if p1 is not None else None, at, ldo
+        chain[i] = lib.ChainLayer(*y)
+        read += [(y[0], y[0] + 4 * N * ldw), (y[4], y[4] + 4 * N)]
+        if p1 is not None:
+            read.append((y[5], y[5] + 4 * N))
+        written.append((at, at + 4 * M * ldo))
         keep += [a, w, p0, p1, out]
-    if not fits(chain, len(chain), *shape):
-        return None
-    written = _written(layers) if written is None else written
-    if _meets(_span(x), written) or any(_meets(s, written[:i]) for i, s in enumerate(written)):
+    if not fits(chain, len(chain), *shape) or any(_meets(s, read) or _meets(s, written[:i]) for i, s in enumerate(written)):
         return None
     return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
 
 
-def _settled(layers, written):
-    """Whether weights and parameters are complete once the pass's first launch runs, which is when layers behind it
-    may read or expand theirs: the pass begins with an input layer, and writes none of them itself (one layer's
-    output as another's weight).  Otherwise its layers run as they do when called by themselves."""
-    return layers[0].settles and not any(_meets(_span(t), written) for l in layers for t in l.read_ahead())
-
-
-def _pass_calls(layers, in_pass, written):
-    """[(entry point, arguments, what they point to)] of one pass."""
-    chain = _chain_call(layers, written) if in_pass else None
-    return [chain] if chain else [l._call_args(in_pass) for l in layers]
+def _pass_calls(layers):
+    """[(entry point, arguments, what they point to)] of one pass, and whether it is one in which weights and parameters are
+    complete once the first launch runs, which is when layers behind it may read or expand theirs: it begins
+    with an input layer, and writes none of them itself (one layer's output as another's weight).  Otherwise the
+    layers run as they do when called by themselves."""
+    if layers[0].settles:
+        chain = _chain_call(layers)
+        if chain:
+            return [chain], True
+        calls = [l._call_args(True) for l in layers]
+        memory = [l.memory(args) for l, (_, args, _) in zip(layers, calls)]
+        written = [s for _, spans in memory for s in spans]
+        if not any(_meets(s, written) for ahead, _ in memory for s in ahead):
+            return calls, True
+    return [l._call_args(False) for l in layers], False
 
 
 class _Calls:
@@ -309,16 +304,13 @@ class _Calls:
 
     def __init__(self, layers):
         device = layers[0].output_gpu.device
-        written = _written(layers)
-        self.in_pass = _settled(layers, written)
         while True:
             self.scratch = ops.shared_scratch(device)
-            prepared = _pass_calls(layers, self.in_pass, written)
+            prepared, self.in_pass = _pass_calls(layers)
             if self.scratch is ops.shared_scratch(device):                   # (else replaced by a larger one on the way)
                 break
         self.calls = [(lib.bound(name), args) for name, args, _ in prepared]
         self.chain = prepared[0][0] == "tcbnn_fc_chain"
-        self.apart = written if self.chain else ()       # from the input, see _chain_call
         self.kept = [t for _, _, keep in prepared for t in keep if t is not layers[0].input_gpu]
 
     def note(self, layers):
@@ -347,7 +339,11 @@ class _Calls:
 
     def serves(self, x):
         """Whether the calls can be made on another input tensor as they are."""
-        return not self.apart or not _meets(_span(x), self.apart)
+        if not self.chain:
+            return True
+        _, M, K, ld, bits, chain, _ = self.calls[0][1]                       # (apart from what it writes, see _chain_call)
+        at = x.data_ptr()
+        return not _meets((at, at + 4 * M * K), [(bits, bits + 4 * M * ld)] + [(y.out, y.out + 4 * M * y.ldo) for y in chain])
 
     def first(self, layers):
         """The first call, on the input that layers[0] now has."""

@@ -69,6 +69,14 @@ def _live_chunked(t, live):
     return t.reshape(-1)[:live * P * Q * ch].reshape(live, P, Q, ch)
 
 
+def _span(t):
+    """[first, last) address of a tensor's elements."""
+    at = t.data_ptr()
+    if t.is_contiguous():
+        return at, at + t.nbytes
+    return at, at + (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride()))) * t.element_size()
+
+
 def _dev():
     if not torch.cuda.is_available():
         raise RuntimeError("tcbnn_b200 needs a CUDA device; there is no CPU path")
@@ -104,9 +112,10 @@ class _Layer:
         """Changes with every attribute that is set, except that a live batch that comes back is the same."""
         return self.generation, self.live
 
-    def read_ahead(self):
-        """Tensors that a pass may read before the layers in front have run."""
-        return ()
+    def memory(self, args):
+        """Of a prepared call: [first, last) addresses of what a pass may read before the layers in front have run, and
+        of what the call writes."""
+        return (), tuple(_span(t) for t in (self.output_gpu, getattr(self, "output_residual_gpu", None)) if t is not None)
 
     def forward(self):
         name, args, _ = self._call_args(False)
@@ -167,6 +176,10 @@ class In128LayerParam(_Layer):
         weights = (ops._l.FcWeight * len(layers))(*(l.fc_weight() for l in layers))
         return "tcbnn_pack_rows_w", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out),
                                      ops._ptr(nxt), weights, len(layers)), (x, out, nxt)
+
+    def memory(self, args):
+        _, rows, _, words, out = args[:5]
+        return (), ((out, out + 4 * rows * words),)
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -232,8 +245,9 @@ class Fc128LayerParam(_Layer):
         ops._need_cuda(w)
         return ops._l.FcWeight(w.data_ptr(), w.shape[0], self.input_width, w.shape[1], self.weight_units.data_ptr())
 
-    def read_ahead(self):
-        return self.weight_gpu, self.bn_gpu
+    def memory(self, args):
+        _, w, thr, M, _, N, _, ldw, out, ldo = args[:10]
+        return ((w, w + 4 * N * ldw), (thr, thr + 4 * N)), ((out, out + 4 * M * ldo),)
 
     def kernel_launches(self):
         # (where a finishing launch computes the bits, the next layer's input is expanded from them)
@@ -292,8 +306,9 @@ class Out128LayerParam(_Layer):
         self.input_gpu = prev_layer_gpu.reshape(self.input_height, -1)
         return self
 
-    def read_ahead(self):
-        return self.weight_gpu, self.bn_scale_gpu, self.bn_bias_gpu
+    def memory(self, args):
+        _, w, scale, bias, M, _, N, _, ldw, out, ldo = args[:11]
+        return ((w, w + 4 * N * ldw), (scale, scale + 4 * N), (bias, bias + 4 * N)), ((out, out + 4 * M * ldo),)
 
     def kernel_launches(self):
         return ops.gemm_call_launches(ops.GEMM_AFFINE, self.live, self.input_gpu, self.weight_gpu, self.input_width, self.workspace)
