@@ -229,11 +229,12 @@ def _input_facts(layers):
     return t.data_ptr(), t.size(), t.stride(), t.dtype, t.device
 
 
-def _meets(span, spans):
-    lo, hi = span
-    for start, end in spans:
-        if lo < end and start < hi:
-            return True
+def _meet(some, others):
+    """Whether an address range of one list overlaps one of the other."""
+    for lo, hi in some:
+        for start, end in others:
+            if lo < end and start < hi:
+                return True
     return False
 
 
@@ -242,13 +243,14 @@ def _chain_call(layers):
     layers, more rows or wider layers than it takes, inputs that are not the layer in front's outputs, or buffers that
     are not all apart (rows are not worked on at the same time)."""
     first, last = layers[0], layers[-1]
-    if (type(first).__name__ != "In128LayerParam" or type(last).__name__ != "Out128LayerParam" or
-            any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
+    if type(first).__name__ != "In128LayerParam":
         return None
     x, bits = first.input_gpu, first.output_gpu
     M, K, ld = shape = first.live, first.input_width, bits.shape[1]
     fits = lib.load().tcbnn_fc_chain_fits
     if not fits(None, len(layers) - 1, *shape):          # (asked first: the list below costs the host 25 us)
+        return None
+    if type(last).__name__ != "Out128LayerParam" or any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1]):
         return None
     keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
     at, end = bits.data_ptr(), x.data_ptr()
@@ -268,7 +270,7 @@ def _chain_call(layers):
             read.append((y[5], y[5] + 4 * N))
         written.append((at, at + 4 * M * ldo))
         keep += [a, w, p0, p1, out]
-    if not fits(chain, len(chain), *shape) or any(_meets(s, read) or _meets(s, written[:i]) for i, s in enumerate(written)):
+    if not fits(chain, len(chain), *shape) or _meet(read, written) or any(_meet((s,), written[:i]) for i, s in enumerate(written)):
         return None
     return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
 
@@ -282,10 +284,12 @@ def _pass_calls(layers):
         chain = _chain_call(layers)
         if chain:
             return [chain], True
-        calls = [l._call_args(True) for l in layers]
-        memory = [l.memory(args) for l, (_, args, _) in zip(layers, calls)]
-        written = [s for _, spans in memory for s in spans]
-        if not any(_meets(s, written) for ahead, _ in memory for s in ahead):
+        calls, ahead, written = [], [], []
+        for l in layers:
+            call = l._call_args(True)
+            calls.append(call)
+            l.memory(call[1], ahead, written)
+        if not _meet(ahead, written):
             return calls, True
     return [l._call_args(False) for l in layers], False
 
@@ -343,7 +347,7 @@ class _Calls:
             return True
         _, M, K, ld, bits, chain, _ = self.calls[0][1]                       # (apart from what it writes, see _chain_call)
         at = x.data_ptr()
-        return not _meets((at, at + 4 * M * K), [(bits, bits + 4 * M * ld)] + [(y.out, y.out + 4 * M * y.ldo) for y in chain])
+        return not _meet([(at, at + 4 * M * K)], [(bits, bits + 4 * M * ld)] + [(y.out, y.out + 4 * M * y.ldo) for y in chain])
 
     def first(self, layers):
         """The first call, on the input that layers[0] now has."""

@@ -112,10 +112,10 @@ class _Layer:
         """Changes with every attribute that is set, except that a live batch that comes back is the same."""
         return self.generation, self.live
 
-    def memory(self, args):
-        """Of a prepared call: [first, last) addresses of what a pass may read before the layers in front have run, and
-        of what the call writes."""
-        return (), tuple(_span(t) for t in (self.output_gpu, getattr(self, "output_residual_gpu", None)) if t is not None)
+    def memory(self, args, ahead, written):
+        """Adds, for a prepared call, the [first, last) addresses of what a pass may read before the layers in front have
+        run to `ahead`, of what the call writes to `written`."""
+        written += [_span(t) for t in (self.output_gpu, getattr(self, "output_residual_gpu", None)) if t is not None]
 
     def forward(self):
         name, args, _ = self._call_args(False)
@@ -177,9 +177,8 @@ class In128LayerParam(_Layer):
         return "tcbnn_pack_rows_w", (ops._ptr(x), self.live, self.input_width, out.shape[1], ops._ptr(out),
                                      ops._ptr(nxt), weights, len(layers)), (x, out, nxt)
 
-    def memory(self, args):
-        _, rows, _, words, out = args[:5]
-        return (), ((out, out + 4 * rows * words),)
+    def memory(self, args, ahead, written):
+        written.append((args[4], args[4] + 4 * args[1] * args[3]))
 
     def get_output_gpu(self):
         return self.output_gpu
@@ -245,9 +244,10 @@ class Fc128LayerParam(_Layer):
         ops._need_cuda(w)
         return ops._l.FcWeight(w.data_ptr(), w.shape[0], self.input_width, w.shape[1], self.weight_units.data_ptr())
 
-    def memory(self, args):
-        _, w, thr, M, _, N, _, ldw, out, ldo = args[:10]
-        return ((w, w + 4 * N * ldw), (thr, thr + 4 * N)), ((out, out + 4 * M * ldo),)
+    def memory(self, args, ahead, written):
+        _, w, thr, M, _, N, _, ldw, out, ldo, *_ = args
+        ahead += (w, w + 4 * N * ldw), (thr, thr + 4 * N)
+        written.append((out, out + 4 * M * ldo))
 
     def kernel_launches(self):
         # (where a finishing launch computes the bits, the next layer's input is expanded from them)
@@ -306,9 +306,10 @@ class Out128LayerParam(_Layer):
         self.input_gpu = prev_layer_gpu.reshape(self.input_height, -1)
         return self
 
-    def memory(self, args):
-        _, w, scale, bias, M, _, N, _, ldw, out, ldo = args[:11]
-        return ((w, w + 4 * N * ldw), (scale, scale + 4 * N), (bias, bias + 4 * N)), ((out, out + 4 * M * ldo),)
+    def memory(self, args, ahead, written):
+        _, w, scale, bias, M, _, N, _, ldw, out, ldo, *_ = args
+        ahead += (w, w + 4 * N * ldw), (scale, scale + 4 * N), (bias, bias + 4 * N)
+        written.append((out, out + 4 * M * ldo))
 
     def kernel_launches(self):
         return ops.gemm_call_launches(ops.GEMM_AFFINE, self.live, self.input_gpu, self.weight_gpu, self.input_width, self.workspace)
