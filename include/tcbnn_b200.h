@@ -109,8 +109,8 @@ typedef struct tcbnn_fc_weight {
 } tcbnn_fc_weight;
 /* An MLP in one launch: fp32 rows [M][K] packed to bits[M][ld_words] (tcbnn_pack_rows), hidden layers
  * (tcbnn_fc_layer: p0 = thresholds, p1 unused, out = words) and, last, an output layer (tcbnn_out_layer: p0 = scale,
- * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which (without
- * layers: whether any n of them could be taken on so many rows of K).
+ * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which, and
+ * tcbnn_fc_chain_pays where that is faster than the layers one by one (widths: K, then the outputs of the n layers).
  * Results are those of the layers called one by one.  Rows are worked on at different times: no buffer that is written
  * (bits, every out) may overlap another one or anything that is read. */
 typedef struct tcbnn_chain_layer {
@@ -122,6 +122,7 @@ typedef struct tcbnn_chain_layer {
     int ldo;
 } tcbnn_chain_layer;
 int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words);
+int tcbnn_fc_chain_pays(const int* widths, int n, int M);
 int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n,
                    void* stream);
 size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows);

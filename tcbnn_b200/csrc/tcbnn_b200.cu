@@ -550,18 +550,18 @@ __global__ void __launch_bounds__(umma::kChainThreads, 1) k_fc_chain(const __gri
     umma::fc_chain_cta(g, dyn_smem_chain);
 }
 
-// Rows per cluster of a chain of n layers on M rows of K, 0: none that the kernel takes, whatever the layers.
-int chain_rows(int n, int M, int K, int ld, int sms) {
-    if (g_gemm_path == 1 || n < 1 || n > umma::kChainMaxLayers || M < 64 || K < 1 || ld < 1 || ld * 32 < K) return 0;
-    // as many clusters as run at once (GPCs hold no whole number of them), the rows dealt out evenly
+// Rows per cluster of a chain on M rows: as many clusters as run at once (GPCs hold no whole number of them), the rows
+// dealt out evenly; 0: more than one launch takes, or fewer.
+int chain_rows(int M, int sms) {
     const int clusters = sms / umma::kChainCtas * 7 / 8;
-    if (clusters < 1 || M > 64 * clusters) return 0;
+    if (clusters < 1 || M < 64 || M > 64 * clusters) return 0;
     return M <= 16 * clusters ? 16 : M <= 32 * clusters ? 32 : 64;
 }
 
 // Fills `a` with the layers and their places in tensor memory; false: not a chain that the kernel takes.
 bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, int sms, umma::ChainArgs* a) {
-    a->rows = chain_rows(n, M, K, ld, sms);
+    if (g_gemm_path == 1 || n < 1 || n > umma::kChainMaxLayers || K < 1 || ld < 1 || ld * 32 < K) return false;
+    a->rows = chain_rows(M, sms);
     if (!a->rows) return false;
     a->units = 0;
     a->n = n;
@@ -605,6 +605,30 @@ GemmRoute gemm_route(const GemmArgs& g, const void* workspace, size_t workspace_
     const bool umma_fits = r.plan.use && g_gemm_path != 1 && workspace && ((uintptr_t)workspace & 255) == 0;
     r.kind = gemm_takes_bits(g, r.plan, umma_fits, u, sms, &r.bits) ? GEMM_ROUTE_PACKED : umma_fits ? GEMM_ROUTE_EXPANDED : GEMM_ROUTE_B1;
     return r;
+}
+
+// Whether one launch is faster than input packing and n layers one by one: widths[0] inputs, then every layer's
+// outputs.  In one launch, us of GPU time (to 8 % on 200 shapes, replayed): set-up and the input's way by its columns and the
+// rows of a cluster, then each layer's hand-over and MMAs; one by one the calls' estimates, which in a pass come out
+// up to a third too long, as weights are read ahead: hence the tenth.  Of those 200, 64 to 960 rows, 71 were faster in one launch;
+// this takes 74, none more than 1.09 slower than its layers, and leaves none that would gain more than 1.12.  Taken whatever the
+// layers, as it was, 784 -> 10 on 700 rows took 10.7 us against 4.1, 784 -> 128 -> 10 13.1 against 7.2, 784 -> 1024 -> 1024 -> 1024 -> 10
+// 19.4 against 15.8 (and 12.5 against 14.8 on 100 rows, which it still takes).
+bool chain_pays(const int* widths, int n, int M, int sms) {
+    const int rows = chain_rows(M, sms);
+    if (!rows || n > umma::kChainMaxLayers || g_gemm_path == 1) return false;
+    double chain = 5.75 + 0.0095 * rows, layers = 2.0;
+    for (int l = 0; l < n; l++) {
+        if (widths[l] < 1 || widths[l + 1] < 1) return false;
+        const int kb = (widths[l] + 63) / 64;
+        chain += l ? 0.75 + 0.0203 * rows + 0.05 * kb : 0.0055 * rows * kb;
+        GemmArgs g = {};                                 // (rows of whole 16 bytes, and scratch enough)
+        g.M = M; g.N = widths[l + 1]; g.K = widths[l]; g.mode = l + 1 == n ? GEMM_OUT_AFFINE : GEMM_FC_BITS;
+        g.lda = g.ldw = (g.K + 127) / 128 * 4;
+        const GemmRoute r = gemm_route(g, (const void*)256, SIZE_MAX, GemmUnits{}, sms);
+        layers += r.kind == GEMM_ROUTE_PACKED ? r.bits.us : r.kind == GEMM_ROUTE_EXPANDED ? gemm_umma_us(r.plan, g, GemmUnits{}) : gemm_small_us(g);
+    }
+    return chain < 0.9 * layers;
 }
 
 int run_gemm(GemmArgs g, void* workspace, size_t workspace_bytes, cudaStream_t st, const GemmUnits& u = GemmUnits{}) {
@@ -1676,9 +1700,14 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
 int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words) {
     int sms;
     umma::ChainArgs a;
-    if (sm_count(&sms)) return 0;
-    if (!layers) return chain_rows(n, M, K, ld_words, sms) ? 1 : 0;
+    if (!layers || sm_count(&sms)) return 0;
     return chain_plan(layers, n, M, K, ld_words, sms, &a) ? 1 : 0;
+}
+
+int tcbnn_fc_chain_pays(const int* widths, int n, int M) {
+    int sms;
+    if (!widths || n < 1 || sm_count(&sms)) return 0;
+    return chain_pays(widths, n, M, sms) ? 1 : 0;
 }
 
 int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n, void* stream) {

@@ -16,6 +16,7 @@ Topologies follow the reference drivers, not the textbook networks:
   * alexnet, vgg16_imagenet : alexnet.cu:141-178, imagenet_vgg.cu:217-280 (11x11 / 5x5 filters,
                  192 / 384 channels, pooled layers at 224 x 224).
 """
+import ctypes as C
 import weakref
 
 import numpy as np
@@ -238,20 +239,25 @@ def _meet(some, others):
     return False
 
 
+def _chain_pays(layers):
+    """Whether an MLP's pass in one call is worth asking for: on so many rows, and faster than its layers' calls
+    (tcbnn_fc_chain_pays)."""
+    if type(layers[0]).__name__ != "In128LayerParam" or len(layers) < 2:
+        return False
+    widths = [l.output_width for l in layers]
+    return lib.load().tcbnn_fc_chain_pays((C.c_int * len(widths))(*widths), len(widths) - 1, layers[0].live)
+
+
 def _chain_call(layers):
     """The one call that makes an MLP's whole pass (tcbnn_fc_chain), or None where it does not apply: other
     layers, more rows or wider layers than it takes, inputs that are not the layer in front's outputs, or buffers that
     are not all apart (rows are not worked on at the same time)."""
     first, last = layers[0], layers[-1]
-    if type(first).__name__ != "In128LayerParam":
+    if (type(first).__name__ != "In128LayerParam" or type(last).__name__ != "Out128LayerParam" or
+            any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
         return None
     x, bits = first.input_gpu, first.output_gpu
     M, K, ld = shape = first.live, first.input_width, bits.shape[1]
-    fits = lib.load().tcbnn_fc_chain_fits
-    if not fits(None, len(layers) - 1, *shape):          # (asked first: the list below costs the host 25 us)
-        return None
-    if type(last).__name__ != "Out128LayerParam" or any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1]):
-        return None
     keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
     at, end = bits.data_ptr(), x.data_ptr()
     read, written = [(end, end + 4 * M * K)], [(at, at + 4 * M * ld)]
@@ -270,7 +276,7 @@ def _chain_call(layers):
             read.append((y[5], y[5] + 4 * N))
         written.append((at, at + 4 * M * ldo))
         keep += [a, w, p0, p1, out]
-    if not fits(chain, len(chain), *shape) or _meet(read, written) or any(_meet((s,), written[:i]) for i, s in enumerate(written)):
+    if not lib.load().tcbnn_fc_chain_fits(chain, len(chain), *shape) or _meet(read, written) or any(_meet((s,), written[:i]) for i, s in enumerate(written)):
         return None
     return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
 
@@ -281,7 +287,7 @@ def _pass_calls(layers):
     with an input layer, and writes none of them itself (one layer's output as another's weight).  Otherwise the
     layers run as they do when called by themselves."""
     if layers[0].settles:
-        chain = _chain_call(layers)
+        chain = _chain_call(layers) if _chain_pays(layers) else None       # (its list costs the host 25 us)
         if chain:
             return [chain], True
         calls, ahead, written = [], [], []

@@ -201,7 +201,8 @@ WIDTHS = [(784, 1024, 1024, 1024, 10), (100, 130, 1000, 64, 7), (1, 1, 1), (845,
 @pytest.mark.parametrize("batch", [64, 65, 241, 300, 700])
 def test_mlp_in_one_launch_is_its_layers_one_by_one(cuda, widths, batch):
     """Every layer's packed output and the logits of a pass in one launch, for 16, 32 and 64 rows per cluster with
-    a ragged last one, against the same layers called by themselves."""
+    a ragged last one, against the same layers called by themselves; and of the network's own passes, which
+    take the one launch or the layers' by what is faster."""
     spec = models.mlp_spec(batch, widths[0], 1, widths[-1])
     spec["layers"] = [spec["layers"][0]] + [dict(type="fc", name="Fc%d" % i, N=n) for i, n in enumerate(widths[1:-1])] + [spec["layers"][-1]]
     w, x = models.synthetic_weights(spec, 41), models.synthetic_input(spec, 42)
@@ -209,22 +210,44 @@ def test_mlp_in_one_launch_is_its_layers_one_by_one(cuda, widths, batch):
     assert models._chain_call(net.layers) is not None
     for l in plain.layers:
         l.forward()
-    for _ in range(4):                                               # (a replayed graph by the last)
+    def one_launch():
+        name, args, _ = models._chain_call(net.layers)
+        lib.call(name, *args, ops._stream())
+    for one_pass in [one_launch] + [net.forward] * 4:                # (a replayed graph by the last)
         for l in net.layers:
             l.output_gpu.fill_(0)
-        net.forward()
+        one_pass()
         for l, p in zip(net.layers, plain.layers):
             assert torch.equal(l.output_gpu, p.output_gpu), l.name
     for fewer in (batch - 1, batch // 3):                            # in the same buffers; in one launch or, below 64 rows, in several
-        for l in net.layers:
-            l.output_gpu.fill_(0)
         net.set_batch(fewer)
         assert (models._chain_call(net.layers) is not None) == (fewer >= 64)
-        net.forward()
-        for l, p in zip(net.layers, plain.layers):
-            assert torch.equal(l.output_gpu[:fewer], p.output_gpu[:fewer]), l.name
-            assert not l.output_gpu[fewer:].any()
+        for one_pass in ([one_launch] if fewer >= 64 else []) + [net.forward]:
+            for l in net.layers:
+                l.output_gpu.fill_(0)
+            one_pass()
+            for l, p in zip(net.layers, plain.layers):
+                assert torch.equal(l.output_gpu[:fewer], p.output_gpu[:fewer]), l.name
+                assert not l.output_gpu[fewer:].any()
     assert ops.gemm_status() == 0
+
+
+@pytest.mark.parametrize("widths", [(784, 10), (784, 128, 10), (200, 1000), (784, 1024, 1000), (784, 1024, 1024, 1024, 10)])
+def test_one_launch_is_not_taken_where_the_layers_are_faster(cuda, widths):
+    """A pass takes no longer than its layers' launches, within a fifth: in one launch 784 -> 10 took 10.7 us on 700 rows where
+    the two layers take 4.1."""
+    for batch in (64, 200, 400, 700, 960):
+        spec = models.mlp_spec(batch, widths[0], 1, widths[-1])
+        spec["layers"] = [spec["layers"][0]] + [dict(type="fc", name="Fc%d" % i, N=n) for i, n in enumerate(widths[1:-1])] + [spec["layers"][-1]]
+        net = models.Network(spec, models.synthetic_weights(spec, 73), models.synthetic_input(spec, 74))
+        own = models._Pass(models._Calls(net.layers), net.layers)
+        layers = [(lib.bound(name), args) for name, args, _ in (l._call_args(True) for l in net.layers)]
+
+        def one_by_one():
+            for f, args in layers:
+                assert f(*args, ops._stream()) == 0
+        took, theirs = _graph_us(own.run), _graph_us(one_by_one)
+        assert took < 1.2 * theirs, (batch, took, theirs, own.common.chain)
 
 
 def test_mlp_with_another_layers_input_is_not_one_launch(cuda):
@@ -246,14 +269,14 @@ def test_mlp_with_another_layers_input_is_not_one_launch(cuda):
 @pytest.mark.parametrize("graph", [False, True])
 def test_mlp_in_one_launch_follows_a_layers_input_given_another_storage(cuda, graph):
     """The rows of a layer's input tensor are exchanged in place, behind passes that are replayed by then."""
-    spec = models.mlp_spec(72)
+    spec = models.mlp_spec(200)
     w, x = models.synthetic_weights(spec, 47), models.synthetic_input(spec, 48)
     net, plain = models.Network(spec, w, x), models.Network(spec, w, x, handover=False)
     one_pass = net.forward_graph if graph else net.forward
-    net.layers[2].input_gpu = net.layers[1].output_gpu.view(72, -1)
+    net.layers[2].input_gpu = net.layers[1].output_gpu.view(200, -1)
     for _ in range(4):
         want = one_pass().clone()
-    assert models._chain_call(net.layers) is not None
+    assert models._Calls(net.layers).chain
     other = torch.randint(-2 ** 31, 2 ** 31, net.layers[2].input_gpu.shape, dtype=torch.int64, device=cuda).to(torch.int32)
     net.layers[2].input_gpu.data = other
     plain.layers[2].set_input_gpu(other)

@@ -13,8 +13,12 @@ class _Library:
         self.asked = []
 
     def tcbnn_fc_chain_fits(self, layers, n, M, K, ld):
-        self.asked.append((None if layers is None else n, M))
+        self.asked.append("fits")
         return int(64 <= M <= 960)
+
+    def tcbnn_fc_chain_pays(self, widths, n, M):
+        self.asked.append((list(widths), n, M))
+        return int(64 <= M <= 960 and widths[n] < 1000)
 
 
 @pytest.fixture
@@ -187,10 +191,12 @@ def test_another_input_tensor_costs_the_first_call_only(library, batch):
     assert p.calls[0][0] == name and p.calls[0][1][1:4] == args[1:4]
 
 
-def test_rows_are_asked_for_before_a_chain_is_built(library, monkeypatch):
-    """Batches that one launch does not take cost no list of layers."""
+@pytest.mark.parametrize("batch,widths", [(8, WIDTHS), (100, (784, 1000))])
+def test_what_does_not_pay_in_one_launch_is_not_built(library, monkeypatch, batch, widths):
+    """Passes that one launch would make slower, or cannot take, cost no list of layers."""
     def build(*a):
         raise AssertionError("built")
-    layers = _mlp(8, WIDTHS)
+    layers = _mlp(batch, widths)
     monkeypatch.setattr(lib, "ChainLayer", build)
-    assert models._chain_call(layers) is None and library.asked == [(None, 8)]
+    assert _names(layers)[0] == "tcbnn_pack_rows_w"
+    assert library.asked == [(list(widths), len(widths) - 1, batch)]
