@@ -1035,10 +1035,12 @@ int launch_conv_umma_pair_epi(umma::ConvWsArgs& a, unsigned grid, size_t smem, c
 // 3x3 stride-1 layers whose filter block of 128 output channels does not fit beside a patch ring (more than 256
 // input channels) run 64 channels at a time, at 54 clocks per MMA where 32 are math: the operands' way out of
 // shared memory.  A pair of SMs shares a block of 128, half each, for 256 positions: 68 clocks per SM for twice the
-// work.  Taken where it has fewer clocks left, which leaves out launches of a tile or two per CTA: *use = the plan
-// applies.  7 x 7 x 512 at batch 1024 68.5 -> 43.9 us, with int16 residuals 73.1 -> 46.8; 8 x 8 x 512 pooled 85.9 -> 54.5;
-// 28 x 28 x 512 at batch 32 29.6 -> 21.5.  Not with a pooled int32 residual, where n-tiles get uneven shares of the GPU
-// (8 x 8 x 512 at batch 201: 31.4 us, 37.1 in pairs).
+// work.  Taken where it has fewer clocks left: *use = the plan applies.  7 x 7 x 512 at batch 1024 68.5 -> 43.9 us, with int16
+// residuals 73.1 -> 46.8; 8 x 8 x 512 pooled 85.9 -> 54.5; 28 x 28 x 512 at batch 32 29.6 -> 21.5.
+// Left out: layers with residuals or sums whose pairs have one tile each, where a CTA's single epilogue of 128 columns is exposed
+// and two of 64 were not (14 x 14 x 512 -> 512 at batch 20, int32 saved: 13.2 us, 14.7 in pairs; 3 to 4 % on average over
+// 27 shapes, plain layers gain 3); and pooled int32 residuals, where n-tiles get uneven shares of the GPU (of eleven shapes eight
+// slower in pairs, by 3 to 21 %, three the same to 2 %: 8 x 8 x 512 at batch 201 33.9 us, 38.3 in pairs, 7 x 7 x 512 at 1024 123, 148).
 int launch_conv_umma_pair(umma::ConvWsArgs& a, int sms, cudaStream_t st, bool* use) {
     *use = false;
     const long long mtiles = (a.NV + 127) / 128;
@@ -1046,8 +1048,9 @@ int launch_conv_umma_pair(umma::ConvWsArgs& a, int sms, cudaStream_t st, bool* u
     if ((a.res_in && a.residual_pool && a.res_in_bytes == 4) || a.O % 128 || a.R != 3 || a.S != 3 || a.stride != 1 || ntiles > sms / 2 || tail <= 0 || tail > 256) return 0;
     const long long per = sms / 2 / ntiles, per64 = sms / (a.O / 64);
     if (per64 < 1) return 0;
-    const double pairs = (double)(((mtiles + 1) / 2 + per - 1) / per) * 68.0, singles = (double)((mtiles + per64 - 1) / per64) * 54.0;
-    if (pairs >= singles) return 0;
+    const bool plain = !a.res_in && !a.res_out && !a.acc_out;
+    const long long rounds = ((mtiles + 1) / 2 + per - 1) / per;           // tiles per pair
+    if ((double)rounds * 68.0 >= (double)((mtiles + per64 - 1) / per64) * 54.0 || (rounds < 2 && !plain)) return 0;
     const long long elements = a.pre_positions * (a.C / 32) * 2;
     if (elements >= (1LL << 31)) return 0;
     size_t smem = 0;
@@ -1067,7 +1070,6 @@ int launch_conv_umma_pair(umma::ConvWsArgs& a, int sms, cudaStream_t st, bool* u
     a.nt_heavy = 0; a.per_heavy = a.per_light = 0;
     const long long want = (mtiles + 1) / 2;
     const unsigned grid = (unsigned)((per < want ? per : want) * ntiles * 2);
-    const bool plain = !a.res_in && !a.res_out && !a.acc_out;
     const bool chunked = !a.acc_out && (!a.res_in || a.res_in_chunked) && (!a.res_out || a.res_out_chunked);
     if (plain) return launch_conv_umma_pair_epi<umma::kEpiTile>(a, grid, smem, head, rest, st);
     if (chunked) return launch_conv_umma_pair_epi<umma::kEpiTilePool>(a, grid, smem, head, rest, st);

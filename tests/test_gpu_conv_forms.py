@@ -129,8 +129,9 @@ def _check_pairs(cuda, form, images, pairs=True):
     assert any("k_conv_umma_pair" in name for name in _kernels(call)) == pairs
 
 
-# B, H, W, C, O, residual in / out.  3x3 layers of more than 256 channels run on pairs of SMs from two tiles per CTA on.  Here
-# a pair has one tile or none: odd numbers of tiles (a pair whose second CTA has none), one block per stage.
+# B, H, W, C, O, residual in / out.  3x3 layers of more than 256 channels run on pairs of SMs from two tiles per CTA on, with
+# residuals or sums from two tiles per pair.  Here a pair has one tile or none: odd numbers of tiles (a pair whose second
+# CTA has none), one block per stage.
 PAIR_FORMS = [
     (29, 8, 8, 512, 512, None, None), (121, 7, 7, 512, 256, None, None), (121, 8, 8, 384, 128, None, None), (30, 8, 9, 448, 512, None, None),
     (29, 8, 8, 512, 512, "int16", "int16"), (33, 8, 8, 512, 512, "int32", "int32"), (29, 8, 8, 512, 512, None, "int32"),
@@ -141,7 +142,7 @@ PAIR_FORMS = [
 
 @pytest.mark.parametrize("form", PAIR_FORMS)
 def test_wide_layers_on_pairs_of_sms(cuda, form):
-    _check_pairs(cuda, form, [(0, form[0])], pairs=form[5] != "pooled int32")
+    _check_pairs(cuda, form, [(0, form[0])], pairs=form[5] is None and form[6] is None)
 
 
 # Four or five tiles per pair and an odd number in all (159, 633, 635): both epilogue groups, accumulators handed back to the
@@ -150,7 +151,7 @@ PAIR_RUNS = [
     (251, 8, 8, 512, 512, None, None), (1000, 8, 8, 384, 128, None, None), (25, 56, 56, 384, 128, None, None),
     (251, 8, 8, 512, 512, "int16", "int16"), (251, 8, 8, 512, 512, "int32", "int32"), (251, 8, 8, 512, 512, None, "int16"),
     (251, 8, 8, 512, 512, None, "int32"), (251, 8, 8, 512, 512, "chunked", "chunked"), (251, 8, 8, 512, 512, None, "chunked"),
-    (323, 6, 8, 512, 512, "pooled chunked", "chunked"), (251, 8, 8, 512, 512, "acc", None),
+    (323, 6, 8, 512, 512, "pooled chunked", "chunked"), (251, 8, 8, 512, 512, "acc", None), (323, 6, 8, 512, 512, "pooled int32", "int32"),
 ]
 
 
@@ -158,4 +159,4 @@ PAIR_RUNS = [
 def test_wide_layers_with_several_tiles_per_pair(cuda, form):
     B = form[0]
     n = 1 if B < 50 else 4
-    _check_pairs(cuda, form, [(0, n), (B // 3, B // 3 + n), (B // 2, B // 2 + n), (B - n, B)])
+    _check_pairs(cuda, form, [(0, n), (B // 3, B // 3 + n), (B // 2, B // 2 + n), (B - n, B)], pairs=form[5] != "pooled int32")
