@@ -15,7 +15,10 @@ namespace tcbnn {
 
 constexpr int kSmallMaxWarps = 16;
 
-template <int MT, int NTL>
+// AHEAD: W and the parameters are loaded in front of A, ahead of the wait for the launch in front where they are settled
+// (GemmArgs::settled): a layer of an MLP on a few rows is a chain of latencies.  What it holds meanwhile costs the 16 x 8
+// tile eight registers and one block of four per SM, see launch_gemm_small.
+template <int MT, int NTL, bool AHEAD>
 __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int NW, int* red) {
     constexpr int R = 16 * MT, C = 8 * NTL, CP = C + 2;    // rows, columns, padded row of the exchange buffer
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -39,11 +42,11 @@ __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int 
     for (int i = 0; i < 2 * MT; i++) sa[i] = 0;
 #pragma unroll
     for (int j = 0; j < NTL; j++) pw[j] = 0;
-    // Launched as a programmatic dependent.  A layer of an MLP on a few rows is a chain of latencies, and of these
-    // the weights' and the parameters' are out of the way where they may be read ahead of the wait (settled).
     const uint32_t* wp[NTL];
+    auto rows_w = [&] {
 #pragma unroll
-    for (int j = 0; j < NTL; j++) wp[j] = g.W + (size_t)min(n0 + j * 8 + gq, g.N - 1) * g.ldw;
+        for (int j = 0; j < NTL; j++) wp[j] = g.W + (size_t)min(n0 + j * 8 + gq, g.N - 1) * g.ldw;
+    };
     // U steps' loads are issued together: the chain is the loads' latency
     constexpr int U = MT * NTL >= 4 ? 2 : 4;
     uint2 b[U][NTL];
@@ -65,13 +68,17 @@ __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int 
             if (g.mode == GEMM_OUT_AFFINE) f1 = ld_dep(g.p1 + col);
         }
     };
-    if (g.settled) { load_w(kw * 4); load_p(0); }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!g.settled) { load_w(kw * 4); load_p(0); }
+    if constexpr (AHEAD) {
+        rows_w();
+        if (g.settled) { load_w(kw * 4); load_p(0); }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // launched as a programmatic dependent
+    if (AHEAD && !g.settled) { load_w(kw * 4); load_p(0); }
     if (n0 < g.N) {
         const uint32_t* ap[2 * MT];
 #pragma unroll
         for (int i = 0; i < 2 * MT; i++) ap[i] = g.A + (size_t)min(m0 + i * 8 + gq, g.M - 1) * g.lda;   // rows past M re-read row M-1
+        if constexpr (!AHEAD) rows_w();
         for (int kb = kw * 4; kb < KP; kb += KW * 4 * U) {
             uint2 a[U][2 * MT];
 #pragma unroll
@@ -79,8 +86,12 @@ __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int 
                 const int kp = kb + u * KW * 4 + t;
 #pragma unroll
                 for (int i = 0; i < 2 * MT; i++) a[u][i] = kp < KP ? ld_dep(reinterpret_cast<const uint2*>(ap[i] + 2 * kp)) : make_uint2(0u, 0u);
+                if constexpr (!AHEAD) {
+#pragma unroll
+                    for (int j = 0; j < NTL; j++) b[u][j] = kp < KP ? ld_dep(reinterpret_cast<const uint2*>(wp[j] + 2 * kp)) : make_uint2(0u, 0u);
+                }
             }
-            if (kb != kw * 4) load_w(kb);
+            if (AHEAD && kb != kw * 4) load_w(kb);
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 if (kb + u * KW * 4 >= KP) break;
@@ -120,19 +131,19 @@ __device__ __forceinline__ void gemm_small_block(const GemmArgs& g, int KW, int 
         const int row = m0 + r, col = nb + w * C + c;
         const bool in = e < total && row < g.M && col < ncols;
         int v = g.K;
-        if (e0 > 0) load_p(e0);
+        if (AHEAD && e0 > 0) load_p(e0);
         if (in)
             for (int k = 0; k < KW; k++) v += red[(size_t)(w * KW + k) * R * CP + r * CP + c];
         if (g.mode == GEMM_FC_BITS) {
             // (float)K - 2*(float)c >= thr[n]  (kernel.cuh:210-213)
-            const bool bit = in && col < g.N && (float)v >= f0;
+            const bool bit = in && col < g.N && (float)v >= (AHEAD ? f0 : ld_dep(g.p0 + col));
             const uint32_t bits = __ballot_sync(0xffffffffu, bit) >> (lane & 24);
             if (in && (lane & 7) == 0)                     // column `col` at bit 31 - col % 32 of its word
                 reinterpret_cast<unsigned char*>((uint32_t*)g.out + (size_t)row * g.ldo + (col >> 5))[3 - ((col & 31) >> 3)] =
                     (unsigned char)(__brev(bits & 0xFFu) >> 24);
         } else if (in) {
             if (g.mode == GEMM_INT32) ((int32_t*)g.out)[(size_t)row * g.ldo + col] = v;
-            else ((float*)g.out)[(size_t)row * g.ldo + col] = __fmaf_rn((float)v, f0, f1);
+            else ((float*)g.out)[(size_t)row * g.ldo + col] = AHEAD ? __fmaf_rn((float)v, f0, f1) : __fmaf_rn((float)v, ld_dep(g.p0 + col), ld_dep(g.p1 + col));
         }
     }
 }

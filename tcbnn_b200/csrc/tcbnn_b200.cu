@@ -158,10 +158,10 @@ __global__ void k_conv_prepare(const uint32_t* fbits, int O, int R, int S, int C
     conv_prepare(fbits, O, R, S, Cw, W_in, KP, wq, ktab, pwt, pwtot);
 }
 
-template <int MT, int NTL>
+template <int MT, int NTL, bool AHEAD>
 __global__ void __launch_bounds__(32 * kSmallMaxWarps, 1) k_gemm_small(GemmArgs g, int KW, int NW) {
     extern __shared__ __align__(16) int small_red[];
-    gemm_small_block<MT, NTL>(g, KW, NW, small_red);
+    gemm_small_block<MT, NTL, AHEAD>(g, KW, NW, small_red);
 }
 
 int launch_check(const char* what) {
@@ -200,11 +200,15 @@ int gemm_use_splits(int M, int N, int K, int sms, size_t workspace_bytes) {
 
 // ---- b1 GEMM of small problems (bgemm_small.cuh) -------------------------------------------
 template <int MT, int NTL>
-int launch_gemm_small(const GemmArgs& g, int KW, int NW, cudaStream_t st) {
+int launch_gemm_small(const GemmArgs& g, int KW, int NW, int sms, cudaStream_t st) {
     const int ncols = g.mode == GEMM_FC_BITS ? (g.N + 31) & ~31 : g.N;
     const long long grid = (long long)((g.M + 16 * MT - 1) / (16 * MT)) * ((ncols + 8 * NTL * NW - 1) / (8 * NTL * NW));
     if (grid >= (1LL << 31)) return fail("gemm: more than 2^31 tiles");
-    const cudaError_t e = launch_dependent(k_gemm_small<MT, NTL>, (unsigned)grid, 32 * KW * NW,
+    // Weights first while the blocks of that form are all resident: 28 warps per SM of the 16 x 8 tile (70 registers), 32 of the other.
+    // 8 x 1024 -> 1024 alone 2.5 -> 2.1 us, 109 x 355 -> 1237 4.2 -> 3.4; but 546 x 1182 -> 114, 525 blocks of 8, 3.6 -> 4.4, 7955 x 369 -> 19
+    // 4.0 -> 4.9, 2 x 17231 -> 1542, 193 blocks of 16, 7.3 -> 8.5.
+    const bool ahead = MT > 1 || grid <= (long long)(28 / (KW * NW)) * sms;
+    const cudaError_t e = launch_dependent(ahead ? k_gemm_small<MT, NTL, true> : k_gemm_small<MT, NTL, false>, (unsigned)grid, 32 * KW * NW,
                                            (size_t)KW * NW * 16 * MT * (8 * NTL + 2) * 4, st, g, KW, NW);
     if (e != cudaSuccess) return fail("gemm (small): %s", cudaGetErrorString(e));
     return 0;
@@ -226,10 +230,10 @@ int run_gemm_small(const GemmArgs& g, int sms, cudaStream_t st) {
     const int NWmax = 8 / KW > 1 ? 8 / KW : 1;
     auto groups = [&](int cols) { int nw = 1; while (nw < NWmax && nw * cols < g.N) nw *= 2; return nw; };
     const double per_sm = 12.0 / steps;
-    if (g.M <= 16 || tiles(32, 16) < (per_sm > 1.0 ? per_sm : 1.0) * sms) return launch_gemm_small<1, 1>(g, KW, groups(8), st);
+    if (g.M <= 16 || tiles(32, 16) < (per_sm > 1.0 ? per_sm : 1.0) * sms) return launch_gemm_small<1, 1>(g, KW, groups(8), sms, st);
     if (KW > 8) KW = 8;
-    if (g.N <= 16 || tiles(32, 32) < (per_sm > 1.5 ? per_sm : 1.5) * sms) return launch_gemm_small<2, 2>(g, KW, groups(16), st);
-    return launch_gemm_small<2, 4>(g, KW, groups(32), st);
+    if (g.N <= 16 || tiles(32, 32) < (per_sm > 1.5 ? per_sm : 1.5) * sms) return launch_gemm_small<2, 2>(g, KW, groups(16), sms, st);
+    return launch_gemm_small<2, 4>(g, KW, groups(32), sms, st);
 }
 
 // ---- tcgen05 bit GEMM (bgemm_umma.cuh) -----------------------------------------------------

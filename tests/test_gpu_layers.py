@@ -81,6 +81,31 @@ def test_small_gemm_tiles(cuda, M, N, K):
         ops.set_gemm_path(0)
 
 
+# 16 x 8 tiles: 444 blocks of eight warps, one block row more, 444 of one, 148 and 149 of sixteen.  Up to these (148 SMs) the weights
+# are loaded first, settled ones ahead of the wait for the launch in front.
+@pytest.mark.parametrize("M,N,K", [(592, 96, 2100), (593, 96, 2100), (1184, 300, 130), (1185, 300, 130), (16, 1184, 16400), (15, 1185, 16400), (3, 5, 70)])
+def test_small_gemm_weights_first(cuda, M, N, K):
+    g = util.rng(M + N + K)
+    ld = orc.step128_words(K)
+    A, W = (util.mask_row_pad(util.rand_words(g, (r, ld)), K) for r in (M, N))
+    thr, scale, bias = ((g.standard_normal(N) * k).astype(np.float32) for k in (np.sqrt(K), 1, 1))
+    a, w, dthr, dscale, dbias = (dev(t, cuda) for t in (A, W, thr, scale, bias))
+    words = orc.step128_words(N)
+    try:
+        ops.set_gemm_path(1)
+        assert np.array_equal(ops.bgemm(a, w, K).cpu().numpy(), orc.bgemm(A, W, K))
+        for settled in (0, 1):
+            bits, out = torch.zeros((M, words), dtype=torch.int32, device=cuda), torch.zeros((M, N), device=cuda)
+            lib.call("tcbnn_fc_layer_p", a.data_ptr(), w.data_ptr(), dthr.data_ptr(), M, K, N, ld, ld, bits.data_ptr(), words, None, 0, None, None,
+                     None, settled, ops._stream())
+            assert np.array_equal(host_u32(bits), orc.fc_layer(A, W, thr, K)), settled
+            lib.call("tcbnn_out_layer_p", a.data_ptr(), w.data_ptr(), dscale.data_ptr(), dbias.data_ptr(), M, K, N, ld, ld, out.data_ptr(), N, None, 0,
+                     settled, ops._stream())
+            np.testing.assert_allclose(out.cpu().numpy(), orc.out_layer(A, W, scale, bias, K), rtol=1e-5, atol=1e-5)
+    finally:
+        ops.set_gemm_path(0)
+
+
 UMMA_GEMM_CASES = [
     # M, N, K, pair, splits: large enough for the tcgen05 GEMM (M*N*K >= 2^30, less with a forced
     # plan), ragged on purpose.
