@@ -94,7 +94,7 @@ int tcbnn_fc_layer(const uint32_t* A, const uint32_t* W, const float* thr, int M
                    size_t workspace_bytes, void* stream);
 /* The same with operands in the tcgen05 GEMM's own form ("units": +-1 4-bit values in 4 KB blocks), for
  * chains of FC layers.  tcbnn_fc_units_bytes(M, N, K, rows) is the size of `rows` rows of K for a layer of
- * that shape, 0 where the layer does not run on that kernel.  w_units: the layer's weight as
+ * that shape, 0 where no call of it runs on that kernel (tcbnn_gemm_route: whether a given one does).  w_units: the layer's weight as
  * tcbnn_fc_expand_weight or tcbnn_pack_rows_w last expanded it -- a weight written to since has to be expanded
  * again; a_units: its input, written by the producer; next_units: the output
  * bits also go there, as the next layer's a_units (K = N here).  tcbnn_pack_rows_x writes the first
@@ -107,24 +107,6 @@ typedef struct tcbnn_fc_weight {
     int N, K, ldw;
     void* units;            /* tcbnn_fc_units_bytes(M, N, K, N) */
 } tcbnn_fc_weight;
-/* An MLP in one launch: fp32 rows [M][K] packed to bits[M][ld_words] (tcbnn_pack_rows), hidden layers
- * (tcbnn_fc_layer: p0 = thresholds, p1 unused, out = words) and, last, an output layer (tcbnn_out_layer: p0 = scale,
- * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which, and
- * tcbnn_fc_chain_pays where that is faster than the layers one by one (widths: K, then the outputs of the n layers).
- * Results are those of the layers called one by one.  Rows are worked on at different times: no buffer that is written
- * (bits, every out) may overlap another one or anything that is read. */
-typedef struct tcbnn_chain_layer {
-    const uint32_t* W;      /* [N][ldw] packed weight, 16-byte aligned, ldw a multiple of 4 */
-    int ldw, K, N;
-    const float* p0;
-    const float* p1;
-    void* out;              /* [M][ldo] */
-    int ldo;
-} tcbnn_chain_layer;
-int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words);
-int tcbnn_fc_chain_pays(const int* widths, int n, int M);
-int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n,
-                   void* stream);
 size_t tcbnn_fc_units_bytes(int M, int N, int K, int rows);
 int tcbnn_fc_expand_weight(const uint32_t* W, int N, int K, int ldw, void* units, void* stream);
 int tcbnn_fc_layer_x(const uint32_t* A, const uint32_t* W, const float* thr, int M, int K, int N,
@@ -143,6 +125,24 @@ int tcbnn_pack_rows_x(const float* x, int rows, int cols, int ld_words, uint32_t
                       void* stream);
 int tcbnn_pack_rows_w(const float* x, int rows, int cols, int ld_words, uint32_t* out, void* units,
                       const tcbnn_fc_weight* weights, int n_weights, void* stream);
+/* An MLP in one launch: fp32 rows [M][K] packed to bits[M][ld_words] (tcbnn_pack_rows), hidden layers
+ * (tcbnn_fc_layer: p0 = thresholds, p1 unused, out = words) and, last, an output layer (tcbnn_out_layer: p0 = scale,
+ * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which, and
+ * tcbnn_fc_chain_pays where that is faster than the layers one by one (widths: K, then the outputs of the n layers).
+ * Results are those of the layers called one by one.  Rows are worked on at different times: no buffer that is written
+ * (bits, every out) may overlap another one or anything that is read. */
+typedef struct tcbnn_chain_layer {
+    const uint32_t* W;      /* [N][ldw] packed weight, 16-byte aligned, ldw a multiple of 4 */
+    int ldw, K, N;
+    const float* p0;
+    const float* p1;
+    void* out;              /* [M][ldo] */
+    int ldo;
+} tcbnn_chain_layer;
+int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words);
+int tcbnn_fc_chain_pays(const int* widths, int n, int M);
+int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n,
+                   void* stream);
 /* Output layer: out[m][n] = fma((float)(K - 2*popc), scale[n], bias[n]), fp32 [M][ldo].
  * Out128LayerFMT, kernel.cuh:230-280. */
 int tcbnn_out_layer(const uint32_t* A, const uint32_t* W, const float* scale, const float* bias,

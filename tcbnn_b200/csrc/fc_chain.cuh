@@ -5,10 +5,11 @@
 // bgemm_bits.cuh) while the input is still being packed and earlier layers run; a layer is a dozen MMAs of 128 x
 // rows x 64, and its bits go as +-1 nibbles straight into the shared memory of the eight CTAs (st.async: the store
 // itself completes the receiver's barrier, no release at cluster scope, which takes over a thousand clocks).
-// What bounds it is that chain, whatever the rows: 9000 clocks until the input has arrived everywhere, then 2700 a layer (16
-// MMAs at 80, reading the accumulator, turning its bits, sending them).  MLP 784 -> 1024 -> 1024 -> 1024 -> 10, five
-// launches against this one: 128 rows 16.2 -> 12.2 us, 300 25.7 -> 14.9, 777 46.2 -> 19.1; 64 rows 11.4 and 12.2 of GPU time, of
-// which one launch costs a replayed pass less; 8 rows 8.5 and 11.7, so fewer than 64 stay with the layers' launches.
+// What bounds it is that chain: 9000 clocks until the input has arrived everywhere (more of a cluster's rows, more of it), then 2700 a layer
+// (16 MMAs at 80, reading the accumulator, turning its bits, sending them).  GPU time of MLP 784 -> 1024 -> 1024 -> 1024 -> 10, five
+// launches (weights read ahead, operands packed) against this one: 64 rows 11.4 and 12.2 us, 100 14.8 and 12.5, 200 14.1 and 12.6, 400
+// 15.6 and 15.2, 700 15.8 and 19.4; 256 -> 256 -> 256 -> 256 -> 10 on 100 rows 11.9 and 9.9; 784 -> 10 on 700 4.1 and 10.7.  So it is taken
+// where an estimate of both says so (chain_pays).  8 rows 8.5 and 11.7: fewer than 64 stay with the layers' launches.
 //
 //   warps 0-3   epilogue of a quarter of the CTA's outputs each
 //   warps 4-19  W expanders : four groups of four, 512 bits of K in turn

@@ -137,7 +137,8 @@ inline std::string generate_source(const SpecHandle& h, const std::vector<unsign
     // accumulator shows (it gets its zero there); a channel whose first term is a -v sums the
     // negatives of everything and is turned round at the end; and channels that agree in both terms share
     // their sum until the third (28 different ones of 64 are usual): 136 adds less of 640 for 64 channels of a
-    // 3 x 3 filter, 3 % of a 7 x 7 one.
+    // 3 x 3 filter, 3 % of a 7 x 7 one.  Measured on the first layers of the networks here, 44 calls, 0.986 of the time
+    // without it on average, between 0.90 and 1.06: what the assembler makes of a given filter differs by more than the adds.
     auto minus = [&](int tap, int o) { return codes[(size_t)tap * Oall + OB + o] < 4; };       // pattern k is minus pattern 7 - k
     auto mag = [&](int tap, int o) { const int k = codes[(size_t)tap * Oall + OB + o]; return k >= 4 ? k : 7 - k; };
     std::vector<int> shared(O, 0);                       // the channel's sum of two taps

@@ -588,9 +588,11 @@ bool chain_plan(const tcbnn_chain_layer* layers, int n, int M, int K, int ld, in
     return umma::chain_smem_bytes(a->rows, a->units) <= 200 * 1024;
 }
 
-// The packed operands' kernel where the estimates say that it is clearly the faster one.  Of 83 shapes, most of them
-// drawn at random (1..8192 x 10..8192 x 64..16384), it takes 27, 1.04 to 4.4 times faster but for one that stays
-// the same; seven of the others would have gained 8 to 45 %.
+// The packed operands' kernel where the estimates say that it is clearly the faster one: by 15 % of what the expanded operands'
+// kernel takes, 10 % of the b1 kernel's.  Of 109 shapes drawn at random (1..8192 x 10..8192 x 64..16384, threshold bits) it takes 28, up
+// to 8.8 times faster, none more than 4 % slower; seven of the others would have gained, by 8 to 31 %.  What refuses them: the two
+// allowances, on estimates that are short for the b1 kernel on 30 to 400 rows and less than 600 of K (37 x 546 -> 2927 4.8 us, estimated
+// 3.9, here 4.0) and for the expanded operands' at one or two tiles per CTA (499 x 983 -> 5693 8.5 us, 7.6, 6.5).
 bool gemm_takes_bits(const GemmArgs& g, const GemmUmmaPlan& plan, bool umma_fits, const GemmUnits& u, int sms, GemmBitsPlan* bits) {
     if (((g.lda | g.ldw) & 3) || (((uintptr_t)g.A | (uintptr_t)g.W) & 15)) return false;
     if (g_gemm_path == 2) return *bits = gemm_bits_plan(g.M, g.N, g.K, g.mode, sms), bits->cols > 0;
