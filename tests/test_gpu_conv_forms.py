@@ -74,15 +74,6 @@ def test_first_layer_sums_of_few_taps(cuda, R, S, O, same):
     spec.release()
 
 
-def _kernels(call):
-    from torch.profiler import ProfilerActivity, profile
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        call()
-        torch.cuda.synchronize()
-    return [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA]
-
-
 def _check_pairs(cuda, form, images, pairs=True):
     """A layer three times in a row, compared with the oracle on ranges of its images; pairs: whether it runs on pairs
     of SMs."""
@@ -126,7 +117,7 @@ def _check_pairs(cuda, form, images, pairs=True):
                 assert np.array_equal(gr[lo:hi].cpu().numpy().astype(np.int32), er), (lo, hi)
             if rin == "acc":
                 assert np.array_equal(ga[lo:hi].cpu().numpy(), ea), (lo, hi)
-    assert any("k_conv_umma_pair" in name for name in _kernels(call)) == pairs
+    assert any("k_conv_umma_pair" in name for name in util.kernels_launched(call)) == pairs
 
 
 # B, H, W, C, O, residual in / out.  3x3 layers of more than 256 channels run on pairs of SMs from two tiles per CTA on, with

@@ -286,26 +286,17 @@ def test_mlp_in_one_launch_follows_a_layers_input_given_another_storage(cuda, gr
     assert torch.equal(got, plain.layers[-1].output_gpu) and not torch.equal(got, want)
 
 
-def _kernels_seen(call):
-    from torch.profiler import ProfilerActivity, profile
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        call()
-        torch.cuda.synchronize()
-    return sum(e.device_type == torch.autograd.DeviceType.CUDA and ("k_" in e.name or "tcbnn_spec" in e.name) for e in p.events())
-
-
 @pytest.mark.parametrize("which,batch", [("mlp", 8), ("mlp", 100), ("mlp", 1100), ("mlp", 2000), ("vgg_cifar", 70), ("resnet_cifar", 33)])
 def test_launches_a_pass_makes(cuda, which, batch):
-    """What a network says a pass launches, against the kernels the profiler sees."""
+    """What a network says a pass launches, against the kernels in a graph of it."""
     spec = getattr(models, which + "_spec")(batch)
     net = models.Network(spec, models.synthetic_weights(spec, 71), models.synthetic_input(spec, 72))
     net.forward()
-    assert _kernels_seen(net.forward) == net.kernel_launches()
+    assert len(util.kernels_launched(net.forward)) == net.kernel_launches()
 
 
 def test_launches_a_call_makes(cuda):
-    """What a layer says it launches, against the kernels the profiler sees."""
+    """What a layer says it launches, against the kernels in a graph of its call."""
     for M, N, K in [(32, 128, 256), (1024, 1000, 512), (2048, 4096, 9216), (200, 256, 200000)]:
         ld = orc.step128_words(K)
         a, w = (torch.zeros((r, ld), dtype=torch.int32, device=cuda) for r in (M, N))
@@ -313,7 +304,7 @@ def test_launches_a_call_makes(cuda):
         ws = ops.gemm_workspace(M, N, K, cuda)
         for room in (ws, None):
             ops.fc_layer(a, w, thr, K, out=out, workspace=room)
-            seen = _kernels_seen(lambda: ops.fc_layer(a, w, thr, K, out=out, workspace=room))
+            seen = len(util.kernels_launched(lambda: ops.fc_layer(a, w, thr, K, out=out, workspace=room)))
             assert ops.gemm_call_launches(ops.GEMM_BITS, M, a, w, K, room) == seen, (M, N, K, room is None)
             assert seen <= ops.gemm_launches(M, N, K, room)
 

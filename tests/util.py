@@ -112,3 +112,30 @@ def reader_images(kind, batch):
     m = np.array(mean, np.float32).reshape(1, 3, 1, 1)
     s_ = np.array(sd, np.float32).reshape(1, 3, 1, 1)
     return (v / np.float32(255.0) - m) / s_
+
+
+def kernels_launched(call):
+    """Names of the kernels that a call launches, read from a graph captured of it (it has run before)."""
+    import torch
+    from cuda.bindings import driver
+
+    def ok(answer):
+        assert answer[0] == driver.CUresult.CUDA_SUCCESS, answer[0]
+        return answer[1] if len(answer) == 2 else answer[1:]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        graph.capture_begin(capture_error_mode="thread_local")
+        try:
+            call()
+        finally:
+            graph.capture_end()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes, _ = ok(driver.cuGraphGetNodes(raw, ok(driver.cuGraphGetNodes(raw))[1]))
+    names = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(node))
+            name = ok(driver.cuKernelGetName(params.kern) if int(params.kern) else driver.cuFuncGetName(params.func))
+            names.append(name.decode())
+    return names
