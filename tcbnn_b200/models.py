@@ -17,6 +17,7 @@ Topologies follow the reference drivers, not the textbook networks:
                  192 / 384 channels, pooled layers at 224 x 224).
 """
 import ctypes as C
+import functools
 import weakref
 
 import numpy as np
@@ -239,13 +240,19 @@ def _meet(some, others):
     return False
 
 
+@functools.lru_cache(maxsize=256)
+def _one_launch_pays(widths, rows, settings, device):
+    """tcbnn_fc_chain_pays, under the process-wide settings and on the device that it is asked for."""
+    return lib.load().tcbnn_fc_chain_pays((C.c_int * len(widths))(*widths), len(widths) - 1, rows)
+
+
 def _chain_pays(layers):
     """Whether an MLP's pass in one call is worth asking for: on so many rows, and faster than its layers' calls
-    (tcbnn_fc_chain_pays)."""
-    if type(layers[0]).__name__ != "In128LayerParam" or len(layers) < 2:
+    (tcbnn_fc_chain_pays, which takes 64 to 960 rows on 148 SMs: others are not asked about, 5 us in a first pass)."""
+    first = layers[0]
+    if type(first).__name__ != "In128LayerParam" or not 64 <= first.live <= 960 or len(layers) < 2:
         return False
-    widths = [l.output_width for l in layers]
-    return lib.load().tcbnn_fc_chain_pays((C.c_int * len(widths))(*widths), len(widths) - 1, layers[0].live)
+    return _one_launch_pays(tuple([l.output_width for l in layers]), first.live, lib.settings_generation, torch._C._cuda_getDevice())
 
 
 def _chain_call(layers):
