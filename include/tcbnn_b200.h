@@ -130,7 +130,7 @@ int tcbnn_pack_rows_w(const float* x, int rows, int cols, int ld_words, uint32_t
  * p1 = bias, out = float).  For few rows and layers of at most 1024 outputs: tcbnn_fc_chain_fits says which, and
  * tcbnn_fc_chain_pays where that is faster than the layers one by one (widths: K, then the outputs of the n layers).
  * Results are those of the layers called one by one.  Rows are worked on at different times: no buffer that is written
- * (bits, every out) may overlap another one or anything that is read. */
+ * (bits, every out) may overlap another one or anything that is read, which tcbnn_fc_chain_apart says of a call. */
 typedef struct tcbnn_chain_layer {
     const uint32_t* W;      /* [N][ldw] packed weight, 16-byte aligned, ldw a multiple of 4 */
     int ldw, K, N;
@@ -141,6 +141,7 @@ typedef struct tcbnn_chain_layer {
 } tcbnn_chain_layer;
 int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, int ld_words);
 int tcbnn_fc_chain_pays(const int* widths, int n, int M);
+int tcbnn_fc_chain_apart(const float* x, int M, int K, int ld_words, const uint32_t* bits, const tcbnn_chain_layer* layers, int n);
 int tcbnn_fc_chain(const float* x, int M, int K, int ld_words, uint32_t* bits, const tcbnn_chain_layer* layers, int n,
                    void* stream);
 /* Output layer: out[m][n] = fma((float)(K - 2*popc), scale[n], bias[n]), fp32 [M][ldo].

@@ -1712,6 +1712,31 @@ int tcbnn_fc_chain_fits(const tcbnn_chain_layer* layers, int n, int M, int K, in
     return chain_plan(layers, n, M, K, ld_words, sms, &a) ? 1 : 0;
 }
 
+int tcbnn_fc_chain_apart(const float* x, int M, int K, int ld_words, const uint32_t* bits, const tcbnn_chain_layer* layers, int n) {
+    struct Span { uintptr_t first, end; };
+    Span read[1 + 3 * umma::kChainMaxLayers], written[1 + umma::kChainMaxLayers];
+    if (n < 0 || n > umma::kChainMaxLayers || !layers) return 0;
+    auto span = [](const void* p, long long words) { return Span{(uintptr_t)p, (uintptr_t)p + 4 * (p ? (size_t)words : 0)}; };
+    int reads = 0, writes = 0;
+    read[reads++] = span(x, (long long)M * K);
+    written[writes++] = span(bits, (long long)M * ld_words);
+    for (int l = 0; l < n; l++) {
+        const tcbnn_chain_layer& y = layers[l];
+        read[reads++] = span(y.W, (long long)y.N * y.ldw);
+        read[reads++] = span(y.p0, y.N);
+        read[reads++] = span(y.p1, y.N);
+        written[writes++] = span(y.out, (long long)M * y.ldo);
+    }
+    auto meet = [](const Span& a, const Span& b) { return a.first < b.end && b.first < a.end; };
+    for (int i = 0; i < writes; i++) {
+        for (int j = 0; j < reads; j++)
+            if (meet(written[i], read[j])) return 0;
+        for (int j = 0; j < i; j++)
+            if (meet(written[i], written[j])) return 0;
+    }
+    return 1;
+}
+
 int tcbnn_fc_chain_pays(const int* widths, int n, int M) {
     int sms;
     if (!widths || n < 1 || sm_count(&sms)) return 0;

@@ -51,6 +51,7 @@ SIGNATURES = {
     "tcbnn_bgemm": (_I, [_P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
     "tcbnn_fc_layer": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _P, _I, _P, _SZ, _P]),
     "tcbnn_fc_chain_fits": (_I, [C.POINTER(ChainLayer), _I, _I, _I, _I]),
+    "tcbnn_fc_chain_apart": (_I, [_P, _I, _I, _I, _P, C.POINTER(ChainLayer), _I]),
     "tcbnn_fc_chain_pays": (_I, [C.POINTER(_I), _I, _I]),
     "tcbnn_fc_chain": (_I, [_P, _I, _I, _I, _P, C.POINTER(ChainLayer), _I, _P]),
     "tcbnn_fc_units_bytes": (_SZ, [_I, _I, _I, _I]),

@@ -264,28 +264,23 @@ def _chain_call(layers):
             any(type(l).__name__ != "Fc128LayerParam" for l in layers[1:-1])):
         return None
     x, bits = first.input_gpu, first.output_gpu
-    M, K, ld = shape = first.live, first.input_width, bits.shape[1]
+    shape = first.live, first.input_width, bits.shape[1]
     keep, chain = [x, bits], (lib.ChainLayer * (len(layers) - 1))()
-    at, end = bits.data_ptr(), x.data_ptr()
-    read, written = [(end, end + 4 * M * K)], [(at, at + 4 * M * ld)]
     for i, (prev, l) in enumerate(zip(layers, layers[1:])):
         a, w, out = l.input_gpu, l.weight_gpu, l.output_gpu
         p0, p1 = (l.bn_scale_gpu, l.bn_bias_gpu) if l is last else (l.bn_gpu, None)
-        if (l.live != M or a.data_ptr() != at or a.shape[1] != prev.output_gpu.shape[1] or l.input_width != prev.output_width):
+        if (l.live != first.live or a.data_ptr() != prev.output_gpu.data_ptr() or a.shape[1] != prev.output_gpu.shape[1]
+                or l.input_width != prev.output_width):
             return None
         ops._need_cuda(a, w, p0, p1)
-        (N, ldw), ldo = w.shape, out.shape[1]
-        at = out.data_ptr()
-        y = w.data_ptr(), ldw, l.input_width, N, p0.data_ptr(), p1.data_ptr() if p1 is not None else None, at, ldo
-        chain[i] = lib.ChainLayer(*y)
-        read += [(y[0], y[0] + 4 * N * ldw), (y[4], y[4] + 4 * N)]
-        if p1 is not None:
-            read.append((y[5], y[5] + 4 * N))
-        written.append((at, at + 4 * M * ldo))
+        chain[i] = lib.ChainLayer(w.data_ptr(), w.shape[1], l.input_width, w.shape[0], p0.data_ptr(), p1.data_ptr() if p1 is not None else None,
+                                  out.data_ptr(), out.shape[1])
         keep += [a, w, p0, p1, out]
-    if not lib.load().tcbnn_fc_chain_fits(chain, len(chain), *shape) or _meet(read, written) or any(_meet((s,), written[:i]) for i, s in enumerate(written)):
+    args = (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain))
+    library = lib.load()
+    if not library.tcbnn_fc_chain_fits(chain, len(chain), *shape) or not library.tcbnn_fc_chain_apart(*args):
         return None
-    return "tcbnn_fc_chain", (ops._ptr(x), *shape, ops._ptr(bits), chain, len(chain)), tuple(t for t in keep if t is not None)
+    return "tcbnn_fc_chain", args, tuple(t for t in keep if t is not None)
 
 
 def _pass_calls(layers):
@@ -356,11 +351,7 @@ class _Calls:
 
     def serves(self, x):
         """Whether the calls can be made on another input tensor as they are."""
-        if not self.chain:
-            return True
-        _, M, K, ld, bits, chain, _ = self.calls[0][1]                       # (apart from what it writes, see _chain_call)
-        at = x.data_ptr()
-        return not _meet([(at, at + 4 * M * K)], [(bits, bits + 4 * M * ld)] + [(y.out, y.out + 4 * M * y.ldo) for y in chain])
+        return not self.chain or bool(lib.load().tcbnn_fc_chain_apart(ops._ptr(x), *self.calls[0][1][1:]))
 
     def first(self, layers):
         """The first call, on the input that layers[0] now has."""

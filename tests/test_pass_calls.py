@@ -11,6 +11,7 @@ from tcbnn_b200 import lib, models, ops, param
 class _Library:
     def __init__(self):
         self.asked = []
+        self.tcbnn_fc_chain_apart = lib.load().tcbnn_fc_chain_apart     # (asks no GPU)
 
     def tcbnn_fc_chain_fits(self, layers, n, M, K, ld):
         self.asked.append("fits")
